@@ -417,7 +417,7 @@ def _exact_fstat(case, x):
         Nv = 4.0 * (((dA.conj()[:, None] * A).real + (dE.conj()[:, None] * E).real) * w[:, None]).sum(-1)
         wc = w.to(A.dtype)
         M = 4.0 * (torch.einsum("nfi,ngi,ni->nfg", A.conj(), A, wc) + torch.einsum("nfi,ngi,ni->nfg", E.conj(), E, wc)).real
-        a = torch.linalg.solve(M, Nv[:, :, None])[:, :, 0]
+        a = _dev(np.linalg.solve(M.cpu().numpy(), Nv[:, :, None].cpu().numpy())[:, :, 0])
         logl = 0.5 * (Nv * a).sum(-1)
         a1, a2, a3, a4 = a.unbind(-1)
         s1 = torch.sqrt((a1 + a4) ** 2 + (a2 - a3) ** 2)
@@ -515,13 +515,13 @@ class _Spline:
     def __init__(self, x, y, even):
         n, self.x, self.even = len(x), x, even
         h = x[1:] - x[:-1]
-        A = torch.eye(n, dtype=torch.float64, device=x.device)
-        i = torch.arange(1, n - 1, device=x.device)
-        A[i, i - 1], A[i, i], A[i, i + 1] = h[:-1], 2.0 * (x[2:] - x[:-2]), h[1:]
+        xs, i = x.cpu().numpy(), np.arange(1, n - 1)
+        A = np.eye(n)
+        A[i, i - 1], A[i, i], A[i, i + 1] = xs[1:-1] - xs[:-2], 2.0 * (xs[2:] - xs[:-2]), xs[2:] - xs[1:-1]
         r = torch.zeros_like(y)
         s = (y[..., 1:] - y[..., :-1]) / h
         r[..., 1:-1] = 3.0 * (s[..., 1:] - s[..., :-1])
-        c2 = torch.linalg.solve(A, r.reshape(-1, n).T).T.reshape(y.shape)
+        c2 = _dev(np.linalg.solve(A, r.reshape(-1, n).T.cpu().numpy()).T).reshape(y.shape)
         self.c0, self.c2 = y[..., :-1], c2[..., :-1]
         self.c1 = s - h * (c2[..., 1:] + 2.0 * c2[..., :-1]) / 3.0
         self.c3 = (c2[..., 1:] - c2[..., :-1]) / (3.0 * h)
