@@ -1346,7 +1346,7 @@ extern "C" int glass_gpu_noise_logl_batch_sgwb(glass_gpu_ctx *ctx, int nprop, co
     cudaFree(nd.partial);
     nd.partial = nullptr;
     nd.partial_models = 0;
-    GLASS_CUDA(cudaMalloc(&nd.partial, sizeof(double) * (size_t)want * noise_chunks(nd.N)), "cudaMalloc(noise partial)");
+    GLASS_CUDA(cudaMalloc(&nd.partial, sizeof(double) * noise_partials(nd.N, want)), "cudaMalloc(noise partial)");
     nd.partial_models = want;
   }
   int nl = 0;
@@ -1538,7 +1538,7 @@ extern "C" int glass_gpu_noise_wavelet_logl_batch_sgwb(glass_gpu_ctx *ctx, int m
     cudaFree(w.partial);
     w.partial = nullptr;
     w.partial_models = 0;
-    GLASS_CUDA(cudaMalloc(&w.partial, sizeof(double) * (size_t)want * noise_wv_chunks(w)), "cudaMalloc(noise wv partial)");
+    GLASS_CUDA(cudaMalloc(&w.partial, sizeof(double) * noise_wv_partials(w, want)), "cudaMalloc(noise wv partial)");
     w.partial_models = want;
   }
   int nl = 0;

@@ -14,13 +14,26 @@
 // proposals per chain per sweep.  Everything that depends on frequency alone
 // (the TDI and arm transfer functions, f^(-7/3), the data's auto- and
 // cross-spectra) is tabulated once per bin when the data are set; a batch then
-// costs one pass over the table per model: per bin the link levels enter
-// linearly, the foreground takes its exp/pow/tanh, and the inverse and
-// log-determinant follow the reference's Cholesky-like elimination.
+// costs one pass over the table per model.
 //
-// FP64, compiled without multiply-add contraction.  The inverse's entries are
-// the cofactors times 1/det instead of the reference's
-// exp(log|cofactor| - log det) (the same numbers to a few ulp).
+// FP64.  The FP64 pipe bounds every kernel here (2 multiply-adds per SM and
+// clock, 1/64 of FP32), so the FP64 instructions per model and bin are what is
+// counted; integer work and loads are free beside them:
+//  * the levels enter through 15 sums per model and five products of transfer
+//    functions per bin (15 operations for the six covariance entries);
+//  * the inverse is the cofactors over the determinant, with one reciprocal
+//    (the reference takes exp(log|cofactor| - log det): the same numbers to a
+//    few ulp of the covariance's conditioning);
+//  * the log-determinants are summed as the product of their mantissas and the
+//    sum of their exponents, one log per warp;
+//  * the foreground's tanh is 1 / (1 + exp(2 (f - fk) / f2)), whose exponential
+//    is a geometric sequence along a thread's bins, and its power law
+//    exp(alpha (log f - log f1)) with log f tabulated.
+// 420 -> 85 FP64 instructions per model and bin with the foreground; 1024
+// models on 15360 bins 12.44 -> 2.45 ms, wavelet cells 202 -> 35 and 22.7 ->
+// 3.56 ms (1024 models, 58880 cells, modulated foreground).  Compiled without
+// multiply-add contraction (the SGWB templates keep the reference's operation
+// order); the code below writes its multiply-adds out.
 
 #include <math.h>
 
@@ -34,12 +47,18 @@ namespace glass {
 
 namespace {
 
-constexpr int kNoiseThreads = 256;
-constexpr int kNoiseBinsPerThread = 8;
-constexpr int kNoiseChunk = kNoiseThreads * kNoiseBinsPerThread;  // bins per CTA
+constexpr int kNoiseThreads = 128;
+// Bins per thread of the Fourier kernels.  The most that still gives every SM
+// a few CTAs, so that one model on a few thousand bins uses the whole chip (a
+// warp's FP64 instruction holds its SM's pipe for 16 clocks: 2048 bins on one
+// SM take 16x what they take on 16); at the most, a CTA's model constants and
+// its reduction are 2% of its work.
+constexpr int kNoiseMaxBins = 16;
+constexpr int kNoiseTargetCtas = 608;  // 4 per SM of a 152-SM GPU
 
 struct NoiseArgs {
-  int N, nchunks, nprop;
+  int N, nchunks, nprop, R;  // R bins per thread
+  double fstep;              // 128 bins, in Hz
   const double *tab;  // kNoiseTabRows rows of N
   const double *inst;  // [nprop][12]
   const double *sgal;  // [nprop][5] or null
@@ -49,49 +68,169 @@ struct NoiseArgs {
   double *partial;     // [nprop][nchunks]
 };
 
-// Instrument covariance of one bin at link levels in[12] (sacc[6], soms[6]),
-// from the bin's cos(f/f*), -8 sin^2(f/f*) and transfer functions
-// (noise/src/glass_noise_model.c:445-546; acc_tf is 0 at f >= 10 mHz, where the
-// reference leaves out the acceleration terms: adding exact zeros changes
-// nothing), normalised by 4.
-__device__ __forceinline__ void noise_inst_cov(double cosx, double tdi, double acc_tf, double oms_tf,
-                                               const double *in, double &cxx, double &cyy, double &czz, double &cxy,
-                                               double &cxz, double &cyz) {
-  const double A12 = in[0] * acc_tf, A21 = in[1] * acc_tf, A23 = in[2] * acc_tf;
-  const double A32 = in[3] * acc_tf, A13 = in[4] * acc_tf, A31 = in[5] * acc_tf;
-  const double O12 = in[6] * oms_tf, O21 = in[7] * oms_tf, O23 = in[8] * oms_tf;
-  const double O32 = in[9] * oms_tf, O13 = in[10] * oms_tf, O31 = in[11] * oms_tf;
-  double c00 = (O12 + O21 + O13 + O31) * .25;
-  double c11 = (O23 + O32 + O21 + O12) * .25;
-  double c22 = (O31 + O13 + O32 + O23) * .25;
-  double c01 = (O12 + O21) * .5;
-  double c02 = (O13 + O31) * .5;
-  double c12 = (O32 + O23) * .5;
-  c00 += ((A12 + A13) + ((A21 + A31)) * cosx * cosx);
-  c11 += ((A23 + A21) + ((A32 + A12)) * cosx * cosx);
-  c22 += ((A31 + A32) + ((A13 + A23)) * cosx * cosx);
-  c01 += 2. * (A12 + A21);
-  c02 += 2. * (A13 + A31);
-  c12 += 2. * (A32 + A23);
-  c00 *= -2. * tdi;
-  c11 *= -2. * tdi;
-  c22 *= -2. * tdi;
-  c01 *= tdi * cosx;
-  c02 *= tdi * cosx;
-  c12 *= tdi * cosx;
-  cxx = c00 / 4.0;
-  cyy = c11 / 4.0;
-  czz = c22 / 4.0;
-  cxy = c01 / 4.0;
-  cxz = c02 / 4.0;
-  cyz = c12 / 4.0;
+// ------------------------------------------------------ FP64 building blocks
+// 1/x for normal x of moderate exponent: the hardware's ~20-bit estimate and
+// one step of Householder's cubic iteration, r (1 + e + e^2) with e = 1 - x r.
+__device__ __forceinline__ double rcp_fast(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
+// exp by table and short polynomial (Tang, ACM Trans. Math. Softw. 15, 1989):
+// x = (64 m + k) ln2/64 + r, exp x = 2^m t[k] (1 + r + ... + r^5/120), t[k] =
+// 2^(k/64), |r| <= ln2/128.  10 FP64 instructions; arguments beyond +-708 and
+// NaN go to the library's.
+constexpr int kExpTab = 64;
+__device__ __forceinline__ double exp_tab(double x, const double *t) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40862000) return exp(x);
+  constexpr double kLn2 = 0.693147180559945309417, kLn2Lo = 2.3190468138462996e-17;  // ln 2 = kLn2 + kLn2Lo
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adds to the nearest integer
+  const double z = fma(x, kExpTab / kLn2, kMagic);
+  const int n = __double2loint(z);
+  const double kd = z - kMagic;
+  double r = fma(kd, -kLn2 / kExpTab, x);
+  r = fma(kd, -kLn2Lo / kExpTab, r);
+  double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+  q = fma(r, q, 1.0 / 6.0);
+  q = fma(r, q, 0.5);
+  q = fma(r * r, q, r);
+  const double T = t[n & (kExpTab - 1)];
+  const double y = fma(T, q, T);
+  return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
+}
+__device__ __forceinline__ void exp_tab_fill(double *t) {
+  for (int k = threadIdx.x; k < kExpTab; k += blockDim.x) t[k] = exp2(k * (1.0 / kExpTab));
+}
+
+// A sum of logarithms of positive normal numbers as the product of their
+// mantissas, kept in [1, 2), and the sum of their exponents.
+struct LogSum {
+  double m = 1.0;
+  int e = 0;
+};
+__device__ __forceinline__ double mantissa(double x, int &e) {
+  const int hi = __double2hiint(x);
+  e += (hi >> 20) - 1023;
+  return __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+}
+__device__ __forceinline__ void log_add(LogSum &s, double x) {
+  const double m = mantissa(x, s.e);
+  s.m = mantissa(s.m * m, s.e);
+}
+// Positive, finite and 2^-959 < x < 2^961: rcp_fast and log_add apply.
+__device__ __forceinline__ bool plain_positive(double x) {
+  return (unsigned)(__double2hiint(x) - 0x04000000) < 0x78000000u;
+}
+
+// The CTA's sum of chi and of the logarithms (valid in thread 0).
+__device__ __forceinline__ double block_total(double chi, LogSum ld) {
+  __shared__ double red[kNoiseThreads / 32], redm[kNoiseThreads / 32];
+  __shared__ int rede[kNoiseThreads / 32];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    chi += __shfl_xor_sync(0xffffffffu, chi, off);
+    ld.m *= __shfl_xor_sync(0xffffffffu, ld.m, off);  // below 2^32
+  }
+  ld.e = __reduce_add_sync(0xffffffffu, ld.e);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) {
+    red[warp] = chi;
+    redm[warp] = ld.m;
+    rede[warp] = ld.e;
+  }
+  __syncthreads();
+  double s = 0.0;
+  if (warp == 0) {
+    if (lane < kNoiseThreads / 32) s = red[lane] + fma((double)rede[lane], 0.693147180559945309417, log(redm[lane]));
+#pragma unroll
+    for (int off = kNoiseThreads / 64; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  }
+  return s;
+}
+
+// ------------------------------------------------------ one model's constants
+// The sums of link levels that the covariance entries use
+// (noise/src/glass_noise_model.c:445-546): per diagonal entry xx, yy, zz the
+// metrology sum o / 4 and the acceleration sums a and b (b times cos^2), per
+// off-diagonal entry xy, xz, yz the metrology sum p / 2 and the acceleration
+// sum 2 q; and the foreground's parameters (map_array_to_foreground_params,
+// :67-74).
+struct NoiseModel {
+  double lev[15];  // o, a, b, p, q: three each
+  double Amp, l1, alpha, fk, i2, f10, estep;
+  int chain;  // the foreground's exponential may run as a geometric sequence
+};
+// Level indices of each sum in o, a, b, p, q (12: none), levels in the order
+// 12, 21, 23, 32, 13, 31 (acceleration, then metrology).
+__constant__ unsigned char kLevelIdx[15][4] = {
+    {6, 7, 10, 11}, {8, 9, 7, 6},   {11, 10, 9, 8},  {0, 4, 12, 12}, {2, 1, 12, 12},
+    {5, 3, 12, 12}, {1, 5, 12, 12}, {3, 0, 12, 12},  {4, 2, 12, 12}, {6, 7, 12, 12},
+    {10, 11, 12, 12}, {9, 8, 12, 12}, {0, 1, 12, 12}, {4, 5, 12, 12}, {3, 2, 12, 12}};
+
+// By the CTA's first warp; the caller synchronises.  fstep: the frequency step
+// between a thread's bins.
+__device__ __forceinline__ void noise_model_load(NoiseModel &M, const double *in, const double *sg, double fstep) {
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  if (lane < 15) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = kLevelIdx[lane][k];
+      s += i < 12 ? in[i] : 0.0;
+    }
+    M.lev[lane] = s * (lane < 3 ? 0.25 : lane < 9 ? 1.0 : lane < 12 ? 0.5 : 2.0);
+  }
+  if (sg) {
+    const double v = lane < 5 ? sg[lane] : 0.0, x = lane == 2 ? 0.0 : v;
+    const double e = exp(x);
+    const double f2 = __shfl_sync(0xffffffffu, e, 4);
+    if (lane == 0) M.Amp = e;
+    if (lane == 1) {
+      M.l1 = v;
+      M.f10 = e * 10;
+    }
+    if (lane == 2) M.alpha = v;
+    if (lane == 3) M.fk = e;
+    if (lane == 4) {
+      // a step of the sequence by more than e^1 could leave the exponent range
+      // within a thread's bins and not come back
+      const double st = 2.0 * fstep / f2;
+      M.i2 = 2.0 / f2;
+      M.estep = exp(st);
+      M.chain = st < 1.0;
+    }
+  }
+}
+
+// The six covariance entries of one bin or layer from the model's sums and the
+// transfer products (table rows kTabU1 .. kTabV2).
+__device__ __forceinline__ void noise_inst_cov(const NoiseModel &M, double u1, double u2, double u3, double v1,
+                                               double v2, double *c) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    c[k] = fma(u1, M.lev[k], fma(u2, M.lev[3 + k], u3 * M.lev[6 + k]));
+    c[3 + k] = fma(v1, M.lev[9 + k], v2 * M.lev[12 + k]);
+  }
+}
+
+// exp(2 (f - fk) / f2), for the foreground's 0.5 (1 + tanh((fk - f) / f2)) =
+// 1 / (1 + E).
+__device__ __forceinline__ double noise_gal_exp(const NoiseModel &M, double f, const double *t) {
+  return exp_tab((f - M.fk) * M.i2, t);
+}
 // The galactic foreground's PSD at f (utils/src/glass_galaxy.c:40-44), zero
-// above 10 f1 as in noise/src/glass_noise_model.c:627-631; fp73 = f^(-7/3).
-__device__ __forceinline__ double noise_sgal(double f, double fp73, double Amp, double f1, double alpha, double fk,
-                                             double f2) {
-  return (f > f1 * 10) ? 0.0 : Amp * fp73 * exp(-pow(f / f1, alpha)) * 0.5 * (1. + tanh((fk - f) / f2));
+// above 10 f1 as in noise/src/glass_noise_model.c:627-631; fp73 = f^(-7/3),
+// lf = log f, E as above.
+__device__ __forceinline__ double noise_sgal(const NoiseModel &M, double f, double fp73, double lf, double E,
+                                             const double *t) {
+  if (f > M.f10) return 0.0;
+  const double u = exp_tab(M.alpha * (lf - M.l1), t);
+  const int h = __double2hiint(E);
+  const double w = (h >= 0x7e000000 && h <= 0x7ff00000) ? 0.0 : rcp_fast(1.0 + E);  // E beyond 2^993: tanh = -1
+  return M.Amp * fp73 * exp_tab(-u, t) * w;
 }
 
 // ------------------------------------------------------------------ SGWB
@@ -173,94 +312,95 @@ __device__ __forceinline__ void noise_inv3(double cxx, double cyy, double czz, d
   iv[5] = (cxy * cxz - cxx * cyz) * idet;
 }
 
-__device__ __forceinline__ void noise_gal_params(const double *sg, double &Amp, double &f1, double &alpha,
-                                                 double &fk, double &f2) {
-  // map_array_to_foreground_params (noise/src/glass_noise_model.c:67-74)
-  Amp = exp(sg[0]);
-  f1 = exp(sg[1]);
-  alpha = sg[2];
-  fk = exp(sg[3]);
-  f2 = exp(sg[4]);
-}
-
-__device__ __forceinline__ double block_sum(double v, double *red) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
+// chi^2 + log det of one cell by the elimination above, for covariances the
+// fast form does not take (not positive, not finite, or with a determinant at
+// the ends of the exponent range).
+__device__ __noinline__ double noise_cell_general(double cxx, double cyy, double czz, double cxy, double cxz,
+                                                  double cyz, const double *P) {
+  double iv[6], ld;
+  noise_inv3(cxx, cyy, czz, cxy, cxz, cyz, iv, ld);
   double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kNoiseThreads / 32; w++) s += red[w];
-  return s;
+#pragma unroll
+  for (int k = 0; k < 6; k++) s += P[k] * iv[k];
+  return s + ld;
 }
 
-// One CTA per (bin chunk, model): per-bin covariance, inverse, likelihood
-// terms; the chunk's sum goes to partial[model][chunk].
+// Adds tr(C^-1 P) and log det C of one cell, c = xx, yy, zz, xy, xz, yz and
+// P = xx, yy, zz, 2 xy, 2 xz, 2 yz: 12 operations for the cofactors, 3 for the
+// determinant, 6 for the trace's numerator, 3 for the reciprocal, 2 for the sums.
+// The determinant's cancellation where the channels are nearly degenerate
+// (third pivot ~1e-7 of the first at 0.1 mHz) is that of the elimination's.
+__device__ __forceinline__ void noise_cell(const double *c, const double *P, double &chi, LogSum &ld) {
+  const double cxx = c[0], cyy = c[1], czz = c[2], cxy = c[3], cxz = c[4], cyz = c[5];
+  const double m2 = fma(cxx, cyy, -(cxy * cxy));
+  const double m4 = fma(cxy, cyz, -(cxz * cyy));
+  const double m5 = fma(cxy, cxz, -(cxx * cyz));
+  const double det = fma(czz, m2, fma(cyz, m5, cxz * m4));
+  // all leading minors positive, as the reference's logarithms need
+  if (__double2hiint(cxx) > 0 && __double2hiint(m2) > 0 && plain_positive(det)) {
+    const double m0 = fma(cyy, czz, -(cyz * cyz));
+    const double m1 = fma(czz, cxx, -(cxz * cxz));
+    const double m3 = fma(cxz, cyz, -(czz * cxy));
+    double num = m0 * P[0];
+    num = fma(m1, P[1], num);
+    num = fma(m2, P[2], num);
+    num = fma(m3, P[3], num);
+    num = fma(m4, P[4], num);
+    num = fma(m5, P[5], num);
+    chi = fma(num, rcp_fast(det), chi);
+    log_add(ld, det);
+  } else {
+    chi += noise_cell_general(cxx, cyy, czz, cxy, cxz, cyz, P);
+  }
+}
+
+// One CTA per (chunk of 128 R bins, model): per-bin covariance, inverse and
+// likelihood terms; the chunk's sum goes to partial[model][chunk].  Bound by
+// the FP64 pipe (see the top of the file).
 __global__ void __launch_bounds__(kNoiseThreads) noise_logl_kernel(NoiseArgs a) {
-  __shared__ double red[kNoiseThreads / 32];
+  __shared__ double et[kExpTab];
+  __shared__ NoiseModel M;
   const int chunk = blockIdx.x, p = blockIdx.y;
-  const double *in = a.inst + 12 * (size_t)p;
   const bool gal = a.sgal != nullptr;
-  double Amp = 0, f1 = 0, alpha = 0, fk = 0, f2 = 0;
-  if (gal) noise_gal_params(a.sgal + 5 * (size_t)p, Amp, f1, alpha, fk, f2);
+  noise_model_load(M, a.inst + 12 * (size_t)p, gal ? a.sgal + 5 * (size_t)p : nullptr, a.fstep);
+  if (gal) exp_tab_fill(et);
+  __syncthreads();
   const double *sgp = a.sgwb ? a.sgwb + 4 * (size_t)p : nullptr;
-  const int N = a.N;
-  const double *F = a.tab + (size_t)kTabF * N, *COSX = a.tab + (size_t)kTabCosx * N;
-  const double *TDI = a.tab + (size_t)kTabTdi * N, *ACC = a.tab + (size_t)kTabAcc * N;
-  const double *OMS = a.tab + (size_t)kTabOms * N, *TG = a.tab + (size_t)kTabTgal * N;
-  const double *P73 = a.tab + (size_t)kTabFp73 * N;
-  const double *XX = a.tab + (size_t)kTabXX * N, *YY = a.tab + (size_t)kTabYY * N;
-  const double *ZZ = a.tab + (size_t)kTabZZ * N, *XY = a.tab + (size_t)kTabXY * N;
-  const double *XZ = a.tab + (size_t)kTabXZ * N, *YZ = a.tab + (size_t)kTabYZ * N;
-  double acc = 0.0;
+  const size_t N = a.N;
+  double chi = 0.0, E = 0.0;
+  LogSum ld;
 #pragma unroll 1
-  for (int r = 0; r < kNoiseBinsPerThread; r++) {
-    const int n = chunk * kNoiseChunk + r * kNoiseThreads + threadIdx.x;
-    if (n >= N) break;
-    const double f = F[n];
-    double cxx = 0.0, cyy = 0.0, czz = 0.0, cxy = 0.0, cxz = 0.0, cyz = 0.0;
-    if (f != 0.0) {
-      noise_inst_cov(COSX[n], TDI[n], ACC[n], OMS[n], in, cxx, cyy, czz, cxy, cxz, cyz);
-      if (gal) {
-        // utils/src/glass_galaxy.c:40-44, skipped above 10 f1 as the reference does
-        const double t = TG[n];
-        const double Sgal = noise_sgal(f, P73[n], Amp, f1, alpha, fk, f2);
-        const double d = t * Sgal / 4.0, o = -0.5 * t * Sgal / 4.0;
-        cxx += d;
-        cyy += d;
-        czz += d;
-        cxy += o;
-        cxz += o;
-        cyz += o;
-      }
-      if (sgp) {
-        // added last, as the instrument sampler combines the three
-        // (noise/src/glass_noise_sampler.c:559-568)
-        const double S = sgwb_psd(a.sg_type, f, sgp);
-        const double *R = a.rsg;
-        cxx += R[n] * S;
-        cyy += R[(size_t)N + n] * S;
-        czz += R[2 * (size_t)N + n] * S;
-        cxy += R[3 * (size_t)N + n] * S;
-        cxz += R[4 * (size_t)N + n] * S;
-        cyz += R[5 * (size_t)N + n] * S;
+  for (int r = 0; r < a.R; r++) {
+    const int n = (chunk * a.R + r) * kNoiseThreads + threadIdx.x;
+    if (n >= a.N) break;
+    const double *t = a.tab + n;
+    double c[6], P[6];
+    noise_inst_cov(M, t[kTabU1 * N], t[kTabU2 * N], t[kTabU3 * N], t[kTabV1 * N], t[kTabV2 * N], c);
+    if (gal) {
+      const double f = t[kTabF * N];
+      E = (r > 0 && M.chain) ? E * M.estep : noise_gal_exp(M, f, et);
+      const double S = noise_sgal(M, f, t[kTabFp73 * N], t[kTabLogf * N], E, et);
+      const double d = 0.25 * t[kTabTgal * N] * S;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        c[k] += d;
+        c[3 + k] = fma(-0.5, d, c[3 + k]);
       }
     }
-    double iv[6], logdetC;
-    noise_inv3(cxx, cyy, czz, cxy, cxz, cyz, iv, logdetC);
-    double l = 0.0;
-    l -= 0.5 * XX[n] * iv[0] * 2;
-    l -= 0.5 * YY[n] * iv[1] * 2;
-    l -= 0.5 * ZZ[n] * iv[2] * 2;
-    l -= XY[n] * iv[3] * 2;
-    l -= XZ[n] * iv[4] * 2;
-    l -= YZ[n] * iv[5] * 2;
-    l -= logdetC;
-    acc += l;
+    if (sgp) {
+      // added last, as the instrument sampler combines the three
+      // (noise/src/glass_noise_sampler.c:559-568)
+      const double f = t[kTabF * N];
+      const double S = f != 0.0 ? sgwb_psd(a.sg_type, f, sgp) : 0.0;
+#pragma unroll
+      for (int k = 0; k < 6; k++) c[k] = fma(a.rsg[k * N + n], S, c[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) P[k] = t[(kTabXX + k) * N];
+    noise_cell(c, P, chi, ld);
   }
-  const double s = block_sum(acc, red);
-  if (threadIdx.x == 0) a.partial[(size_t)p * a.nchunks + chunk] = s;
+  const double s = block_total(chi, ld);
+  if (threadIdx.x == 0) a.partial[(size_t)p * a.nchunks + chunk] = -s;
 }
 
 // The one- and two-channel forms: the instrument covariance of
@@ -273,48 +413,48 @@ __global__ void __launch_bounds__(kNoiseThreads) noise_logl_kernel(NoiseArgs a) 
 // (noise/src/glass_noise_model.c:1104-1134).  sin^2(f/f*) is the table's
 // -8 sin^2 times -1/8 (exact).
 __global__ void __launch_bounds__(kNoiseThreads) noise_ch12_kernel(NoiseArgs a, int nch) {
-  __shared__ double red[kNoiseThreads / 32];
+  __shared__ double et[kExpTab];
+  __shared__ NoiseModel M;
   const int chunk = blockIdx.x, p = blockIdx.y;
   const double *in = a.inst + 12 * (size_t)p;
   const bool gal = a.sgal != nullptr;
-  double Amp = 0, f1 = 0, alpha = 0, fk = 0, f2 = 0;
-  if (gal) noise_gal_params(a.sgal + 5 * (size_t)p, Amp, f1, alpha, fk, f2);
+  noise_model_load(M, in, gal ? a.sgal + 5 * (size_t)p : nullptr, a.fstep);
+  if (gal) exp_tab_fill(et);
+  __syncthreads();
   const double sacc12 = in[0], soms12 = in[6];
-  const int N = a.N;
-  const double *F = a.tab + (size_t)kTabF * N, *COSX = a.tab + (size_t)kTabCosx * N;
-  const double *TDI = a.tab + (size_t)kTabTdi * N, *ACC = a.tab + (size_t)kTabAcc * N;
-  const double *OMS = a.tab + (size_t)kTabOms * N, *TG = a.tab + (size_t)kTabTgal * N;
-  const double *P73 = a.tab + (size_t)kTabFp73 * N, *C2X = a.tab + (size_t)kTabCos2x * N;
-  const double *P0 = a.tab + (size_t)kTabP0 * N, *P1 = a.tab + (size_t)kTabP1 * N;
-  double acc = 0.0;
+  const size_t N = a.N;
+  double chi = 0.0, E = 0.0;
+  LogSum ld;
 #pragma unroll 1
-  for (int r = 0; r < kNoiseBinsPerThread; r++) {
-    const int n = chunk * kNoiseChunk + r * kNoiseThreads + threadIdx.x;
-    if (n >= N) break;
-    const double f = F[n];
+  for (int r = 0; r < a.R; r++) {
+    const int n = (chunk * a.R + r) * kNoiseThreads + threadIdx.x;
+    if (n >= a.N) break;
+    const double *t = a.tab + n;
+    const double f = t[kTabF * N];
     double c = 0.0;
     if (f != 0.0) {
-      const double cosx = COSX[n], sx2 = TDI[n] * -0.125;
-      const double Spm = sacc12 * ACC[n], Sop = soms12 * OMS[n];
+      const double cosx = t[kTabCosx * N], sx2 = t[kTabTdi * N] * -0.125;
+      const double Spm = sacc12 * t[kTabAcc * N], Sop = soms12 * t[kTabOms * N];
       c = (nch == 1) ? 16. * sx2 * (2. * (1.0 + cosx * cosx) * Spm + Sop)
-                     : 8. * sx2 * (2. * Spm * (3. + 2. * cosx + C2X[n]) + Sop * (2. + cosx));
-      c = c / 4.0;
+                     : 8. * sx2 * (2. * Spm * (3. + 2. * cosx + t[kTabCos2x * N]) + Sop * (2. + cosx));
+      c = c * 0.25;
       if (gal) {
-        const double Sgal = noise_sgal(f, P73[n], Amp, f1, alpha, fk, f2);
-        c += (nch == 1 ? Sgal : 1.5 * TG[n] * Sgal) / 4.0;
+        E = (r > 0 && M.chain) ? E * M.estep : noise_gal_exp(M, f, et);
+        const double Sgal = noise_sgal(M, f, t[kTabFp73 * N], t[kTabLogf * N], E, et);
+        c += (nch == 1 ? Sgal : 1.5 * t[kTabTgal * N] * Sgal) * 0.25;
       }
     }
-    const double ic = 1. / c;
-    double l = -0.5 * (2.0 * (P0[n] * ic));
-    double ld = log(c);
-    if (nch == 2) {
-      l -= 0.5 * (2.0 * (P1[n] * ic));
-      ld += log(c);
+    const double P = nch == 2 ? t[kTabP0 * N] + t[kTabP1 * N] : t[kTabP0 * N];
+    if (plain_positive(c)) {
+      chi = fma(P, rcp_fast(c), chi);
+      log_add(ld, c);
+      if (nch == 2) log_add(ld, c);
+    } else {
+      chi += P * (1. / c) + (nch == 2 ? 2.0 : 1.0) * log(c);
     }
-    acc += l - ld;
   }
-  const double s = block_sum(acc, red);
-  if (threadIdx.x == 0) a.partial[(size_t)p * a.nchunks + chunk] = s;
+  const double s = block_total(chi, ld);
+  if (threadIdx.x == 0) a.partial[(size_t)p * a.nchunks + chunk] = -s;
 }
 
 // Per model: the chunks' sums in order, and the constant -3 N log(2 pi).
@@ -338,148 +478,105 @@ struct NoiseWvArgs {
   double *out;  // logl (modes 0/1) or partial (mode 2)
 };
 
-// The background's variance in layer j (generate_sgwb_model_wavelet
-// :843-892: the Fourier model at the layer centre over ND, zero in the DC
-// layer): sg6 = xx, yy, zz, xy, xz, yz.
-__device__ __forceinline__ void noise_wv_sgwb(const NoiseWvArgs &a, int j, const double *sgp, double *sg6) {
-  const int NL = a.Nlayer;
-  const double f = a.tab[(size_t)kTabF * NL + j];
-  const double S = f != 0.0 ? sgwb_psd(a.sg_type, f, sgp) : 0.0;
+// One layer's covariances in the wavelet domain: the Fourier model at the layer
+// centre over ND (generate_instrument_noise_model_wavelet :561-610), plus the
+// background's (generate_sgwb_model_wavelet :843-892, zero in the DC layer), in
+// c6 = xx, yy, zz, xy, xz, yz; returns the foreground's (generate_galactic_
+// foreground_model_wavelet :656-722), the same for the three diagonal and, with
+// the isotropic -1/2 undone, for the three off-diagonal entries.
+__device__ __forceinline__ double noise_wv_layer(const NoiseWvArgs &a, const NoiseModel &M, int j, bool gal,
+                                                 const double *sgp, const double *et, double *c6) {
+  const size_t NL = a.Nlayer;
+  const double *t = a.tab + j;
+  const double f = t[kTabF * NL];
+  noise_inst_cov(M, t[kTabU1 * NL], t[kTabU2 * NL], t[kTabU3 * NL], t[kTabV1 * NL], t[kTabV2 * NL], c6);
 #pragma unroll
-  for (int e = 0; e < 6; e++) sg6[e] = f != 0.0 ? a.rsg[(size_t)e * NL + j] * S * a.inv_ND : 0.0;
-}
-
-// Instrument (and foreground) variance of one layer in the wavelet domain:
-// the Fourier model at the layer centre over ND (generate_instrument_noise_
-// model_wavelet :561-610, generate_galactic_foreground_model_wavelet :656-722,
-// whose off-diagonals have the isotropic -1/2 undone).  inst6, conf6: xx, yy,
-// zz, xy, xz, yz.
-__device__ __forceinline__ void noise_wv_layer(const NoiseWvArgs &a, int j, const double *in, bool gal, double Amp,
-                                               double f1, double alpha, double fk, double f2, double *inst6,
-                                               double *conf6) {
-  const int NL = a.Nlayer;
-  const double f = a.tab[(size_t)kTabF * NL + j];
-  double cxx = 0, cyy = 0, czz = 0, cxy = 0, cxz = 0, cyz = 0;
-  if (f != 0.0)
-    noise_inst_cov(a.tab[(size_t)kTabCosx * NL + j], a.tab[(size_t)kTabTdi * NL + j], a.tab[(size_t)kTabAcc * NL + j],
-                   a.tab[(size_t)kTabOms * NL + j], in, cxx, cyy, czz, cxy, cxz, cyz);
-  inst6[0] = cxx * a.inv_ND;
-  inst6[1] = cyy * a.inv_ND;
-  inst6[2] = czz * a.inv_ND;
-  inst6[3] = cxy * a.inv_ND;
-  inst6[4] = cxz * a.inv_ND;
-  inst6[5] = cyz * a.inv_ND;
-  double dg = 0.0, og = 0.0;
-  if (gal && f != 0.0) {
-    const double t = a.tab[(size_t)kTabTgal * NL + j];
-    const double Sgal = noise_sgal(f, a.tab[(size_t)kTabFp73 * NL + j], Amp, f1, alpha, fk, f2);
-    dg = t * Sgal / 4.0;
-    og = -0.5 * t * Sgal / 4.0;
-    og *= -2.0;
+  for (int e = 0; e < 6; e++) c6[e] *= a.inv_ND;
+  if (sgp && f != 0.0) {
+    const double S = sgwb_psd(a.sg_type, f, sgp) * a.inv_ND;
+#pragma unroll
+    for (int e = 0; e < 6; e++) c6[e] = fma(a.rsg[e * NL + j], S, c6[e]);
   }
-  conf6[0] = conf6[1] = conf6[2] = dg * a.inv_ND;
-  conf6[3] = conf6[4] = conf6[5] = og * a.inv_ND;
+  if (!gal || f == 0.0) return 0.0;
+  const double S = noise_sgal(M, f, t[kTabFp73 * NL], t[kTabLogf * NL], noise_gal_exp(M, f, et), et);
+  return 0.25 * t[kTabTgal * NL] * S * a.inv_ND;
 }
 
 // Modes 0/1: the covariance is the same for every cell of a layer, so a
 // layer's cells contribute -Q/2 (ixx Sxx + ... + 2 ixy Sxy ...) - Q/2 Ncoarse
 // log det with S the layer's sums of the cell statistics.  One CTA per model.
 __global__ void __launch_bounds__(kNoiseThreads) noise_wv_stationary_kernel(NoiseWvArgs a) {
-  __shared__ double red[kNoiseThreads / 32];
+  __shared__ double et[kExpTab];
+  __shared__ NoiseModel M;
   const int p = blockIdx.x;
-  const double *in = a.inst + 12 * (size_t)p;
   const bool gal = a.mode == 1;
-  double Amp = 0, f1 = 0, alpha = 0, fk = 0, f2 = 0;
-  if (gal) noise_gal_params(a.sgal + 5 * (size_t)p, Amp, f1, alpha, fk, f2);
-  const int NL = a.Nlayer;
-  const double Qd = (double)a.Q;
+  noise_model_load(M, a.inst + 12 * (size_t)p, gal ? a.sgal + 5 * (size_t)p : nullptr, 0.0);
+  if (gal) exp_tab_fill(et);
+  __syncthreads();
+  const size_t NL = a.Nlayer;
   const double *sgp = a.sgwb ? a.sgwb + 4 * (size_t)p : nullptr;
-  double acc = 0.0;
-  for (int j = threadIdx.x; j < NL; j += blockDim.x) {
-    double c6[6], g6[6];
-    noise_wv_layer(a, j, in, gal, Amp, f1, alpha, fk, f2, c6, g6);
-    if (gal) {  // generate_full_stationary_covariance_matrix_coarse (:1003-1010)
-      c6[0] += g6[0];
-      c6[1] += g6[1];
-      c6[2] += g6[2];
-      c6[3] -= g6[3] / 2.;
-      c6[4] -= g6[4] / 2.;
-      c6[5] -= g6[5] / 2.;
-    }
-    if (sgp) {  // added last (:1012-1019)
-      double s6[6];
-      noise_wv_sgwb(a, j, sgp, s6);
+  const double cells = (double)a.Ncoarse, icells = 1.0 / cells;
+  double chi = 0.0;
+  LogSum ld;
+  for (int j = threadIdx.x; j < a.Nlayer; j += blockDim.x) {
+    double c6[6], P[6];
+    // generate_full_stationary_covariance_matrix_coarse (:1003-1010)
+    const double g = noise_wv_layer(a, M, j, gal, sgp, et, c6);
 #pragma unroll
-      for (int e = 0; e < 6; e++) c6[e] += s6[e];
+    for (int e = 0; e < 3; e++) {
+      c6[e] += g;
+      c6[3 + e] = fma(-0.5, g, c6[3 + e]);
+      P[e] = a.tab[(kTabXX + e) * NL + j] * icells;
+      P[3 + e] = a.tab[(kTabXY + e) * NL + j] * icells;
     }
-    double iv[6], ld;
-    noise_inv3(c6[0], c6[1], c6[2], c6[3], c6[4], c6[5], iv, ld);
-    double s = 0.0;
-    s -= 0.5 * Qd * iv[0] * a.tab[(size_t)kTabXX * NL + j];
-    s -= 0.5 * Qd * iv[1] * a.tab[(size_t)kTabYY * NL + j];
-    s -= 0.5 * Qd * iv[2] * a.tab[(size_t)kTabZZ * NL + j];
-    s -= Qd * iv[3] * a.tab[(size_t)kTabXY * NL + j];
-    s -= Qd * iv[4] * a.tab[(size_t)kTabXZ * NL + j];
-    s -= Qd * iv[5] * a.tab[(size_t)kTabYZ * NL + j];
-    s -= 0.5 * Qd * ld * (double)a.Ncoarse;
-    acc += s;
+    noise_cell(c6, P, chi, ld);
   }
-  const double s = block_sum(acc, red);
-  if (threadIdx.x == 0) a.out[p] = s;
+  const double s = block_total(chi, ld);
+  if (threadIdx.x == 0) a.out[p] = -0.5 * (double)a.Q * cells * s;
 }
 
 // Mode 2: the foreground modulated per cell (generate_full_dynamic_covariance_
 // matrix_coarse :923-981).  One CTA per (chunk of LJ layers, model); the
 // chunk's layer covariances go to shared memory, then every cell is inverted
 // and summed with its statistics (my_noise_log_likelihood_wavelet_coarse
-// :1211-1241).
+// :1211-1241): 6 FP64 operations for its covariance, 26 in noise_cell.
 constexpr int kNoiseWvMaxLJ = 64;
 __global__ void __launch_bounds__(kNoiseThreads) noise_wv_dynamic_kernel(NoiseWvArgs a) {
-  __shared__ double red[kNoiseThreads / 32];
-  __shared__ double lay[kNoiseWvMaxLJ][18];
+  __shared__ double et[kExpTab];
+  __shared__ double lay[kNoiseWvMaxLJ][7];
+  __shared__ NoiseModel M;
   const int chunk = blockIdx.x, p = blockIdx.y;
-  const double *in = a.inst + 12 * (size_t)p;
-  double Amp, f1, alpha, fk, f2;
-  noise_gal_params(a.sgal + 5 * (size_t)p, Amp, f1, alpha, fk, f2);
+  noise_model_load(M, a.inst + 12 * (size_t)p, a.sgal + 5 * (size_t)p, 0.0);
+  exp_tab_fill(et);
+  __syncthreads();
   const double *sgp = a.sgwb ? a.sgwb + 4 * (size_t)p : nullptr;
   const int j0 = chunk * a.LJ;
   const int nl = min(a.LJ, a.Nlayer - j0);
-  for (int t = threadIdx.x; t < nl; t += blockDim.x) {
-    noise_wv_layer(a, j0 + t, in, true, Amp, f1, alpha, fk, f2, &lay[t][0], &lay[t][6]);
-    if (sgp)
-      noise_wv_sgwb(a, j0 + t, sgp, &lay[t][12]);
-    else
-      for (int e = 12; e < 18; e++) lay[t][e] = 0.0;
+  if ((int)threadIdx.x < nl) {
+    double c6[6];
+    lay[threadIdx.x][6] = noise_wv_layer(a, M, j0 + threadIdx.x, true, sgp, et, c6);
+#pragma unroll
+    for (int e = 0; e < 6; e++) lay[threadIdx.x][e] = c6[e];
   }
   __syncthreads();
   const int Nc = a.Ncoarse;
   const size_t Npix = (size_t)a.Nlayer * Nc;
-  const double Qd = (double)a.Q;
-  double acc = 0.0;
+  double chi = 0.0;
+  LogSum ld;
+#pragma unroll 1
   for (int idx = threadIdx.x; idx < nl * Nc; idx += blockDim.x) {
     const int jj = idx / Nc, q = idx - jj * Nc;
-    double c6[6];
+    const double *P0 = a.P + (size_t)j0 * Nc + idx;
+    double c6[6], P[6];
 #pragma unroll
-    for (int e = 0; e < 6; e++) c6[e] = lay[jj][e] + lay[jj][6 + e] * a.mod[(size_t)e * Nc + q];
-    if (sgp) {  // the stationary background last (:964-971)
-#pragma unroll
-      for (int e = 0; e < 6; e++) c6[e] += lay[jj][12 + e];
+    for (int e = 0; e < 6; e++) {
+      c6[e] = fma(lay[jj][6], a.mod[(size_t)e * Nc + q], lay[jj][e]);
+      P[e] = P0[e * Npix];
     }
-    double iv[6], ld;
-    noise_inv3(c6[0], c6[1], c6[2], c6[3], c6[4], c6[5], iv, ld);
-    const size_t k = (size_t)(j0 + jj) * Nc + q;
-    double s = 0.0;
-    s -= 0.5 * Qd * iv[0] * a.P[k];
-    s -= 0.5 * Qd * iv[1] * a.P[Npix + k];
-    s -= 0.5 * Qd * iv[2] * a.P[2 * Npix + k];
-    s -= Qd * iv[3] * a.P[3 * Npix + k];
-    s -= Qd * iv[4] * a.P[4 * Npix + k];
-    s -= Qd * iv[5] * a.P[5 * Npix + k];
-    s -= 0.5 * Qd * ld;
-    acc += s;
+    noise_cell(c6, P, chi, ld);
   }
-  const double s = block_sum(acc, red);
-  if (threadIdx.x == 0) a.out[(size_t)p * a.nchunks + chunk] = s;
+  const double s = block_total(chi, ld);
+  if (threadIdx.x == 0) a.out[(size_t)p * a.nchunks + chunk] = -0.5 * (double)a.Q * s;
 }
 
 __global__ void noise_wv_const_kernel(double *logl, int nprop, double cst) {
@@ -520,9 +617,23 @@ __device__ __forceinline__ int spline_knot_below(int K, const double *x, double 
   return lo;
 }
 
-__global__ void __launch_bounds__(kNoiseThreads) spline_noise_kernel(SplineNoiseArgs a) {
+constexpr int kSplineThreads = 256;
+
+__device__ __forceinline__ double block_sum(double v, double *red) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kSplineThreads / 32; w++) s += red[w];
+  return s;
+}
+
+__global__ void __launch_bounds__(kSplineThreads) spline_noise_kernel(SplineNoiseArgs a) {
   extern __shared__ double sm[];
-  __shared__ double red[kNoiseThreads / 32];
+  __shared__ double red[kSplineThreads / 32];
   const int p = blockIdx.x, K = a.nknots[p], KM = a.kmax;
   if (K < 2 || K > KM) {  // the whole CTA leaves before any barrier
     if (threadIdx.x == 0) a.logl[p] = __longlong_as_double(0x7ff8000000000000LL);
@@ -582,42 +693,6 @@ __global__ void __launch_bounds__(kNoiseThreads) spline_noise_kernel(SplineNoise
 // grid f_n = fmin + n/T (noise/src/glass_noise_model.c:1384-1385), the
 // transfer functions of :415-446 and :620-624, and the data's auto- and
 // cross-spectra of :1251-1263.
-void noise_build_table(double T, double fmin, int N, const double *X, const double *Y, const double *Z,
-                       double *tab) {
-  const double fstar = kCLIGHT / (2.0 * M_PI * kLARM);
-  const double acc_units = 2.81837551648e-19;  // 1/(2 pi c)^2
-  const double oms_units = 4.39256635604e-16;  // (2 pi / c)^2
-  const double acc_fmax = 0.01;
-  for (int n = 0; n < N; n++) {
-    const double f = fmin + (double)n / T;
-    double *col[kNoiseTabRows];
-    for (int r = 0; r < kNoiseTabRows; r++) col[r] = tab + (size_t)r * N + n;
-    *col[kTabF] = f;
-    if (f != 0.0) {
-      const double x = f / fstar, f2 = f * f;
-      const double sx = sin(x);
-      *col[kTabCosx] = cos(x);
-      *col[kTabTdi] = -8.0 * (sx * sx);
-      *col[kTabAcc] = (f < acc_fmax) ? acc_units / f2 * (1.0 + pow(0.4e-3 / f, 2)) * (1.0 + pow(f / 8.0e-3, 4)) : 0.0;
-      *col[kTabOms] = oms_units * f2 * (1.0 + pow(2.0e-3 / f, 4));
-      const double xg = f / (kCLIGHT / (kPI2 * kLARM));
-      *col[kTabTgal] = 4. * xg * xg * sin(xg) * sin(xg);
-      *col[kTabFp73] = pow(f, -7. / 3.);
-    } else {
-      *col[kTabCosx] = *col[kTabTdi] = *col[kTabAcc] = *col[kTabOms] = *col[kTabTgal] = *col[kTabFp73] = 0.0;
-    }
-    const double rex = X[2 * n], imx = X[2 * n + 1];
-    const double rey = Y[2 * n], imy = Y[2 * n + 1];
-    const double rez = Z[2 * n], imz = Z[2 * n + 1];
-    *col[kTabXX] = rex * rex + imx * imx;
-    *col[kTabYY] = rey * rey + imy * imy;
-    *col[kTabZZ] = rez * rez + imz * imz;
-    *col[kTabXY] = rex * rey + imx * imy;
-    *col[kTabXZ] = rex * rez + imx * imz;
-    *col[kTabYZ] = rey * rez + imy * imz;
-  }
-}
-
 static void noise_freq_rows(double f, double *tab, int N, int n) {
   const double fstar = kCLIGHT / (2.0 * M_PI * kLARM);
   const double acc_units = 2.81837551648e-19;  // 1/(2 pi c)^2
@@ -636,8 +711,33 @@ static void noise_freq_rows(double f, double *tab, int N, int n) {
     const double xg = f / (kCLIGHT / (kPI2 * kLARM));
     *col[kTabTgal] = 4. * xg * xg * sin(xg) * sin(xg);
     *col[kTabFp73] = pow(f, -7. / 3.);
+    *col[kTabLogf] = log(f);
   } else {
     *col[kTabCosx] = *col[kTabTdi] = *col[kTabAcc] = *col[kTabOms] = *col[kTabTgal] = *col[kTabFp73] = 0.0;
+    *col[kTabLogf] = 0.0;
+  }
+  // the covariance's products (the reference's c_ij / 4)
+  const double cx = *col[kTabCosx], td = *col[kTabTdi];
+  *col[kTabU1] = -0.5 * td * *col[kTabOms];
+  *col[kTabU2] = -0.5 * td * *col[kTabAcc];
+  *col[kTabU3] = *col[kTabU2] * cx * cx;
+  *col[kTabV1] = 0.25 * td * cx * *col[kTabOms];
+  *col[kTabV2] = 0.25 * td * cx * *col[kTabAcc];
+}
+
+void noise_build_table(double T, double fmin, int N, const double *X, const double *Y, const double *Z,
+                       double *tab) {
+  for (int n = 0; n < N; n++) {
+    noise_freq_rows(fmin + (double)n / T, tab, N, n);
+    const double rex = X[2 * n], imx = X[2 * n + 1];
+    const double rey = Y[2 * n], imy = Y[2 * n + 1];
+    const double rez = Z[2 * n], imz = Z[2 * n + 1];
+    tab[(size_t)kTabXX * N + n] = rex * rex + imx * imx;
+    tab[(size_t)kTabYY * N + n] = rey * rey + imy * imy;
+    tab[(size_t)kTabZZ * N + n] = rez * rez + imz * imz;
+    tab[(size_t)kTabXY * N + n] = 2.0 * (rex * rey + imx * imy);
+    tab[(size_t)kTabXZ * N + n] = 2.0 * (rex * rez + imx * imz);
+    tab[(size_t)kTabYZ * N + n] = 2.0 * (rey * rez + imy * imz);
   }
 }
 
@@ -674,7 +774,8 @@ void noise_wv_build(int NT, double df, int lmin, int Nlayer, int Q, const double
         syz += wy * wz;
       }
       const size_t kc = (size_t)q + (size_t)j * Nc;
-      const double v[6] = {sxx * invQ, syy * invQ, szz * invQ, sxy * invQ, sxz * invQ, syz * invQ};
+      const double v[6] = {sxx * invQ, syy * invQ, szz * invQ, 2.0 * (sxy * invQ), 2.0 * (sxz * invQ),
+                           2.0 * (syz * invQ)};  // the off-diagonal terms count twice
       for (int e = 0; e < 6; e++) {
         P[(size_t)e * Npix + kc] = v[e];
         S[e] += v[e];
@@ -759,16 +860,20 @@ int noise_sgwb_rows(int nresp, const double *resp, int N, const double *f, doubl
   return 0;
 }
 
-static int noise_wv_lj(const NoiseWvDev &w) {
+// Layers per CTA of the modulated form: about 4096 cells, fewer where the
+// batch is too small to give every SM a few CTAs (a CTA's model constants and
+// layer covariances cost about as much as 300 cells).
+static int noise_wv_lj(const NoiseWvDev &w, int nprop) {
   int lj = 4096 / (w.Ncoarse > 0 ? w.Ncoarse : 1);
   if (lj < 1) lj = 1;
   if (lj > kNoiseWvMaxLJ) lj = kNoiseWvMaxLJ;
+  while (lj > 1 && (long long)((w.Nlayer + lj - 1) / lj) * nprop < kNoiseTargetCtas) lj = (lj + 1) / 2;
   return lj;
 }
 
-int noise_wv_chunks(const NoiseWvDev &w) {
-  const int lj = noise_wv_lj(w);
-  return (w.Nlayer + lj - 1) / lj;
+size_t noise_wv_partials(const NoiseWvDev &w, int nprop) {
+  const size_t most = (size_t)nprop * ((w.Nlayer + noise_wv_lj(w, 1 << 30) - 1) / noise_wv_lj(w, 1 << 30));
+  return most > 4 * (size_t)kNoiseTargetCtas + 4 * (size_t)nprop ? most : 4 * (size_t)kNoiseTargetCtas + 4 * (size_t)nprop;
 }
 
 cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const double *inst, const double *sgal,
@@ -777,8 +882,8 @@ cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const
   a.Nlayer = w.Nlayer;
   a.Ncoarse = w.Ncoarse;
   a.Q = w.Q;
-  a.LJ = noise_wv_lj(w);
-  a.nchunks = noise_wv_chunks(w);
+  a.LJ = noise_wv_lj(w, nprop);
+  a.nchunks = (w.Nlayer + a.LJ - 1) / a.LJ;
   a.mode = mode;
   a.inv_ND = 1.0 / (double)((long long)w.NF * w.NT);
   a.tab = w.tab;
@@ -828,7 +933,20 @@ cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const
   return cudaGetLastError();
 }
 
-int noise_chunks(int N) { return (N + kNoiseChunk - 1) / kNoiseChunk; }
+static int noise_bins_per_thread(int N, int nprop) {
+  int R = kNoiseMaxBins;
+  while (R > 1 && (long long)((N + kNoiseThreads * R - 1) / (kNoiseThreads * R)) * nprop < kNoiseTargetCtas) R /= 2;
+  return R;
+}
+
+// What any batch of at most nprop models needs: below the largest chunk the
+// rule stops at the first size that reaches the target, at most twice it.
+size_t noise_partials(int N, int nprop) {
+  const int chunk = kNoiseThreads * kNoiseMaxBins;
+  const size_t most = (size_t)nprop * ((N + chunk - 1) / chunk);
+  const size_t few = 2 * (size_t)kNoiseTargetCtas + 2 * (size_t)nprop;
+  return most > few ? most : few;
+}
 
 static size_t spline_smem(int nch, int kmax) { return sizeof(double) * (size_t)kmax * (1 + 6 * nch); }
 
@@ -851,7 +969,7 @@ cudaError_t spline_noise_launch(const SplineNoiseDev &s, int nprop, int kmax, co
   a.knot_f = knot_f;
   a.knot_C = knot_C;
   a.logl = logl;
-  spline_noise_kernel<<<nprop, kNoiseThreads, spline_smem(s.nch, kmax), stream>>>(a);
+  spline_noise_kernel<<<nprop, kSplineThreads, spline_smem(s.nch, kmax), stream>>>(a);
   if (nlaunch) *nlaunch = 1;
   return cudaGetLastError();
 }
@@ -860,7 +978,9 @@ cudaError_t noise_logl_launch(const NoiseDev &nd, int nprop, const double *inst,
                               const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch) {
   NoiseArgs a;
   a.N = nd.N;
-  a.nchunks = noise_chunks(nd.N);
+  a.R = noise_bins_per_thread(nd.N, nprop);
+  a.nchunks = (nd.N + kNoiseThreads * a.R - 1) / (kNoiseThreads * a.R);
+  a.fstep = kNoiseThreads / nd.T;
   a.nprop = nprop;
   a.tab = nd.tab;
   a.inst = inst;

@@ -6,10 +6,13 @@ namespace glass {
 
 // Rows of the per-bin table (each N doubles): the frequency, cos(f/f*), the
 // TDI transfer function -8 sin^2(f/f*), the acceleration and optical-metrology
-// transfer functions, the foreground's 4 x^2 sin^2 x and f^(-7/3), and the
-// data's XX, YY, ZZ, XY, XZ, YZ spectra.
+// transfer functions, the foreground's 4 x^2 sin^2 x, f^(-7/3) and log f, the
+// transfer products of the XYZ covariance's diagonal (metrology, acceleration,
+// acceleration cos^2) and off-diagonal entries (metrology, acceleration), and
+// the data's XX, YY, ZZ, 2 XY, 2 XZ, 2 YZ spectra.
 enum {
-  kTabF = 0, kTabCosx, kTabTdi, kTabAcc, kTabOms, kTabTgal, kTabFp73,
+  kTabF = 0, kTabCosx, kTabTdi, kTabAcc, kTabOms, kTabTgal, kTabFp73, kTabLogf,
+  kTabU1, kTabU2, kTabU3, kTabV1, kTabV2,
   kTabXX, kTabYY, kTabZZ, kTabXY, kTabXZ, kTabYZ, kNoiseTabRows
 };
 // One- and two-channel data (Michelson X; or A and E) keep the data's power
@@ -37,7 +40,7 @@ struct NoiseWvDev {
   double df = 0;
   bool has_mod = false;
   double *tab = nullptr;      // kNoiseTabRows x Nlayer: layer-centre factors, then per-layer sums of P over q
-  double *P = nullptr;        // 6 x Nlayer Ncoarse cell statistics (xx, yy, zz, xy, xz, yz)
+  double *P = nullptr;        // 6 x Nlayer Ncoarse cell statistics (xx, yy, zz, 2 xy, 2 xz, 2 yz)
   double *mod = nullptr;      // 6 x Ncoarse modulation of the foreground (or unused)
   double *rsg = nullptr;      // 6 x Nlayer: the SGWB response at the layer centres, or null
   double *partial = nullptr;  // per-model chunk sums
@@ -51,10 +54,11 @@ struct NoiseWvDev {
 // kTabXX .. kTabYZ).
 void noise_wv_build(int NT, double df, int lmin, int Nlayer, int Q, const double *X, const double *Y, const double *Z,
                     double *tab, double *P);
-int noise_wv_chunks(const NoiseWvDev &w);
+// doubles that w.partial needs for any batch of at most nprop models
+size_t noise_wv_partials(const NoiseWvDev &w, int nprop);
 // mode 0 instrument, 1 stationary foreground, 2 modulated foreground; plus,
 // with sgwb (4 per model, template sg_type), the stochastic background;
-// w.partial must hold nprop x noise_wv_chunks(w) (mode 2).
+// w.partial must hold noise_wv_partials(w, nprop) (mode 2).
 cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const double *inst, const double *sgal,
                                  int sg_type, const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch);
 
@@ -79,11 +83,12 @@ struct SplineNoiseDev {
 // knot_C[(p nch + c) kmax ..] (device pointers)
 cudaError_t spline_noise_launch(const SplineNoiseDev &s, int nprop, int kmax, const int *nknots, const double *knot_f,
                                 const double *knot_C, double *logl, cudaStream_t stream, int *nlaunch);
-int noise_chunks(int N);
+// doubles that nd.partial needs for any batch of at most nprop models
+size_t noise_partials(int N, int nprop);
 // logl[p] for noise models inst[12 p ..] (sacc[6], soms[6]) and sgal[5 p ..]
 // (or null: instrument only), plus, with sgwb[4 p ..] (or null), the SGWB of
-// template sg_type (three channels only); nd.partial must hold nprop x
-// noise_chunks(N).  Three channels: my_noise_log_likelihood; one or two:
+// template sg_type (three channels only); nd.partial must hold
+// noise_partials(N, nprop).  Three channels: my_noise_log_likelihood; one or two:
 // noise_log_likelihood (no 2 pi constant), link levels sacc[0], soms[0].
 cudaError_t noise_logl_launch(const NoiseDev &nd, int nprop, const double *inst, const double *sgal, int sg_type,
                               const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch);
