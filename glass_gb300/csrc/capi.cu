@@ -952,14 +952,14 @@ extern "C" int glass_gpu_grad_fisher_batch_host(glass_gpu_ctx *ctx, int nitems, 
 
 // ------------------------------------------------------------ F-statistic
 // Scratch of the F-statistic batches: cells per launch sequence bounded so
-// that the filter series (16 N complex doubles per cell at the segment's
+// that the filter series (8 N complex doubles per cell at the segment's
 // largest filter size) stay within kFsSeriesBudget.
 static constexpr size_t kFsSeriesBudget = (size_t)2 << 30;
 
 static int ensure_fs_work(glass_gpu_ctx *ctx, int ncells) {
   int maxN = fs_max_size(ctx->bank.NFFT);
   if (maxN > kMaxN) maxN = kMaxN;
-  const size_t per_cell = (size_t)16 * maxN * sizeof(double2);
+  const size_t per_cell = (size_t)8 * maxN * sizeof(double2);
   size_t chunk = kFsSeriesBudget / per_cell;
   if (chunk < 256) chunk = 256;
   size_t want = 256;
@@ -1896,7 +1896,7 @@ static cudaError_t legacy_enqueue(LegacyThread &L, int fmt, double T, int BW, in
   if (e != cudaSuccess) return e;
   e = fd_waveform_launch(reinterpret_cast<const OrbitSample64 *>(L.d_in + LegacyThread::kPosOffset),
                          reinterpret_cast<const ItemF64 *>(L.d_in), BW, fmt, NI, T, fstar_of_orbit(), L.d_d6, L.d_out,
-                         L.tab.tw64[bin_index(BW)], s);
+                         L.tab.tw64[bin_index(BW)], L.tab.tw64[bin_index(kSincosTab)], s);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(L.h_out, L.d_out, sizeof(double) * nout, cudaMemcpyDeviceToHost, s);
 }
@@ -1914,7 +1914,7 @@ static int legacy_waveform_run(int fmt, double T, const double *params, int NPar
   // plan kernels run, with the reference's operation order
   SourceGeom geo;
   source_geometry(p, NParams, T, geo);
-  make_item_f64(geo, BW, *L.h_item());
+  make_item_f64(geo, BW, fstar_of_orbit(), *L.h_item());
   bool all = (fmt == GLASS_FMT_SANGRIA) || NI > 1;
   size_t nout = all ? 10 * (size_t)BW : 2 * (size_t)BW;
   cudaStream_t s = L.stream;
@@ -1975,6 +1975,7 @@ extern "C" int glass_ucb_waveform(const double *orbit_xyz, const char *format, d
       o.z[i] = xyz[3 * i + 2];
     }
     o.t = t;
+    orbit_arms(o);
   }
   return legacy_waveform_run(fmt, T, params, NParams, X, Y, Z, A, E, BW, NI);
 }
@@ -2003,6 +2004,7 @@ extern "C" void ucb_waveform(struct Orbit *orbit, char *format, double T, double
         s.z[i] = z[i + 1];
       }
       s.t = t;
+      orbit_arms(s);
     }
     rc = legacy_waveform_run(fmt, T, params, NParams, X, Y, Z, A, E, BW, NI);
   }

@@ -1,0 +1,97 @@
+// FP64 building blocks counted in FP64 instructions.
+//
+// GB300's FP64 pipe does 2 multiply-adds per SM and clock, 1/64 of FP32: a
+// warp's FP64 instruction holds it for 16 clocks, and integer work, loads and
+// selects are free beside it.  The forms here spend table loads and integer
+// operations to save FP64 instructions, at the accuracy of the library's.
+#pragma once
+#include <math.h>
+
+namespace glass {
+
+// 1/x for normal x of moderate exponent: the hardware's ~20-bit estimate and
+// one step of Householder's cubic iteration, r (1 + e + e^2) with e = 1 - x r.
+__device__ __forceinline__ double rcp_fast(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+constexpr double kRoundMagic = 6755399441055744.0;  // 1.5 2^52: adding it rounds to the nearest integer
+
+// exp by table and short polynomial (Tang, ACM Trans. Math. Softw. 15, 1989):
+// x = (64 m + k) ln2/64 + r, exp x = 2^m t[k] (1 + r + ... + r^5/120), t[k] =
+// 2^(k/64), |r| <= ln2/128.  10 FP64 instructions; arguments beyond +-708 and
+// NaN go to the library's.
+constexpr int kExpTab = 64;
+__device__ __forceinline__ double exp_tab(double x, const double *t) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40862000) return exp(x);
+  constexpr double kLn2 = 0.693147180559945309417, kLn2Lo = 2.3190468138462996e-17;  // ln 2 = kLn2 + kLn2Lo
+  const double z = fma(x, kExpTab / kLn2, kRoundMagic);
+  const int n = __double2loint(z);
+  const double kd = z - kRoundMagic;
+  double r = fma(kd, -kLn2 / kExpTab, x);
+  r = fma(kd, -kLn2Lo / kExpTab, r);
+  double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+  q = fma(r, q, 1.0 / 6.0);
+  q = fma(r, q, 0.5);
+  q = fma(r * r, q, r);
+  const double T = t[n & (kExpTab - 1)];
+  const double y = fma(T, q, T);
+  return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
+}
+__device__ __forceinline__ void exp_tab_fill(double *t) {
+  for (int k = threadIdx.x; k < kExpTab; k += blockDim.x) t[k] = exp2(k * (1.0 / kExpTab));
+}
+
+// sin x and cos x by table and short polynomials (the same method): x = k
+// 2 pi/1024 + r, |r| <= pi/1024, and the angle-sum formulas.  tw: the 1024-point
+// FFT twiddles exp(-2 pi i k/1024).  14 FP64 instructions (the library's take
+// about 25); within 1 ulp of 1 like theirs.  |x| >= 1e5 (where the reduction's
+// two-part 2 pi/1024 would lose accuracy) and non-finite x go to the library's.
+constexpr int kSincosTab = 1024;
+__device__ __forceinline__ void sincos_tab(double x, const double2 *tw, double *s, double *c) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) {
+    sincos(x, s, c);
+    return;
+  }
+  constexpr double k2Pi = 6.283185307179586477, k2PiLo = 2.4492935982947064e-16;  // 2 pi = k2Pi + k2PiLo
+  const double z = fma(x, kSincosTab / k2Pi, kRoundMagic);
+  const double kd = z - kRoundMagic;
+  double r = fma(kd, -k2Pi / kSincosTab, x);
+  r = fma(kd, -k2PiLo / kSincosTab, r);
+  const double2 t = tw[__double2loint(z) & (kSincosTab - 1)];  // cos, -sin of the table angle
+  const double r2 = r * r;
+  const double sn = fma(r * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), r);
+  const double cm1 = r2 * fma(r2, 1.0 / 24.0, -0.5);
+  *c = fma(t.y, sn, fma(t.x, cm1, t.x));
+  *s = fma(t.x, sn, -fma(t.y, cm1, t.y));
+}
+
+// sin(x) / x: the Taylor series for |x| <= 1 (to x^10/11! for |x| <= 0.2, to
+// x^16/17! beyond: truncation below 1e-17), else the quotient.
+__device__ __forceinline__ double sinc64(double x) {
+  const double z = x * x;
+  const int h = __double2hiint(z);
+  if (h <= 0x3fa47ae1) {  // z <= 0.04
+    double p = fma(z, -1.0 / 39916800.0, 1.0 / 362880.0);
+    p = fma(z, p, -1.0 / 5040.0);
+    p = fma(z, p, 1.0 / 120.0);
+    p = fma(z, p, -1.0 / 6.0);
+    return fma(z, p, 1.0);
+  }
+  if (h < 0x3ff00000) {  // z < 1
+    double p = fma(z, 1.0 / 355687428096000.0, -1.0 / 1307674368000.0);
+    p = fma(z, p, 1.0 / 6227020800.0);
+    p = fma(z, p, -1.0 / 39916800.0);
+    p = fma(z, p, 1.0 / 362880.0);
+    p = fma(z, p, -1.0 / 5040.0);
+    p = fma(z, p, 1.0 / 120.0);
+    p = fma(z, p, -1.0 / 6.0);
+    return fma(z, p, 1.0);
+  }
+  return sin(x) / x;
+}
+
+}  // namespace glass

@@ -179,14 +179,16 @@ __device__ __forceinline__ df df_reduce_2pi_df(df x) {
 // so that dplus*DPr + dcross*DCr = r.Mr.r for an arm direction r.  Symmetric
 // tensors are stored as xx, xy, xz, yy, yz, zz.
 
-// Plain-FP64 path.
+// Plain-FP64 path.  The polarisation tensors are e+ = v v - u u and ex = u v +
+// v u, so an arm r has r.e+.r = (r.v)^2 - (r.u)^2 and r.ex.r = 2 (r.u)(r.v).
 struct ItemF64 {
   int seg, N, imin, pad;
-  double k[3];
-  double ep[6], ec[6];        // polarisation tensors e+, ex
-  double DPr, DPi, DCr, DCi;  // amplitude-free polarisation factors
-  double f0, fdot, phi0, dfq;  // dfq = 2 pi q / T (ucb/src/glass_ucb_waveform.c:818)
-  double amp_s;               // amp / (2N)
+  double k[3], u[3], v[3];      // propagation direction, polarisation axes (v[2] = 0)
+  double DPr, DPi, DC2r, DC2i;  // amplitude-free polarisation factors, DC twice
+  double f0, phi0, dfq;         // dfq = 2 pi q / T (ucb/src/glass_ucb_waveform.c:818)
+  double w0, wd, ae;            // 2 pi f0, pi fdot, (2/3) fdot / f0
+  double h0, hd;                // f0 / (2 f*), fdot / (2 f*)
+  double amp_s;                 // amp / (2N)
 };
 
 // Mixed path: FP32 for everything but the carrier phase, which is carried as
@@ -238,11 +240,22 @@ struct __align__(16) ItemGrad {
 };
 
 // Per-sample orbit tables, one per waveform size.  Positions of the three
-// spacecraft (FP64, metres) and the sample time; and, for the mixed path,
-// u = t/T and the guiding-centre angle cos/sin(2 pi t / YEAR) as double-floats.
+// spacecraft (FP64, metres), the sample time and the arm vectors over L; and,
+// for the mixed path, u = t/T and the guiding-centre angle cos/sin(2 pi t /
+// YEAR) as double-floats.
 struct OrbitSample64 {
   double x[3], y[3], z[3], t;
+  double r[3][3];  // (x_j - x_i) / L of arms 12, 13, 23
 };
+// Fills the arm vectors from the positions.
+__host__ __device__ inline void orbit_arms(OrbitSample64 &o) {
+  for (int a = 0; a < 3; a++) {
+    const int i = a == 2 ? 1 : 0, j = a == 0 ? 1 : 2;
+    o.r[a][0] = (o.x[j] - o.x[i]) / kLARM;
+    o.r[a][1] = (o.y[j] - o.y[i]) / kLARM;
+    o.r[a][2] = (o.z[j] - o.z[i]) / kLARM;
+  }
+}
 struct OrbitSampleMix {
   float u_hi, u_lo, ca_hi, ca_lo;
   float sa_hi, sa_lo, pad0, pad1;

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "../../include/glass_gb300.h"
+#include "fp64_math.cuh"
 #include "glass_common.cuh"
 #include "noise.cuh"
 
@@ -67,42 +68,6 @@ struct NoiseArgs {
   const double *rsg;   // SGWB response, 6 rows of N
   double *partial;     // [nprop][nchunks]
 };
-
-// ------------------------------------------------------ FP64 building blocks
-// 1/x for normal x of moderate exponent: the hardware's ~20-bit estimate and
-// one step of Householder's cubic iteration, r (1 + e + e^2) with e = 1 - x r.
-__device__ __forceinline__ double rcp_fast(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
-// exp by table and short polynomial (Tang, ACM Trans. Math. Softw. 15, 1989):
-// x = (64 m + k) ln2/64 + r, exp x = 2^m t[k] (1 + r + ... + r^5/120), t[k] =
-// 2^(k/64), |r| <= ln2/128.  10 FP64 instructions; arguments beyond +-708 and
-// NaN go to the library's.
-constexpr int kExpTab = 64;
-__device__ __forceinline__ double exp_tab(double x, const double *t) {
-  if ((__double2hiint(x) & 0x7fffffff) >= 0x40862000) return exp(x);
-  constexpr double kLn2 = 0.693147180559945309417, kLn2Lo = 2.3190468138462996e-17;  // ln 2 = kLn2 + kLn2Lo
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adds to the nearest integer
-  const double z = fma(x, kExpTab / kLn2, kMagic);
-  const int n = __double2loint(z);
-  const double kd = z - kMagic;
-  double r = fma(kd, -kLn2 / kExpTab, x);
-  r = fma(kd, -kLn2Lo / kExpTab, r);
-  double q = fma(r, 1.0 / 120.0, 1.0 / 24.0);
-  q = fma(r, q, 1.0 / 6.0);
-  q = fma(r, q, 0.5);
-  q = fma(r * r, q, r);
-  const double T = t[n & (kExpTab - 1)];
-  const double y = fma(T, q, T);
-  return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
-}
-__device__ __forceinline__ void exp_tab_fill(double *t) {
-  for (int k = threadIdx.x; k < kExpTab; k += blockDim.x) t[k] = exp2(k * (1.0 / kExpTab));
-}
 
 // A sum of logarithms of positive normal numbers as the product of their
 // mantissas, kept in [1, 2), and the sum of their exponents.

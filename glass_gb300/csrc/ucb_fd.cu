@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(64) fd_plan64_kernel(PlanArgs a) {
       SourceGeom g;
       source_geometry(p, 8, T, g);
       ItemF64 c;
-      make_item_f64(g, N, c);
+      make_item_f64(g, N, a.fstar, c);
       c.seg = seg;
       c.N = N;
       c.imin = imin;
@@ -291,6 +291,7 @@ __global__ void fd_orbit_table_kernel(FdTablesDev tab, double T, double t0) {
     o.z[i] = -kSQ3 * R * (ca * cb + sa * sb);
   }
   o.t = t;
+  orbit_arms(o);
   tab.pos64[b][n] = o;
   OrbitSampleMix m;
   df u = df_from_double(t / T), cd = df_from_double(ca), sd = df_from_double(sa);
@@ -516,6 +517,7 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
     sa.mix[b] = tab.mix[b];
     sa.geo[b] = tab.geo[b];
   }
+  sa.tw1024 = tab.tw64[fd_bin_of(kSincosTab)];
   sa.series = work.series;
   sa.nitems = nitems;
   sa.series_len = (long long)(work.series_bytes / (mix ? sizeof(float2) : sizeof(double2)));
@@ -721,12 +723,12 @@ size_t fd_series_bytes(int nitems, int NFFT, int precision) {
 // FP64 pipe of many SMs, not one); then one CTA per Michelson channel (X, Y,
 // Z) FFTs its two series and applies the format's TDI weights per bin.  A and
 // E follow in fd_ae_kernel from the stored X, Y, Z (utils/src/glass_lisa.c:429-441).
-__global__ void fd_single_slow_kernel(const OrbitSample64 *pos, const ItemF64 *item, int N, double fstar, double L,
+__global__ void fd_single_slow_kernel(const OrbitSample64 *pos, const ItemF64 *item, int N, const double2 *tw1024,
                                       double2 *d6) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
   double2 d[6];
-  slow_sample64(*item, pos[n], fstar, L, d);
+  slow_sample64(*item, pos[n], tw1024, d);
 #pragma unroll
   for (int a = 0; a < 6; a++) d6[(size_t)a * N + n] = d[a];
 }
@@ -757,7 +759,7 @@ __global__ void __launch_bounds__(LegacyCfg<N>::GT) fd_waveform_kernel(const Ite
     buf[N + n] = csub(d6[(size_t)va * N + n], d6[(size_t)vb * N + n]);
   }
   __syncthreads();
-  group_fft<N, GT, 2, 1, double2, 64>(buf, tw, lane);  // CTA barrier: the CTA may be a partial warp
+  group_fft<N, GT, 2, 1, double2, true>(buf, tw, lane);  // CTA barrier: the CTA may be a partial warp
   const double sqT = sqrt(T);
   const long long q = (long long)(item->f0 * T);
   const double amp_s = item->amp_s;
@@ -821,9 +823,10 @@ static cudaError_t launch_waveform(const ItemF64 *item, const double2 *d6, int f
 }
 
 cudaError_t fd_waveform_launch(const OrbitSample64 *pos, const ItemF64 *item, int N, int format, int NI, double T,
-                               double fstar, double2 *d6, double *out, const double2 *tw, cudaStream_t stream) {
+                               double fstar, double2 *d6, double *out, const double2 *tw, const double2 *tw1024,
+                               cudaStream_t stream) {
   int nch = (format != 0 && NI <= 1) ? 1 : 3;
-  fd_single_slow_kernel<<<(N + 31) / 32, 32, 0, stream>>>(pos, item, N, fstar, kLARM, d6);
+  fd_single_slow_kernel<<<(N + 31) / 32, 32, 0, stream>>>(pos, item, N, tw1024, d6);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   e = cudaErrorInvalidValue;

@@ -125,7 +125,7 @@ struct FsWorkDev {
   void *cells = nullptr;     // [cap] per-cell constants
   int *bin_count = nullptr;  // [16]
   int *bin_list = nullptr;   // [9*cap]
-  void *series = nullptr;    // 16 series of N complex doubles per cell
+  void *series = nullptr;    // 8 series of N complex doubles per cell
   size_t series_bytes = 0;
 };
 size_t fs_cell_bytes();
@@ -157,9 +157,10 @@ cudaError_t fs_finalize(const double *logl0, const int *pos, const double *scan,
 // pos: N orbit samples (device), item: the source's FP64 constants (device,
 // from source_geometry + make_item_f64), d6: 6 N complex scratch, out: 10*N
 // doubles (device) = X,Y,Z,A,E.  tw: the N-point FP64 twiddle table
-// (FdTablesDev::tw64 of the size).
+// (FdTablesDev::tw64 of the size), tw1024: the 1024-point one.
 cudaError_t fd_waveform_launch(const OrbitSample64 *pos, const ItemF64 *item, int N, int format, int NI, double T,
-                               double fstar, double2 *d6, double *out, const double2 *tw, cudaStream_t stream);
+                               double fstar, double2 *d6, double *out, const double2 *tw, const double2 *tw1024,
+                               cudaStream_t stream);
 
 
 }  // namespace glass

@@ -6,6 +6,7 @@
 
 #include <type_traits>
 
+#include "fp64_math.cuh"
 #include "ucb_fd.cuh"
 
 namespace glass {
@@ -50,6 +51,17 @@ __device__ __forceinline__ void group_sync() {
   }
 }
 
+// The same for the groups of one CTA that run on their own (some may have left):
+// groups above a warp use a named barrier each, id 1 + group.
+template <int GT>
+__device__ __forceinline__ void group_bar(int g) {
+  if constexpr (GT <= 32) {
+    __syncwarp();
+  } else {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(GT) : "memory");
+  }
+}
+
 // ----------------------------------------------------------------------- FFT
 // In-place forward DFT (exp(-2 pi i k n / N), unnormalised) of NSER series of
 // length N held series-major in shared memory, by a group of GT threads.
@@ -60,8 +72,16 @@ __device__ __forceinline__ void group_sync() {
 // lets the stage overwrite its own input.  CH series are processed per round to
 // bound register use; rounds touch disjoint series, so a round's loads need no
 // barrier after the previous round's stores, only one at the end of the stage.
-template <int N, int GT, int NSER, int CH, typename C, int SYNC_GT = GT>
-__device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane) {
+// SYNC_CTA: the group is the whole CTA, which may be a partial warp; else the
+// groups of the CTA synchronise on their own (group_bar of group g).
+template <int N, int GT, int NSER, int CH, typename C, bool SYNC_CTA = false>
+__device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane, int g = 0) {
+  auto sync = [&] {
+    if constexpr (SYNC_CTA)
+      __syncthreads();
+    else
+      group_bar<GT>(g);
+  };
   constexpr int LOG = ilog2c(N);
   constexpr int NR4 = LOG / 2;
   constexpr int B4 = N / 4 / GT;
@@ -93,7 +113,7 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane) {
 #pragma unroll
           for (int m = 0; m < 4; ++m) v[s][b][m] = buf[(c0 + s) * N + i + m * (N / 4)];
         }
-      group_sync<SYNC_GT>();
+      sync();
 #pragma unroll
       for (int s = 0; s < CH; ++s)
 #pragma unroll
@@ -113,7 +133,7 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane) {
           o[3 * p] = csub(bb, d);
         }
     }
-    group_sync<SYNC_GT>();
+    sync();
     p *= 4;
   }
   if constexpr (LOG & 1) {
@@ -133,7 +153,7 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane) {
           v[s][b][0] = buf[(c0 + s) * N + i];
           v[s][b][1] = buf[(c0 + s) * N + i + N / 2];
         }
-      group_sync<SYNC_GT>();
+      sync();
 #pragma unroll
       for (int s = 0; s < CH; ++s)
 #pragma unroll
@@ -146,7 +166,7 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane) {
           buf[(c0 + s) * N + j + p] = csub(v[s][b][0], u1);
         }
     }
-    group_sync<SYNC_GT>();
+    sync();
   }
 }
 
@@ -444,7 +464,7 @@ static __device__ int bandwidth_dev(double L, double fstar, double f, double fdo
 // utils/src/glass_lisa.c:1566-1596).
 struct SourceGeom {
   double f0, fdot, phi0, amp, eps, dfq;
-  double k[3], ep[6], ec[6];
+  double k[3], u[3], v[3], ep[6], ec[6];
   double DPr, DPi, DCr, DCi;
 };
 
@@ -470,6 +490,10 @@ static __host__ __device__ void source_geometry(const double *p, int NP, double 
   sincos(phi, &sinph, &cosph);
   double u[3] = {costh * cosph, costh * sinph, -sinth};
   double v[3] = {sinph, -cosph, 0.};
+  for (int i = 0; i < 3; i++) {
+    g.u[i] = u[i];
+    g.v[i] = v[i];
+  }
   g.k[0] = -sinth * cosph;
   g.k[1] = -sinth * sinph;
   g.k[2] = -costh;
@@ -481,20 +505,24 @@ static __host__ __device__ void source_geometry(const double *p, int NP, double 
     }
 }
 
-static __host__ __device__ void make_item_f64(const SourceGeom &g, int N, ItemF64 &c) {
-  for (int i = 0; i < 3; i++) c.k[i] = g.k[i];
-  for (int i = 0; i < 6; i++) {
-    c.ep[i] = g.ep[i];
-    c.ec[i] = g.ec[i];
+static __host__ __device__ void make_item_f64(const SourceGeom &g, int N, double fstar, ItemF64 &c) {
+  for (int i = 0; i < 3; i++) {
+    c.k[i] = g.k[i];
+    c.u[i] = g.u[i];
+    c.v[i] = g.v[i];
   }
   c.DPr = g.DPr;
   c.DPi = g.DPi;
-  c.DCr = g.DCr;
-  c.DCi = g.DCi;
+  c.DC2r = 2.0 * g.DCr;
+  c.DC2i = 2.0 * g.DCi;
   c.f0 = g.f0;
-  c.fdot = g.fdot;
   c.phi0 = g.phi0;
   c.dfq = g.dfq;
+  c.w0 = kPI2 * g.f0;
+  c.wd = kPI * g.fdot;
+  c.ae = 0.66666666666666666666 * g.fdot / g.f0;
+  c.h0 = 0.5 * g.f0 / fstar;
+  c.hd = 0.5 * g.fdot / fstar;
   c.amp_s = g.amp / (2.0 * (double)N);
 }
 
@@ -603,92 +631,89 @@ __device__ __forceinline__ void fast_sincos(float x, float *s, float *c) {
   *c = ((qi + 1) & 2) ? -cc : cc;
 }
 
-// Delay of spacecraft i's sample, xi = t - k.x_i / c, and the carrier
-// argument w0 xi - phi0 - dfq t + wd xi^2 (ucb/src/glass_ucb_waveform.c:858-870),
-// every operation rounded on its own.
-__device__ __forceinline__ double slow_xi64(const ItemF64 &c, const OrbitSample64 &o, int i) {
-  const double kx = __dadd_rn(__dadd_rn(__dmul_rn(o.x[i], c.k[0]), __dmul_rn(o.y[i], c.k[1])), __dmul_rn(o.z[i], c.k[2]));
-  return __dsub_rn(o.t, __ddiv_rn(kx, kCLIGHT));
-}
-__device__ __forceinline__ double slow_arg2_64(const ItemF64 &c, double t, double w0, double wd, double xi) {
-  const double a2 = __dsub_rn(__dsub_rn(__dmul_rn(w0, xi), c.phi0), __dmul_rn(c.dfq, t));
-  return __dadd_rn(a2, __dmul_rn(__dmul_rn(wd, xi), xi));
-}
-// One arm from its spacecraft's terms and its own projections
-// (ucb/src/glass_ucb_waveform.c:880-922).
-__device__ __forceinline__ double2 slow_arm64(const ItemF64 &c, double fon, double aev, double arg2, double dp,
-                                              double dcr, double kr) {
-  const double arg1 = 0.5 * fon * (1.0 + kr);
-  const double sinc = 0.25 * sin(arg1) / arg1;
-  const double t1r = aev * (dp * c.DPr + dcr * c.DCr);
-  const double t1i = aev * (dp * c.DPi + dcr * c.DCi);
-  double s2, c2;
-  sincos(__dsub_rn(arg1, arg2), &s2, &c2);
-  return make_double2(sinc * (t1r * c2 + t1i * s2), sinc * (-t1r * s2 + t1i * c2));
+// ------------------------------------------------------------ FP64 slow part
+// The six arm series d_ij at one sample (order 12, 13, 21, 23, 31, 32),
+// amplitude-free (ucb/src/glass_ucb_waveform.c:840-922).  The carrier argument
+// arg2 reaches ~1e6 rad, where every rounding step is worth ~1e-10 rad: the
+// delay xi and the carrier phase round every product and sum separately
+// (explicit round-to-nearest operations), as the reference's C does; everything
+// else is arranged for few FP64 instructions, which bound the kernel (the pipe
+// is 87% busy): arm vectors from the sample table, antenna patterns from the
+// arms' projections on the polarisation axes, per-proposal constants instead of
+// divisions, sinc by series and sincos by table.  640 -> 320 FP64 instructions
+// per sample; the FP64 step of 3072 proposals (32..1024 samples) 1169 -> 633 us,
+// with the spectral unit below.
+
+// kx / c, correctly rounded: the product with 1/c and one exact-residual step.
+__device__ __forceinline__ double div_clight(double kx) {
+  constexpr double ic = 1.0 / kCLIGHT;
+  const double q = kx * ic;
+  return fma(fma(-q, kCLIGHT, kx), ic, q);
 }
 
-// The six arm series d_ij at one sample (order 12, 13, 21, 23, 31, 32),
-// amplitude-free, in FP64 with the reference's own sequence of operations
-// (ucb/src/glass_ucb_waveform.c:840-922).  The carrier argument arg2 reaches
-// ~1e6 rad, where every rounding step is worth ~1e-10 rad: the delay xi and
-// the carrier phase round every product and sum separately (explicit
-// round-to-nearest operations, which multiply-add contraction leaves alone),
-// as the reference's C does; everything else may contract.
-__device__ __forceinline__ void slow_sample64(const ItemF64 &c, const OrbitSample64 &o, double fstar, double L,
+// Arms 12, 13, 23: r.e+.r, half of r.ex.r, and k.r.
+struct ArmGeom64 {
+  double dp[3], dc[3], kr[3];
+};
+__device__ __forceinline__ void slow_geom64(const ItemF64 &c, const OrbitSample64 &o, ArmGeom64 &g) {
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const double x = o.r[a][0], y = o.r[a][1], z = o.r[a][2];
+    const double ru = fma(z, c.u[2], fma(y, c.u[1], x * c.u[0]));
+    const double rv = fma(y, c.v[1], x * c.v[0]);
+    g.kr[a] = fma(z, c.k[2], fma(y, c.k[1], x * c.k[0]));
+    g.dp[a] = fma(rv, rv, -(ru * ru));
+    g.dc[a] = ru * rv;
+  }
+}
+
+// Spacecraft i: the carrier argument, half the instantaneous frequency over f*
+// and a quarter of the amplitude evolution (sinc's factor).
+__device__ __forceinline__ void slow_sc64(const ItemF64 &c, const OrbitSample64 &o, int i, double &arg2, double &h,
+                                          double &aev) {
+  const double kx = __dadd_rn(__dadd_rn(__dmul_rn(o.x[i], c.k[0]), __dmul_rn(o.y[i], c.k[1])), __dmul_rn(o.z[i], c.k[2]));
+  const double xi = __dsub_rn(o.t, div_clight(kx));
+  const double a2 = __dsub_rn(__dsub_rn(__dmul_rn(c.w0, xi), c.phi0), __dmul_rn(c.dfq, o.t));
+  arg2 = __dadd_rn(a2, __dmul_rn(__dmul_rn(c.wd, xi), xi));
+  h = fma(c.hd, xi, c.h0);
+  aev = 0.25 * fma(c.ae, xi, 1.0);
+}
+
+// The transfer function times exp(-i (arg1 - arg2)) of one arm: (cos, sin)
+// scaled by sinc(arg1) aev / 4, arg1 = h (1 + kr).
+__device__ __forceinline__ double2 slow_transfer64(double h, double kr, double arg2, double aev, const double2 *tw) {
+  const double x = fma(h, kr, h);
+  double s, c;
+  sincos_tab(__dsub_rn(x, arg2), tw, &s, &c);
+  const double m = aev * sinc64(x);
+  return make_double2(c * m, s * m);
+}
+
+// tw: the 1024-point twiddles (sincos_tab).
+__device__ __forceinline__ void slow_sample64(const ItemF64 &c, const OrbitSample64 &o, const double2 *tw,
                                               double2 d[6]) {
-  double r12[3] = {(o.x[1] - o.x[0]) / L, (o.y[1] - o.y[0]) / L, (o.z[1] - o.z[0]) / L};
-  double r13[3] = {(o.x[2] - o.x[0]) / L, (o.y[2] - o.y[0]) / L, (o.z[2] - o.z[0]) / L};
-  double r23[3] = {(o.x[2] - o.x[1]) / L, (o.y[2] - o.y[1]) / L, (o.z[2] - o.z[1]) / L};
-  double dp12 = quad(c.ep, r12[0], r12[1], r12[2]), dc12 = quad(c.ec, r12[0], r12[1], r12[2]);
-  double dp13 = quad(c.ep, r13[0], r13[1], r13[2]), dc13 = quad(c.ec, r13[0], r13[1], r13[2]);
-  double dp23 = quad(c.ep, r23[0], r23[1], r23[2]), dc23 = quad(c.ec, r23[0], r23[1], r23[2]);
-  double kr12 = c.k[0] * r12[0] + c.k[1] * r12[1] + c.k[2] * r12[2];
-  double kr13 = c.k[0] * r13[0] + c.k[1] * r13[1] + c.k[2] * r13[2];
-  double kr23 = c.k[0] * r23[0] + c.k[1] * r23[1] + c.k[2] * r23[2];
-  const double t = o.t;
-  const double w0 = kPI2 * c.f0, wd = kPI * c.fdot, ae = 0.66666666666666666666 * c.fdot / c.f0;
-  double fon[3], arg2[3], aev[3];
+  ArmGeom64 g;
+  slow_geom64(c, o, g);
+  double tr[3], ti[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    tr[a] = fma(g.dc[a], c.DC2r, g.dp[a] * c.DPr);
+    ti[a] = fma(g.dc[a], c.DC2i, g.dp[a] * c.DPi);
+  }
+  // arms of spacecraft i: 12, 13 | 21, 23 | 31, 32
+  constexpr int arm[6] = {0, 1, 0, 2, 1, 2};
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const double xi = slow_xi64(c, o, i);
-    fon[i] = (c.f0 + c.fdot * xi) / fstar;
-    arg2[i] = slow_arg2_64(c, t, w0, wd, xi);
-    aev[i] = 1.0 + ae * xi;
-  }
-  const int ai[6] = {0, 0, 1, 1, 2, 2};
-  const double dps[6] = {dp12, dp13, dp12, dp23, dp13, dp23};
-  const double dcs[6] = {dc12, dc13, dc12, dc23, dc13, dc23};
-  const double krs[6] = {kr12, kr13, -kr12, kr23, -kr13, -kr23};
+    double arg2, h, aev;
+    slow_sc64(c, o, i, arg2, h, aev);
 #pragma unroll
-  for (int a = 0; a < 6; a++) {
-    int i = ai[a];
-    d[a] = slow_arm64(c, fon[i], aev[i], arg2[i], dps[a], dcs[a], krs[a]);
+    for (int e = 0; e < 2; e++) {
+      const int q = 2 * i + e, a = arm[q];
+      const bool back = i == 2 || (i == 1 && e == 0);  // 21, 31, 32 run against the tabulated arm
+      const double2 w = slow_transfer64(h, back ? -g.kr[a] : g.kr[a], arg2, aev, tw);
+      d[q] = make_double2(fma(tr[a], w.x, ti[a] * w.y), fma(ti[a], w.x, -(tr[a] * w.y)));
+    }
   }
-}
-
-// The two arms of spacecraft i (12, 13 | 21, 23 | 31, 32) with the same
-// operations as slow_sample64, for a slow part that spreads the arms of a
-// sample over three warps.
-__device__ __forceinline__ void slow_arms64(const ItemF64 &c, const OrbitSample64 &o, double fstar, double L, int i,
-                                            double2 d[2]) {
-  // arm vectors: spacecraft 0 needs r12, r13; 1 needs r12 (as r21 = -r12), r23; 2 needs r13, r23
-  const int pb = i == 2 ? 2 : 1;  // first vector r_{0 pb}: r12 (i = 0, 1) or r13 (i = 2)
-  const int qa = i == 0 ? 0 : 1;  // second vector r_{qa 2}: r13 (i = 0) or r23 (i = 1, 2)
-  const int pa = 0, qb = 2;
-  const double u[3] = {(o.x[pb] - o.x[pa]) / L, (o.y[pb] - o.y[pa]) / L, (o.z[pb] - o.z[pa]) / L};
-  const double v[3] = {(o.x[qb] - o.x[qa]) / L, (o.y[qb] - o.y[qa]) / L, (o.z[qb] - o.z[qa]) / L};
-  const double dpu = quad(c.ep, u[0], u[1], u[2]), dcu = quad(c.ec, u[0], u[1], u[2]);
-  const double dpv = quad(c.ep, v[0], v[1], v[2]), dcv = quad(c.ec, v[0], v[1], v[2]);
-  const double kru = c.k[0] * u[0] + c.k[1] * u[1] + c.k[2] * u[2];
-  const double krv = c.k[0] * v[0] + c.k[1] * v[1] + c.k[2] * v[2];
-  const double w0 = kPI2 * c.f0, wd = kPI * c.fdot, ae = 0.66666666666666666666 * c.fdot / c.f0;
-  const double xi = slow_xi64(c, o, i);
-  const double fon = (c.f0 + c.fdot * xi) / fstar;
-  const double arg2 = slow_arg2_64(c, o.t, w0, wd, xi);
-  const double aev = 1.0 + ae * xi;
-  // arm order: i = 0: 12 (u), 13 (v); i = 1: 21 (-u), 23 (v); i = 2: 31 (-u), 32 (-v)
-  d[0] = slow_arm64(c, fon, aev, arg2, dpu, dcu, i == 0 ? kru : -kru);
-  d[1] = slow_arm64(c, fon, aev, arg2, dpv, dcv, i == 2 ? -krv : krv);
 }
 
 // Carrier phase common to the three spacecraft, reduced mod 2 pi:
@@ -818,6 +843,18 @@ __device__ __forceinline__ void ae_combos(const C d[6], C out[4]) {
   out[1] = csub(cadd(d13, d31), cadd(d23, d21));                                     // a1
   out[2] = cadd(csub(csub(cadd(d12, d31), d13), d32), cscale(csub(d21, d23), 2));    // e2
   out[3] = cadd(csub(csub(cadd(d13, d21), d23), d31), cscale(csub(d12, d32), 2));    // e1
+}
+
+// The same in FP64 with 12 instead of 16 complex additions (the doublings
+// contracted): u = d12 - d32, v = d31 - d13, w = d21 - d23.
+__device__ __forceinline__ void ae_combos64(const double2 d[6], double2 out[4]) {
+  const double2 d12 = d[0], d13 = d[1], d21 = d[2], d23 = d[3], d31 = d[4], d32 = d[5];
+  const double2 P = cadd(d31, d13), u = csub(d12, d32), v = csub(d31, d13), w = csub(d21, d23);
+  const double2 uv = cadd(u, v), wv = csub(w, v);
+  out[0] = csub(P, cadd(d32, d12));                                            // a2
+  out[1] = csub(P, cadd(d23, d21));                                            // a1
+  out[2] = make_double2(fma(2.0, w.x, uv.x), fma(2.0, w.y, uv.y));             // e2
+  out[3] = make_double2(fma(2.0, u.x, wv.x), fma(2.0, u.y, wv.y));             // e1
 }
 
 // ------------------------------------------------------------- kernel args
@@ -977,6 +1014,7 @@ struct SlowArgs {
   const ItemF64 *items64;
   const ItemMix *itemsmix;
   const OrbitSample64 *pos64[kNumBins];
+  const double2 *tw1024 = nullptr;  // FP64: the sine/cosine table
   const OrbitSampleMix *mix[kNumBins];
   const GeoSampleMix *geo[kNumBins] = {};  // mixed only
   void *series;  // float2 (mixed) or double2 (FP64)
@@ -1098,7 +1136,11 @@ __global__ void __launch_bounds__(BLOCK) fd_slow_kernel(SlowArgs a) {
   cs[kNumBins] = acc;
   const int nchunks = acc;
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // FP64: consecutive chunks go to different CTAs, so that the chunks of one
+  // or a few proposals spread over the SMs (four warps on one SM share its FP64
+  // pipe and take four times as long as on four)
+  const int warp = MIX ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5)
+                       : (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   C *series = reinterpret_cast<C *>(a.series);
 #pragma unroll 1
@@ -1120,10 +1162,11 @@ __global__ void __launch_bounds__(BLOCK) fd_slow_kernel(SlowArgs a) {
     C d[6], cmb[4];
     if constexpr (MIX) {
       slow_sample_mix(a.itemsmix[item], a.mix[b][n], a.geo[b][n], a.invLf, a.AUcf, a.invTf, d);
+      ae_combos(d, cmb);
     } else {
-      slow_sample64(a.items64[item], a.pos64[b][n], a.fstar, a.L, d);
+      slow_sample64(a.items64[item], a.pos64[b][n], a.tw1024, d);
+      ae_combos64(d, cmb);
     }
-    ae_combos(d, cmb);
     const long long o0 = ((long long)cb * 32 + (long long)slot * N) * 4 + n;
     if (!chk(o0 >= 0 && o0 + 3LL * N < a.series_len, kChkSeriesWrite)) continue;
     C *out = series + o0;
@@ -1153,15 +1196,15 @@ struct SpecSmem {
       sizeof(TW) * (size_t)SN + sizeof(C) * (size_t)SN * (size_t)SpecCfg<N>::GPC * NSER + sizeof(double) * 3 * 32;
 };
 
-// Sum over the threads of one group (result valid in lane 0 of the group).
+// Sum over the threads of group g (result valid in lane 0 of the group).
 template <int GT>
-__device__ __forceinline__ double group_sum(double v, double *red, int lane) {
+__device__ __forceinline__ double group_sum(double v, double *red, int lane, int g) {
 #pragma unroll
   for (int off = (GT < 32 ? GT : 32) / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   if constexpr (GT > 32) {
-    __syncthreads();
+    group_bar<GT>(g);
     if ((lane & 31) == 0) red[lane >> 5] = v;
-    __syncthreads();
+    group_bar<GT>(g);
     if (lane == 0) {
       double s = 0;
       for (int w = 0; w < GT / 32; w++) s += red[w];
@@ -1265,6 +1308,9 @@ __device__ __forceinline__ void acc_resid_sq(float whi, float wlo, float h, floa
 }
 
 // a b + c, complex, with fused multiply-adds
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
 __device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
@@ -1295,6 +1341,11 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
   const int NFFT = a.NFFT;
   const int slot = base + g;
   const bool valid = slot < count;
+  if constexpr (!MIX) {
+    // a warp with no proposal leaves: its FP64 instructions would hold the
+    // SM's pipe (groups share no barrier)
+    if (base + (GT >= 32 ? g : (int)(threadIdx.x & ~31u) / GT) >= count) return;
+  }
   const int sl = valid ? slot : count - 1;
   // checked build: an index outside its buffer is recorded, the group reads
   // from the buffers' starts instead (it still runs its FFT and barriers) and
@@ -1330,8 +1381,9 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
   // bins (w)
   float rS = 0.f, rE = 0.f, eS = 0.f, eE = 0.f, fh = 0.f;
   float4 ev = make_float4(0.f, 0.f, 0.f, 0.f);
-  double acc = 0.0, hacc = 0.0;
-  double accE = 0.0;
+  // FP64: sums of w.h and |h|^2 per channel of the template before its
+  // amplitude amp_s, which enters at the end
+  double wacc[2] = {0.0, 0.0}, hacc[2] = {0.0, 0.0};
 #pragma unroll 1
   for (int pass = 0; pass < PASSES; ++pass) {
     if constexpr (MIX) {
@@ -1341,8 +1393,8 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
       for (int s = 0; s < NSER; ++s)
 #pragma unroll
         for (int r = 0; r < B; ++r) buf[s * N + lane + GT * r] = src[(size_t)(pass * NSER + s) * N + lane + GT * r];
-      group_sync<GT>();
-      group_fft<N, GT, NSER, (CH < NSER ? CH : NSER)>(buf, tw, lane);
+      group_bar<GT>(g);
+      group_fft<N, GT, NSER, (CH < NSER ? CH : NSER)>(buf, tw, lane, g);
     }
 #pragma unroll
     for (int r = 0; r < B; ++r) {
@@ -1388,24 +1440,24 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
       } else {
         if (j < 0 || j >= NFFT) continue;
         const size_t sj = (size_t)seg * NFFT + j;
-        const double s = a.items64[item].amp_s;
-        // series (2 ch, 2 ch + 1) of this pass hold the A (chan 0) or E (chan 1) pair
+        // series (2 ch, 2 ch + 1) of this pass hold the A (chan 0) or E (chan 1)
+        // pair: 12 FP64 instructions per bin and channel
 #pragma unroll
         for (int ch = 0; ch < NSER / 2; ++ch) {
           const int chan = pass * (NSER / 2) + ch;
           const double2 w = a.w64[2 * sj + chan];
           const double2 g2 = a.g64[4 * sj + 2 * chan], g1 = a.g64[4 * sj + 2 * chan + 1];
-          double2 h = cadd(cmul(buf[(2 * ch) * N + k], g2), cmul(buf[(2 * ch + 1) * N + k], g1));
-          h = cscale(h, s);
-          if (PERCH && chan == 1)
-            accE += 2.0 * (w.x * h.x + w.y * h.y) - (h.x * h.x + h.y * h.y);
-          else
-            acc += 2.0 * (w.x * h.x + w.y * h.y) - (h.x * h.x + h.y * h.y);
-          hacc += h.x * h.x + h.y * h.y;
+          const double2 h = cfma(buf[(2 * ch) * N + k], g2, cmul(buf[(2 * ch + 1) * N + k], g1));
+          const int at = PERCH ? chan : 0;
+          wacc[at] = fma(w.x, h.x, fma(w.y, h.y, wacc[at]));
+          hacc[at] = fma(h.x, h.x, fma(h.y, h.y, hacc[at]));
         }
       }
     }
-    group_sync<GT>();
+    if constexpr (MIX)
+      group_sync<GT>();
+    else
+      group_bar<GT>(g);
   }
   df sa, sh, saE;
   if constexpr (MIX) {
@@ -1419,9 +1471,11 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
     sh = group_sum_df<GT>(fh, redf + 32, lane);
     if (est_on) ev = group_sum4<GT>(ev, reinterpret_cast<float *>(red), lane);
   } else {
-    acc = group_sum<GT>(acc, red, lane);
-    hacc = group_sum<GT>(hacc, red + 32, lane);
-    if constexpr (PERCH) accE = group_sum<GT>(accE, red + 64, lane);
+#pragma unroll
+    for (int ch = 0; ch < (PERCH ? 2 : 1); ++ch) {
+      wacc[ch] = group_sum<GT>(wacc[ch], red, lane, g);
+      hacc[ch] = group_sum<GT>(hacc[ch], red + 32, lane, g);
+    }
   }
   if (valid && inb && lane == 0) {
     double term, hh;
@@ -1466,14 +1520,17 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
         }
       }
     } else {
+      // 2 (w|h) - |h|^2 with the amplitude s
+      const double s = a.items64[item].amp_s;
+      term = s * (2.0 * wacc[0] - s * hacc[0]);
       if constexpr (PERCH) {
-        a.term_ch[2 * (size_t)item] = acc;
-        a.term_ch[2 * (size_t)item + 1] = accE;
-        term = acc + accE;
-      } else {
-        term = acc;
+        const double tE = s * (2.0 * wacc[1] - s * hacc[1]);
+        a.term_ch[2 * (size_t)item] = term;
+        a.term_ch[2 * (size_t)item + 1] = tE;
+        term += tE;
+        hacc[0] += hacc[1];
       }
-      hh = 2.0 * hacc;
+      hh = 2.0 * (s * s) * hacc[0];
     }
     const double tx = a.term_x ? a.term_x[item] : 0.0;
     a.dlogl[item] = term - tx;
@@ -1481,7 +1538,11 @@ __device__ __forceinline__ void spec_unit(const SpecArgs &a, const int *bin_list
     if (a.hh) a.hh[item] = hh;
     if (a.status) a.status[item] = isfinite(term) ? 0 : 1;
   }
-  if constexpr (GT > 32) __syncthreads();
+  if constexpr (MIX) {
+    if constexpr (GT > 32) __syncthreads();
+  } else {
+    group_bar<GT>(g);
+  }
 }
 
 template <int N, bool MIX, bool PERCH = false>
@@ -1913,10 +1974,5 @@ static cudaError_t launch_slow(const SlowArgs &a, int num_sms, cudaStream_t stre
   fd_slow_kernel<MIX, BLOCK><<<occ * num_sms, BLOCK, 0, stream>>>(a);
   return cudaGetLastError();
 }
-
-// The slow part of a few proposals (the FP64 re-evaluation of flagged mixed
-// ones): one warp per CTA, so that the chunks of 32 samples spread over the
-// SMs instead of filling the first few (an FP64 sample costs ~700 FP64
-// instructions and the FP64 pipe of an SM issues a warp's in 16 cycles).
 
 }  // namespace glass

@@ -217,6 +217,7 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
     sa.pos64[b] = tab.pos64[b];
     sa.mix[b] = tab.mix[b];
   }
+  sa.tw1024 = tab.tw64[fd_bin_of(kSincosTab)];
   sa.series = na->series;
   sa.nitems = nitems;
   sa.series_len = 4 * kNaMaxSamples;

@@ -1,5 +1,5 @@
 // F-statistic of sky/frequency cells for sm_103a, FP64 (compiled without
-// multiply-add contraction, like the FP64 likelihood path).
+// multiply-add contraction; multiply-adds are written out).
 //
 // The reference evaluates one cell at a time (get_Fstat_logL,
 // ucb/src/glass_ucb_fstatistic.c:646-703): four filter waveforms by
@@ -10,17 +10,35 @@
 // (ucb/src/glass_ucb_proposal.c:1085-1182) calls it for every cell of a
 // frequency x sky grid, with OpenMP over the sky rows.
 //
-// Here a batch of cells runs as three stages, with the cells binned by their
-// filter size N = ucb_bandwidth(f0, fdot, cos theta, A = 1e-22) in 16..4096:
-//   plan   one thread per cell: the per-cell geometry (shared by the four
-//          filters) and the four filters' polarisation factors and phases;
-//   slow   one thread per (cell, sample): the six arm series of all four
-//          filters, sharing every filter-independent quantity, with each
-//          filter's own arithmetic in the reference's order;
-//   spec   per size, one group of N/4 threads per cell: FFT of each filter's
-//          four A/E series, TDI weights and whitening per bin (the likelihood
-//          path's tables), then N^i and M^ij over the segment bins
-//          0 < k < NFFT, and the 4x4 solve in one lane.
+// The four filters are two templates and their quarter turns.  At inclination
+// pi/2 only the plus amplitude is left, so with H the response to e+ (psi = 0)
+// and G the response to -ex (psi = pi/4, phase pi), the filters (psi, phase) =
+// (0, 0), (pi/4, pi), (0, 3pi/2), (pi/4, pi/2) are H, G, iH, iG, exactly.  (The
+// reference rounds each filter's carrier argument, ~1e6 rad, on its own, which
+// moves its filters by ~1e-10 rad from these; the results agree to that.)  So
+// N = (d.H, d.G, d.iH, d.iG) is two complex products, and of M only |H|^2,
+// |G|^2 and the complex H*.G are left:
+//   M = [ HH  Re  0  -Im ]     Re + i Im = sum H* G
+//       [ Re  GG  Im  0  ]
+//       [ 0   Im  HH  Re ]
+//       [ -Im 0   Re  GG ]
+//
+// A batch of cells runs in four stages, the cells binned by their filter size
+// N = ucb_bandwidth(f0, fdot, cos theta, A = 1e-22) in 16..4096:
+//   plan    one thread per cell: the per-cell geometry;
+//   slow    one thread per (cell, sample): the six arms' transfer factors
+//           (slow_transfer64) once, with both real polarisation patterns;
+//   spec    per size, one group of N/4 threads per cell: FFT of H's and G's
+//           two series per channel, TDI weights and whitening per bin (the
+//           likelihood path's tables), and the eight sums over the segment
+//           bins 0 < k < NFFT;
+//   finish  one thread per cell: the 4x4 solve, logL and the fit.
+// All four are bound by the FP64 pipe (85% busy by ncu).  Against four filters,
+// each with its own series, transforms and ten products, 1440 -> 340 FP64
+// instructions per sample in the slow part and 656 -> 235 in the spectral part;
+// the solve, one lane of a warp per cell before, runs full warps.  51200 cells
+// of 64 samples: 13.43 -> 3.51 ms.
+//
 // The A/E inner products of the reference weight both channels with the A
 // channel's noise C[0][0]; with templates and data whitened by their own
 // channel's noise, the E terms are multiplied by invC_A/invC_E per bin, which
@@ -35,22 +53,14 @@ namespace glass {
 namespace {
 
 constexpr int kFsBins = 9;  // N = 16 << b
-constexpr int kFsSeries = 16;  // 4 filters x (A2, A1, E2, E1)
-
-// The four filters (ucb/src/glass_ucb_fstatistic.c:262-265): amplitude 2,
-// inclination pi/2, and these polarisations and phases.
-__constant__ double kFsPsi[4] = {0.0, M_PI_4, 0.0, M_PI_4};
-__constant__ double kFsPhase[4] = {0.0, M_PI, 3.0 * M_PI_2, M_PI_2};
-// each phase as a quadrant k (phase = k pi/2 to the rounding of the double),
-// and k pi/2 as a double-double hi + lo
-__constant__ int kFsQuadrant[4] = {0, 2, 3, 1};
-__constant__ double kFsKPio2Hi[4] = {0.0, 1.5707963267948966, 3.141592653589793, 4.71238898038469};
-__constant__ double kFsKPio2Lo[4] = {0.0, 6.123233995736766e-17, 1.2246467991473532e-16, 1.8369701987210297e-16};
+constexpr int kFsSeries = 8;  // (H, G) x (A2, A1, E2, E1)
 
 struct FsCell {
-  ItemF64 it;        // the cell's geometry, f0, fdot, q, amp/(2N), segment, N, imin
-  double DP[4][4];   // DPr, DPi, DCr, DCi of each filter
-  double phi0[4];
+  ItemF64 it;     // the cell's geometry, f0, fdot, q, amp/(2N), segment, N, imin
+  // over the segment bins, whitened, before the amplitude: |H|^2, |G|^2, Re and
+  // Im of H* G, Re and Im of d* H, Re and Im of d* G
+  double sum[8];
+  int live;       // evaluated (the others' results are written by the plan)
 };
 
 struct FsPlanArgs {
@@ -68,7 +78,7 @@ struct FsPlanArgs {
 
 struct FsSlowArgs {
   int cap;
-  double fstar, L;
+  const double2 *tw1024;
   const int *bin_count, *bin_list;
   const FsCell *fc;
   const OrbitSample64 *pos64[kNumBins];
@@ -78,14 +88,12 @@ struct FsSlowArgs {
 struct FsSpecArgs {
   int NFFT, cap, bin;
   const int *bin_count, *bin_list;
-  const FsCell *fc;
-  double2 *series;
+  FsCell *fc;
+  const double2 *series;
   const double2 *tw;  // twiddles of size N (size 16: every other entry of size 32's)
   int tw_stride;
   const double2 *w64, *g64;
   const double *rho;
-  double *logl, *fparams;
-  int *status;
 };
 
 // ------------------------------------------------------------ 4x4 algebra
@@ -172,7 +180,7 @@ __device__ void fs_write(const FsPlanArgs &a, int i, const double *o, int st) {
 // ------------------------------------------------------------------- plan
 // One thread per cell.  Filter parameters as get_filters sets them
 // (ucb/src/glass_ucb_fstatistic.c:241-344): f0 T, cos theta, phi, ln 2,
-// cos(pi/2), psi, phase, fdot T^2.
+// cos(pi/2), psi, phase (0, 0 for H), fdot T^2.
 __global__ void __launch_bounds__(128) fs_plan_kernel(FsPlanArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int b = -1;
@@ -201,34 +209,28 @@ __global__ void __launch_bounds__(128) fs_plan_kernel(FsPlanArgs a) {
         fs_finish(Nv, m, o);
         fs_write(a, i, o, GLASS_ITEM_OUTSIDE);
       } else {
-        FsCell c;
+        ItemF64 c;
         double p[8];
         p[0] = f0 * a.T;
         p[1] = costh;
         p[2] = phi;
         p[3] = log(2.0);
         p[4] = cos(M_PI_2);
+        p[5] = p[6] = 0.0;
         p[7] = fdot * (a.T * a.T);
-        for (int f = 0; f < 4; f++) {
-          p[5] = kFsPsi[f];
-          p[6] = kFsPhase[f];
-          SourceGeom g;
-          source_geometry(p, 8, a.T, g);
-          if (f == 0) make_item_f64(g, N, c.it);
-          c.DP[f][0] = g.DPr;
-          c.DP[f][1] = g.DPi;
-          c.DP[f][2] = g.DCr;
-          c.DP[f][3] = g.DCi;
-          c.phi0[f] = g.phi0;
-        }
-        c.it.seg = seg;
-        c.it.N = N;
-        c.it.imin = (int)lo;
-        a.fc[i] = c;
+        SourceGeom g;
+        source_geometry(p, 8, a.T, g);
+        make_item_f64(g, N, a.fstar, c);
+        c.amp_s *= 0.5;  // the plus factor (1 + cos^2 iota) / 2, left out of H and G
+        c.seg = seg;
+        c.N = N;
+        c.imin = (int)lo;
+        a.fc[i].it = c;
         b = 31 - __clz(N) - 4;
       }
     }
   }
+  if (i < a.ncells) a.fc[i].live = b >= 0;
   // warp-aggregated binning: one atomic per distinct size per warp
   const int lane = threadIdx.x & 31;
   const unsigned active = __ballot_sync(0xffffffffu, b >= 0);
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(128) fs_plan_kernel(FsPlanArgs a) {
 }
 
 // Start (in samples of one series) of size bin `bin` in the scratch: sizes in
-// increasing order, cells of one size back to back, 16 series of N each.
+// increasing order, cells of one size back to back, 8 series of N each.
 __device__ __forceinline__ long long fs_bin_start(const int *bin_count, int bin) {
   long long acc = 0;
 #pragma unroll
@@ -253,10 +255,9 @@ __device__ __forceinline__ long long fs_bin_start(const int *bin_count, int bin)
 }
 
 // ------------------------------------------------------------------- slow
-// One thread per (cell, sample): the six arm series of the four filters
-// (ucb/src/glass_ucb_waveform.c:840-922 for each filter; every quantity that
-// does not depend on the filter is computed once, with the same operations),
-// combined to the four A/E series and stored at [cell][filter][series][n].
+// One thread per (cell, sample): the six arm series of H and G (ucb/src/
+// glass_ucb_waveform.c:840-922 with real polarisation factors), combined to the
+// four A/E series each and stored at [cell][template][series][n].
 __global__ void __launch_bounds__(256) fs_slow_kernel(FsSlowArgs a) {
   long long cs[kFsBins + 1];
   long long acc = 0;
@@ -278,95 +279,36 @@ __global__ void __launch_bounds__(256) fs_slow_kernel(FsSlowArgs a) {
     const int slot = (int)(local >> (b + 4));
     const int n = (int)(local & (N - 1));
     const int cell = a.bin_list[(size_t)b * a.cap + slot];
-    const FsCell &c = a.fc[cell];
+    const ItemF64 &c = a.fc[cell].it;
     // size 16 samples are every other sample of size 32 (same times exactly)
-    const OrbitSample64 o = b == 0 ? a.pos64[0][2 * n] : a.pos64[b - 1][n];
-    const double L = a.L, fstar = a.fstar;
-    double r12[3] = {(o.x[1] - o.x[0]) / L, (o.y[1] - o.y[0]) / L, (o.z[1] - o.z[0]) / L};
-    double r13[3] = {(o.x[2] - o.x[0]) / L, (o.y[2] - o.y[0]) / L, (o.z[2] - o.z[0]) / L};
-    double r23[3] = {(o.x[2] - o.x[1]) / L, (o.y[2] - o.y[1]) / L, (o.z[2] - o.z[1]) / L};
-    const ItemF64 &it = c.it;
-    const double dp12 = quad(it.ep, r12[0], r12[1], r12[2]), dc12 = quad(it.ec, r12[0], r12[1], r12[2]);
-    const double dp13 = quad(it.ep, r13[0], r13[1], r13[2]), dc13 = quad(it.ec, r13[0], r13[1], r13[2]);
-    const double dp23 = quad(it.ep, r23[0], r23[1], r23[2]), dc23 = quad(it.ec, r23[0], r23[1], r23[2]);
-    const double kr12 = it.k[0] * r12[0] + it.k[1] * r12[1] + it.k[2] * r12[2];
-    const double kr13 = it.k[0] * r13[0] + it.k[1] * r13[1] + it.k[2] * r13[2];
-    const double kr23 = it.k[0] * r23[0] + it.k[1] * r23[1] + it.k[2] * r23[2];
-    const double t = o.t;
-    const double w0 = kPI2 * it.f0, wd = kPI * it.fdot, ae = 0.66666666666666666666 * it.fdot / it.f0;
-    const double dfqt = it.dfq * t;
-    double w0x[3], wdx[3], aev[3], fon[3];
+    const OrbitSample64 &o = b == 0 ? a.pos64[0][2 * n] : a.pos64[b - 1][n];
+    ArmGeom64 g;
+    slow_geom64(c, o, g);
+    constexpr int arm[6] = {0, 1, 0, 2, 1, 2};
+    double2 w[6], d[6], cmb[4];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      const double kdotx = (o.x[i] * it.k[0] + o.y[i] * it.k[1] + o.z[i] * it.k[2]) / kCLIGHT;
-      const double xi = t - kdotx;
-      fon[i] = (it.f0 + it.fdot * xi) / fstar;
-      w0x[i] = w0 * xi;
-      wdx[i] = wd * xi * xi;
-      aev[i] = 1.0 + ae * xi;
-    }
-    const int ai[6] = {0, 0, 1, 1, 2, 2};
-    const double dps[6] = {dp12, dp13, dp12, dp23, dp13, dp23};
-    const double dcs[6] = {dc12, dc13, dc12, dc23, dc13, dc23};
-    const double krs[6] = {kr12, kr13, -kr12, kr23, -kr13, -kr23};
-    double arg1[6], sinc[6];
+      double arg2, h, aev;
+      slow_sc64(c, o, i, arg2, h, aev);
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-      arg1[q] = 0.5 * fon[ai[q]] * (1.0 + krs[q]);
-      sinc[q] = 0.25 * sin(arg1[q]) / arg1[q];
-    }
-    const int Nn = N;
-    double2 *out = a.series + fs_bin_start(a.bin_count, b) + (long long)slot * kFsSeries * Nn + n;
-    // Filter 0 (phase 0) takes sincos of its arguments x0 = arg1 - arg2.  The
-    // other filters' arguments xf, rounded exactly as the reference rounds
-    // them, differ from x0 by their phase k pi/2 plus ~1e-10 (the rounding of
-    // w0 xi - phi0 at |w0 xi| ~ 1e6): sincos(xf) is sincos(x0) turned by the
-    // quadrant k and by eps = xf - x0 - k pi/2, taken exactly (two-sum, and
-    // k pi/2 as a double-double); |eps| < 1e-9, so cos eps = 1 and sin eps =
-    // eps to double precision.
-    double s0[6], c0[6], x0[6];
-#pragma unroll 1
-    for (int f = 0; f < 4; f++) {
-      double arg2[3];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        double a2 = w0x[i] - c.phi0[f] - dfqt;
-        a2 += wdx[i];
-        arg2[i] = a2;
+      for (int e = 0; e < 2; e++) {
+        const int q = 2 * i + e;
+        const bool back = i == 2 || (i == 1 && e == 0);
+        const double2 t = slow_transfer64(h, back ? -g.kr[arm[q]] : g.kr[arm[q]], arg2, aev, a.tw1024);
+        w[q] = make_double2(t.x, -t.y);
       }
-      const double DPr = c.DP[f][0], DPi = c.DP[f][1], DCr = c.DP[f][2], DCi = c.DP[f][3];
-      const int k = kFsQuadrant[f];
-      const double khi = kFsKPio2Hi[k], klo = kFsKPio2Lo[k];
-      double2 d[6], cmb[4];
-#pragma unroll
-      for (int q = 0; q < 6; q++) {
-        const int i = ai[q];
-        const double t1r = aev[i] * (dps[q] * DPr + dcs[q] * DCr);
-        const double t1i = aev[i] * (dps[q] * DPi + dcs[q] * DCi);
-        const double x = arg1[q] - arg2[i];
-        double s2, c2;
-        if (f == 0) {
-          sincos(x, &s2, &c2);
-          s0[q] = s2;
-          c0[q] = c2;
-          x0[q] = x;
-        } else {
-          const double dh = x - x0[q];
-          const double bb = dh - x;
-          const double dl = (x - (dh - bb)) + (-x0[q] - bb);
-          const double eps = ((dh - khi) + dl) - klo;
-          const double rs = (k & 1) ? c0[q] : s0[q];
-          const double rc = (k & 1) ? -s0[q] : c0[q];
-          const double qs = (k & 2) ? -rs : rs, qc = (k & 2) ? -rc : rc;
-          s2 = qs + qc * eps;
-          c2 = qc - qs * eps;
-        }
-        d[q] = make_double2(sinc[q] * (t1r * c2 + t1i * s2), sinc[q] * (-t1r * s2 + t1i * c2));
-      }
-      ae_combos(d, cmb);
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) out[(size_t)(4 * f + kk) * Nn] = cmb[kk];
     }
+    double2 *out = a.series + fs_bin_start(a.bin_count, b) + (long long)slot * kFsSeries * N + n;
+#pragma unroll
+    for (int q = 0; q < 6; q++) d[q] = cscale(w[q], g.dp[arm[q]]);
+    ae_combos64(d, cmb);
+#pragma unroll
+    for (int k = 0; k < 4; k++) out[(size_t)k * N] = cmb[k];
+#pragma unroll
+    for (int q = 0; q < 6; q++) d[q] = cscale(w[q], 2.0 * g.dc[arm[q]]);
+    ae_combos64(d, cmb);
+#pragma unroll
+    for (int k = 0; k < 4; k++) out[(size_t)(4 + k) * N] = cmb[k];
   }
 }
 
@@ -376,126 +318,118 @@ struct FsCfg {
   static constexpr int GT = N / 4;
   static constexpr int CTA = GT >= 128 ? GT : 128;
   static constexpr int GPC = CTA / GT;
-  static constexpr int NSER = N == 4096 ? 2 : 4;  // series in shared memory at once
-  static constexpr int PASSES = 4 / NSER;
-  static constexpr size_t smem = sizeof(double2) * (size_t)N * (1 + (size_t)GPC * NSER) + sizeof(double) * 32 * GPC;
+  static constexpr size_t smem = sizeof(double2) * (size_t)N * (1 + (size_t)GPC * 2) + sizeof(double) * 32 * GPC;
 };
 
+// One channel of one template at a time (two series in shared memory): H's bins
+// stay in registers while G's series are transformed, then the channel's share
+// of the eight sums is taken.
 template <int N>
 __global__ void __launch_bounds__(FsCfg<N>::CTA) fs_spec_kernel(FsSpecArgs a) {
   using Cfg = FsCfg<N>;
-  constexpr int GT = Cfg::GT, GPC = Cfg::GPC, NSER = Cfg::NSER, PASSES = Cfg::PASSES;
+  constexpr int GT = Cfg::GT, GPC = Cfg::GPC;
   constexpr int B = N / GT;  // bins per thread (4)
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int count = a.bin_count[a.bin];
+  if (count == 0) return;
   double2 *tw = reinterpret_cast<double2 *>(smem_raw);
   double2 *bufs = tw + N;
-  double *reds = reinterpret_cast<double *>(bufs + (size_t)GPC * NSER * N);
+  double *reds = reinterpret_cast<double *>(bufs + (size_t)GPC * 2 * N);
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = a.tw[(size_t)i * a.tw_stride];
   __syncthreads();
-  const int count = a.bin_count[a.bin];
-  double2 *ser_bin = a.series + fs_bin_start(a.bin_count, a.bin);
+  const double2 *ser_bin = a.series + fs_bin_start(a.bin_count, a.bin);
   const int *list = a.bin_list + (size_t)a.bin * a.cap;
   const int g = threadIdx.x / GT, lane = threadIdx.x % GT;
-  double2 *buf = bufs + (size_t)g * NSER * N;
+  double2 *buf = bufs + (size_t)g * 2 * N;
   double *red = reds + 32 * g;
   const int NFFT = a.NFFT;
   for (int base = blockIdx.x * GPC; base < count; base += gridDim.x * GPC) {
     const int slot = base + g;
     const bool valid = slot < count;
+    if (base + (GT >= 32 ? g : (int)(threadIdx.x & ~31u) / GT) >= count) break;  // a warp with no cell
     const int sl = valid ? slot : count - 1;
     const int cell = list[sl];
     const ItemF64 &it = a.fc[cell].it;
-    const int seg = it.seg, imin = it.imin;
-    const double s = it.amp_s;
-    double2 *ser = ser_bin + (size_t)sl * kFsSeries * N;
+    const int imin = it.imin;
+    const size_t seg0 = (size_t)it.seg * NFFT;
+    const double2 *ser = ser_bin + (size_t)sl * kFsSeries * N;
+    double sum[8] = {};
 #pragma unroll 1
-    for (int f = 0; f < 4; ++f) {
+    for (int chan = 0; chan < 2; ++chan) {
+      double2 hb[B];
 #pragma unroll 1
-      for (int pass = 0; pass < PASSES; ++pass) {
+      for (int f = 0; f < 2; ++f) {
 #pragma unroll
-        for (int q = 0; q < NSER; ++q)
+        for (int q = 0; q < 2; ++q)
 #pragma unroll
           for (int r = 0; r < B; ++r)
-            buf[q * N + lane + GT * r] = ser[(size_t)(4 * f + pass * NSER + q) * N + lane + GT * r];
-        group_sync<GT>();
-        group_fft<N, GT, NSER, 2>(buf, tw, lane);
-        // template bins of this filter, in place of its A2 (A) and E2 (E) series
+            buf[q * N + lane + GT * r] = ser[(size_t)(4 * f + 2 * chan + q) * N + lane + GT * r];
+        group_bar<GT>(g);
+        group_fft<N, GT, 2, 2>(buf, tw, lane, g);
 #pragma unroll
         for (int r = 0; r < B; ++r) {
           const int k = lane + GT * r;
-          const int m = (k + N / 2) & (N - 1);  // fftshift
-          const int j = imin + m;
-#pragma unroll
-          for (int ch = 0; ch < NSER / 2; ++ch) {
-            const int chan = pass * (NSER / 2) + ch;
-            double2 h = make_double2(0.0, 0.0);
-            if (j > 0 && j < NFFT) {
-              const size_t sj = (size_t)seg * NFFT + j;
-              const double2 g2 = a.g64[4 * sj + 2 * chan], g1 = a.g64[4 * sj + 2 * chan + 1];
-              h = cscale(cadd(cmul(buf[(2 * ch) * N + k], g2), cmul(buf[(2 * ch + 1) * N + k], g1)), s);
+          const int j = imin + ((k + N / 2) & (N - 1));  // fftshift
+          double2 h = make_double2(0.0, 0.0);
+          if (j > 0 && j < NFFT) {
+            const size_t sj = seg0 + j;
+            const double2 g2 = a.g64[4 * sj + 2 * chan], g1 = a.g64[4 * sj + 2 * chan + 1];
+            h = cfma(buf[k], g2, cmul(buf[N + k], g1));
+            if (f == 1) {
+              const double2 w = a.w64[2 * sj + chan];
+              double2 H = hb[r], G = h;  // the second factors, weighted
+              if (chan == 1) {
+                const double rho = a.rho[sj];
+                H = cscale(H, rho);
+                G = cscale(G, rho);
+              }
+              sum[0] = fma(hb[r].x, H.x, fma(hb[r].y, H.y, sum[0]));
+              sum[1] = fma(h.x, G.x, fma(h.y, G.y, sum[1]));
+              sum[2] = fma(hb[r].x, G.x, fma(hb[r].y, G.y, sum[2]));
+              sum[3] = fma(hb[r].x, G.y, fma(-hb[r].y, G.x, sum[3]));
+              sum[4] = fma(w.x, H.x, fma(w.y, H.y, sum[4]));
+              sum[5] = fma(w.x, H.y, fma(-w.y, H.x, sum[5]));
+              sum[6] = fma(w.x, G.x, fma(w.y, G.y, sum[6]));
+              sum[7] = fma(w.x, G.y, fma(-w.y, G.x, sum[7]));
             }
-            if (valid) ser[(size_t)(4 * f + 2 * chan) * N + m] = h;
           }
+          if (f == 0) hb[r] = h;
         }
-        group_sync<GT>();
+        group_bar<GT>(g);
       }
     }
-    // N^i and M^ij over this thread's bins (the spectra it wrote itself)
-    double nacc[4] = {0, 0, 0, 0}, macc[10] = {};
 #pragma unroll
-    for (int r = 0; r < B; ++r) {
-      const int k = lane + GT * r;
-      const int m = (k + N / 2) & (N - 1);
-      const int j = imin + m;
-      if (!(j > 0 && j < NFFT)) continue;
-      const size_t sj = (size_t)seg * NFFT + j;
-      const double2 wA = a.w64[2 * sj], wE = a.w64[2 * sj + 1];
-      const double rho = a.rho[sj];
-      double2 hA[4], hE[4];
+    for (int q = 0; q < 8; ++q) sum[q] = group_sum<GT>(sum[q], red, lane, g);
+    if (valid && lane == 0)
 #pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        hA[f] = ser[(size_t)(4 * f) * N + m];
-        hE[f] = ser[(size_t)(4 * f + 2) * N + m];
-      }
-#pragma unroll
-      for (int f = 0; f < 4; ++f)
-        nacc[f] += (wA.x * hA[f].x + wA.y * hA[f].y) + rho * (wE.x * hE[f].x + wE.y * hE[f].y);
-      int idx = 0;
-#pragma unroll
-      for (int f = 0; f < 4; ++f)
-#pragma unroll
-        for (int h = f; h < 4; ++h, ++idx)
-          macc[idx] += (hA[f].x * hA[h].x + hA[f].y * hA[h].y) + rho * (hE[f].x * hE[h].x + hE[f].y * hE[h].y);
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) nacc[f] = group_sum<GT>(nacc[f], red, lane);
-#pragma unroll
-    for (int q = 0; q < 10; ++q) macc[q] = group_sum<GT>(macc[q], red, lane);
-    if (valid && lane == 0) {
-      double Nv[4], m[16], o[5];
-#pragma unroll
-      for (int f = 0; f < 4; ++f) Nv[f] = 4.0 * nacc[f];
-      int idx = 0;
-#pragma unroll
-      for (int f = 0; f < 4; ++f)
-#pragma unroll
-        for (int h = f; h < 4; ++h, ++idx) m[4 * f + h] = m[4 * h + f] = 4.0 * macc[idx];
-      int st = 0;
-      if (!fs_finish(Nv, m, o)) {
-        const double nan = __longlong_as_double(0x7ff8000000000000ULL);
-        for (int q = 0; q < 5; q++) o[q] = nan;
-        st = GLASS_ITEM_NONFINITE;
-      } else if (!isfinite(o[0])) {
-        st = GLASS_ITEM_NONFINITE;
-      }
-      a.logl[cell] = o[0];
-      if (a.fparams)
-#pragma unroll
-        for (int q = 0; q < 4; q++) a.fparams[4 * (size_t)cell + q] = o[1 + q];
-      if (a.status) a.status[cell] = st;
-    }
-    if constexpr (GT > 32) __syncthreads();
+      for (int q = 0; q < 8; ++q) a.fc[cell].sum[q] = sum[q];
   }
+}
+
+// ----------------------------------------------------------------- finish
+__global__ void __launch_bounds__(128) fs_finish_kernel(const FsCell *fc, int ncells, double *logl, double *fparams,
+                                                        int *status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= ncells || !fc[i].live) return;
+  const double s = 4.0 * fc[i].it.amp_s, s2 = s * fc[i].it.amp_s;
+  const double *v = fc[i].sum;
+  const double Nv[4] = {s * v[4], s * v[6], -(s * v[5]), -(s * v[7])};
+  const double hh = s2 * v[0], gg = s2 * v[1], re = s2 * v[2], im = s2 * v[3];
+  double m[16] = {hh, re, 0.0, -im, re, gg, im, 0.0, 0.0, im, hh, re, -im, 0.0, re, gg};
+  double o[5];
+  int st = 0;
+  if (!fs_finish(Nv, m, o)) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+    for (int q = 0; q < 5; q++) o[q] = nan;
+    st = GLASS_ITEM_NONFINITE;
+  } else if (!isfinite(o[0])) {
+    st = GLASS_ITEM_NONFINITE;
+  }
+  logl[i] = o[0];
+  if (fparams)
+#pragma unroll
+    for (int q = 0; q < 4; q++) fparams[4 * (size_t)i + q] = o[1 + q];
+  if (status) status[i] = st;
 }
 
 template <int N>
@@ -669,8 +603,7 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
 
     FsSlowArgs sa;
     sa.cap = w.cap;
-    sa.fstar = bank.fstar;
-    sa.L = kLARM;
+    sa.tw1024 = tab.tw64[fd_bin_of(kSincosTab)];
     sa.bin_count = w.bin_count;
     sa.bin_list = w.bin_list;
     sa.fc = (const FsCell *)w.cells;
@@ -693,14 +626,11 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
     ca.cap = w.cap;
     ca.bin_count = w.bin_count;
     ca.bin_list = w.bin_list;
-    ca.fc = (const FsCell *)w.cells;
-    ca.series = (double2 *)w.series;
+    ca.fc = (FsCell *)w.cells;
+    ca.series = (const double2 *)w.series;
     ca.w64 = bank.w64;
     ca.g64 = bank.g64;
     ca.rho = rho;
-    ca.logl = logl + off;
-    ca.fparams = fparams ? fparams + 4 * (size_t)off : nullptr;
-    ca.status = status ? status + off : nullptr;
     for (int b = 0; b < kFsBins; b++) {
       const int N = 16 << b;
       if (N > maxN || N > kMaxN) break;
@@ -721,6 +651,9 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
       launches++;
       if (e != cudaSuccess) return e;
     }
+    fs_finish_kernel<<<(n + 127) / 128, 128, 0, stream>>>((const FsCell *)w.cells, n, pa.logl, pa.fparams, pa.status);
+    launches++;
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (nlaunch) *nlaunch = launches;
   return cudaSuccess;
