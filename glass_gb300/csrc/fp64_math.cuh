@@ -69,6 +69,20 @@ __device__ __forceinline__ void sincos_tab(double x, const double2 *tw, double *
   *s = fma(t.x, sn, -fma(t.y, cm1, t.y));
 }
 
+// cos x alone: 12 FP64 instructions.
+__device__ __forceinline__ double cos_tab(double x, const double2 *tw) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) return cos(x);
+  constexpr double k2Pi = 6.283185307179586477, k2PiLo = 2.4492935982947064e-16;
+  const double z = fma(x, kSincosTab / k2Pi, kRoundMagic);
+  const double kd = z - kRoundMagic;
+  double r = fma(kd, -k2Pi / kSincosTab, x);
+  r = fma(kd, -k2PiLo / kSincosTab, r);
+  const double2 t = tw[__double2loint(z) & (kSincosTab - 1)];
+  const double r2 = r * r;
+  const double sn = fma(r * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), r);
+  return fma(t.y, sn, fma(t.x, r2 * fma(r2, 1.0 / 24.0, -0.5), t.x));
+}
+
 // sin(x) / x: the Taylor series for |x| <= 1 (to x^10/11! for |x| <= 0.2, to
 // x^16/17! beyond: truncation below 1e-17), else the quotient.
 __device__ __forceinline__ double sinc64(double x) {

@@ -13,7 +13,7 @@ constexpr int kWvMaxLayers = 3;  // ucb_wavelet_layers gives 1..3 layers
 
 // Per-source plan record, written by the plan kernel.
 struct WvSrc {
-  double k[3], ep[9], ec[9];
+  double k[3], u[3], v[3];  // propagation direction, polarisation axes (v[2] = 0)
   double Ap, Ac, c2p, s2p;
   double fhet;
   int jmin, nl, jlo, c;  // first layer, layer count, first kept layer, kept layers per pixel time
@@ -28,9 +28,15 @@ struct WvGridDev {
   const double *orb_t;    // [norb] orbit node times (even grid of the barycentre splines)
   const double *tssb;     // [norb] t0 + i Tobs/(norb-1) (grid of the TDI splines)
   const double *geo;      // [norb][21]: S/C positions / c (9), unit arms (9), arm lengths / c (3) at tssb
-  const double *fac_orb;  // [3][norb]: h, l, mu of the spline system on orb_t
-  const double *fac_ssb;  // [3][norb]: same on tssb
+  const double *fac_orb;  // [5][norb]: h, l, mu, 1/h, 1/l of the spline system on orb_t
+  const double *fac_ssb;  // [5][norb]: same on tssb
+  double orb_inv, orb_off;  // 1/dx and -x0/dx - 1/2 of orb_t's even lookup (dx = x1 - x0)
+  const double2 *tw1024;    // e^{-2 pi i k / 1024}: the sine and cosine table
   const double *r0ds[kWvMaxLayers + 1];  // [NT (nl+1)][3] S/C 1 position / c at the downsampled times
+  // the downsampled times, and their offset from the TDI spline node below
+  // them and its index
+  const double *tds[kWvMaxLayers + 1], *dds[kWvMaxLayers + 1];
+  const int *jds[kWvMaxLayers + 1];
   const double *win[kWvMaxLayers + 1];   // [NT/2 + 1] window of an (nl+1)-layer grid
   const double2 *tw[kWvMaxLayers + 1];   // [NT (nl+1)] e^{-2 pi i k / (NT (nl+1))}
   const double *res;      // [3][N] residual X, Y, Z
@@ -54,6 +60,7 @@ struct WvWorkDev {
   double *resp = nullptr;  // [cap][7][norb] M (3), Mf (3), phase at S/C 1
   double *tdi = nullptr;   // [cap][3][2][4][norb] per-channel amplitude / phase splines
   double *coef = nullptr;  // [cap][3][kWvMaxLayers NT] coefficients, list order first
+  double *carrier = nullptr;  // [cap][(kWvMaxLayers + 1) NT] barycentre phase at S/C 1 of every sample (FP64 path)
   // the mixed likelihood's re-evaluation list: total[0] counts the sources
   // re-evaluated over the context's life, count[0] those of the current
   // launch, list[k] their indices
