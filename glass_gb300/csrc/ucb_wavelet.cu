@@ -42,6 +42,7 @@
 
 #include <algorithm>
 
+#include "fft_dit.cuh"
 #include "fp64_math.cuh"
 #include "glass_common.cuh"
 #include "ucb_wavelet.cuh"
@@ -479,135 +480,6 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     spline_coeffs(Q, zp, i, N, fac, cp);
   }
 #undef WV_TDI_PTRS
-}
-
-// ------------------------------------------------------------ FFTs
-// Radices of an in-place decimation-in-time FFT: 3s, then 4s, then a 2.
-struct RadixPlan {
-  int n;
-  int r[24];
-  int pre[24];  // R_0 ... R_{s-1}
-};
-
-__device__ __forceinline__ void radix_plan(int L, RadixPlan &P) {
-  P.n = 0;
-  int rem = L, pre = 1;
-  while (rem % 3 == 0) {
-    P.r[P.n] = 3;
-    P.pre[P.n++] = pre;
-    pre *= 3;
-    rem /= 3;
-  }
-  while (rem % 4 == 0) {
-    P.r[P.n] = 4;
-    P.pre[P.n++] = pre;
-    pre *= 4;
-    rem /= 4;
-  }
-  while (rem % 2 == 0) {
-    P.r[P.n] = 2;
-    P.pre[P.n++] = pre;
-    pre *= 2;
-    rem /= 2;
-  }
-}
-
-// Input position of element x: its stage digits read in reverse.
-__device__ __forceinline__ int digit_rev(int x, const RadixPlan &P) {
-  int pos = 0;
-  for (int s = P.n - 1; s >= 0; s--) {
-    const int d = x % P.r[s];
-    x /= P.r[s];
-    pos += d * P.pre[s];
-  }
-  return pos;
-}
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-template <typename C>
-__device__ __forceinline__ C mkc(decltype(C::x) x, decltype(C::x) y) {
-  C r;
-  r.x = x;
-  r.y = y;
-  return r;
-}
-
-// In-place mixed-radix FFT of a[L] held in digit-reversed order; result in
-// natural order.  tw[j * twmul] = e^{-2 pi i j / L}; sign -1 forward, +1
-// inverse (unnormalised).  Whole CTA.  C = double2 or float2.
-template <typename C>
-__device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ tw, int twmul, int sign) {
-  using R = decltype(C::x);
-  constexpr bool kF64 = sizeof(R) == 8;
-  int p = 1;
-  for (int st = 0; st < P.n; st++) {
-    const int Rd = P.r[st], q = p * Rd, nb = L / Rd;
-    const int tstep = (L / q) * twmul;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      const int b = t / p, k = t - b * p;
-      C *base = a + (size_t)b * q + k;
-      if (Rd == 4) {
-        C v0 = base[0], v1 = base[p], v2 = base[2 * p], v3 = base[3 * p];
-        if (!kF64 || st > 0) {  // FP64: the first stage's factors are 1
-          C w1 = tw[k * tstep], w2 = tw[2 * k * tstep], w3 = tw[3 * k * tstep];
-          if (sign > 0) {
-            w1.y = -w1.y;
-            w2.y = -w2.y;
-            w3.y = -w3.y;
-          }
-          v1 = cmul(v1, w1);
-          v2 = cmul(v2, w2);
-          v3 = cmul(v3, w3);
-        }
-        const C t0 = mkc<C>(v0.x + v2.x, v0.y + v2.y), t1 = mkc<C>(v0.x - v2.x, v0.y - v2.y);
-        const C t2 = mkc<C>(v1.x + v3.x, v1.y + v3.y), t3 = mkc<C>(v1.x - v3.x, v1.y - v3.y);
-        const C t3r = sign < 0 ? mkc<C>(t3.y, -t3.x) : mkc<C>(-t3.y, t3.x);
-        base[0] = mkc<C>(t0.x + t2.x, t0.y + t2.y);
-        base[p] = mkc<C>(t1.x + t3r.x, t1.y + t3r.y);
-        base[2 * p] = mkc<C>(t0.x - t2.x, t0.y - t2.y);
-        base[3 * p] = mkc<C>(t1.x - t3r.x, t1.y - t3r.y);
-      } else if (Rd == 2) {
-        C v0 = base[0], v1 = base[p];
-        C w1 = tw[k * tstep];
-        if (sign > 0) w1.y = -w1.y;
-        v1 = cmul(v1, w1);
-        base[0] = mkc<C>(v0.x + v1.x, v0.y + v1.y);
-        base[p] = mkc<C>(v0.x - v1.x, v0.y - v1.y);
-      } else {
-        C v0 = base[0], v1 = base[p], v2 = base[2 * p];
-        if (!kF64 || st > 0) {
-          C w1 = tw[k * tstep], w2 = tw[2 * k * tstep];
-          if (sign > 0) {
-            w1.y = -w1.y;
-            w2.y = -w2.y;
-          }
-          v1 = cmul(v1, w1);
-          v2 = cmul(v2, w2);
-        }
-        const R s3 = (R)0.86602540378443864676 * (R)sign;
-        const C sm = mkc<C>(v1.x + v2.x, v1.y + v2.y), df = mkc<C>(v1.x - v2.x, v1.y - v2.y);
-        if constexpr (kF64) {
-          const C m1 = mkc<C>(fma(-0.5, sm.x, v0.x), fma(-0.5, sm.y, v0.y));
-          base[0] = mkc<C>(v0.x + sm.x, v0.y + sm.y);
-          base[p] = mkc<C>(fma(-s3, df.y, m1.x), fma(s3, df.x, m1.y));
-          base[2 * p] = mkc<C>(fma(s3, df.y, m1.x), fma(-s3, df.x, m1.y));
-          continue;
-        }
-        const C m1 = mkc<C>(v0.x - (R)0.5 * sm.x, v0.y - (R)0.5 * sm.y);
-        const C m2 = mkc<C>(-s3 * df.y, s3 * df.x);
-        base[0] = mkc<C>(v0.x + sm.x, v0.y + sm.y);
-        base[p] = mkc<C>(m1.x + m2.x, m1.y + m2.y);
-        base[2 * p] = mkc<C>(m1.x - m2.x, m1.y - m2.y);
-      }
-    }
-    __syncthreads();
-    p = q;
-  }
 }
 
 // ------------------------------------------------------------ layers
@@ -1427,7 +1299,7 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
 // The FP64 layers of n sources (or of those on a device list of at most n).
 static cudaError_t launch_layers64(const WvGridDev &g, const WvWorkDev &w, int n, const int *count, const int *list,
                                    cudaStream_t s) {
-  const size_t sm = sizeof(double2) * (size_t)g.NT * (kWvMaxLayers + 1) / 2 + sizeof(double2) * g.NT;
+  const size_t sm = sizeof(double2) * ((size_t)g.NT * (kWvMaxLayers + 1) / 2 + g.NT);
   const cudaError_t e = cudaFuncSetAttribute(wv_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   wv_carrier_kernel<<<dim3(kCarrierSlices, n), 256, 0, s>>>(g, w.src, w.ssb, w.carrier, count, list);

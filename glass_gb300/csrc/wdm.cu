@@ -13,20 +13,39 @@
 //  * the real FFT of ND samples is a complex FFT of M = ND/2 packed samples
 //    (x[2n] + i x[2n+1]), done four-step as M1 x M2: FFTs down the M2 columns
 //    with the exp(-2 pi i n2 k1 / M) twiddle folded in, then FFTs along the M1
-//    rows; the real spectrum is unpacked on the fly where it is read;
-//  * one CTA per layer for the windowed NT-point transforms;
-//  * the inverse overlap-add runs in two launches (even, then odd layers): the
-//    supports of same-parity layers are disjoint, so no atomics are needed and
-//    the sum order is fixed;
-//  * all FFTs are mixed-radix (3, 4, 2) Stockham transforms in shared memory
-//    with ping-pong buffers, so NF = 1536 (the reference's default grid) works.
-// Templated on the arithmetic type: FP64 (parity with the reference) and FP32.
+//    rows;
+//  * one CTA per layer, or pair of layers, for the windowed NT-point transforms;
+//  * grids of the form 2^a 3^b, so NF = 1536 (the reference's default grid) works.
+//
+// FP64 (parity with the reference) is bound by the FP64 pipe, so FP64
+// instructions per sample are what counts, and warps enough to keep the pipe
+// full:
+//  * all FFTs run in place (fft_dit.cuh; twiddles from L1), 16 bytes of shared
+//    memory per point instead of 48 with ping-pong buffers and a twiddle copy: 16
+//    and more warps per SM instead of 8, which kept the pipe 65% busy;
+//  * two layers share a transform.  Of a layer's inverse FFT each pixel uses the
+//    real or the imaginary part; multiplied by (-i)^n (a shift of the spectrum by
+//    NT/4) those are the real part, up to a sign s(n) of period four, so layers a
+//    and b are the real and imaginary part of the inverse FFT of H_a + i H_b, H
+//    the Hermitian parts.  The inverse runs the same backwards;
+//  * the real spectrum is unpacked in the row pass and packed in the inverse's
+//    column pass, where both bins k and M - k are at hand (one product for the two).
+// 107 -> 66 FP64 instructions per sample forward, 104 -> 70 inverse.  2^21 samples
+// (1024 x 2048) forward 538 -> 333 us; 6.3 M samples (1536 x 4096) inverse 1787 ->
+// 1030 us.
+//
+// FP32 (GLASS_PREC_MIXED), and in FP64 the layers of grids whose NT is not a
+// multiple of 4, run one layer per CTA on ping-pong Stockham transforms; there
+// the inverse's overlap-add runs in two launches (even, then odd layers: the
+// supports of same-parity layers are disjoint, so no atomics are needed and the
+// sum order is fixed).
 #include <math.h>
 
 #include <mutex>
 #include <type_traits>
 #include <vector>
 
+#include "fft_dit.cuh"
 #include "wdm.cuh"
 
 namespace glass {
@@ -228,11 +247,12 @@ __device__ __forceinline__ C real_bin(const C *Z, long long M, long long k, cons
 }
 
 // Forward layers: one CTA per layer m in [0, NF].  The spectrum is either X
-// (bins 0..M given) or unpacked on the fly from Z, the FFT of the packed samples.
+// (bins 0..M given, times scale) or unpacked on the fly from Z, the FFT of the
+// packed samples.
 template <typename C>
 __global__ void wdm_fwd_layer_kernel(const C *Z, const C *X, long long M, int NF, int NT,
                                      const decltype(C().x) *phif, const C *twNT, const C *tlo, const C *thi, int K,
-                                     decltype(C().x) *wdm) {
+                                     decltype(C().x) scale, decltype(C().x) *wdm) {
   using R = decltype(C().x);
   extern __shared__ __align__(16) unsigned char sm_raw[];
   C *tw = reinterpret_cast<C *>(sm_raw);
@@ -257,7 +277,7 @@ __global__ void wdm_fwd_layer_kernel(const C *Z, const C *X, long long M, int NF
   }
   __syncthreads();
   C *r = block_fft(a, b, NT, 1, tw, +1);
-  const R inv = (R)1 / (R)NT;
+  const R inv = scale / (R)NT;  // scale 1 (FP32): exact
   const R sq2 = (R)1.41421356237309504880;
   for (int n = threadIdx.x; n < NT; n += blockDim.x) {
     const C v = r[n];
@@ -272,11 +292,11 @@ __global__ void wdm_fwd_layer_kernel(const C *Z, const C *X, long long M, int NF
   }
 }
 
-// Inverse layers of one parity: X[i] += window * FFT(prefactors) for the
+// Inverse layers of one parity: X[i] += scale * window * FFT(prefactors) for the
 // layer's support; layers m = parity, parity + 2, ...
 template <typename C>
 __global__ void wdm_inv_layer_kernel(const decltype(C().x) *wdm, int NF, int NT, int parity,
-                                     const decltype(C().x) *phif, const C *twNT, C *X) {
+                                     const decltype(C().x) *phif, const C *twNT, decltype(C().x) scale, C *X) {
   using R = decltype(C().x);
   extern __shared__ __align__(16) unsigned char sm_raw[];
   C *tw = reinterpret_cast<C *>(sm_raw);
@@ -305,7 +325,6 @@ __global__ void wdm_inv_layer_kernel(const decltype(C().x) *wdm, int NF, int NT,
   int imin = center - NT / 2, imax = center + NT / 2;
   if (imin < 0) imin = 0;
   if (imax > ND / 2 + 1) imax = (int)(ND / 2 + 1);
-  const R scale = (R)NF / (R)2;
   for (int i = imin + threadIdx.x; i < imax; i += blockDim.x) {
     const int iind = i > center ? i - center : center - i;
     const C v = (m == 0 || m == NF) ? r[(2 * i) % NT] : r[i % NT];
@@ -335,6 +354,255 @@ __global__ void wdm_pack_kernel(const C *X, long long M, const C *tlo, const C *
   const C e = twiddle2(tlo, thi, k, K, +1);
   const C ed = cm(e, d);
   Z[k] = mk<C>(s.x - ed.y, s.y + ed.x);
+}
+
+// ------------------------------------------------------------------ FP64
+// exp(sign 2 pi i p / P) from the two-level tables, in FP64.
+__device__ __forceinline__ double2 root2(const double2 *lo, const double2 *hi, long long p, int K, int sign) {
+  const double2 t = cmul(hi[p / K], lo[p % K]);
+  return make_double2(t.x, sign < 0 ? t.y : -t.y);
+}
+
+// Four-step pass 1, one column per CTA (16-byte accesses: two CTAs read each
+// sector, which L2 serves; the FP64 pipe is the bound, and 1024 CTAs balance
+// over 152 SMs where 256 of four columns leave a sixth of them idle).
+__global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, double2 *dst, int M1, int M2,
+                                                        const double2 *tw1, const double2 *tlo, const double2 *thi,
+                                                        int K) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(M1, P);
+  const int c = blockIdx.x;
+  for (int n1 = threadIdx.x; n1 < M1; n1 += blockDim.x) sm64[digit_rev(n1, P)] = src[(size_t)n1 * M2 + c];
+  __syncthreads();
+  dit_fft(sm64, M1, P, tw1, 1, -1);
+  for (int k1 = threadIdx.x; k1 < M1; k1 += blockDim.x)
+    dst[(size_t)k1 * M2 + c] = cmul(sm64[k1], root2(tlo, thi, (long long)c * k1, K, -1));
+}
+
+// The inverse's pass 1 on columns c and M2 - c, whose elements are bins k and M -
+// k of the real spectrum X (bins 0..M, the imaginary parts of bins 0 and M
+// ignored as an inverse real FFT does): with s = X_k + X*_{M-k}, d = X_k - X*_{M-k}
+// and w = e^{2 pi i k/ND} d, the packed spectrum is Z_k = s + i w, Z_{M-k} = s* + i w*.
+__global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, double2 *dst, int M1, int M2,
+                                                             const double2 *tw1, const double2 *mlo,
+                                                             const double2 *mhi, const double2 *nlo,
+                                                             const double2 *nhi, int K) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(M1, P);
+  const long long M = (long long)M1 * M2;
+  const int c = blockIdx.x, cm = c == 0 ? 0 : M2 - c;
+  const bool two = cm != c;
+  const int bo = two ? M1 : 0;  // column M2 - c's place
+  // column c's rows, each with its mirror: row M1 - n1 of column 0 (row 0 with bin
+  // M), else row M1 - 1 - n1 of column M2 - c; a lone column's mirrors repeat it
+  const int rows = two ? M1 : c == 0 ? M1 / 2 + 1 : (M1 + 1) / 2;
+  for (int n1 = threadIdx.x; n1 < rows; n1 += blockDim.x) {
+    const long long k = (long long)n1 * M2 + c;
+    double2 xk = X[k], xm = X[M - k];
+    if (k == 0) xk.y = xm.y = 0.0;
+    const double2 s = make_double2(xk.x + xm.x, xk.y - xm.y), d = make_double2(xk.x - xm.x, xk.y + xm.y);
+    const double2 w = cmul(root2(nlo, nhi, k, K, +1), d);
+    sm64[digit_rev(n1, P)] = make_double2(s.x - w.y, s.y + w.x);
+    if (k > 0) {
+      const int nm = c == 0 ? M1 - n1 : M1 - 1 - n1;
+      if (two || nm != n1) sm64[bo + digit_rev(nm, P)] = make_double2(s.x + w.y, w.x - s.y);
+    }
+  }
+  __syncthreads();
+  dit_fft(sm64, M1, P, tw1, 1, +1, two ? 2 : 1);
+  for (int t = threadIdx.x; t < (two ? 2 * M1 : M1); t += blockDim.x) {
+    const int which = t >= M1, k1 = t - which * M1, col = which ? cm : c;
+    dst[(size_t)k1 * M2 + col] = cmul(sm64[t], root2(mlo, mhi, (long long)col * k1, K, +1));
+  }
+}
+
+// The inverse's pass 2, one row per CTA: output index k1 + M1 k2.
+__global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, double2 *dst, int M1, int M2,
+                                                        const double2 *tw2) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(M2, P);
+  const int r = blockIdx.x;
+  for (int t = threadIdx.x; t < M2; t += blockDim.x) sm64[digit_rev(t, P)] = src[(size_t)r * M2 + t];
+  __syncthreads();
+  dit_fft(sm64, M2, P, tw2, 1, +1);
+  for (int k2 = threadIdx.x; k2 < M2; k2 += blockDim.x) dst[(size_t)r + (size_t)M1 * k2] = sm64[k2];
+}
+
+// The forward's pass 2 on rows k1 and M1 - k1, whose elements are bins k = k1 +
+// M1 k2 and M - k of the packed spectrum Z, unpacked to twice the real spectrum:
+// with s = Z_k + Z*_{M-k}, d = Z_k - Z*_{M-k} and w = e^{-2 pi i k/ND} d, 2 X_k = s - i w
+// and 2 X_{M-k} = s* - i w*.
+__global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *src, double2 *X, int M1, int M2,
+                                                               const double2 *tw2, const double2 *nlo,
+                                                               const double2 *nhi, int K) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(M2, P);
+  const long long M = (long long)M1 * M2;
+  const int r = blockIdx.x, rm = r == 0 ? 0 : M1 - r;
+  const bool two = rm != r;
+  for (int t = threadIdx.x; t < (two ? 2 * M2 : M2); t += blockDim.x) {
+    const int which = t >= M2, k2 = t - which * M2;
+    sm64[which * M2 + digit_rev(k2, P)] = src[(size_t)(which ? rm : r) * M2 + k2];
+  }
+  __syncthreads();
+  dit_fft(sm64, M2, P, tw2, 1, -1, two ? 2 : 1);
+  const int bo = two ? M2 : 0;
+  const int n = two ? M2 : r == 0 ? M2 / 2 + 1 : (M2 + 1) / 2;
+  for (int k2 = threadIdx.x; k2 < n; k2 += blockDim.x) {
+    const long long k = (long long)r + (long long)M1 * k2;
+    const double2 zk = sm64[k2], zm = sm64[bo + (r == 0 ? (k2 == 0 ? 0 : M2 - k2) : M2 - 1 - k2)];
+    const double2 s = make_double2(zk.x + zm.x, zk.y - zm.y), d = make_double2(zk.x - zm.x, zk.y + zm.y);
+    const double2 w = cmul(root2(nlo, nhi, k, K, -1), d);
+    X[k] = make_double2(s.x + w.y, s.y - w.x);
+    if (2 * k != M) X[M - k] = make_double2(s.x - w.y, -(s.y + w.x));
+  }
+}
+
+// Layers of pair q: 0: the grid's first and last (0, NF); q >= 1: 2 q - 1 and 2 q
+// (the second absent where it would be NF).
+__host__ __device__ __forceinline__ int layer_pairs(int NF) { return 1 + NF / 2; }
+
+// Forward layers, a pair per CTA, from scale times the real spectrum X (scale:
+// what the window must be multiplied with, 1/NT and the Hermitian parts' half
+// included).  The first and last layer use the real parts of even n alone, as
+// they are (no shift).
+__global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, int NF, int NT, const double *phif,
+                                                             const double2 *twNT, double scale, double *wdm) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(NT, P);
+  const int q = blockIdx.x, h = NT / 2;
+  const bool edge = q == 0;
+  const int ma = edge ? 0 : 2 * q - 1, mb = edge ? NF : 2 * q;
+  const bool has_b = edge || mb < NF;
+  if (!edge && ma >= NF) return;
+  if (edge) scale *= 1.41421356237309504880;
+  auto bin = [&](int m, int k) {
+    const int j = k - h;
+    double2 v = make_double2(0.0, 0.0);
+    if (j == -h || (m == 0 && j < 0) || (m == NF && j > 0)) return v;
+    double w = scale * phif[j < 0 ? -j : j];
+    if (edge && j == 0) w *= 0.5;
+    v = X[(size_t)m * h + j];
+    v = make_double2(v.x * w, v.y * w);
+    return (!edge && (m & 1)) ? make_double2(-v.y, v.x) : v;
+  };
+  for (int e = threadIdx.x; e <= h; e += blockDim.x) {
+    int k, kp, p, pp;
+    if (edge) {
+      k = p = e;
+      kp = pp = e == 0 ? 0 : NT - e;
+    } else {
+      k = e <= NT / 4 ? e : NT / 4 + e;
+      kp = e <= NT / 4 ? h - k : 3 * h - k;
+      p = k < NT / 4 ? k + 3 * (NT / 4) : k - NT / 4;
+      pp = kp < NT / 4 ? kp + 3 * (NT / 4) : kp - NT / 4;
+    }
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 a0 = bin(ma, k), a1 = bin(ma, kp), b0 = has_b ? bin(mb, k) : zero, b1 = has_b ? bin(mb, kp) : zero;
+    const double ax = a0.x + a1.x, ay = a0.y - a1.y, bx = b0.x + b1.x, by = b0.y - b1.y;
+    sm64[digit_rev(p, P)] = make_double2(ax - by, ay + bx);
+    if (pp != p) sm64[digit_rev(pp, P)] = make_double2(ax + by, bx - ay);
+  }
+  __syncthreads();
+  dit_fft(sm64, NT, P, twNT, 1, +1);
+  if (edge) {
+    for (int n = 2 * threadIdx.x; n < NT; n += 2 * blockDim.x) {
+      wdm[n] = sm64[n].x;
+      wdm[n + 1] = sm64[n].y;
+    }
+  } else {
+    for (int n = threadIdx.x; n < NT; n += blockDim.x) {
+      const double2 v = sm64[n];
+      wdm[n + (size_t)NT * ma] = (n & 2) ? -v.x : v.x;
+      if (has_b) wdm[n + (size_t)NT * mb] = (n & 2) ? -v.y : v.y;
+    }
+  }
+}
+
+// Inverse layers, a pair per CTA: the FFT of u_a + i u_b, u a layer's coefficients
+// with their signs, gives both layers' spectra, windowed and added into the bins
+// of X.  No bin is cleared beforehand and the sum order is fixed: pairs 2q - 1, 2q
+// reach bins [(q - 1) NT, (q + 1/2) NT); those of odd q store (first launch), those
+// of even q add where a neighbour has stored and store between (second).  The
+// first layer adds in the second launch; the last stores in the first where the
+// pair below it is of even q, else adds in the second.  blockIdx: the launch's
+// pairs, then its edge layers (first, last).
+__global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, int NF, int NT, int launch,
+                                                             const double *phif, const double2 *twNT, double scale,
+                                                             double2 *X) {
+  extern __shared__ __align__(16) double2 sm64[];
+  RadixPlan P;
+  radix_plan(NT, P);
+  const int h = NT / 2, pairs = NF / 2, mine = launch == 0 ? (pairs + 1) / 2 : pairs / 2;
+  const bool edge = (int)blockIdx.x >= mine;
+  const int q = 2 * blockIdx.x + 1 + launch;
+  const int ma = 2 * q - 1, mb = 2 * q;
+  const bool has_b = mb < NF;
+  const bool last = edge && (launch == 0 || (int)blockIdx.x > mine);  // the edge CTA's layer is NF
+  for (int n = threadIdx.x; n < NT; n += blockDim.x) {
+    double2 v = make_double2(0.0, 0.0);
+    if (edge) {
+      v.x = wdm[(2 * n) % NT + last];
+    } else {
+      // layer a is odd, b even: the reference's (-i)^(n + m odd) as -i (-i)^n and
+      // (-i)^n times these signs
+      v.x = wdm[n + (size_t)NT * ma];
+      if (has_b) v.y = wdm[n + (size_t)NT * mb];
+      if ((n + 1) & 2) v.x = -v.x;
+      if (n & 2) v.y = -v.y;
+    }
+    sm64[digit_rev(n, P)] = v;
+  }
+  __syncthreads();
+  dit_fft(sm64, NT, P, twNT, 1, -1);
+  if (edge) {
+    const double c = scale * 0.70710678118654752440;
+    const long long M = (long long)NF * h;
+    // layer 0: bins 0 .. h - 1; layer NF: M - h .. M, bin M its own
+    for (int i = threadIdx.x; i < (last ? h + 1 : h); i += blockDim.x) {
+      const long long k = last ? M - i : i;
+      const double2 a = sm64[(int)((2 * k) % NT)];
+      const double w = c * phif[i];
+      if (last && (i == 0 || launch == 0))
+        X[k] = make_double2(w * a.x, w * a.y);
+      else
+        X[k] = make_double2(fma(w, a.x, X[k].x), fma(w, a.y, X[k].y));
+    }
+    return;
+  }
+  const double c = 0.5 * scale;
+  // spectrum of layer a (real part's) or b at bin k of its own transform, twice
+  auto part = [&](bool second, int k) {
+    const double2 f = sm64[k], g = sm64[k == 0 ? 0 : NT - k];
+    return second ? make_double2(f.y + g.y, g.x - f.x) : make_double2(f.x + g.x, f.y - g.y);
+  };
+  // bin i of layer m: R_m[i mod NT] = nu U_m[(i + NT/4) mod NT], nu = -i for layer a
+  const int i0 = (q - 1) * NT, ca = ma * h, cb = ca + h;
+  const int top = has_b ? NT : h;  // the upper layer's upper half
+  for (int t = threadIdx.x; t < top + h; t += blockDim.x) {
+    const int i = i0 + t, k = (t + NT / 4) % NT;  // i0 is a multiple of NT
+    double2 v = make_double2(0.0, 0.0);
+    if (t < NT) {
+      const double2 a = part(false, k);
+      const double w = c * phif[i < ca ? ca - i : i - ca];
+      v = make_double2(w * a.y, -(w * a.x));
+    }
+    if (has_b && t >= h) {
+      const double2 b = part(true, k);
+      const double w = c * phif[i < cb ? cb - i : i - cb];
+      v = make_double2(fma(w, b.x, v.x), fma(w, b.y, v.y));
+    }
+    if (launch == 1 && (t < h || t >= top)) {  // the first launch has stored there
+      const double2 x = X[i];
+      v = make_double2(v.x + x.x, v.y + x.y);
+    }
+    X[i] = v;
+  }
 }
 
 template <typename C>
@@ -518,125 +786,181 @@ static cudaError_t four_step(const WdmPlan &P, const C *src, C *tmp, C *dst, int
 
 static unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 
-template <typename C>
-static cudaError_t forward_t(const WdmPlan &P, const double *time, double *wdm, cudaStream_t s) {
-  using R = decltype(C().x);
-  constexpr bool kF64 = std::is_same<R, double>::value;
+// ---- FP64
+static size_t smem64(int points) { return sizeof(double2) * (size_t)points; }
+static int threads64(int points, int most) {  // one radix-4 butterfly per thread
+  int t = (points / 4 + 31) / 32 * 32;
+  return t < 32 ? 32 : t > most ? most : t;
+}
+template <typename K, typename... Args>
+static cudaError_t launch64(K kernel, int grid, int points, int most, cudaStream_t s, Args... args) {
+  cudaError_t e;
+  if (smem64(points) > 48 * 1024 && (e = set_smem((const void *)kernel, smem64(points))) != cudaSuccess) return e;
+  kernel<<<grid, threads64(points, most), smem64(points), s>>>(args...);
+  return cudaGetLastError();
+}
+
+// scale times the real spectrum X -> coefficients.
+static cudaError_t fwd_layers64(const WdmPlan &P, const double2 *X, double scale, double *wdm, cudaStream_t s) {
+  const int NF = P.NF, NT = P.NT;
+  if (NT % 4 == 0)
+    return launch64(wdm_fwd_pair64_kernel, layer_pairs(NF), NT, 256, s, X, NF, NT, (const double *)P.win,
+                    (const double2 *)P.twNT, 0.5 * scale / NT, wdm);
+  const size_t sm = fft_smem<double2>(NT, 1);
+  const cudaError_t e = set_smem((const void *)wdm_fwd_layer_kernel<double2>, sm);
+  if (e != cudaSuccess) return e;
+  wdm_fwd_layer_kernel<double2><<<NF + 1, 256, sm, s>>>(nullptr, X, P.M, NF, NT, (const double *)P.win,
+                                                        (const double2 *)P.twNT, (const double2 *)P.nlo,
+                                                        (const double2 *)P.nhi, P.K, scale, wdm);
+  return cudaGetLastError();
+}
+
+static cudaError_t forward64(const WdmPlan &P, const double *time, double *wdm, cudaStream_t s) {
+  const long long ND = (long long)P.NF * P.NT;
+  const double2 *packed = reinterpret_cast<const double2 *>(time);
+  cudaError_t e;
+  if ((uintptr_t)time % 16) {  // the packed complex view needs 16-byte alignment
+    if ((e = cudaMemcpyAsync(P.rbuf, time, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
+    packed = reinterpret_cast<const double2 *>(P.rbuf);
+  }
+  if ((e = launch64(wdm_col64_kernel, P.M2, P.M1, 256, s, packed, (double2 *)P.bufB, P.M1, P.M2,
+                    (const double2 *)P.tw1, (const double2 *)P.mlo, (const double2 *)P.mhi, P.K)) != cudaSuccess)
+    return e;
+  if ((e = launch64(wdm_row_unpack64_kernel, P.M1 / 2 + 1, 2 * P.M2, 512, s, (const double2 *)P.bufB,
+                    (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.nlo,
+                    (const double2 *)P.nhi, P.K)) != cudaSuccess)
+    return e;
+  return fwd_layers64(P, (const double2 *)P.bufX, 0.5, wdm, s);
+}
+
+// WDM -> scale times the spectrum, bins 0..M of P.bufX.
+static cudaError_t inverse_layers64(const WdmPlan &P, const double *wdm, double scale, cudaStream_t s) {
+  const int NF = P.NF, NT = P.NT;
+  const double *win = (const double *)P.win;
+  const double2 *tw = (const double2 *)P.twNT;
+  double2 *X = (double2 *)P.bufX;
+  cudaError_t e;
+  scale *= 0.5 * NF;
+  if (NT % 4 == 0) {
+    const int pairs = NF / 2;  // (1, 2), (3, 4), ...
+    const bool last_first = pairs % 2 == 0;  // the last layer's place: see the kernel
+    if ((e = launch64(wdm_inv_pair64_kernel, (pairs + 1) / 2 + last_first, NT, 256, s, wdm, NF, NT, 0, win, tw, scale,
+                      X)) != cudaSuccess)
+      return e;
+    return launch64(wdm_inv_pair64_kernel, pairs / 2 + 1 + !last_first, NT, 256, s, wdm, NF, NT, 1, win, tw, scale, X);
+  }
+  wdm_zero_kernel<double2><<<blocks_for(P.M + 1), 256, 0, s>>>(X, P.M + 1);
+  const size_t sm = fft_smem<double2>(NT, 1);
+  if ((e = set_smem((const void *)wdm_inv_layer_kernel<double2>, sm)) != cudaSuccess) return e;
+  for (int parity = 0; parity < 2; parity++)
+    wdm_inv_layer_kernel<double2><<<(NF - parity) / 2 + 1, 256, sm, s>>>(wdm, NF, NT, parity, win, tw, scale, X);
+  return cudaGetLastError();
+}
+
+static cudaError_t inverse64(const WdmPlan &P, const double *wdm, double *time, cudaStream_t s) {
   const long long ND = (long long)P.NF * P.NT;
   cudaError_t e;
-  const C *packed;
-  R *out;
-  if (kF64) {
-    if ((uintptr_t)time % 16) {  // the packed complex view needs 16-byte alignment
-      if ((e = cudaMemcpyAsync(P.rbuf, time, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-        return e;
-      packed = reinterpret_cast<const C *>(P.rbuf);
-    } else {
-      packed = reinterpret_cast<const C *>(time);
-    }
-    out = reinterpret_cast<R *>(wdm);
-  } else {
-    wdm_cast_kernel<C><<<blocks_for(ND), 256, 0, s>>>(time, (R *)P.rbuf, ND);
-    packed = reinterpret_cast<const C *>(P.rbuf);
-    out = (R *)P.rbuf;  // consumed by the first FFT pass before the layers write
+  if ((e = inverse_layers64(P, wdm, 1.0 / (double)ND, s)) != cudaSuccess) return e;
+  if ((e = launch64(wdm_pack_col64_kernel, P.M2 / 2 + 1, 2 * P.M1, 512, s, (const double2 *)P.bufX,
+                    (double2 *)P.bufB, P.M1, P.M2, (const double2 *)P.tw1, (const double2 *)P.mlo,
+                    (const double2 *)P.mhi, (const double2 *)P.nlo, (const double2 *)P.nhi, P.K)) != cudaSuccess)
+    return e;
+  const bool direct = (uintptr_t)time % 16 == 0;
+  double2 *dst = reinterpret_cast<double2 *>(direct ? (void *)time : P.rbuf);
+  if ((e = launch64(wdm_row64_kernel, P.M1, P.M2, 256, s, (const double2 *)P.bufB, dst, P.M1, P.M2,
+                    (const double2 *)P.tw2)) != cudaSuccess)
+    return e;
+  if (!direct) return cudaMemcpyAsync(time, P.rbuf, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s);
+  return cudaSuccess;
+}
+
+// wdm -> ND/2 + 1 complex bins (ND + 2 doubles), wavelet_transform_inverse_freq
+static cudaError_t to_freq64(const WdmPlan &P, const double *wdm, double *freq, cudaStream_t s) {
+  const cudaError_t e = inverse_layers64(P, wdm, 1.0, s);
+  if (e != cudaSuccess) return e;
+  return cudaMemcpyAsync(freq, P.bufX, sizeof(double2) * (size_t)(P.M + 1), cudaMemcpyDeviceToDevice, s);
+}
+
+// ND/2 + 1 complex bins -> wdm, wavelet_transform_freq
+static cudaError_t from_freq64(const WdmPlan &P, const double *freq, double *wdm, cudaStream_t s) {
+  const double2 *X = reinterpret_cast<const double2 *>(freq);
+  if ((uintptr_t)freq % 16) {
+    const cudaError_t e =
+        cudaMemcpyAsync(P.bufX, freq, sizeof(double2) * (size_t)(P.M + 1), cudaMemcpyDeviceToDevice, s);
+    if (e != cudaSuccess) return e;
+    X = (const double2 *)P.bufX;
   }
-  if ((e = four_step<C>(P, packed, (C *)P.bufB, (C *)P.bufA, -1, (R)1, s)) != cudaSuccess) return e;
-  const size_t sm = fft_smem<C>(P.NT, 1);
-  if ((e = set_smem((const void *)wdm_fwd_layer_kernel<C>, sm)) != cudaSuccess) return e;
-  wdm_fwd_layer_kernel<C><<<P.NF + 1, 256, sm, s>>>((const C *)P.bufA, nullptr, P.M, P.NF, P.NT, (const R *)P.win,
-                                                     (const C *)P.twNT, (const C *)P.nlo, (const C *)P.nhi, P.K,
-                                                     out);
+  return fwd_layers64(P, X, 1.0, wdm, s);
+}
+
+// ---- FP32 (double at the boundary)
+static cudaError_t forward32(const WdmPlan &P, const double *time, double *wdm, cudaStream_t s) {
+  const long long ND = (long long)P.NF * P.NT;
+  cudaError_t e;
+  float *out = (float *)P.rbuf;  // consumed by the first FFT pass before the layers write
+  wdm_cast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>(time, out, ND);
+  if ((e = four_step<float2>(P, (const float2 *)P.rbuf, (float2 *)P.bufB, (float2 *)P.bufA, -1, 1.f, s)) != cudaSuccess)
+    return e;
+  const size_t sm = fft_smem<float2>(P.NT, 1);
+  if ((e = set_smem((const void *)wdm_fwd_layer_kernel<float2>, sm)) != cudaSuccess) return e;
+  wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>((const float2 *)P.bufA, nullptr, P.M, P.NF, P.NT,
+                                                         (const float *)P.win, (const float2 *)P.twNT,
+                                                         (const float2 *)P.nlo, (const float2 *)P.nhi, P.K, 1.f, out);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (!kF64) wdm_uncast_kernel<C><<<blocks_for(ND), 256, 0, s>>>(out, wdm, ND);
+  wdm_uncast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>(out, wdm, ND);
   return cudaGetLastError();
 }
 
 // WDM -> spectrum: bins 0..M summed into P.bufX by the windowed layer transforms.
-template <typename C>
-static cudaError_t inverse_layers_t(const WdmPlan &P, const double *wdm, cudaStream_t s) {
-  using R = decltype(C().x);
-  constexpr bool kF64 = std::is_same<R, double>::value;
-  const long long ND = (long long)P.NF * P.NT, M = P.M;
+static cudaError_t inverse_layers32(const WdmPlan &P, const double *wdm, cudaStream_t s) {
+  const long long ND = (long long)P.NF * P.NT;
   const int NT = P.NT, NF = P.NF;
-  cudaError_t e;
-  const R *in;
-  if (kF64) {
-    in = reinterpret_cast<const R *>(wdm);
-  } else {
-    wdm_cast_kernel<C><<<blocks_for(ND), 256, 0, s>>>(wdm, (R *)P.rbuf, ND);
-    in = (const R *)P.rbuf;
-  }
-  wdm_zero_kernel<C><<<blocks_for(M + 1), 256, 0, s>>>((C *)P.bufX, M + 1);
-  const size_t sm = fft_smem<C>(NT, 1);
-  if ((e = set_smem((const void *)wdm_inv_layer_kernel<C>, sm)) != cudaSuccess) return e;
+  wdm_cast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>(wdm, (float *)P.rbuf, ND);
+  wdm_zero_kernel<float2><<<blocks_for(P.M + 1), 256, 0, s>>>((float2 *)P.bufX, P.M + 1);
+  const size_t sm = fft_smem<float2>(NT, 1);
+  const cudaError_t e = set_smem((const void *)wdm_inv_layer_kernel<float2>, sm);
+  if (e != cudaSuccess) return e;
   // even layers, then odd: same-parity layers have disjoint supports
   for (int parity = 0; parity < 2; parity++)
-    wdm_inv_layer_kernel<C><<<(NF - parity) / 2 + 1, 256, sm, s>>>(in, NF, NT, parity, (const R *)P.win,
-                                                                    (const C *)P.twNT, (C *)P.bufX);
+    wdm_inv_layer_kernel<float2><<<(NF - parity) / 2 + 1, 256, sm, s>>>((const float *)P.rbuf, NF, NT, parity,
+                                                                        (const float *)P.win, (const float2 *)P.twNT,
+                                                                        (float)NF / 2.f, (float2 *)P.bufX);
   return cudaGetLastError();
 }
 
-template <typename C>
-static cudaError_t inverse_t(const WdmPlan &P, const double *wdm, double *time, cudaStream_t s) {
-  using R = decltype(C().x);
-  constexpr bool kF64 = std::is_same<R, double>::value;
+static cudaError_t inverse32(const WdmPlan &P, const double *wdm, double *time, cudaStream_t s) {
   const long long ND = (long long)P.NF * P.NT, M = P.M;
   cudaError_t e;
-  if ((e = inverse_layers_t<C>(P, wdm, s)) != cudaSuccess) return e;
-  wdm_pack_kernel<C><<<blocks_for(M), 256, 0, s>>>((const C *)P.bufX, M, (const C *)P.nlo, (const C *)P.nhi, P.K,
-                                                   (C *)P.bufA);
-  const bool direct = kF64 && (uintptr_t)time % 16 == 0;
-  C *dst = direct ? reinterpret_cast<C *>(time) : reinterpret_cast<C *>(P.rbuf);
-  if ((e = four_step<C>(P, (const C *)P.bufA, (C *)P.bufB, dst, +1, (R)(1.0 / (double)ND), s)) != cudaSuccess)
+  if ((e = inverse_layers32(P, wdm, s)) != cudaSuccess) return e;
+  wdm_pack_kernel<float2><<<blocks_for(M), 256, 0, s>>>((const float2 *)P.bufX, M, (const float2 *)P.nlo,
+                                                        (const float2 *)P.nhi, P.K, (float2 *)P.bufA);
+  if ((e = four_step<float2>(P, (const float2 *)P.bufA, (float2 *)P.bufB, (float2 *)P.rbuf, +1,
+                             (float)(1.0 / (double)ND), s)) != cudaSuccess)
     return e;
-  if (!kF64)
-    wdm_uncast_kernel<C><<<blocks_for(ND), 256, 0, s>>>((const R *)P.rbuf, time, ND);
-  else if (!direct)
-    return cudaMemcpyAsync(time, P.rbuf, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s);
+  wdm_uncast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>((const float *)P.rbuf, time, ND);
   return cudaGetLastError();
 }
 
-// wdm -> ND/2 + 1 complex bins (ND + 2 doubles), wavelet_transform_inverse_freq
-template <typename C>
-static cudaError_t to_freq_t(const WdmPlan &P, const double *wdm, double *freq, cudaStream_t s) {
-  using R = decltype(C().x);
-  constexpr bool kF64 = std::is_same<R, double>::value;
+static cudaError_t to_freq32(const WdmPlan &P, const double *wdm, double *freq, cudaStream_t s) {
   const long long n = 2 * (P.M + 1);
-  cudaError_t e;
-  if ((e = inverse_layers_t<C>(P, wdm, s)) != cudaSuccess) return e;
-  if (kF64) return cudaMemcpyAsync(freq, P.bufX, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
-  wdm_uncast_kernel<C><<<blocks_for(n), 256, 0, s>>>((const R *)P.bufX, freq, n);
+  const cudaError_t e = inverse_layers32(P, wdm, s);
+  if (e != cudaSuccess) return e;
+  wdm_uncast_kernel<float2><<<blocks_for(n), 256, 0, s>>>((const float *)P.bufX, freq, n);
   return cudaGetLastError();
 }
 
-// ND/2 + 1 complex bins -> wdm, wavelet_transform_freq
-template <typename C>
-static cudaError_t from_freq_t(const WdmPlan &P, const double *freq, double *wdm, cudaStream_t s) {
-  using R = decltype(C().x);
-  constexpr bool kF64 = std::is_same<R, double>::value;
+static cudaError_t from_freq32(const WdmPlan &P, const double *freq, double *wdm, cudaStream_t s) {
   const long long ND = (long long)P.NF * P.NT, n = 2 * (P.M + 1);
-  cudaError_t e;
-  const C *X;
-  R *out;
-  if (kF64) {
-    if ((uintptr_t)freq % 16) {
-      if ((e = cudaMemcpyAsync(P.bufX, freq, sizeof(double) * n, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-      X = (const C *)P.bufX;
-    } else {
-      X = reinterpret_cast<const C *>(freq);
-    }
-    out = reinterpret_cast<R *>(wdm);
-  } else {
-    wdm_cast_kernel<C><<<blocks_for(n), 256, 0, s>>>(freq, (R *)P.bufX, n);
-    X = (const C *)P.bufX;
-    out = (R *)P.rbuf;
-  }
-  const size_t sm = fft_smem<C>(P.NT, 1);
-  if ((e = set_smem((const void *)wdm_fwd_layer_kernel<C>, sm)) != cudaSuccess) return e;
-  wdm_fwd_layer_kernel<C><<<P.NF + 1, 256, sm, s>>>(nullptr, X, P.M, P.NF, P.NT, (const R *)P.win, (const C *)P.twNT,
-                                                     (const C *)P.nlo, (const C *)P.nhi, P.K, out);
+  wdm_cast_kernel<float2><<<blocks_for(n), 256, 0, s>>>(freq, (float *)P.bufX, n);
+  const size_t sm = fft_smem<float2>(P.NT, 1);
+  cudaError_t e = set_smem((const void *)wdm_fwd_layer_kernel<float2>, sm);
+  if (e != cudaSuccess) return e;
+  wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>(nullptr, (const float2 *)P.bufX, P.M, P.NF, P.NT,
+                                                         (const float *)P.win, (const float2 *)P.twNT,
+                                                         (const float2 *)P.nlo, (const float2 *)P.nhi, P.K, 1.f,
+                                                         (float *)P.rbuf);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (!kF64) wdm_uncast_kernel<C><<<blocks_for(ND), 256, 0, s>>>(out, wdm, ND);
+  wdm_uncast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>((const float *)P.rbuf, wdm, ND);
   return cudaGetLastError();
 }
 
@@ -662,19 +986,19 @@ void wdm_release(WdmPlan &P) {
 }
 
 cudaError_t wdm_forward(const WdmPlan &P, const double *time, double *wdm, cudaStream_t s) {
-  return P.precision == 1 ? forward_t<float2>(P, time, wdm, s) : forward_t<double2>(P, time, wdm, s);
+  return P.precision == 1 ? forward32(P, time, wdm, s) : forward64(P, time, wdm, s);
 }
 
 cudaError_t wdm_inverse(const WdmPlan &P, const double *wdm, double *time, cudaStream_t s) {
-  return P.precision == 1 ? inverse_t<float2>(P, wdm, time, s) : inverse_t<double2>(P, wdm, time, s);
+  return P.precision == 1 ? inverse32(P, wdm, time, s) : inverse64(P, wdm, time, s);
 }
 
 cudaError_t wdm_to_freq(const WdmPlan &P, const double *wdm, double *freq, cudaStream_t s) {
-  return P.precision == 1 ? to_freq_t<float2>(P, wdm, freq, s) : to_freq_t<double2>(P, wdm, freq, s);
+  return P.precision == 1 ? to_freq32(P, wdm, freq, s) : to_freq64(P, wdm, freq, s);
 }
 
 cudaError_t wdm_from_freq(const WdmPlan &P, const double *freq, double *wdm, cudaStream_t s) {
-  return P.precision == 1 ? from_freq_t<float2>(P, freq, wdm, s) : from_freq_t<double2>(P, freq, wdm, s);
+  return P.precision == 1 ? from_freq32(P, freq, wdm, s) : from_freq64(P, freq, wdm, s);
 }
 
 // Meyer window of utils/src/glass_wavelet.c:305-349 with the regularised
