@@ -17,7 +17,7 @@
 //     Taylor series) and sinc, and the per-sample
 //     geometry and per-proposal constants as hi + lo floats;
 //   fd_hp_kernel:      thread-block clusters of 4 CTAs, one proposal each:
-//     CTA r transforms series r in its shared memory (radix-4 Stockham,
+//     CTA r transforms series r in place in its shared memory (radix 4,
 //     twiddles as hi + lo floats), then CTAs 2c and 2c + 1 form channel c's
 //     whitened template per bin from their own spectrum and their partner's
 //     (read through distributed shared memory), each over half of the bins,
@@ -35,24 +35,35 @@ namespace glass {
 constexpr int kHpThreads = 256;
 
 // -------------------------------------------------------- slow part, df
-// The two arms of spacecraft i (12, 13 | 21, 23 | 31, 32) at one sample, as
-// slow_sample_mix computes them, in double-float throughout.  tab: the
-// sine/cosine table of df_sincos_tab.
-__device__ __forceinline__ void slow_arms_hp(const ItemMix &c, const OrbitSampleMix &o, const GeoSampleMix &gm,
-                                             const GeoSampleMix &gl, const SlowArgs &K, const float4 *tab, int i,
-                                             dc d[2]) {
+// k.(x_i - x_gc) of spacecraft i (metres).
+__device__ __forceinline__ df kdot_hp(const ItemMix &c, const GeoSampleMix &gm, const GeoSampleMix &gl, int i) {
   const df k0 = {c.k[0], c.kl[0]}, k1 = {c.k[1], c.kl[1]}, k2 = {c.k[2], c.kl[2]};
-  // k.(x_j - x_gc) for the three spacecraft (metres)
-  df kd[3];
+  return df_add(df_add(df_mul(k0, df{gm.f[3 * i], gl.f[3 * i]}), df_mul(k1, df{gm.f[3 * i + 1], gl.f[3 * i + 1]})),
+                df_mul(k2, df{gm.f[3 * i + 2], gl.f[3 * i + 2]}));
+}
+// r^T M r of arm a (0: 12, 1: 13, 2: 23), M = m (DP e+ + DC ex) as hi + lo.
+__device__ __forceinline__ dc arm_hp(const ItemMix &c, const GeoSampleMix &gm, const GeoSampleMix &gl, int a) {
+  df mr = {0.f, 0.f}, mi = {0.f, 0.f};
 #pragma unroll
-  for (int j = 0; j < 3; j++)
-    kd[j] = df_add(df_add(df_mul(k0, df{gm.f[3 * j], gl.f[3 * j]}), df_mul(k1, df{gm.f[3 * j + 1], gl.f[3 * j + 1]})),
-                   df_mul(k2, df{gm.f[3 * j + 2], gl.f[3 * j + 2]}));
+  for (int t = 0; t < 6; t++) {
+    const df mo = {gm.f[9 + 6 * a + t], gl.f[9 + 6 * a + t]};
+    mr = df_add(mr, df_mul(df{c.Mr[t], c.Mrl[t]}, mo));
+    mi = df_add(mi, df_mul(df{c.Mi[t], c.Mil[t]}, mo));
+  }
+  return {mr, mi};
+}
+
+// The two arms of spacecraft i (12, 13 | 21, 23 | 31, 32) at one sample, as
+// slow_sample_mix computes them, in double-float throughout, from the three
+// spacecraft's kdot_hp and the three arms' arm_hp.  tab: the sine/cosine table of
+// df_sincos_tab.
+__device__ __forceinline__ void slow_arms_hp(const ItemMix &c, const OrbitSampleMix &o, const df kd[3], const dc m[3],
+                                             const SlowArgs &K, const float4 *tab, int i, dc d[2]) {
+  const df k0 = {c.k[0], c.kl[0]}, k1 = {c.k[1], c.kl[1]};
   // this spacecraft's two arms as unique arms (0: 12, 1: 13, 2: 23) with the
   // orientation signs of k.r: 12 +0, 13 +1 | 21 -0, 23 +2 | 31 -1, 32 -2
   const int ua[2] = {i == 2 ? 1 : 0, i == 0 ? 1 : 2};
   const bool neg[2] = {i != 0, i == 2};
-  const int ends[3][2] = {{0, 1}, {0, 2}, {1, 2}};
   const df psi0 = carrier_phase_mix(c, o);
   const df u = {o.u_hi, o.u_lo}, ca = {o.ca_hi, o.ca_lo}, sa = {o.sa_hi, o.sa_lo};
   const df tgc = df_mul(K.AUcd, df_add(df_mul(k0, ca), df_mul(k1, sa)));  // guiding-centre delay (s)
@@ -65,21 +76,13 @@ __device__ __forceinline__ void slow_arms_hp(const ItemMix &c, const OrbitSample
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const int a = ua[q];
-    df kr = df_mul(df_add(kd[ends[a][1]], df_neg(kd[ends[a][0]])), K.invLd);
+    df kr = df_mul(df_add(kd[a == 0 ? 1 : 2], df_neg(kd[a == 2 ? 1 : 0])), K.invLd);
     if (neg[q]) kr = df_neg(kr);
-    // r^T M r with M = m (DP e+ + DC ex) as hi + lo
-    df mr = {0.f, 0.f}, mi = {0.f, 0.f};
-#pragma unroll
-    for (int t = 0; t < 6; t++) {
-      const df mo = {gm.f[9 + 6 * a + t], gl.f[9 + 6 * a + t]};
-      mr = df_add(mr, df_mul(df{c.Mr[t], c.Mrl[t]}, mo));
-      mi = df_add(mi, df_mul(df{c.Mi[t], c.Mil[t]}, mo));
-    }
     const df h1 = df_add(df{1.f, 0.f}, kr);
     const df arg1 = df_mul(df{0.5f * fon.hi, 0.5f * fon.lo}, h1);
     const df sc = df_sinc(arg1, tab);
     const df sinc = {0.25f * sc.hi, 0.25f * sc.lo};
-    const df t1r = df_mul(aev, mr), t1i = df_mul(aev, mi);
+    const df t1r = df_mul(aev, m[a].re), t1i = df_mul(aev, m[a].im);
     df s2, c2;
     df_sincos_tab(df_add(arg1, df_neg(arg2)), tab, &s2, &c2);
     const df re = df_add(df_mul(t1r, c2), df_mul(t1i, s2));
@@ -89,8 +92,9 @@ __device__ __forceinline__ void slow_arms_hp(const ItemMix &c, const OrbitSample
 }
 
 // One CTA of three warps per 32 consecutive samples of one binned proposal,
-// grid-stride over all of them: warp i computes the arms of spacecraft i (a
-// third of the dependent chain of a sample each, on separate SM
+// grid-stride over all of them: warp i computes k.x of spacecraft i and the
+// antenna pattern of arm i, shared with the other two, then the arms of
+// spacecraft i (a third of the dependent chain of a sample each, on separate SM
 // sub-partitions); warps 0 and 1 then form the A and E arm combinations of
 // ae_combos in double-float.
 // sin(k pi / 32), cos(k pi / 32) as hi + lo floats {s.hi, s.lo, c.hi, c.lo},
@@ -98,10 +102,9 @@ __device__ __forceinline__ void slow_arms_hp(const ItemMix &c, const OrbitSample
 static __device__ float4 g_hp_sincos[64];
 
 __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
-  __shared__ dc s_d[6][32];
+  __shared__ dc s_d[6][32], s_m[3][32];
+  __shared__ float2 s_kd[3][32];
   __shared__ float4 s_tab[64];
-  if (threadIdx.x < 64) s_tab[threadIdx.x] = g_hp_sincos[threadIdx.x];
-  __syncthreads();
   int cs[kNumBins + 1];
   int acc = 0;
 #pragma unroll
@@ -110,6 +113,9 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
     if ((32 << b) <= a.NFFT) acc += a.bin_count[b] << b;
   }
   cs[kNumBins] = acc;
+  if ((int)blockIdx.x >= acc) return;
+  if (threadIdx.x < 64) s_tab[threadIdx.x] = g_hp_sincos[threadIdx.x];
+  __syncthreads();
   const int lane = threadIdx.x & 31, sc = threadIdx.x >> 5;
   float4 *series = reinterpret_cast<float4 *>(a.series);
 #pragma unroll 1
@@ -134,8 +140,22 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
     if (!iok) item = 0;
     const long long o0 = ((long long)cb * 32 + (long long)slot * N) * 4 + n;
     const bool wok = lok && iok && chk(o0 >= 0 && o0 + 3LL * N < a.series_len, kChkSeriesWrite);
+    const ItemMix &c = a.itemsmix[item];
+    const GeoSampleMix &gm = a.geo[b][n], &gl = a.geolo[b][n];
+    const df kx = kdot_hp(c, gm, gl, sc);
+    s_kd[sc][lane] = make_float2(kx.hi, kx.lo);
+    s_m[sc][lane] = arm_hp(c, gm, gl, sc);
+    __syncthreads();
+    df kd[3];
+    dc m[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const float2 v = s_kd[q][lane];
+      kd[q] = {v.x, v.y};
+      m[q] = s_m[q][lane];
+    }
     dc d2[2];
-    slow_arms_hp(a.itemsmix[item], a.mix[b][n], a.geo[b][n], a.geolo[b][n], a, s_tab, sc, d2);
+    slow_arms_hp(c, a.mix[b][n], kd, m, a, s_tab, sc, d2);
     s_d[2 * sc][lane] = d2[0];
     s_d[2 * sc + 1][lane] = d2[1];
     __syncthreads();
@@ -162,8 +182,9 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
 }
 
 // ------------------------------------------------------- spectral stage, df
-// The proposal of entry k (in size order): item, size, segment, placement,
-// size bin and series offset (float4 elements).
+// The proposal of entry k (largest sizes first, so that the long ones start
+// early): item, size, segment, placement, size bin and series offset (float4
+// elements).  cs[b]: the first entry of size bin b.
 struct HpEntry {
   int item, N, seg, imin, bin;
   long long off;
@@ -172,9 +193,9 @@ struct HpEntry {
 };
 
 __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *cs) {
-  int bin = 0;
+  int bin = kNumBins - 1;
 #pragma unroll
-  for (int b = 1; b < kNumBins; b++)
+  for (int b = kNumBins - 2; b >= 0; b--)
     if (k >= cs[b]) bin = b;
   const int slot = k - cs[bin];
   HpEntry e;
@@ -199,74 +220,89 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
   return e;
 }
 
+// Latency-bound: a batch lists tens of proposals, each a chain of dependent loads,
+// five or six FFT stages and cluster barriers, so what matters is that all of
+// them are resident at once and that the chain is short.  In place and with the
+// twiddles in L1 a CTA takes 16 bytes per point (64 KB at N = 4096, where
+// ping-pong buffers and a twiddle copy took 192 KB and left one CTA per SM); the
+// bank's entries of a thread's first bins are loaded before the transform.  61
+// proposals of up to 1024 points 19.1 -> 16.7 us, 73 of up to 2048 on 8192-bin
+// segments 60.8 -> 42.2 us.
 template <bool PERCH>
-__global__ void __launch_bounds__(kHpThreads) fd_hp_kernel(HpArgs a) {
+__global__ void __launch_bounds__(kHpThreads, 3) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 red[32];
-  __shared__ float4 s_part;  // this CTA's {rr hi, rr lo, hw hi, hw lo}
-  const int NM = a.nmax, NFFT = a.NFFT;
-  dc *xb = reinterpret_cast<dc *>(smem_raw), *yb = xb + NM;
-  float4 *tws = reinterpret_cast<float4 *>(yb + NM);
+  __shared__ float4 s_part[2];  // this CTA's {rr hi, rr lo, hw hi, hw lo}, by turns
+  const int NFFT = a.NFFT;
+  dc *S = reinterpret_cast<dc *>(smem_raw);
   const int r = (int)cluster.block_rank(), ch = r >> 1;
   const int ncl = (int)(gridDim.x >> 2);
-  int cs[kNumBins + 1];
+  int cs[kNumBins];
   int total = 0;
 #pragma unroll
-  for (int b = 0; b < kNumBins; b++) {
+  for (int b = kNumBins - 1; b >= 0; b--) {
     cs[b] = total;
     if ((32 << b) <= NFFT) total += a.bin_count[b];
   }
-  cs[kNumBins] = total;
-  int cur = -1;
-  for (int k = (int)(blockIdx.x >> 2); k < total; k += ncl) {
+  if (total == 0) return;  // nothing listed: the counters are zero already
+  int turn = 0;
+  for (int k = (int)(blockIdx.x >> 2); k < total; k += ncl, turn ^= 1) {
     const HpEntry e = hp_entry(a, k, cs);
-    const int N = e.N;
-    if (e.bin != cur) {
-      const float4 *tw = a.tw32x[e.bin];
-      for (int n = threadIdx.x; n < N; n += blockDim.x) tws[n] = tw[n];
-      cur = e.bin;
-    }
+    const int N = e.N, ln = e.bin + 5;
     const float4 *src = a.series + e.off + (long long)r * N;
-    for (int n = threadIdx.x; n < N; n += blockDim.x) xb[n] = dc_from(src[n]);
+    for (int n = threadIdx.x; n < N; n += blockDim.x) S[hp_at(hp_rev(n, ln))] = dc_from(src[n]);
+    // the bank's entries of bin q of this CTA's half
+    const int half = N >> 1, q0 = (r & 1) * half;
+    struct Bin {
+      float4 gh, gl, wh, wl;
+    };
+    auto load_bin = [&](int q, Bin &t) {
+      const int j = e.imin + ((q + half) & (N - 1));  // fftshift
+      if (q >= q0 + half || j < 0 || j >= NFFT) return false;
+      const size_t sj = (size_t)e.seg * NFFT + j;
+      t = {a.g32[2 * sj + ch], a.g32lo[2 * sj + ch], a.w32[sj], a.w32lo[sj]};
+      return true;
+    };
+    Bin first;
+    const bool has_first = load_bin(q0 + (int)threadIdx.x, first);
     __syncthreads();
-    dc *S = hp_fft(xb, yb, N, tws);
+    hp_fft(S, ln, a.tw32x[e.bin]);
     cluster.sync();  // every spectrum of the proposal is complete
     const dc *Sp = cluster.map_shared_rank(S, (unsigned)(r ^ 1));
     const dc *S0 = (r & 1) ? Sp : S, *S1 = (r & 1) ? S : Sp;  // the channel's series 2c, 2c + 1
     df rr = {0.f, 0.f}, hw = {0.f, 0.f};
-    const int half = N >> 1, q0 = (r & 1) * half;
     for (int q = q0 + threadIdx.x; q < q0 + half; q += blockDim.x) {
-      const int j = e.imin + ((q + half) & (N - 1));  // fftshift
-      if (j < 0 || j >= NFFT) continue;
-      const size_t sj = (size_t)e.seg * NFFT + j;
-      const float4 gh = a.g32[2 * sj + ch], gl = a.g32lo[2 * sj + ch];
-      dc h = dc_add(dc_mul(S0[q], dc_from(make_float2(gh.x, gh.y), make_float2(gl.x, gl.y))),
-                    dc_mul(S1[q], dc_from(make_float2(gh.z, gh.w), make_float2(gl.z, gl.w))));
+      Bin t = first;
+      if (!(q == q0 + (int)threadIdx.x ? has_first : load_bin(q, t))) continue;
+      const int qs = hp_at(q);
+      dc h = dc_add(dc_mul(S0[qs], dc_from(make_float2(t.gh.x, t.gh.y), make_float2(t.gl.x, t.gl.y))),
+                    dc_mul(S1[qs], dc_from(make_float2(t.gh.z, t.gh.w), make_float2(t.gl.z, t.gl.w))));
       h = dc_scale2(h, e.amp_p2);
-      const float4 wh = a.w32[sj], wl = a.w32lo[sj];
-      const dc w = ch == 0 ? dc_from(make_float2(wh.x, wh.y), make_float2(wl.x, wl.y))
-                           : dc_from(make_float2(wh.z, wh.w), make_float2(wl.z, wl.w));
+      const dc w = ch == 0 ? dc_from(make_float2(t.wh.x, t.wh.y), make_float2(t.wl.x, t.wl.y))
+                           : dc_from(make_float2(t.wh.z, t.wh.w), make_float2(t.wl.z, t.wl.w));
       rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
       hw = df_add(hw, df_sq_sum(h));
     }
     rr = hp_block_sum(rr, red);
     hw = hp_block_sum(hw, red);
-    if (threadIdx.x == 0) s_part = make_float4(rr.hi, rr.lo, hw.hi, hw.lo);
+    if (threadIdx.x == 0) s_part[turn] = make_float4(rr.hi, rr.lo, hw.hi, hw.lo);
     cluster.sync();  // partial sums are published; the partner is done with S
     if (r == 0 && threadIdx.x == 0 && e.ok) {
       df s[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
       for (int q = 0; q < 4; q++) {
-        const float4 o = *cluster.map_shared_rank(&s_part, (unsigned)q);
+        const float4 o = *cluster.map_shared_rank(&s_part[turn], (unsigned)q);
         s[q >> 1] = df_add(s[q >> 1], df{o.x, o.y});
         s[2] = df_add(s[2], df{o.z, o.w});
       }
       hp_write(e.item, N, e.seg, e.imin, NFFT, s, a.Q, a.QA, PERCH, a.term_x, a.dlogl, a.term_y, a.hh, a.term_ch,
                a.status);
     }
-    cluster.sync();  // s_part is read before the next proposal overwrites it
+    // the next proposal's sums go to the other s_part, the one after it follows
+    // two more cluster barriers
   }
+  cluster.sync();  // no CTA leaves while CTA 0 may be reading its s_part
   // the last CTA leaves the counters it was given at zero
   if (threadIdx.x == 0) {
     __threadfence();
@@ -277,7 +313,7 @@ __global__ void __launch_bounds__(kHpThreads) fd_hp_kernel(HpArgs a) {
   }
 }
 
-static size_t hp_smem_bytes(int nmax) { return (size_t)nmax * (2 * sizeof(dc) + sizeof(float4)); }
+static size_t hp_smem_bytes(int nmax) { return (size_t)nmax * sizeof(dc); }
 
 template <bool PERCH>
 static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) {

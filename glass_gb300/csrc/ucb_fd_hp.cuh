@@ -1,5 +1,5 @@
 // Double-float (pairs of floats) arithmetic: complex operations, division,
-// sine, cosine and sinc, the CTA-wide Stockham FFT and reduction, and the
+// sine, cosine and sinc, the CTA-wide FFT and reduction, and the
 // result write of the double-float re-evaluation of mixed proposals
 // (ucb_fd_hp.cu).
 #pragma once
@@ -124,50 +124,60 @@ __device__ __forceinline__ df df_sinc(df x, const float4 *tab) {
   return df_div(s, x);
 }
 
-// Stockham FFT of one series of N double-floats by the CTA, ping-ponging
-// between x and y: radix-4 stages (sub-transform size p: butterfly i < N/4,
-// k = i mod p, reads x[i + m N/4], m = 0..3, times exp(-2 pi i m k / (4p)),
-// writes y[(i - k) 4 + k + m p]) and a final radix-2 stage when log2 N is
-// odd.  tw[j] = exp(-2 pi i j / N) as hi + lo floats.  Returns the buffer
-// holding the result.
-__device__ __forceinline__ dc *hp_fft(dc *x, dc *y, int N, const float4 *tw) {
-  int p = 1;
-  for (; 4 * p <= N; p <<= 2) {
-    const int step = N / (4 * p), q = N / 4;
-    for (int i = threadIdx.x; i < q; i += blockDim.x) {
-      const int k = i & (p - 1);
-      dc u0 = x[i], u1 = x[i + q], u2 = x[i + 2 * q], u3 = x[i + 3 * q];
-      if (p > 1) {
+// In-place FFT of one series of N = 2^ln double-floats by the CTA: decimation in
+// time from digit-reversed order (element n at hp_at(hp_rev(n, ln))), radix-4
+// stages (sub-transform size p: butterfly i < N/4, k = i mod p, on x[4 (i - k) + k
+// + m p] times exp(-2 pi i m k / (4p)), m = 0..3) and a final radix-2 stage when
+// log2 N is odd; results in natural order at hp_at.  tw[j] = exp(-2 pi i j / N) as
+// hi + lo floats, read from global memory (L1 after the first touch): 16 bytes of
+// shared memory per point.
+//
+// hp_at: a 16-byte access serves 8 lanes at a time, one per 16-byte column; the
+// permutation within each run of 8 elements puts the strides of the first stages
+// (4 and 16) and of the digit-reversed scatter on different columns.
+__device__ __forceinline__ int hp_at(int i) {
+  return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9) ^ ((i >> 2) & 4)) & 7);
+}
+// base-4 digits of n reversed; with ln odd the lowest bit becomes the highest
+// (the radix-2 stage's digit)
+__device__ __forceinline__ int hp_rev(int n, int ln) {
+  const int top = (ln & 1) ? (n & 1) << (ln - 1) : 0;
+  const int l4 = ln & ~1, m = (ln & 1) ? n >> 1 : n;
+  const unsigned r = __brev((unsigned)m) >> (32 - l4);
+  return top + (int)(((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u));
+}
+__device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__ tw) {
+  const int N = 1 << ln;
+  int lp = 0;
+  for (; lp + 2 <= ln; lp += 2) {
+    const int p = 1 << lp, step = N >> (lp + 2);
+    for (int i = threadIdx.x; i < N / 4; i += blockDim.x) {
+      const int k = i & (p - 1), j = ((i - k) << 2) + k;
+      dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + p), *const x2 = x + hp_at(j + 2 * p),
+               *const x3 = x + hp_at(j + 3 * p);
+      dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
+      if (lp > 0) {
         u1 = dc_mul(u1, dc_from(tw[k * step]));
         u2 = dc_mul(u2, dc_from(tw[2 * k * step]));
         u3 = dc_mul(u3, dc_from(tw[3 * k * step]));
       }
       const dc a = dc_add(u0, u2), b = dc_sub(u0, u2), c = dc_add(u1, u3), d = dc_mi(dc_sub(u1, u3));
-      const int j = (i - k) * 4 + k;
-      y[j] = dc_add(a, c);
-      y[j + p] = dc_add(b, d);
-      y[j + 2 * p] = dc_sub(a, c);
-      y[j + 3 * p] = dc_sub(b, d);
+      *x0 = dc_add(a, c);
+      *x1 = dc_add(b, d);
+      *x2 = dc_sub(a, c);
+      *x3 = dc_sub(b, d);
     }
     __syncthreads();
-    dc *t = x;
-    x = y;
-    y = t;
   }
-  if (p < N) {  // log2 N odd: one radix-2 stage, p = N/2
-    for (int i = threadIdx.x; i < N / 2; i += blockDim.x) {
-      const int k = i & (p - 1);
-      const dc a = x[i], b = dc_mul(x[i + N / 2], dc_from(tw[k]));
-      const int j = (i - k) * 2 + k;
-      y[j] = dc_add(a, b);
-      y[j + p] = dc_sub(a, b);
+  if (lp < ln) {  // log2 N odd: one radix-2 stage, p = N/2
+    for (int k = threadIdx.x; k < N / 2; k += blockDim.x) {
+      dc *const x0 = x + hp_at(k), *const x1 = x + hp_at(k + N / 2);
+      const dc a = *x0, b = dc_mul(*x1, dc_from(tw[k]));
+      *x0 = dc_add(a, b);
+      *x1 = dc_sub(a, b);
     }
     __syncthreads();
-    dc *t = x;
-    x = y;
-    y = t;
   }
-  return x;
 }
 
 // Sum over the CTA of a double-float per thread (valid in thread 0).
