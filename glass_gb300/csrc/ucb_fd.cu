@@ -10,7 +10,7 @@
 //
 // Here a batch of proposals of mixed sizes N (32..4096) is evaluated in three
 // steps on one stream:
-//   1. plan (one thread per proposal, FP64): the reference's bandwidth rule
+//   1. plan (FP64, spread over warps): the reference's bandwidth rule
 //      gives N, the alignment gives the template's first segment bin, and the
 //      per-proposal constants are prepared; proposals are binned by N;
 //   2. slow part (one thread per (proposal, sample), all sizes in one launch):
@@ -40,225 +40,357 @@ cudaError_t fd_launch_spec_fp64(int N, const SpecArgs &a, int nitems, int num_sm
 cudaError_t fd_launch_spec_all_mixed(const SpecAllArgs &A, int num_sms, cudaStream_t stream, bool perch, int cap);
 cudaError_t fd_launch_spec_all_fp64(const SpecAllArgs &A, int num_sms, cudaStream_t stream, bool perch);
 
-// ------------------------------------------------------------- plan kernels
-// Plain-FP64 plan: ucb_bandwidth, ucb_alignment and the per-proposal constants
-// entirely in FP64, one thread per proposal.
-__global__ void __launch_bounds__(64) fd_plan64_kernel(PlanArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int b = -1;
-  if (i < a.nitems) {
-    double p[8];
-    int seg;
-    int st = plan_validate(a, i, p, seg);
-    const double T = a.T, f0 = p[0] / T;
-    int N = 0;
-    if (!st) {
-      N = a.n_fixed > 0 ? a.n_fixed : 2 * bandwidth_dev(a.L, a.fstar, f0, p[7] / (T * T), p[1], exp(p[3]), T, a.NFFT);
-      if (N < kMinN || N > kMaxN) st |= 1;
+// ------------------------------------------------------------- plan kernel
+// The two spreads of the bandwidth rule (ucb/src/glass_ucb_waveform.c:708-722, with
+// AEnoise, utils/src/glass_lisa.c:1188-1198) in FP64, evaluated with one sincos and
+// products: sin(acos(c)) as sqrt((1 - c)(1 + c)), x^10 as ((x^2)^2)^2 x^2, cos 2x as
+// 2 cos^2 x - 1.  These agree with the library forms to a few ulp, so N can
+// differ from the reference's only for a spread within ~1e-15 of a power of
+// two (where the reference's own result depends on its libm).
+__device__ __noinline__ int doppler_spread_fp64(double T, double f0, double fdot, double costheta) {
+  const double sintheta = sqrt((1.0 - costheta) * (1.0 + costheta));
+  return pow2_above_dev(2 * T * ((4. + kPI2 * f0 * (kAU / kCLIGHT) * sintheta) * (1.0 / kYEAR) + fabs(fdot) * T) - 1);
+}
+__device__ __noinline__ int snr_spread_fp64(const PlanArgs &a, double f0, double lnA) {
+  double sf, cf;
+  sincos_tab(div_by(f0, a.fstar, a.invfstar), a.tw1024, &sf, &cf);
+  const double rf = rcp_fast(f0), r = 1.0e-4 * rf, q = 2.0e-5 * rf, q2 = q * q, q4 = q2 * q2;
+  const double red = 1. + 16.0 * (q4 * q4 * q2 + r * r);
+  const double rw = rf * (1.0 / kPI2), rw2 = rw * rw;
+  const double c2x = 2.0 * cf * cf - 1.0;
+  const double sn4L2 = (16.0 / 3.0) * sf * sf *
+                       ((2.0 + cf) * (kSPS + kSLOC) + 2.0 * (3.0 + 2.0 * cf + c2x) * (kSLOC / 2.0 + kSACC * (rw2 * rw2) * red));
+  return pow2_above_dev(exp(lnA) * sqrt(a.T) * sf * (2.0 * a.L) / sqrt(sn4L2) - 1);
+}
+
+// The interval of (int)pow(2, (int)log2(v) + 1), within [Nmin, Nmax], for an FP32
+// estimate v good to 2e-5.
+__device__ __forceinline__ void pow2_above_f32(float v, int Nmin, int Nmax, int &lo, int &hi) {
+  lo = Nmin;
+  hi = Nmax;
+  if (isnan(v)) return;
+  const float v0 = v * 0.99998f, v1 = v * 1.00002f;
+  // the binary exponent of a v >= 1, plus 1 (at most 30 below infinity's)
+  const int e0 = min((__float_as_int(v0) >> 23) - 126, 30), e1 = min((__float_as_int(v1) >> 23) - 126, 30);
+  lo = max(min(v0 >= 1.f ? 1 << e0 : 1, Nmax), Nmin);
+  hi = max(min(v1 >= 1.f ? 1 << e1 : 1, Nmax), Nmin);
+}
+
+// The bandwidth rule of ucb/src/glass_ucb_waveform.c:698-725: N is always the
+// reference's.  FP32 estimates of the two spreads, good to 1e-5 over the range of
+// the test below (ln A rounded: 4e-6; the sine and cosine of f/f* <= 10: 2e-6); a
+// spread is evaluated in FP64 only where its estimate's interval leaves N open (or
+// the estimate overflows, or the input is outside that range), which one proposal
+// in 20,000 does; that lane runs 100 FP64 instructions, while its CTA waits.
+__device__ __forceinline__ int plan_size(const PlanArgs &a, const double *p, double f0) {
+  const int Nmin = 16, half = a.NFFT / 2;
+  const int Nmax = half >= 1 ? (1 << (31 - __clz(half))) : 0;
+  const float Tf = to_f32(a.T), f0f = to_f32(f0), lnA = to_f32(p[3]), p7 = to_f32(p[7]);
+  int D0 = Nmin, D1 = Nmax, S0 = Nmin, S1 = Nmax;
+  if (f0f > 1e-6f && f0f < 0.2f && fabsf(lnA) < 80.f && fabsf(p7) < 1e30f) {
+    // 1 - cos^2 in FP64, as it cancels at the poles
+    const float sinthf = sqrtf(fmaxf(0.f, to_f32(fma(-p[1], p[1], 1.0))));
+    const float bw = 2.f * Tf * (4.f + 6.2831853f * f0f * (float)(kAU / kCLIGHT) * sinthf) * (float)(1.0 / kYEAR) +
+                     2.f * fabsf(p7);
+    pow2_above_f32(bw - 1.f, Nmin, Nmax, D0, D1);
+    // AEnoise times (2L)^2 (AEnoise itself, ~1e-42, is below FP32's normal range)
+    float sx, cx;
+    sincosf(f0f * to_f32(a.invfstar), &sx, &cx);
+    const float c2x = 2.f * cx * cx - 1.f, rf = 1.f / f0f;
+    const float rw = rf * 0.15915494f, rw2 = rw * rw;
+    const float q1 = 2.0e-5f * rf, q2 = q1 * q1, q4 = q2 * q2, r1 = 1.0e-4f * rf;
+    const float red = 1.f + 16.f * (q4 * q4 * q2 + r1 * r1);
+    const float sn4L2 = (16.f / 3.f) * sx * sx *
+                        ((2.f + cx) * (float)(kSPS + kSLOC) +
+                         2.f * (3.f + 2.f * cx + c2x) * ((float)(kSLOC / 2.0) + (float)kSACC * (rw2 * rw2) * red));
+    // (at a zero of the sine its sign, and so the rule's outcome, is FP64's)
+    if (fabsf(sx) > 1e-3f)
+      pow2_above_f32(expf(lnA) * sqrtf(Tf) * sx * (2.f * to_f32(a.L)) * rsqrtf(sn4L2) - 1.f, Nmin, Nmax, S0, S1);
+  }
+  if (max(D0, S0) != max(D1, S1) && D0 != D1) {
+    D0 = doppler_spread_fp64(a.T, f0, div_by(p[7], a.T2, a.invT2), p[1]);
+    D0 = D1 = max(min(D0, Nmax), Nmin);
+  }
+  if (max(D0, S0) != max(D1, S1)) {
+    S0 = snr_spread_fp64(a, f0, p[3]);
+    S0 = max(min(S0, Nmax), Nmin);
+  }
+  return 2 * max(D0, S0);
+}
+
+// Warp-aggregated binning: one atomic per distinct size per warp, begun by
+// bin_begin, which returns its result to the group's first lane, and the list
+// entries written by bin_end (so that the atomic's round trip passes behind other
+// work).
+struct BinSlot {
+  unsigned same;
+  int base;
+};
+__device__ __forceinline__ BinSlot bin_begin(const PlanArgs &a, int b) {
+  BinSlot s = {__match_any_sync(0xffffffffu, b), 0};
+  if (b >= 0 && (int)(threadIdx.x & 31) == __ffs(s.same) - 1) s.base = atomicAdd(&a.bin_count[b], __popc(s.same));
+  return s;
+}
+__device__ __forceinline__ void bin_end(const PlanArgs &a, const BinSlot &s, int i, int b) {
+  const int lane = threadIdx.x & 31, base = __shfl_sync(0xffffffffu, s.base, __ffs(s.same) - 1);
+  const int slot = base + __popc(s.same & ((1u << lane) - 1));
+  if (b >= 0 && chk(slot < a.cap && b < kNumBins, kChkBinList)) a.bin_list[(size_t)b * a.cap + slot] = i;
+}
+
+// u (component r of the sky basis vector along theta) and v (along phi).
+__device__ __forceinline__ double sky_u(int r, double cth, double sth, double sph, double cph) {
+  return r == 2 ? -sth : cth * (r == 0 ? cph : sph);
+}
+__device__ __forceinline__ double sky_v(int r, double sph, double cph) { return r == 2 ? 0.0 : (r == 0 ? sph : -cph); }
+
+// Plan: size and placement of each proposal's template, its constants in the
+// record of the path that follows, and its entry in its size's list.
+//
+// Latency-bound on FP64: an FP64 instruction, or a conversion to or from FP64,
+// occupies a sub-partition for 64 clocks whatever the number of active lanes and
+// of independent ones behind it, so the time is that of the warp with the most
+// of them.  The work of P proposals is therefore spread over the four warps of
+// a CTA (first part: warp 0 the sines and carrier constants, phi and 2 psi side
+// by side in one warp's lanes; warp 1 size and placement, in FP32 up to the rule's
+// boundaries; warp 2 amplitude and sine of theta; warp 3 the frequency constants)
+// and, after a barrier, over all threads (second part: a tensor element each);
+// quotients come from reciprocals of the batch's constants (correctly rounded),
+// sines from the table, hi + lo floats and powers of two by integer arithmetic.
+// P = ceil(n / SMs), 16 .. 32, keeps a batch of a few thousand on one wave.
+// One proposal in FP64 23.6 -> 8.6 us, 3072 mixed 14.9 -> 10.4 us, 4096 for gradients
+// 30 -> 14.2 us.
+template <PlanKind KIND>
+__global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
+  __shared__ double2 s_sc[2][32];  // sine, cosine of phi and of 2 psi
+  __shared__ double s_sth[32], s_amp[32], s_cthsth[32];
+  __shared__ int s_st[32], s_N[32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, P = a.per_cta;
+  const int i0 = blockIdx.x * P, n = min(P, a.nitems - i0);
+  const int i = i0 + l;
+  const double *p = a.params + 8 * (size_t)i;
+  ItemMix *const m = KIND == kPlanGrad ? &a.itemsgrad[l < n ? i : i0].m : a.itemsmix + (l < n ? i : i0);
+  ItemF64 *const c64 = a.items64 + (l < n ? i : i0);
+  if (w == 0) {
+    for (int q = l; q < 2 * n; q += 32) {
+      const int t = q >= n, j = t ? q - n : q;
+      const double *pj = a.params + 8 * (size_t)(i0 + j);
+      const double x = t ? 2. * pj[5] : pj[2];
+      double s, c;
+      sincos_tab(x, a.tw1024, &s, &c);
+      s_sc[t][j] = make_double2(s, c);
     }
-    int imin = 0;
-    if (!st) {
-      imin = (int)((long long)(f0 * T) - N / 2) - a.seg_qmin[seg];
-      if (imin >= a.NFFT || imin + N <= 0) st = 4;
+    if (l < n) {
+      const double f0 = div_by(p[0], a.T, a.invT), fT = f0 * a.T;
+      const double q = trunc_i64(fT);
+      if (KIND == kPlanF64) {
+        c64->f0 = f0;
+        c64->dfq = kPI2 * div_by(q, a.T, a.invT);
+        c64->phi0 = p[6];
+      } else {
+        split_f32(kPI2 * (fT - q), m->eps2pi.hi, m->eps2pi.lo);
+        split_f32(p[6], m->phi0.hi, m->phi0.lo);
+      }
     }
-    if (st) {
-      plan_write_skipped(a, i, st);
+  } else if (w == 1) {
+    if (l < n) {
+      double v[8];
+      int st = 0;
+      const int seg = a.item_seg[i];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        v[k] = p[k];
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v[k]) << 1;  // |v|
+        if (b >= 0x7ffull << 53) st = 1;                                                   // infinite or NaN
+        if ((k == 1 || k == 4) && b > 0x3ffull << 53) st = 1;                              // |cosine| > 1
+      }
+      if (seg < 0 || seg >= a.nseg) st |= 2;
+      int N = 0, imin = 0;
+      if (!st) {
+        const double f0 = div_by(v[0], a.T, a.invT);
+        N = a.n_fixed > 0 ? a.n_fixed : plan_size(a, v, f0);
+        if (N < kMinN || N > kMaxN) {
+          st = 1;
+        } else {
+          imin = (int)((long long)(f0 * a.T) - N / 2) - a.seg_qmin[seg];
+          if (imin >= a.NFFT || imin + N <= 0) st = 4;
+        }
+      }
+      s_st[l] = st;
+      s_N[l] = N;
+      const int4 head = make_int4(seg, N, imin, 0);
+      if (st)
+        plan_write_skipped(a, i, st);
+      else if (KIND == kPlanF64)
+        c64->seg = head.x, c64->N = head.y, c64->imin = head.z, c64->pad = 0;
+      else
+        m->seg = head.x, m->N = head.y, m->imin = head.z, m->pad = 0;
+    }
+  } else if (w == 2) {
+    if (l < n) {
+      s_amp[l] = exp(p[3]);
+      const double cth = p[1], sth = sqrt(fma(-cth, cth, 1.0));
+      s_sth[l] = sth;
+      if (KIND == kPlanGrad) s_cthsth[l] = cth / (sth < 1e-9 ? 1e-9 : sth);  // d/dcos(theta) is singular at the poles
+    }
+  } else if (l < n) {
+    const double f0 = div_by(p[0], a.T, a.invT);
+    if (KIND == kPlanF64) {
+      const double fdot = div_by(p[7], a.T2, a.invT2);
+      c64->w0 = kPI2 * f0;
+      c64->wd = kPI * fdot;
+      c64->ae = 0.66666666666666666666 * fdot / f0;
+      c64->h0 = div_by(0.5 * f0, a.fstar, a.invfstar);
+      c64->hd = div_by(0.5 * fdot, a.fstar, a.invfstar);
     } else {
-      SourceGeom g;
-      source_geometry(p, 8, T, g);
-      ItemF64 c;
-      make_item_f64(g, N, a.fstar, c);
-      c.seg = seg;
-      c.N = N;
-      c.imin = imin;
-      c.pad = 0;
-      a.items64[i] = c;
-      b = fd_bin_of(N);
+      const double fdotT = div_by(p[7], a.T, a.invT);
+      split_f32(div_by(f0, a.fstar, a.invfstar), m->fonfs0, m->fonfs0l);
+      split_f32(div_by(fdotT, a.fstar, a.invfstar), m->fdfs, m->fdfsl);
+      split_f32(0.66666666666666666666 * fdotT / f0, m->aef, m->aefl);
+      split_f32(div_by(kPI2 * f0, kCLIGHT, a.invc), m->w0c, m->w0cl);
+      split_f32(kPI * p[7], m->p7pi_d.hi, m->p7pi_d.lo);
+      m->p7pi = m->p7pi_d.hi;
+      if (KIND == kPlanGrad) {
+        ItemGrad &g = a.itemsgrad[i];
+        g.f0 = to_f32(f0);
+        g.fdot = to_f32(div_by(p[7], a.T2, a.invT2));
+        g.invT = to_f32(a.invT);
+        g.fstar = to_f32(a.fstar);
+      }
     }
   }
-  plan_bin(a, i, b);
+  __syncthreads();
+  const int bin = w == 1 && l < n && s_st[l] == 0 ? fd_bin_of(s_N[l]) : -1;
+  BinSlot slot = {0, 0};
+  if (w == 1) slot = bin_begin(a, bin);
+  for (int q = threadIdx.x; q < (KIND == kPlanF64 ? 2 : 8) * n; q += 128) {
+    const int role = q / n, j = q - role * n;
+    if (s_st[j]) continue;
+    const double *pj = a.params + 8 * (size_t)(i0 + j);
+    const double cth = pj[1], ci = pj[4], sth = s_sth[j];
+    const double sph = s_sc[0][j].x, cph = s_sc[0][j].y, s2 = s_sc[1][j].x, c2 = s_sc[1][j].y;
+    const double amp = scale_pow2(s_amp[j], -(32 - __clz(s_N[j])));  // amp / (2N), N a power of two
+    if (KIND == kPlanF64) {
+      ItemF64 &c = a.items64[i0 + j];
+      if (role == 0) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+          c.u[r] = sky_u(r, cth, sth, sph, cph);
+          c.v[r] = sky_v(r, sph, cph);
+        }
+        c.k[0] = -sth * cph;
+        c.k[1] = -sth * sph;
+        c.k[2] = -cth;
+      } else {
+        const double Ap = (1. + ci * ci) * 0.5;
+        c.DPr = Ap * c2;
+        c.DPi = ci * s2;
+        c.DC2r = 2.0 * (-Ap * s2);
+        c.DC2i = 2.0 * (ci * c2);
+        c.amp_s = amp;
+      }
+      continue;
+    }
+    ItemGrad *const g = KIND == kPlanGrad ? a.itemsgrad + i0 + j : nullptr;
+    ItemMix &c = KIND == kPlanGrad ? g->m : a.itemsmix[i0 + j];
+    const double Ap = (1. + ci * ci) * 0.5;
+    if (role < 6) {
+      // tensor element (r, s) of xx, xy, xz, yy, yz, zz.  amp/(2N) = msc 2^e, msc in
+      // [1, 2): the power of two scales the template exactly in the likelihood
+      // kernels, msc goes into the antenna tensors
+      const int r = role < 3 ? 0 : (role < 5 ? 1 : 2), s = role < 3 ? role : (role < 5 ? role - 2 : 2);
+      double ur = sky_u(r, cth, sth, sph, cph), us = sky_u(s, cth, sth, sph, cph);
+      const double vr = sky_v(r, sph, cph), vs = sky_v(s, sph, cph);
+      double ep = vr * vs - ur * us, ec = ur * vs + vr * us;
+      int ex = ((__double2hiint(amp) >> 20) & 0x7ff) - 1023;
+      if (ex <= -1023 || ex > 1023) ex = ilogb(amp);
+      const double msc = scale_pow2(amp, -ex);
+      split_f32(msc * (Ap * c2 * ep + -Ap * s2 * ec), c.Mr[role], c.Mrl[role]);
+      split_f32(msc * (ci * s2 * ep + ci * c2 * ec), c.Mi[role], c.Mil[role]);
+      if (role == 0) {
+        c.amp_p2 = to_f32(scale_pow2(1.0, ex));
+        split_f32(amp, c.amp_hi, c.amp_lo);
+      }
+      if (KIND == kPlanGrad) {
+        // the tensors and their derivatives by cos(theta) and phi, at least 1e-9
+        // from the poles
+        if (sth < 1e-9) {
+          ur = sky_u(r, cth, 1e-9, sph, cph);
+          us = sky_u(s, cth, 1e-9, sph, cph);
+          ep = vr * vs - ur * us;
+          ec = ur * vs + vr * us;
+        }
+        const double uc[3] = {cph, sph, s_cthsth[j]};
+        const double ucr = r == 0 ? uc[0] : (r == 1 ? uc[1] : uc[2]), ucs = s == 0 ? uc[0] : (s == 1 ? uc[1] : uc[2]);
+        const double upr = r == 2 ? 0.0 : cth * (r == 0 ? -sph : cph), ups = s == 2 ? 0.0 : cth * (s == 0 ? -sph : cph);
+        const double vpr = r == 2 ? 0.0 : (r == 0 ? cph : sph), vps = s == 2 ? 0.0 : (s == 0 ? cph : sph);
+        g->ep[role] = to_f32(ep);
+        g->ec[role] = to_f32(ec);
+        g->dep_c[role] = to_f32(-ucr * us - ur * ucs);
+        g->dec_c[role] = to_f32(ucr * vs + vr * ucs);
+        g->dep_p[role] = to_f32(vpr * vs + vr * vps - upr * us - ur * ups);
+        g->dec_p[role] = to_f32(upr * vs + ur * vps + vpr * us + vr * ups);
+      }
+    } else if (role == 6) {
+      const double kx = -sth * cph, ky = -sth * sph;
+      split_f32(kx, c.k[0], c.kl[0]);
+      split_f32(ky, c.k[1], c.kl[1]);
+      split_f32(-cth, c.k[2], c.kl[2]);
+      c.k[3] = 0.f;
+      const double bscale = kPI2 * div_by(pj[0], a.T, a.invT) * (kAU / kCLIGHT);
+      split_f32(bscale * kx, c.beta1.hi, c.beta1.lo);
+      split_f32(bscale * ky, c.beta2.hi, c.beta2.lo);
+    } else if (KIND == kPlanGrad) {
+      const double t = s_cthsth[j], sg = sth < 1e-9 ? 1e-9 : sth;
+      g->dk_c[0] = to_f32(t * cph);
+      g->dk_c[1] = to_f32(t * sph);
+      g->dk_c[2] = -1.f;
+      g->dk_c[3] = 0.f;
+      g->dk_p[0] = to_f32(sg * sph);
+      g->dk_p[1] = to_f32(-sg * cph);
+      g->dk_p[2] = g->dk_p[3] = 0.f;
+      const float ac = to_f32(Ap * c2), as = to_f32(Ap * s2), cc = to_f32(ci * c2), cs = to_f32(ci * s2);
+      g->DP[0] = ac;
+      g->DP[1] = cs;
+      g->DC[0] = -as;
+      g->DC[1] = cc;
+      g->dDP_i[0] = cc;
+      g->dDP_i[1] = to_f32(s2);
+      g->dDC_i[0] = -cs;
+      g->dDC_i[1] = to_f32(c2);
+      g->dDP_s[0] = -2.f * as;
+      g->dDP_s[1] = 2.f * cc;
+      g->dDC_s[0] = -2.f * ac;
+      g->dDC_s[1] = -2.f * cs;
+    }
+  }
+  if (w == 1) {
+    __syncwarp();
+    bin_end(a, slot, i, bin);
+  }
+}
+
+cudaError_t fd_launch_plan(PlanKind kind, PlanArgs a, const FdTablesDev &tab, int per_cta, int num_sms,
+                           cudaStream_t stream) {
+  const int per = num_sms > 0 ? (a.nitems + num_sms - 1) / num_sms : 16;
+  a.per_cta = per_cta > 0 ? per_cta : (per < 16 ? 16 : (per > 32 ? 32 : per));
+  a.invT = 1.0 / a.T;
+  a.T2 = a.T * a.T;
+  a.invT2 = 1.0 / a.T2;
+  a.invfstar = 1.0 / a.fstar;
+  a.invc = 1.0 / kCLIGHT;
+  a.tw1024 = tab.tw64[fd_bin_of(kSincosTab)];
+  const int grid = (a.nitems + a.per_cta - 1) / a.per_cta;
+  switch (kind) {
+    case kPlanF64: fd_plan_kernel<kPlanF64><<<grid, 128, 0, stream>>>(a); break;
+    case kPlanMix: fd_plan_kernel<kPlanMix><<<grid, 128, 0, stream>>>(a); break;
+    default: fd_plan_kernel<kPlanGrad><<<grid, 128, 0, stream>>>(a); break;
+  }
+  return cudaGetLastError();
 }
 
 // Sets a CUDA-graph conditional node's value to (*count > 0).
 __global__ void fd_cond_kernel(const int *count, cudaGraphConditionalHandle h) {
   if (threadIdx.x == 0) cudaGraphSetConditional(h, *(volatile const int *)count > 0 ? 1u : 0u);
-}
-
-// Mixed-precision plan, warp-specialised: GB300's FP64 pipe issues a warp
-// instruction only every few tens of cycles, so the FP64 work of a proposal is
-// split over four warps that run in parallel on different SM sub-partitions,
-// each writing its share of the ItemMix record directly: warp 0 the bandwidth
-// rule (FP32, FP64 only near a size boundary) and placement, warp 1 the sky
-// direction, polarisation tensors and Doppler constants, warp 2 the
-// polarisation factors and the FP32 frequency constants, warp 3 the amplitude
-// and the double-float carrier constants.  The antenna tensors Mr, Mi are then
-// assembled in FP64 by all 128 threads; only the N-dependent fields wait for
-// the barrier.  Same results as planmix_item (the FP32 constants to rounding).
-// Proposals per CTA: ceil(n / SMs) lanes of each role warp, at least 16, so
-// that a batch of a few thousand proposals is one wave over every SM (the
-// kernel is latency-bound; a second CTA on some SMs doubles their time).
-
-__global__ void __launch_bounds__(128) fd_planmix_kernel(PlanArgs a) {
-  __shared__ double s_ep[32][6], s_ec[32][6], s_dp[32][4], s_amp[32];
-  __shared__ int s_st[32], s_N[32], s_imin[32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int i = blockIdx.x * a.per_cta + l;
-  const bool in = l < a.per_cta && i < a.nitems;
-  double p[8];
-  int seg = 0, st = 1;
-  if (in) st = plan_validate(a, i, p, seg);
-  const double T = a.T;
-  ItemMix *c = a.itemsmix + (in ? i : 0);
-  if (in && !st) {
-    const double f0 = p[0] / T;
-    if (w == 0) {
-      int N;
-      if (a.n_fixed > 0) {
-        N = a.n_fixed;
-      } else {
-        const float Tf = (float)T, f0f = (float)f0, costhf = (float)p[1];
-        const float fdotf = (float)(p[7] / (T * T));
-        const float ampf = expf((float)p[3]);
-        const float sinthf = sqrtf(fmaxf(0.f, (1.f - costhf) * (1.f + costhf)));
-        const int Nmin = 16;
-        const int half = a.NFFT / 2;
-        const int Nmax = half >= 1 ? (1 << (31 - __clz(half))) : 0;
-        float bw = 2.f * Tf * ((4.f + 6.2831853f * f0f * (float)(kAU / kCLIGHT) * sinthf) / (float)kYEAR +
-                               fabsf(fdotf) * Tf);
-        int DS = pow2_above_f32(bw - 1.f);
-        if (DS < 0) DS = doppler_spread_fp64(T, f0, p[7] / (T * T), p[1]);
-        if (DS > Nmax) DS = Nmax;
-        if (DS < Nmin) DS = Nmin;
-        const float x = f0f / (float)a.fstar;
-        float sx, cx;
-        sincosf(x, &sx, &cx);
-        const float c2x = 2.f * cx * cx - 1.f;
-        const float wf = 6.2831853f * f0f, w2 = wf * wf;
-        const float q1 = 2.0e-5f / f0f, q2 = q1 * q1, q4 = q2 * q2, r1 = 1.0e-4f / f0f;
-        const float red = 1.f + 16.f * (q4 * q4 * q2 + r1 * r1);
-        const float twoL = 2.f * (float)a.L;
-        const float sn4L2 = (16.f / 3.f) * sx * sx *
-                            ((2.f + cx) * (float)(kSPS + kSLOC) +
-                             2.f * (3.f + 2.f * cx + c2x) * ((float)(kSLOC / 2.0) + (float)kSACC / (w2 * w2) * red));
-        const float snrm = ampf * sqrtf(Tf) * sx * twoL / sqrtf(sn4L2);
-        int SS = pow2_above_f32(snrm - 1.f);
-        if (SS < 0) SS = snr_spread_fp64(T, f0, p[3], a.L, a.fstar);
-        if (SS > Nmax) SS = Nmax;
-        if (SS < Nmin) SS = Nmin;
-        N = 2 * ((DS > SS) ? DS : SS);
-      }
-      int stw = 0, imin = 0;
-      if (N < kMinN || N > kMaxN) {
-        stw = 1;
-      } else {
-        imin = (int)((long long)(f0 * T) - N / 2) - a.seg_qmin[seg];
-        if (imin >= a.NFFT || imin + N <= 0) stw = 4;
-      }
-      s_st[l] = stw;
-      s_N[l] = N;
-      s_imin[l] = imin;
-    } else if (w == 1) {
-      const double cth = p[1], sth = sqrt(1.0 - cth * cth);
-      double sph, cph;
-      sincos(p[2], &sph, &cph);
-      const double u[3] = {cth * cph, cth * sph, -sth}, v[3] = {sph, -cph, 0.};
-      const double kx = -sth * cph, ky = -sth * sph;
-      c->k[0] = (float)kx;
-      c->k[1] = (float)ky;
-      c->k[2] = (float)(-cth);
-      c->k[3] = 0.f;
-      c->kl[0] = (float)(kx - (double)c->k[0]);
-      c->kl[1] = (float)(ky - (double)c->k[1]);
-      c->kl[2] = (float)(-cth - (double)c->k[2]);
-      int idx = 0;
-#pragma unroll
-      for (int r = 0; r < 3; r++)
-#pragma unroll
-        for (int q = r; q < 3; q++, idx++) {
-          s_ep[l][idx] = v[r] * v[q] - u[r] * u[q];
-          s_ec[l][idx] = u[r] * v[q] + v[r] * u[q];
-        }
-      const double bscale = kPI2 * f0 * (kAU / kCLIGHT);
-      c->beta1 = df_from_double(bscale * kx);
-      c->beta2 = df_from_double(bscale * ky);
-    } else if (w == 2) {
-      const double cosi = p[4];
-      double sinps, cosps;
-      sincos(2. * p[5], &sinps, &cosps);
-      const double Aplus = (1. + cosi * cosi) * 0.5, Across = -cosi;
-      s_dp[l][0] = Aplus * cosps;
-      s_dp[l][1] = -Across * sinps;
-      s_dp[l][2] = -Aplus * sinps;
-      s_dp[l][3] = -Across * cosps;
-      const double fdotT = p[7] / T;  // fdot T
-      c->fonfs0 = (float)(f0 / a.fstar);
-      c->fonfs0l = (float)(f0 / a.fstar - (double)c->fonfs0);
-      c->fdfs = (float)(fdotT / a.fstar);
-      c->fdfsl = (float)(fdotT / a.fstar - (double)c->fdfs);
-      c->aef = (float)(0.66666666666666666666 * fdotT / f0);
-      c->aefl = (float)(0.66666666666666666666 * fdotT / f0 - (double)c->aef);
-      c->w0c = (float)(kPI2 * f0 / kCLIGHT);
-      c->w0cl = (float)(kPI2 * f0 / kCLIGHT - (double)c->w0c);
-      c->p7pi = (float)(kPI * p[7]);
-    } else {
-      s_amp[l] = exp(p[3]);
-      const double fT = f0 * T;
-      const long long q = (long long)fT;
-      c->eps2pi = df_from_double(kPI2 * (fT - (double)q));
-      c->phi0 = df_from_double(p[6]);
-      c->p7pi_d = df_from_double(kPI * p[7]);
-    }
-  } else if (w == 0) {
-    s_st[l] = st;
-    s_N[l] = 0;
-    s_imin[l] = 0;
-  }
-  __syncthreads();
-  const int stt = in ? (st | s_st[l]) : 1;
-  // amp/(2N) = m 2^e, m in [1, 2): the power of two scales the template
-  // exactly in the likelihood kernels, m goes into the antenna tensors
-  double msc = 1.0;
-  if (in && !stt) {
-    const double sc = scalbn(s_amp[l], -(32 - __clz(s_N[l])));  // amp / (2N), N a power of two
-    const int ex = ilogb(sc);
-    msc = scalbn(sc, -ex);
-    if (w == 0) c->amp_p2 = (float)scalbn(1.0, ex);
-  }
-  // antenna tensors: warp w assembles elements 3w/2 .. of the 12 (Mr, Mi) x 6
-  if (in && !stt) {
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const int e = 3 * w + q;  // 0..11: (tensor element, real/imag)
-      const int el = e >> 1;
-      const double DPx = s_dp[l][(e & 1) ? 1 : 0], DCx = s_dp[l][(e & 1) ? 3 : 2];
-      const double md = msc * (DPx * s_ep[l][el] + DCx * s_ec[l][el]);
-      const float m = (float)md, ml = (float)(md - (double)m);
-      if (e & 1) {
-        c->Mi[el] = m;
-        c->Mil[el] = ml;
-      } else {
-        c->Mr[el] = m;
-        c->Mrl[el] = ml;
-      }
-    }
-  }
-  int b = -1;
-  if (w == 0) {
-    if (in && stt) {
-      plan_write_skipped(a, i, stt);
-    } else if (in) {
-      const int N = s_N[l];
-      c->seg = seg;
-      c->N = N;
-      c->imin = s_imin[l];
-      c->pad = 0;
-      const double sc = scalbn(s_amp[l], -(32 - __clz(N)));  // amp / (2N), N a power of two
-      c->amp_hi = (float)sc;
-      c->amp_lo = (float)(sc - (double)c->amp_hi);
-      b = fd_bin_of(N);
-    }
-    plan_bin(a, i, b);
-  }
 }
 
 // ------------------------------------------------------------ orbit tables
@@ -486,17 +618,10 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   const bool timing = work.phase_timing;
   work.phase_recorded = false;
   if (timing && (e = cudaEventRecord(work.phase[0], stream)) != cudaSuccess) return e;
-  {
-    int per = (nitems + num_sms - 1) / (num_sms > 0 ? num_sms : 1);
-    pa.per_cta = per < 16 ? 16 : (per > 32 ? 32 : per);
-    if (work.tune.plan_per_cta >= 8 && work.tune.plan_per_cta <= 32) pa.per_cta = work.tune.plan_per_cta;
-  }
-  if (mix)
-    fd_planmix_kernel<<<(nitems + pa.per_cta - 1) / pa.per_cta, 128, 0, stream>>>(pa);
-  else
-    fd_plan64_kernel<<<(nitems + 63) / 64, 64, 0, stream>>>(pa);
+  const int tune_per = work.tune.plan_per_cta;
+  e = fd_launch_plan(mix ? kPlanMix : kPlanF64, pa, tab, tune_per >= 8 && tune_per <= 32 ? tune_per : 0, num_sms, stream);
   launches++;
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (e != cudaSuccess) return e;
   if (timing && (e = cudaEventRecord(work.phase[1], stream)) != cudaSuccess) return e;
 
   SlowArgs sa;
@@ -704,11 +829,6 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   }
   if (nlaunch) *nlaunch = launches;
   return cudaSuccess;
-}
-
-cudaError_t fd_launch_plan64(const PlanArgs &a, cudaStream_t stream) {
-  fd_plan64_kernel<<<(a.nitems + 63) / 64, 64, 0, stream>>>(a);
-  return cudaGetLastError();
 }
 
 size_t fd_series_bytes(int nitems, int NFFT, int precision) {

@@ -410,35 +410,6 @@ __device__ __forceinline__ int pow2_above_dev(double v) {
   return e > 30 ? (1 << 30) : (1 << e);
 }
 
-// FP64 re-evaluation of the two spreads of the bandwidth rule for the mixed
-// plans, taken when the FP32 estimate lies within 1e-4 of a power of two.
-// Same formulas as ucb/src/glass_ucb_waveform.c:708-722 and AEnoise
-// (utils/src/glass_lisa.c:1188-1198), evaluated with one sincos and products:
-// sin(acos(c)) as sqrt((1 - c)(1 + c)), x^10 as ((x^2)^2)^2 x^2, cos 2x as
-// 2 cos^2 x - 1.  These agree with the library forms to a few ulp, so N can
-// differ from the reference's only for a spread within ~1e-15 of a power of
-// two (where the reference's own result depends on its libm).  A lane that
-// takes this path runs a few hundred FP64 instructions; the library forms
-// (acos, sin, pow) cost several times that on the FP64 pipe and made this rare
-// lane the tail of the whole plan launch.
-__device__ __forceinline__ int doppler_spread_fp64(double T, double f0, double fdot, double costheta) {
-  const double sintheta = sqrt((1.0 - costheta) * (1.0 + costheta));
-  return pow2_above_dev(2 * T * ((4. + kPI2 * f0 * (kAU / kCLIGHT) * sintheta) / kYEAR + fabs(fdot) * T) - 1);
-}
-__device__ __forceinline__ int snr_spread_fp64(double T, double f0, double lnA, double L, double fstar) {
-  const double x = f0 / fstar;
-  double sf, cf;
-  sincos(x, &sf, &cf);
-  const double r = 1.0e-4 / f0, q = 2.0e-5 / f0, q2 = q * q, q4 = q2 * q2;
-  const double red = 1. + 16.0 * (q4 * q4 * q2 + r * r);
-  const double w = kPI2 * f0, w2 = w * w;
-  const double c2x = 2.0 * cf * cf - 1.0;
-  const double sn = (16.0 / 3.0) * sf * sf *
-                    ((2.0 + cf) * (kSPS + kSLOC) + 2.0 * (3.0 + 2.0 * cf + c2x) * (kSLOC / 2.0 + kSACC / (w2 * w2) * red)) /
-                    ((2.0 * L) * (2.0 * L));
-  return pow2_above_dev(exp(lnA) * sqrt(T) * sf / sqrt(sn) - 1);
-}
-
 // ucb/src/glass_ucb_waveform.c:698-725 (ucb_bandwidth).
 static __device__ int bandwidth_dev(double L, double fstar, double f, double fdot, double costheta, double A,
                                     double T, int NFFT) {
@@ -524,42 +495,6 @@ static __host__ __device__ void make_item_f64(const SourceGeom &g, int N, double
   c.h0 = 0.5 * g.f0 / fstar;
   c.hd = 0.5 * g.fdot / fstar;
   c.amp_s = g.amp / (2.0 * (double)N);
-}
-
-static __device__ void make_item_mix(const SourceGeom &g, int N, double T, double fstar, ItemMix &c) {
-  for (int i = 0; i < 3; i++) {
-    c.k[i] = (float)g.k[i];
-    c.kl[i] = (float)(g.k[i] - (double)c.k[i]);
-  }
-  c.k[3] = 0.f;
-  const double s = g.amp / (2.0 * (double)N);
-  const int e = ilogb(s);
-  const double m = scalbn(s, -e);  // in [1, 2)
-  c.amp_p2 = (float)scalbn(1.0, e);
-  for (int i = 0; i < 6; i++) {
-    const double mr = m * (g.DPr * g.ep[i] + g.DCr * g.ec[i]), mi = m * (g.DPi * g.ep[i] + g.DCi * g.ec[i]);
-    c.Mr[i] = (float)mr;
-    c.Mi[i] = (float)mi;
-    c.Mrl[i] = (float)(mr - (double)c.Mr[i]);
-    c.Mil[i] = (float)(mi - (double)c.Mi[i]);
-  }
-  c.fonfs0 = (float)(g.f0 / fstar);
-  c.fonfs0l = (float)(g.f0 / fstar - (double)c.fonfs0);
-  c.fdfs = (float)(g.fdot * T / fstar);
-  c.fdfsl = (float)(g.fdot * T / fstar - (double)c.fdfs);
-  c.aef = (float)(0.66666666666666666666 * g.fdot * T / g.f0);
-  c.aefl = (float)(0.66666666666666666666 * g.fdot * T / g.f0 - (double)c.aef);
-  c.w0c = (float)(kPI2 * g.f0 / kCLIGHT);
-  c.w0cl = (float)(kPI2 * g.f0 / kCLIGHT - (double)c.w0c);
-  c.p7pi = (float)(kPI * g.fdot * T * T);
-  c.amp_hi = (float)s;
-  c.amp_lo = (float)(s - (double)c.amp_hi);
-  c.eps2pi = df_from_double(kPI2 * g.eps);
-  double bscale = kPI2 * g.f0 * (kAU / kCLIGHT);
-  c.beta1 = df_from_double(bscale * g.k[0]);
-  c.beta2 = df_from_double(bscale * g.k[1]);
-  c.phi0 = df_from_double(g.phi0);
-  c.p7pi_d = df_from_double(kPI * g.fdot * T * T);
 }
 
 // ----------------------------------------------------------------- slow part
@@ -861,18 +796,26 @@ __device__ __forceinline__ void ae_combos64(const double2 d[6], double2 out[4]) 
 struct PlanArgs {
   int nitems, nseg, NFFT, cap, precision;
   int n_fixed;  // 0: bandwidth rule
-  int per_cta = 16;  // mixed plan: proposals per CTA (16..32 lanes of each role warp)
+  int per_cta = 16;  // proposals per CTA (8 .. 32)
   double T, fstar, L;
+  double invT, T2, invT2, invfstar, invc;  // reciprocals, for div_by
+  const double2 *tw1024;                   // the sine/cosine table
   const int *item_seg;
   const double *params;
   const double *term_x;
   const int *seg_qmin;
-  ItemF64 *items64;
-  ItemMix *itemsmix;
+  ItemF64 *items64 = nullptr;     // kPlanF64
+  ItemMix *itemsmix = nullptr;    // kPlanMix
+  ItemGrad *itemsgrad = nullptr;  // kPlanGrad, with the outputs grad and fisher (may be null)
+  double *grad = nullptr, *fisher = nullptr;
   int *bin_count, *bin_list;
   double *dlogl, *term_y, *hh;
   int *status;
 };
+enum PlanKind { kPlanF64, kPlanMix, kPlanGrad };
+// Plan of a batch, in kind's item records (ucb_fd.cu); per_cta: 0 for the default.
+cudaError_t fd_launch_plan(PlanKind kind, PlanArgs a, const FdTablesDev &tab, int per_cta, int num_sms,
+                           cudaStream_t stream);
 
 // Outputs of a proposal that is not evaluated (bad input, or a template
 // entirely outside its segment).
@@ -889,119 +832,12 @@ __device__ __forceinline__ void plan_write_skipped(const PlanArgs &a, int i, int
     if (a.hh) a.hh[i] = 0.0;
   }
   if (a.status) a.status[i] = st;
-}
-
-// Warp-aggregated binning: one atomic per distinct size per warp.
-__device__ __forceinline__ void plan_bin(const PlanArgs &a, int i, int b) {
-  const int lane = threadIdx.x & 31;
-  const unsigned active = __ballot_sync(0xffffffffu, b >= 0);
-  if (b >= 0) {
-    const unsigned same = __match_any_sync(active, b);
-    const int first = __ffs(same) - 1;
-    int base = 0;
-    if (lane == first) base = atomicAdd(&a.bin_count[b], __popc(same));
-    base = __shfl_sync(same, base, first);
-    const int slot = base + __popc(same & ((1u << lane) - 1));
-    if (chk(slot < a.cap && b < kNumBins, kChkBinList)) a.bin_list[(size_t)b * a.cap + slot] = i;
+  if (a.grad) {
+    const double v = (st & 3) ? __longlong_as_double(0x7ff8000000000000ULL) : 0.0;
+    for (int k = 0; k < 8; k++) a.grad[8 * (size_t)i + k] = v;
+    if (a.fisher)
+      for (int k = 0; k < 64; k++) a.fisher[64 * (size_t)i + k] = v;
   }
-}
-
-__device__ __forceinline__ int plan_validate(const PlanArgs &a, int i, double *p, int &seg) {
-  bool finite = true;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    p[k] = a.params[8 * (size_t)i + k];
-    finite = finite && isfinite(p[k]);
-  }
-  seg = a.item_seg[i];
-  int st = 0;
-  if (seg < 0 || seg >= a.nseg) st |= 2;
-  if (!finite || fabs(p[1]) > 1.0 || fabs(p[4]) > 1.0) st |= 1;
-  return st;
-}
-
-// (int)pow(2, (int)log2(v) + 1) from an FP32 estimate of v, or -1 when v lies
-// within 1e-4 (relative) of a power of two, where an FP32 estimate could fall
-// on the other side of the boundary than the reference's FP64 value.
-__device__ __forceinline__ int pow2_above_f32(float v) {
-  if (!(v >= 1.0f)) return (v < 0.99f) ? 1 : -1;
-  int e;
-  float m = frexpf(v, &e);  // v = m 2^e, m in [0.5, 1)
-  if (m < 0.50005f || m > 0.99995f) return -1;
-  return e > 30 ? (1 << 30) : (1 << e);  // (int)log2(v) = e - 1
-}
-
-// Mixed-precision plan of proposal i: FP32 except where a constant sets the
-// carrier phase (f0 T - q, the Doppler amplitude 2 pi f0 AU/c k, phi0,
-// pi fdot T^2), and the bandwidth rule, which is evaluated in FP32 and
-// re-evaluated in FP64 only for values near a power-of-two boundary, so N is
-// always the reference's.  N_fixed > 0 replaces the rule by that size.
-// Returns the status bits; fills c when they are 0.
-__device__ __forceinline__ int planmix_item(const PlanArgs &a, int i, int N_fixed, ItemMix &c) {
-  double p[8];
-  int seg;
-  int st = plan_validate(a, i, p, seg);
-  const double T = a.T;
-  const double f0 = p[0] / T;
-  const float Tf = (float)T, f0f = (float)f0, costhf = (float)p[1];
-  const float fdotf = (float)(p[7] / (T * T));
-  const float ampf = expf((float)p[3]);
-  const float sinthf = sqrtf(fmaxf(0.f, 1.f - costhf * costhf));
-  int N = 0;
-  if (!st && N_fixed > 0) {
-    N = N_fixed;
-  } else if (!st) {
-    const int Nmin = 16;
-    const int half = a.NFFT / 2;
-    const int Nmax = half >= 1 ? (1 << (31 - __clz(half))) : 0;
-    // Doppler spread (ucb/src/glass_ucb_waveform.c:708-714)
-    float bw = 2.f * Tf * ((4.f + 6.2831853f * f0f * (float)(kAU / kCLIGHT) * sinthf) / (float)kYEAR + fabsf(fdotf) * Tf);
-    int DS = pow2_above_f32(bw - 1.f);
-    if (DS < 0) DS = doppler_spread_fp64(T, f0, p[7] / (T * T), p[1]);
-    if (DS > Nmax) DS = Nmax;
-    if (DS < Nmin) DS = Nmin;
-    // SNR spread (:717-722) with AEnoise (utils/src/glass_lisa.c:1188-1198)
-    const float x = f0f / (float)a.fstar;
-    float sx, cx;
-    sincosf(x, &sx, &cx);
-    const float c2x = 2.f * cx * cx - 1.f;
-    const float w = 6.2831853f * f0f, w2 = w * w;
-    const float q1 = 2.0e-5f / f0f, q2 = q1 * q1, q4 = q2 * q2, r1 = 1.0e-4f / f0f;
-    const float red = 1.f + 16.f * (q4 * q4 * q2 + r1 * r1);
-    // AEnoise times (2L)^2: AEnoise itself (~1e-42) is below FP32's normal range
-    const float twoL = 2.f * (float)a.L;
-    const float sn4L2 = (16.f / 3.f) * sx * sx *
-                        ((2.f + cx) * (float)(kSPS + kSLOC) +
-                         2.f * (3.f + 2.f * cx + c2x) * ((float)(kSLOC / 2.0) + (float)kSACC / (w2 * w2) * red));
-    const float snrm = ampf * sqrtf(Tf) * sx * twoL / sqrtf(sn4L2);
-    int SS = pow2_above_f32(snrm - 1.f);
-    if (SS < 0) SS = snr_spread_fp64(T, f0, p[3], a.L, a.fstar);
-    if (SS > Nmax) SS = Nmax;
-    if (SS < Nmin) SS = Nmin;
-    N = 2 * ((DS > SS) ? DS : SS);
-    if (N < kMinN || N > kMaxN) st |= 1;
-  }
-  const double fT = f0 * T;
-  const long long q = (long long)fT;
-  int imin = 0;
-  if (!st) {
-    imin = (int)(q - N / 2) - a.seg_qmin[seg];
-    if (imin >= a.NFFT || imin + N <= 0) st = 4;
-  }
-  if (!st) {
-    // Geometry, polarisation and amplitude in FP64, rounded once: an FP32
-    // exp of lnA ~ -50, or FP32 trigonometry of phi and 2 psi, would put a
-    // systematic 1e-7..1e-6 error on the template that shows up in delta
-    // logL even at the likelihood maximum.
-    SourceGeom g;
-    source_geometry(p, 8, T, g);
-    make_item_mix(g, N, T, a.fstar, c);
-    c.seg = seg;
-    c.N = N;
-    c.imin = imin;
-    c.pad = 0;
-  }
-  return st;
 }
 
 // Stage 1: slow part of every (proposal, sample) pair, written to scratch as the

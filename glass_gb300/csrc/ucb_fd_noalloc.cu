@@ -26,7 +26,6 @@ namespace glass {
 
 cudaError_t fd_launch_slow_fp64(const SlowArgs &a, int num_sms, cudaStream_t stream);
 cudaError_t fd_launch_spec_fp64(int N, const SpecArgs &a, int nitems, int num_sms, cudaStream_t stream, bool perch);
-cudaError_t fd_launch_plan64(const PlanArgs &a, cudaStream_t stream);
 int report_error(int code, const char *msg);
 int report_cuda_error(cudaError_t e, const char *where);
 
@@ -191,14 +190,13 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
   pa.term_x = term_x;
   pa.seg_qmin = qmin;
   pa.items64 = na->items;
-  pa.itemsmix = nullptr;
   pa.bin_count = na->bin_count;
   pa.bin_list = na->bin_list;
   pa.dlogl = dlogl;
   pa.term_y = term_y;
   pa.hh = hh;
   pa.status = status;
-  if ((e = fd_launch_plan64(pa, s)) != cudaSuccess) return report_cuda_error(e, "dlogl_fp64_noalloc: plan");
+  if ((e = fd_launch_plan(kPlanF64, pa, tab, 0, 0, s)) != cudaSuccess) return report_cuda_error(e, "dlogl_fp64_noalloc: plan");
 
   SlowArgs sa;
   sa.cap = kNaMaxItems;

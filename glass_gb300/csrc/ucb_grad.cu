@@ -44,84 +44,6 @@ __device__ __forceinline__ float dsinc_f(float x) {
   return p * x;
 }
 
-struct GradPlanArgs {
-  PlanArgs base;
-  int N_fixed;
-  ItemGrad *items;
-  double *grad, *fisher;
-};
-
-__global__ void __launch_bounds__(256) fd_plangrad_kernel(GradPlanArgs ga) {
-  const PlanArgs &a = ga.base;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int b = -1;
-  if (i < a.nitems) {
-    ItemMix c;
-    int st = planmix_item(a, i, ga.N_fixed, c);
-    if (st) {
-      plan_write_skipped(a, i, st);
-      const double v = (st & 3) ? __longlong_as_double(0x7ff8000000000000ULL) : 0.0;
-      for (int k = 0; k < 8; k++) ga.grad[8 * (size_t)i + k] = v;
-      if (ga.fisher)
-        for (int k = 0; k < 64; k++) ga.fisher[64 * (size_t)i + k] = v;
-    } else {
-      ItemGrad g;
-      g.m = c;
-      const double *p = a.params + 8 * (size_t)i;
-      const double T = a.T;
-      const double cth = p[1];
-      double sth = sqrt(1.0 - cth * cth);
-      if (sth < 1e-9) sth = 1e-9;  // d/dcos(theta) is singular at the poles
-      double sph, cph;
-      sincos(p[2], &sph, &cph);
-      const double u[3] = {cth * cph, cth * sph, -sth}, v[3] = {sph, -cph, 0.};
-      const double du_c[3] = {cph, sph, cth / sth}, dv_c[3] = {0., 0., 0.};
-      const double du_p[3] = {-cth * sph, cth * cph, 0.}, dv_p[3] = {cph, sph, 0.};
-      g.dk_c[0] = (float)(cth / sth * cph);
-      g.dk_c[1] = (float)(cth / sth * sph);
-      g.dk_c[2] = -1.f;
-      g.dk_c[3] = 0.f;
-      g.dk_p[0] = (float)(sth * sph);
-      g.dk_p[1] = (float)(-sth * cph);
-      g.dk_p[2] = 0.f;
-      g.dk_p[3] = 0.f;
-      int idx = 0;
-      for (int r = 0; r < 3; r++)
-        for (int s = r; s < 3; s++, idx++) {
-          g.ep[idx] = (float)(v[r] * v[s] - u[r] * u[s]);
-          g.ec[idx] = (float)(u[r] * v[s] + v[r] * u[s]);
-          g.dep_c[idx] = (float)(dv_c[r] * v[s] + v[r] * dv_c[s] - du_c[r] * u[s] - u[r] * du_c[s]);
-          g.dec_c[idx] = (float)(du_c[r] * v[s] + u[r] * dv_c[s] + dv_c[r] * u[s] + v[r] * du_c[s]);
-          g.dep_p[idx] = (float)(dv_p[r] * v[s] + v[r] * dv_p[s] - du_p[r] * u[s] - u[r] * du_p[s]);
-          g.dec_p[idx] = (float)(du_p[r] * v[s] + u[r] * dv_p[s] + dv_p[r] * u[s] + v[r] * du_p[s]);
-        }
-      const double ci = p[4];
-      double s2, c2;
-      sincos(2.0 * p[5], &s2, &c2);
-      const double Ap = 0.5 * (1.0 + ci * ci);
-      g.DP[0] = (float)(Ap * c2);
-      g.DP[1] = (float)(ci * s2);
-      g.DC[0] = (float)(-Ap * s2);
-      g.DC[1] = (float)(ci * c2);
-      g.dDP_i[0] = (float)(ci * c2);
-      g.dDP_i[1] = (float)s2;
-      g.dDC_i[0] = (float)(-ci * s2);
-      g.dDC_i[1] = (float)c2;
-      g.dDP_s[0] = (float)(-2.0 * Ap * s2);
-      g.dDP_s[1] = (float)(2.0 * ci * c2);
-      g.dDC_s[0] = (float)(-2.0 * Ap * c2);
-      g.dDC_s[1] = (float)(-2.0 * ci * s2);
-      g.f0 = (float)(p[0] / T);
-      g.fdot = (float)(p[7] / (T * T));
-      g.invT = (float)(1.0 / T);
-      g.fstar = (float)a.fstar;
-      ga.items[i] = g;
-      b = fd_bin_of(c.N);
-    }
-  }
-  plan_bin(a, i, b);
-}
-
 struct GradConsts {
   float Rf, invLf, AUcf, invTf, AUf, Tf;
 };
@@ -729,8 +651,7 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
   if (!work.counts_zero && (e = cudaMemsetAsync(work.bin_count, 0, sizeof(int) * (kNumBins + 1), stream)) != cudaSuccess)
     return e;
   work.counts_zero = false;
-  GradPlanArgs ga;
-  PlanArgs &pa = ga.base;
+  PlanArgs pa;
   pa.nitems = nitems;
   pa.nseg = bank.nseg;
   pa.NFFT = bank.NFFT;
@@ -744,29 +665,18 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
   pa.params = params;
   pa.term_x = nullptr;
   pa.seg_qmin = bank.qmin;
-  pa.items64 = nullptr;
-  pa.itemsmix = nullptr;
+  pa.itemsgrad = work.itemsgrad;
+  pa.grad = grad;
+  pa.fisher = fisher;
   pa.bin_count = work.bin_count;
   pa.bin_list = work.bin_list;
   pa.dlogl = term_y;
   pa.term_y = nullptr;
   pa.hh = nullptr;
   pa.status = status;
-  ga.N_fixed = N_fixed;
-  ga.items = work.itemsgrad;
-  ga.grad = grad;
-  ga.fisher = fisher;
-  {
-    // one thread per proposal in CTAs of 64..256 threads, as few CTAs as
-    // SMs where the batch allows (the kernel is a latency-bound FP64 chain: a
-    // second CTA on some SMs doubles their time)
-    int per = (nitems + num_sms - 1) / (num_sms > 0 ? num_sms : 1);
-    per = (per + 31) / 32 * 32;
-    per = per < 64 ? 64 : (per > 256 ? 256 : per);
-    fd_plangrad_kernel<<<(nitems + per - 1) / per, per, 0, stream>>>(ga);
-  }
+  e = fd_launch_plan(kPlanGrad, pa, tab, 0, num_sms, stream);
   launches++;
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (e != cudaSuccess) return e;
 
   GradSpecArgs a;
   a.NFFT = bank.NFFT;

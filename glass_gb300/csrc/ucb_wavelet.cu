@@ -81,13 +81,6 @@ __device__ __forceinline__ int even_index(const EvenGrid &e, int n, double v) {
   return min(max(__double2loint(q + kRoundMagic), 0), n - 1);
 }
 
-// a / b, correctly rounded, from rb = 1/b: the product and one exact-residual
-// step (3 FP64 instructions instead of about 9).
-__device__ __forceinline__ double div_by(double a, double b, double rb) {
-  const double q = a * rb;
-  return fma(fma(-q, b, a), rb, q);
-}
-
 // The tile kernels below keep 4 arrays of n doubles per chain in shared memory,
 // chains 4 n + 1 doubles apart: the sequential phases have the chains' threads
 // at the same node index, which an unpadded stride would put on one bank.
