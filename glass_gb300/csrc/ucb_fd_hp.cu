@@ -225,11 +225,12 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // them are resident at once and that the chain is short.  In place and with the
 // twiddles in L1 a CTA takes 16 bytes per point (64 KB at N = 4096, where
 // ping-pong buffers and a twiddle copy took 192 KB and left one CTA per SM); the
-// bank's entries of a thread's first bins are loaded before the transform.  61
-// proposals of up to 1024 points 19.1 -> 16.7 us, 73 of up to 2048 on 8192-bin
-// segments 60.8 -> 42.2 us.
+// bank's entries of a thread's first bins are loaded before the transform, those
+// of each next bin and the twiddles of each next butterfly before the arithmetic of
+// the current one.  61 proposals of up to 1024 points 19.1 -> 16.5 us, 73 of up to
+// 2048 on 8192-bin segments 60.8 -> 38 us.
 template <bool PERCH>
-__global__ void __launch_bounds__(kHpThreads, 3) fd_hp_kernel(HpArgs a) {
+__global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -252,7 +253,15 @@ __global__ void __launch_bounds__(kHpThreads, 3) fd_hp_kernel(HpArgs a) {
     const HpEntry e = hp_entry(a, k, cs);
     const int N = e.N, ln = e.bin + 5;
     const float4 *src = a.series + e.off + (long long)r * N;
-    for (int n = threadIdx.x; n < N; n += blockDim.x) S[hp_at(hp_rev(n, ln))] = dc_from(src[n]);
+    for (int n0 = threadIdx.x; n0 < N; n0 += 4 * kHpThreads) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (n0 + u * kHpThreads < N) v[u] = src[n0 + u * kHpThreads];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (n0 + u * kHpThreads < N) S[hp_at(hp_rev(n0 + u * kHpThreads, ln))] = dc_from(v[u]);
+    }
     // the bank's entries of bin q of this CTA's half
     const int half = N >> 1, q0 = (r & 1) * half;
     struct Bin {
@@ -265,8 +274,8 @@ __global__ void __launch_bounds__(kHpThreads, 3) fd_hp_kernel(HpArgs a) {
       t = {a.g32[2 * sj + ch], a.g32lo[2 * sj + ch], a.w32[sj], a.w32lo[sj]};
       return true;
     };
-    Bin first;
-    const bool has_first = load_bin(q0 + (int)threadIdx.x, first);
+    Bin t;
+    bool has = load_bin(q0 + (int)threadIdx.x, t);
     __syncthreads();
     hp_fft(S, ln, a.tw32x[e.bin]);
     cluster.sync();  // every spectrum of the proposal is complete
@@ -274,16 +283,20 @@ __global__ void __launch_bounds__(kHpThreads, 3) fd_hp_kernel(HpArgs a) {
     const dc *S0 = (r & 1) ? Sp : S, *S1 = (r & 1) ? S : Sp;  // the channel's series 2c, 2c + 1
     df rr = {0.f, 0.f}, hw = {0.f, 0.f};
     for (int q = q0 + threadIdx.x; q < q0 + half; q += blockDim.x) {
-      Bin t = first;
-      if (!(q == q0 + (int)threadIdx.x ? has_first : load_bin(q, t))) continue;
-      const int qs = hp_at(q);
-      dc h = dc_add(dc_mul(S0[qs], dc_from(make_float2(t.gh.x, t.gh.y), make_float2(t.gl.x, t.gl.y))),
-                    dc_mul(S1[qs], dc_from(make_float2(t.gh.z, t.gh.w), make_float2(t.gl.z, t.gl.w))));
-      h = dc_scale2(h, e.amp_p2);
-      const dc w = ch == 0 ? dc_from(make_float2(t.wh.x, t.wh.y), make_float2(t.wl.x, t.wl.y))
-                           : dc_from(make_float2(t.wh.z, t.wh.w), make_float2(t.wl.z, t.wl.w));
-      rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
-      hw = df_add(hw, df_sq_sum(h));
+      Bin next;
+      const bool has_next = load_bin(q + kHpThreads, next);
+      if (has) {
+        const int qs = hp_at(q);
+        dc h = dc_add(dc_mul(S0[qs], dc_from(make_float2(t.gh.x, t.gh.y), make_float2(t.gl.x, t.gl.y))),
+                      dc_mul(S1[qs], dc_from(make_float2(t.gh.z, t.gh.w), make_float2(t.gl.z, t.gl.w))));
+        h = dc_scale2(h, e.amp_p2);
+        const dc w = ch == 0 ? dc_from(make_float2(t.wh.x, t.wh.y), make_float2(t.wl.x, t.wl.y))
+                             : dc_from(make_float2(t.wh.z, t.wh.w), make_float2(t.wl.z, t.wl.w));
+        rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
+        hw = df_add(hw, df_sq_sum(h));
+      }
+      t = next;
+      has = has_next;
     }
     rr = hp_block_sum(rr, red);
     hw = hp_block_sum(hw, red);

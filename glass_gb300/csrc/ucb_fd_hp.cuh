@@ -12,15 +12,22 @@ struct dc {
 };
 __device__ __forceinline__ dc dc_add(dc a, dc b) { return {df_add(a.re, b.re), df_add(a.im, b.im)}; }
 __device__ __forceinline__ dc dc_sub(dc a, dc b) { return {df_add(a.re, df_neg(b.re)), df_add(a.im, df_neg(b.im))}; }
+// a b + c d: the two exact products summed before the one renormalisation
+__device__ __forceinline__ df df_mul2_add(df a, df b, df c, df d) {
+  const df p = two_prod(a.hi, b.hi), q = two_prod(c.hi, d.hi), s = two_sum(p.hi, q.hi);
+  const float l = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo));
+  const float m = __fmaf_rn(c.hi, d.lo, __fmaf_rn(c.lo, d.hi, q.lo));
+  return quick_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(l, m)));
+}
 __device__ __forceinline__ dc dc_mul(dc a, dc b) {
-  return {df_add(df_mul(a.re, b.re), df_neg(df_mul(a.im, b.im))), df_add(df_mul(a.re, b.im), df_mul(a.im, b.re))};
+  return {df_mul2_add(a.re, b.re, df_neg(a.im), b.im), df_mul2_add(a.re, b.im, a.im, b.re)};
 }
 __device__ __forceinline__ dc dc_mi(dc a) { return {a.im, df_neg(a.re)}; }  // -i a
 // complex hi + lo floats (x, y: hi; z, w: lo), as the tables store them: no
 // FP64 conversion in the inner loops (GB300's FP64 pipe runs at 1/64 rate)
 __device__ __forceinline__ dc dc_from(float4 v) { return {{v.x, v.z}, {v.y, v.w}}; }
 __device__ __forceinline__ dc dc_from(float2 hi, float2 lo) { return {{hi.x, lo.x}, {hi.y, lo.y}}; }
-__device__ __forceinline__ df df_sq_sum(dc a) { return df_add(df_mul(a.re, a.re), df_mul(a.im, a.im)); }
+__device__ __forceinline__ df df_sq_sum(dc a) { return df_mul2_add(a.re, a.re, a.im, a.im); }
 // a times an exact power of two
 __device__ __forceinline__ dc dc_scale2(dc a, float p2) {
   return {{a.re.hi * p2, a.re.lo * p2}, {a.im.hi * p2, a.im.lo * p2}};
@@ -146,20 +153,37 @@ __device__ __forceinline__ int hp_rev(int n, int ln) {
   const unsigned r = __brev((unsigned)m) >> (32 - l4);
   return top + (int)(((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u));
 }
+// The twiddles of a thread's next butterfly (of its next stage, after the last of
+// one) are loaded before the arithmetic of the current one: each is used once per
+// series, so every load is a trip to L2.
 __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__ tw) {
   const int N = 1 << ln;
+  float4 w[3] = {};
   int lp = 0;
   for (; lp + 2 <= ln; lp += 2) {
-    const int p = 1 << lp, step = N >> (lp + 2);
+    const int p = 1 << lp;
     for (int i = threadIdx.x; i < N / 4; i += blockDim.x) {
       const int k = i & (p - 1), j = ((i - k) << 2) + k;
       dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + p), *const x2 = x + hp_at(j + 2 * p),
                *const x3 = x + hp_at(j + 3 * p);
       dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
+      const float4 w1 = w[0], w2 = w[1], w3 = w[2];
+      const bool last = i + (int)blockDim.x >= N / 4;
+      const int lq = last ? lp + 2 : lp, in = last ? (int)threadIdx.x : i + (int)blockDim.x;
+      if (lq + 2 <= ln) {
+        const int kn = (in & ((1 << lq) - 1)) << (ln - lq - 2);
+        if (lq > 0) {
+          w[0] = tw[kn];
+          w[1] = tw[2 * kn];
+          w[2] = tw[3 * kn];
+        }
+      } else if (lq < ln) {
+        w[0] = tw[in];  // the radix-2 stage's first
+      }
       if (lp > 0) {
-        u1 = dc_mul(u1, dc_from(tw[k * step]));
-        u2 = dc_mul(u2, dc_from(tw[2 * k * step]));
-        u3 = dc_mul(u3, dc_from(tw[3 * k * step]));
+        u1 = dc_mul(u1, dc_from(w1));
+        u2 = dc_mul(u2, dc_from(w2));
+        u3 = dc_mul(u3, dc_from(w3));
       }
       const dc a = dc_add(u0, u2), b = dc_sub(u0, u2), c = dc_add(u1, u3), d = dc_mi(dc_sub(u1, u3));
       *x0 = dc_add(a, c);
@@ -170,9 +194,12 @@ __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__
     __syncthreads();
   }
   if (lp < ln) {  // log2 N odd: one radix-2 stage, p = N/2
+    if ((int)threadIdx.x >= N / 4 && (int)threadIdx.x < N / 2) w[0] = tw[threadIdx.x];
     for (int k = threadIdx.x; k < N / 2; k += blockDim.x) {
       dc *const x0 = x + hp_at(k), *const x1 = x + hp_at(k + N / 2);
-      const dc a = *x0, b = dc_mul(*x1, dc_from(tw[k]));
+      const float4 w1 = w[0];
+      if (k + (int)blockDim.x < N / 2) w[0] = tw[k + blockDim.x];
+      const dc a = *x0, b = dc_mul(*x1, dc_from(w1));
       *x0 = dc_add(a, b);
       *x1 = dc_sub(a, b);
     }
