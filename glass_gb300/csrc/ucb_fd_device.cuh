@@ -590,16 +590,18 @@ __device__ __forceinline__ double div_clight(double kx) {
 struct ArmGeom64 {
   double dp[3], dc[3], kr[3];
 };
+__device__ __forceinline__ void arm_geom64(const ItemF64 &c, const OrbitSample64 &o, int a, double &dp, double &dc,
+                                           double &kr) {
+  const double x = o.r[a][0], y = o.r[a][1], z = o.r[a][2];
+  const double ru = fma(z, c.u[2], fma(y, c.u[1], x * c.u[0]));
+  const double rv = fma(y, c.v[1], x * c.v[0]);
+  kr = fma(z, c.k[2], fma(y, c.k[1], x * c.k[0]));
+  dp = fma(rv, rv, -(ru * ru));
+  dc = ru * rv;
+}
 __device__ __forceinline__ void slow_geom64(const ItemF64 &c, const OrbitSample64 &o, ArmGeom64 &g) {
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const double x = o.r[a][0], y = o.r[a][1], z = o.r[a][2];
-    const double ru = fma(z, c.u[2], fma(y, c.u[1], x * c.u[0]));
-    const double rv = fma(y, c.v[1], x * c.v[0]);
-    g.kr[a] = fma(z, c.k[2], fma(y, c.k[1], x * c.k[0]));
-    g.dp[a] = fma(rv, rv, -(ru * ru));
-    g.dc[a] = ru * rv;
-  }
+  for (int a = 0; a < 3; a++) arm_geom64(c, o, a, g.dp[a], g.dc[a], g.kr[a]);
 }
 
 // Spacecraft i: the carrier argument, half the instantaneous frequency over f*
@@ -648,6 +650,23 @@ __device__ __forceinline__ void slow_sample64(const ItemF64 &c, const OrbitSampl
       const double2 w = slow_transfer64(h, back ? -g.kr[a] : g.kr[a], arg2, aev, tw);
       d[q] = make_double2(fma(tr[a], w.x, ti[a] * w.y), fma(ti[a], w.x, -(tr[a] * w.y)));
     }
+  }
+}
+
+// The two arms of spacecraft i alone, as slow_sample64 computes them.
+__device__ __forceinline__ void slow_sc_arms64(const ItemF64 &c, const OrbitSample64 &o, const double2 *tw, int i,
+                                               double2 d[2]) {
+  double arg2, h, aev;
+  slow_sc64(c, o, i, arg2, h, aev);
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int a = e == 0 ? (i == 2 ? 1 : 0) : (i == 0 ? 1 : 2);
+    const bool back = i == 2 || (i == 1 && e == 0);
+    double dp, dc, kr;
+    arm_geom64(c, o, a, dp, dc, kr);
+    const double tr = fma(dc, c.DC2r, dp * c.DPr), ti = fma(dc, c.DC2i, dp * c.DPi);
+    const double2 w = slow_transfer64(h, back ? -kr : kr, arg2, aev, tw);
+    d[e] = make_double2(fma(tr, w.x, ti * w.y), fma(ti, w.x, -(tr * w.y)));
   }
 }
 
@@ -979,8 +998,14 @@ __global__ void __launch_bounds__(BLOCK) fd_slow_kernel(SlowArgs a) {
                        : (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   C *series = reinterpret_cast<C *>(a.series);
+  // FP64, at most a chunk per CTA (a few proposals): three warps per chunk, each
+  // the arms of one spacecraft and then a share of the combinations, a third of
+  // the FP64 instructions per warp (of one 128-sample proposal 16.0 -> 11.9 us)
+  const bool split = !MIX && nchunks <= (int)gridDim.x;
+  const int sc = threadIdx.x >> 5;
+  if (split && sc >= 3) return;
 #pragma unroll 1
-  for (int ch = warp; ch < nchunks; ch += nwarps) {
+  for (int ch = split ? (int)blockIdx.x : warp; ch < nchunks; ch += nwarps) {
     int b = 0, cb = 0;
 #pragma unroll
     for (int bb = 1; bb < kNumBins; bb++)
@@ -996,6 +1021,30 @@ __global__ void __launch_bounds__(BLOCK) fd_slow_kernel(SlowArgs a) {
     const int item = a.bin_list[(size_t)b * a.cap + slot];
     if (!chk(item >= 0 && item < a.nitems, kChkItem)) continue;
     C d[6], cmb[4];
+    if constexpr (!MIX) {
+      if (split) {
+        __shared__ double2 s_d[6][32];
+        slow_sc_arms64(a.items64[item], a.pos64[b][n], a.tw1024, sc, d);
+        s_d[2 * sc][lane] = d[0];
+        s_d[2 * sc + 1][lane] = d[1];
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 6; q++) d[q] = s_d[q][lane];
+        const long long o0 = ((long long)cb * 32 + (long long)slot * N) * 4 + n;
+        if (!chk(o0 >= 0 && o0 + 3LL * N < a.series_len, kChkSeriesWrite)) return;
+        C *out = series + o0;
+        ae_combos64(d, cmb);
+        if (sc == 0) {
+          out[0] = cmb[0];
+          out[N] = cmb[1];
+        } else if (sc == 1) {
+          out[2 * (size_t)N] = cmb[2];
+        } else {
+          out[3 * (size_t)N] = cmb[3];
+        }
+        return;
+      }
+    }
     if constexpr (MIX) {
       slow_sample_mix(a.itemsmix[item], a.mix[b][n], a.geo[b][n], a.invLf, a.AUcf, a.invTf, d);
       ae_combos(d, cmb);
@@ -1394,10 +1443,11 @@ __global__ void __launch_bounds__(SpecCfg<N>::CTA) fd_spec_kernel(SpecArgs a) {
   C *bufs = reinterpret_cast<C *>(tw + SN);
   double *red = reinterpret_cast<double *>(bufs + (size_t)GPC * NSER * SN);
 
+  const int count = a.bin_count[a.bin];
+  if ((int)blockIdx.x * GPC >= count) return;
   const TW *twg = reinterpret_cast<const TW *>(a.tw);
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[MIX ? pad16(i) : i] = twg[i];
   __syncthreads();
-  const int count = a.bin_count[a.bin];
   const C *series = reinterpret_cast<const C *>(a.series) + bin_sample_start(a.bin_count, a.NFFT, a.bin) * 4;
   for (int base = blockIdx.x * GPC; base < count; base += gridDim.x * GPC)
     spec_unit<N, MIX, GPC, PERCH>(a, a.bin_list, count, base, series, tw, bufs, red);
@@ -1673,6 +1723,112 @@ struct SpecAllSmem {
   static constexpr size_t bytes = sizeof(TW) * SN + sizeof(C) * 4 * SN + sizeof(double) * 96 * 4;
 };
 
+// In-place FFTs of four series of N = 2^ln points, back to back, by the CTA: radix-4
+// decimation in time from digit-reversed order (hp_rev) and a radix-2 stage when
+// log2 N is odd; results in natural order.  tw[j] = exp(-2 pi i j / N).
+static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const double2 *tw) {
+  int lp = 0;
+  for (; lp + 2 <= ln; lp += 2) {
+    const int p = 1 << lp, lt = ln - lp - 2;
+    for (int t = threadIdx.x; t < 1 << ln; t += blockDim.x) {  // butterflies of the four series in a row
+      const int k = t & (p - 1);
+      double2 *const y = x + ((t - k) << 2) + k;
+      double2 v0 = y[0], v1 = y[p], v2 = y[2 * p], v3 = y[3 * p];
+      if (lp > 0) {
+        v1 = cmul(v1, tw[k << lt]);
+        v2 = cmul(v2, tw[2 * k << lt]);
+        v3 = cmul(v3, tw[3 * k << lt]);
+      }
+      const double2 a = cadd(v0, v2), b = csub(v0, v2), c = cadd(v1, v3), e = csub(v1, v3);
+      y[0] = cadd(a, c);
+      y[p] = make_double2(b.x + e.y, b.y - e.x);
+      y[2 * p] = csub(a, c);
+      y[3 * p] = make_double2(b.x - e.y, b.y + e.x);
+    }
+    __syncthreads();
+  }
+  if (lp < ln) {
+    const int p = 1 << lp;
+    for (int t = threadIdx.x; t < 2 << ln; t += blockDim.x) {
+      const int k = t & (p - 1);
+      double2 *const y = x + ((t - k) << 1) + k;
+      const double2 v0 = y[0], v1 = cmul(y[p], tw[k]);
+      y[0] = cadd(v0, v1);
+      y[p] = csub(v0, v1);
+    }
+    __syncthreads();
+  }
+}
+
+// spec_unit in FP64 for one proposal by the whole CTA, size at run time: for
+// batches of fewer proposals than CTAs, where a group of N/4 threads would leave
+// one warp with all of a small proposal's FP64 instructions (one of 128 points
+// 20.5 -> 12.3 us).
+template <bool PERCH>
+static __device__ __forceinline__ void spec_unit_wide64(const SpecArgs &a, const int *bin_list, int sl, int ln,
+                                                        const double2 *series, const double2 *tw, double2 *buf,
+                                                        double *red) {
+  const int N = 1 << ln, NFFT = a.NFFT, tid = threadIdx.x;
+  const bool lok = chk(sl >= 0 && sl < a.cap, kChkBinList);
+  const int item = lok ? bin_list[sl] : 0;
+  const bool iok = chk(item >= 0 && item < a.nitems, kChkItem);
+  int seg = 0, imin = 0;
+  double s = 0.0;
+  if (iok) {
+    seg = a.items64[item].seg;
+    imin = a.items64[item].imin;
+    s = a.items64[item].amp_s;
+  }
+  const bool sok = chk(seg >= 0 && seg < a.nseg, kChkBankRead);
+  const bool rok = chk((long long)(sl + 1) * 4 * N <= a.series_len, kChkSeriesRead);
+  const bool inb = lok && iok && sok && rok;
+  if (!inb) seg = 0;
+  const double2 *src = series + (inb ? (size_t)sl * 4 * N : 0);
+  for (int i = tid; i < 4 * N; i += blockDim.x) buf[(i & ~(N - 1)) + hp_rev(i & (N - 1), ln)] = src[i];
+  __syncthreads();
+  fft4_dit64(buf, ln, tw);
+  double wA = 0.0, hA = 0.0, wE = 0.0, hE = 0.0;
+  for (int i = tid; i < 2 * N; i += blockDim.x) {
+    const int chan = i >> ln, k = i & (N - 1);
+    const int j = imin + ((k + N / 2) & (N - 1));  // fftshift
+    if (j < 0 || j >= NFFT) continue;
+    const size_t sj = (size_t)seg * NFFT + j;
+    const double2 w = a.w64[2 * sj + chan];
+    const double2 g2 = a.g64[4 * sj + 2 * chan], g1 = a.g64[4 * sj + 2 * chan + 1];
+    const double2 h = cfma(buf[2 * chan * N + k], g2, cmul(buf[(2 * chan + 1) * N + k], g1));
+    if (PERCH && chan) {
+      wE = fma(w.x, h.x, fma(w.y, h.y, wE));
+      hE = fma(h.x, h.x, fma(h.y, h.y, hE));
+    } else {
+      wA = fma(w.x, h.x, fma(w.y, h.y, wA));
+      hA = fma(h.x, h.x, fma(h.y, h.y, hA));
+    }
+  }
+  wA = group_sum<kSpecAllThreads>(wA, red, tid, 0);
+  hA = group_sum<kSpecAllThreads>(hA, red + 32, tid, 0);
+  if (PERCH) {
+    wE = group_sum<kSpecAllThreads>(wE, red + 64, tid, 0);
+    hE = group_sum<kSpecAllThreads>(hE, red + 96, tid, 0);
+  }
+  if (inb && tid == 0) {
+    // 2 (w|h) - |h|^2 with the amplitude s
+    double term = s * (2.0 * wA - s * hA);
+    if (PERCH) {
+      const double tE = s * (2.0 * wE - s * hE);
+      a.term_ch[2 * (size_t)item] = term;
+      a.term_ch[2 * (size_t)item + 1] = tE;
+      term += tE;
+      hA += hE;
+    }
+    const double tx = a.term_x ? a.term_x[item] : 0.0;
+    a.dlogl[item] = term - tx;
+    if (a.term_y) a.term_y[item] = term;
+    if (a.hh) a.hh[item] = 2.0 * (s * s) * hA;
+    if (a.status) a.status[item] = isfinite(term) ? 0 : 1;
+  }
+  __syncthreads();
+}
+
 struct SpecAllArgs {
   SpecArgs a;                    // a.bin_list: all sizes' lists, stride cap; a.tw unused
   const void *tw[kSpecAllBins];  // twiddles per size
@@ -1682,7 +1838,7 @@ struct SpecAllArgs {
 };
 
 template <bool MIX, bool PERCH = false>
-__global__ void __launch_bounds__(kSpecAllThreads, 4) fd_spec_all_kernel(SpecAllArgs A) {
+__global__ void __launch_bounds__(kSpecAllThreads, MIX ? 4 : 2) fd_spec_all_kernel(SpecAllArgs A) {
   using C = typename SpecAllSmem<MIX>::C;
   using TW = typename SpecAllSmem<MIX>::TW;
   const SpecArgs &a = A.a;
@@ -1694,6 +1850,13 @@ __global__ void __launch_bounds__(kSpecAllThreads, 4) fd_spec_all_kernel(SpecAll
   // unit ranges per size, largest first; in shared memory so that they hold
   // no registers while a unit runs
   __shared__ int ustart[kSpecAllBins + 1];
+  // FP64: a CTA per proposal where that leaves none waiting
+  bool wide = false;
+  if constexpr (!MIX) {
+    int n = 0;
+    for (int b = 0; b < A.nbins; b++) n += a.bin_count[b];
+    wide = n <= (int)gridDim.x;
+  }
   if (threadIdx.x == 0) {
     int total = 0;
 #pragma unroll
@@ -1701,7 +1864,7 @@ __global__ void __launch_bounds__(kSpecAllThreads, 4) fd_spec_all_kernel(SpecAll
       const int b = kSpecAllBins - 1 - q;
       ustart[q] = total;
       if (b < A.nbins) {
-        const int gpc = 32 >> b;
+        const int gpc = wide ? 1 : 32 >> b;
         total += (a.bin_count[b] + gpc - 1) / gpc;
       }
     }
@@ -1724,13 +1887,16 @@ __global__ void __launch_bounds__(kSpecAllThreads, 4) fd_spec_all_kernel(SpecAll
       __syncthreads();
       cur = b;
     }
-    const int gpc = 32 >> b;
+    const int gpc = wide ? 1 : 32 >> b;
     const int base = (unit - ustart[q]) * gpc;
     const int count = a.bin_count[b];
     const int *bl = a.bin_list + (size_t)b * a.cap;
     const C *series = reinterpret_cast<const C *>(a.series) + bin_sample_start(a.bin_count, a.NFFT, b) * 4;
     if constexpr (MIX) {
       spec_unit_mix_rt<PERCH>(a, bl, count, base, b + 5, series, tw, bufs, reds);
+      continue;
+    } else if (wide) {
+      spec_unit_wide64<PERCH>(a, bl, base, b + 5, series, tw, bufs, reds);
       continue;
     }
     switch (b) {
