@@ -1924,6 +1924,19 @@ __global__ void __launch_bounds__(kSpecAllThreads, MIX ? 4 : 2) fd_spec_all_kern
   }
 }
 
+// Grids of the persistent kernels: what fills the chip, or less where the batch
+// cannot hold that many units, as a launch's CTAs cost time whether or not they
+// find work (1824 idle ones 4.6 us): a proposal has at most one unit of the spectral
+// stage, and at most slow_chunks(NFFT) chunks of 32 samples.
+static inline int grid_for(int full, long long units) {
+  return (int)(units < full ? (units > 0 ? units : 1) : full);
+}
+static inline long long slow_chunks(int NFFT) {
+  int n = kMaxN;
+  while (n > NFFT && n > 32) n >>= 1;
+  return n / 32;
+}
+
 template <bool MIX, bool PERCH = false>
 static cudaError_t launch_spec_all(const SpecAllArgs &A, int num_sms, cudaStream_t stream, int cap = 0) {
   const size_t smem = SpecAllSmem<MIX>::bytes;
@@ -1937,7 +1950,7 @@ static cudaError_t launch_spec_all(const SpecAllArgs &A, int num_sms, cudaStream
   }, &occ);
   if (e != cudaSuccess) return e;
   if (cap > 0 && cap < occ) occ = cap;
-  fd_spec_all_kernel<MIX, PERCH><<<occ * num_sms, kSpecAllThreads, smem, stream>>>(A);
+  fd_spec_all_kernel<MIX, PERCH><<<grid_for(occ * num_sms, A.a.nitems), kSpecAllThreads, smem, stream>>>(A);
   return cudaGetLastError();
 }
 
@@ -1973,7 +1986,9 @@ static cudaError_t launch_slow(const SlowArgs &a, int num_sms, cudaStream_t stre
   }, &occ);
   if (e != cudaSuccess) return e;
   if (cap > 0 && cap < occ) occ = cap;
-  fd_slow_kernel<MIX, BLOCK><<<occ * num_sms, BLOCK, 0, stream>>>(a);
+  const long long chunks = a.nitems * slow_chunks(a.NFFT);
+  const int grid = grid_for(occ * num_sms, MIX ? (chunks + BLOCK / 32 - 1) / (BLOCK / 32) : chunks);
+  fd_slow_kernel<MIX, BLOCK><<<grid, BLOCK, 0, stream>>>(a);
   return cudaGetLastError();
 }
 

@@ -354,7 +354,7 @@ static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) 
   }, &ncl);
   if (e != cudaSuccess) return e;
   if (ncl < 1) ncl = 1;
-  cfg.gridDim = dim3(4 * ncl);
+  cfg.gridDim = dim3(4 * grid_for(ncl, a.nitems));
   return cudaLaunchKernelEx(&cfg, fd_hp_kernel<PERCH>, a);
 }
 
@@ -386,7 +386,8 @@ cudaError_t fd_launch_reeval(const SlowArgs &sa, const HpArgs &h, bool perch, in
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, fd_slow_hp_kernel, 96, 0);
   }, &occ);
   if (e != cudaSuccess) return e;
-  fd_slow_hp_kernel<<<(occ > 0 ? occ : 1) * num_sms, 96, 0, stream>>>(sa);
+  const int full = (occ > 0 ? occ : 1) * num_sms;
+  fd_slow_hp_kernel<<<grid_for(full, sa.nitems * slow_chunks(sa.NFFT)), 96, 0, stream>>>(sa);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   e = perch ? launch_hp<true>(h, num_sms, stream) : launch_hp<false>(h, num_sms, stream);
   if (nlaunch) *nlaunch += 2;
