@@ -78,6 +78,35 @@ inline cudaError_t launch_setup(LaunchSetup &s, Init init, int *occ) {
   return cudaSuccess;
 }
 
+// Launch of a kernel of a chain, its start overlapped with the end of the one
+// before it in the stream (programmatic dependent launch): its CTAs are placed as
+// that one's leave, and each begins with grid_begin(), which waits until every
+// earlier kernel of the chain has finished and its writes are visible.  Every CTA
+// passes there before anything else, so that a kernel's end implies the ends of all
+// before it.  After anything but a kernel, an ordinary launch.  A boundary between
+// two small kernels in a stream 4.1 -> 1.6 us (in a graph 1.2 -> 1.0); five
+// kernels of a batch of 3072 mixed proposals 92 -> 71 us.  (No kernel lets the
+// next one be placed earlier, by griddepcontrol.launch_dependents: with that at the
+// start of each, the waiting CTAs take room from the running kernel's
+// neighbours, and the same batch takes 102 us.)
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+__device__ __forceinline__ void grid_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Physical constants, identical to utils/src/glass_constants.h:31-89 and
 // utils/src/glass_lisa.h:31 (the carrier phase multiplies them by ~1e5, so
 // they must be the same doubles as the reference's).

@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
   __shared__ double2 s_sc[2][32];  // sine, cosine of phi and of 2 psi
   __shared__ double s_sth[32], s_amp[32], s_cthsth[32];
   __shared__ int s_st[32], s_N[32];
+  grid_begin();
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, P = a.per_cta;
   const int i0 = blockIdx.x * P, n = min(P, a.nitems - i0);
   const int i = i0 + l;
@@ -381,11 +382,10 @@ cudaError_t fd_launch_plan(PlanKind kind, PlanArgs a, const FdTablesDev &tab, in
   a.tw1024 = tab.tw64[fd_bin_of(kSincosTab)];
   const int grid = (a.nitems + a.per_cta - 1) / a.per_cta;
   switch (kind) {
-    case kPlanF64: fd_plan_kernel<kPlanF64><<<grid, 128, 0, stream>>>(a); break;
-    case kPlanMix: fd_plan_kernel<kPlanMix><<<grid, 128, 0, stream>>>(a); break;
-    default: fd_plan_kernel<kPlanGrad><<<grid, 128, 0, stream>>>(a); break;
+    case kPlanF64: return launch_chained(fd_plan_kernel<kPlanF64>, grid, 128, 0, stream, a);
+    case kPlanMix: return launch_chained(fd_plan_kernel<kPlanMix>, grid, 128, 0, stream, a);
+    default: return launch_chained(fd_plan_kernel<kPlanGrad>, grid, 128, 0, stream, a);
   }
-  return cudaGetLastError();
 }
 
 // Sets a CUDA-graph conditional node's value to (*count > 0).
@@ -743,7 +743,10 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   }
   for (int b = kSpecAllBins; b < kSpecAllBins + nb; b++)
     if ((e = cudaStreamWaitEvent(stream, work.join[b], 0)) != cudaSuccess) return e;
-  if (nb > 0 || nall == 0) {  // the size counts only: fb_count follows them
+  // the size counts only: fb_count follows them (the re-evaluation's first kernel
+  // zeroes them where it runs in any case)
+  const bool counts_left = nb > 0 || nall == 0;
+  if (counts_left && (!fallback || cond)) {
     if ((e = cudaMemsetAsync(work.bin_count, 0, sizeof(int) * kNumBins, stream)) != cudaSuccess) return e;
   }
   if (timing && (e = cudaEventRecord(work.phase[3], stream)) != cudaSuccess) return e;
@@ -757,6 +760,7 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
     SlowArgs sh = sa;
     sh.bin_count = work.hp_count;
     sh.bin_list = work.hp_list;
+    sh.zero_counts = counts_left && !cond ? work.bin_count : nullptr;
     sh.series = work.series2;
     sh.series_len = (long long)(work.series_bytes / sizeof(float4));
     for (int b = 0; b < kNumBins; b++) sh.geolo[b] = tab.geolo[b];

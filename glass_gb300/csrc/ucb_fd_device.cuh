@@ -880,6 +880,7 @@ struct SlowArgs {
   // extents for the checked build: proposals, and series elements
   int nitems = 0;
   long long series_len = 0;
+  int *zero_counts = nullptr;  // re-evaluation: non-null, the kNumBins size counts there are left at zero
 };
 
 // Stage 2: FFTs, TDI weights, whitening and the residual power, per size.
@@ -980,6 +981,7 @@ __device__ __forceinline__ long long bin_sample_start(const int *bin_count, int 
 template <bool MIX, int BLOCK = 256>
 __global__ void __launch_bounds__(BLOCK) fd_slow_kernel(SlowArgs a) {
   using C = typename std::conditional<MIX, float2, double2>::type;
+  grid_begin();
   // chunk offsets per size (chunks of 32 samples: N/32 = 2^b per proposal), in registers
   int cs[kNumBins + 1];
   int acc = 0;
@@ -1842,6 +1844,7 @@ __global__ void __launch_bounds__(kSpecAllThreads, MIX ? 4 : 2) fd_spec_all_kern
   using C = typename SpecAllSmem<MIX>::C;
   using TW = typename SpecAllSmem<MIX>::TW;
   const SpecArgs &a = A.a;
+  grid_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int SN = SpecAllSmem<MIX>::SN;
   TW *tw = reinterpret_cast<TW *>(smem_raw);
@@ -1950,8 +1953,8 @@ static cudaError_t launch_spec_all(const SpecAllArgs &A, int num_sms, cudaStream
   }, &occ);
   if (e != cudaSuccess) return e;
   if (cap > 0 && cap < occ) occ = cap;
-  fd_spec_all_kernel<MIX, PERCH><<<grid_for(occ * num_sms, A.a.nitems), kSpecAllThreads, smem, stream>>>(A);
-  return cudaGetLastError();
+  return launch_chained(fd_spec_all_kernel<MIX, PERCH>, grid_for(occ * num_sms, A.a.nitems), kSpecAllThreads, smem,
+                        stream, A);
 }
 
 // Launch of one size's kernel with a grid bounded by the SM count times the
@@ -1988,8 +1991,7 @@ static cudaError_t launch_slow(const SlowArgs &a, int num_sms, cudaStream_t stre
   if (cap > 0 && cap < occ) occ = cap;
   const long long chunks = a.nitems * slow_chunks(a.NFFT);
   const int grid = grid_for(occ * num_sms, MIX ? (chunks + BLOCK / 32 - 1) / (BLOCK / 32) : chunks);
-  fd_slow_kernel<MIX, BLOCK><<<grid, BLOCK, 0, stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(fd_slow_kernel<MIX, BLOCK>, grid, BLOCK, 0, stream, a);
 }
 
 }  // namespace glass

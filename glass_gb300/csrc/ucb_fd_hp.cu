@@ -105,6 +105,9 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
   __shared__ dc s_d[6][32], s_m[3][32];
   __shared__ float2 s_kd[3][32];
   __shared__ float4 s_tab[64];
+  grid_begin();
+  // the batch's size counts, which the spectral stage has read for the last time
+  if (a.zero_counts && blockIdx.x == 0 && threadIdx.x < kNumBins) a.zero_counts[threadIdx.x] = 0;
   int cs[kNumBins + 1];
   int acc = 0;
 #pragma unroll
@@ -233,6 +236,7 @@ template <bool PERCH>
 __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
+  grid_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 red[32];
   __shared__ float4 s_part[2];  // this CTA's {rr hi, rr lo, hw hi, hw lo}, by turns
@@ -332,7 +336,7 @@ template <bool PERCH>
 static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) {
   const size_t smem = hp_smem_bytes(a.nmax);
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 4;
   attr[0].val.clusterDim.y = 1;
@@ -342,6 +346,8 @@ static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_chained
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   static LaunchSetup setup[kNumBins];
   int ncl = 0;
   cudaError_t e = launch_setup(setup[fd_bin_of(a.nmax)], [&](int *o) {
@@ -355,6 +361,7 @@ static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) 
   if (e != cudaSuccess) return e;
   if (ncl < 1) ncl = 1;
   cfg.gridDim = dim3(4 * grid_for(ncl, a.nitems));
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, fd_hp_kernel<PERCH>, a);
 }
 
@@ -387,8 +394,8 @@ cudaError_t fd_launch_reeval(const SlowArgs &sa, const HpArgs &h, bool perch, in
   }, &occ);
   if (e != cudaSuccess) return e;
   const int full = (occ > 0 ? occ : 1) * num_sms;
-  fd_slow_hp_kernel<<<grid_for(full, sa.nitems * slow_chunks(sa.NFFT)), 96, 0, stream>>>(sa);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = launch_chained(fd_slow_hp_kernel, grid_for(full, sa.nitems * slow_chunks(sa.NFFT)), 96, 0, stream, sa);
+  if (e != cudaSuccess) return e;
   e = perch ? launch_hp<true>(h, num_sms, stream) : launch_hp<false>(h, num_sms, stream);
   if (nlaunch) *nlaunch += 2;
   return e;
