@@ -794,6 +794,27 @@ static int dlogl_host_enqueue(glass_gpu_ctx *ctx, int precision, int nitems, boo
   return GLASS_OK;
 }
 
+// A small batch: the kernels read the inputs from the pinned staging block and
+// write the results there, with no copy or gather and scatter kernels between
+// (five launches to three in FP64; a call of 21 mixed proposals 47.5 -> 32.6 us, of
+// one in FP64 36.7 -> 32.2).  The block's
+// layout is dlogl_host_enqueue's.
+static int dlogl_small_enqueue(glass_gpu_ctx *ctx, int precision, int nitems, bool has_tx, size_t out_off) {
+  const size_t nd = (size_t)nitems;
+  char *h = (char *)ctx->h_stage;
+  double *h_params = (double *)h, *h_tx = h_params + 8 * nd;
+  int *h_seg = (int *)(h_tx + nd);
+  double *h_dl = (double *)(h + out_off), *h_ty = h_dl + nd, *h_hh = h_ty + nd;
+  int *h_st = (int *)(h_hh + nd);
+  int nl = 0;
+  const cudaError_t e =
+      fd_dlogl_launch(ctx->bank, ctx->tab, ctx->work, precision, nitems, h_seg, h_params, has_tx ? h_tx : nullptr, h_dl,
+                      h_ty, h_hh, h_st, ctx->n_fixed, ctx->num_sms, ctx->stream, &nl, nullptr, (double *)ctx->d_stage);
+  ctx->last_launches = nl;
+  if (e != cudaSuccess) return cuda_err(e, "dlogl_batch_host launch");
+  return GLASS_OK;
+}
+
 extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int nitems, const int *item_seg,
                                           const double *params, const double *term_x, double *dlogl,
                                           double *term_y, double *hh, int *status) {
@@ -813,7 +834,9 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
   const size_t out_bytes = sizeof(double) * 3 * nd + sizeof(int) * nd;
   const size_t bytes = out_off + out_bytes;
   cudaStream_t s = ctx->stream;
-  if (ctx->host_direct) {
+  const bool small = nitems <= kSmallBatch;
+  if (ctx->n_fixed > ctx->bank.NFFT) return set_err(GLASS_ERR_SIZE, "dlogl_batch: template size above NFFT");
+  if (ctx->host_direct && !small) {
     // + the device copy of the pointer block
     if ((rc = ensure_stage(ctx, out_off + (out_bytes + 15) / 16 * 16 + sizeof(HostIo)))) return rc;
     if ((rc = ensure_work(ctx, nitems))) return rc;
@@ -855,8 +878,12 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
   }
   // buffers first, so that nothing is reallocated while a graph is recorded
   if ((rc = ensure_stage(ctx, bytes))) return rc;
-  if ((rc = ensure_host_stage(ctx, bytes))) return rc;
+  if ((rc = ensure_host_stage(ctx, bytes < (size_t)kSmallBatch * 128 ? (size_t)kSmallBatch * 128 : bytes))) return rc;
   if ((rc = ensure_work(ctx, nitems))) return rc;
+  auto enqueue = [&] {
+    return small ? dlogl_small_enqueue(ctx, precision, nitems, has_tx, out_off)
+                 : dlogl_host_enqueue(ctx, precision, nitems, has_tx, in_bytes, out_off, out_bytes);
+  };
   char *h = (char *)ctx->h_stage;
   memcpy(h, params, sizeof(double) * 8 * nd);
   if (has_tx) memcpy(h + sizeof(double) * 8 * nd, term_x, sizeof(double) * nd);
@@ -867,7 +894,7 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
     GLASS_CUDA(cudaGraphLaunch(it->second, s), "dlogl_batch_host graph launch");
     ctx->last_launches = 3;
   } else {
-    if ((rc = dlogl_host_enqueue(ctx, precision, nitems, has_tx, in_bytes, out_off, out_bytes))) return rc;
+    if ((rc = enqueue())) return rc;
     GLASS_CUDA(cudaStreamSynchronize(s), "dlogl_batch_host sync");
     if (!ctx->work.phase_timing && ctx->host_graphs.size() < 64) {
       // record the sequence for the next calls of this shape (a stream that
@@ -876,7 +903,7 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
       cudaGraph_t g = nullptr;
       cudaGraphExec_t ge = nullptr;
       if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const int rc2 = dlogl_host_enqueue(ctx, precision, nitems, has_tx, in_bytes, out_off, out_bytes);
+        const int rc2 = enqueue();
         const cudaError_t e2 = cudaStreamEndCapture(s, &g);
         if (rc2 == GLASS_OK && e2 == cudaSuccess && cudaGraphInstantiate(&ge, g, 0) == cudaSuccess)
           ctx->host_graphs[key] = ge;

@@ -164,17 +164,25 @@ __global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
   __shared__ double2 s_sc[2][32];  // sine, cosine of phi and of 2 psi
   __shared__ double s_sth[32], s_amp[32], s_cthsth[32];
   __shared__ int s_st[32], s_N[32];
+  __shared__ double s_p[32][9];  // parameters, rows of 9 against bank conflicts
   grid_begin();
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, P = a.per_cta;
   const int i0 = blockIdx.x * P, n = min(P, a.nitems - i0);
   const int i = i0 + l;
-  const double *p = a.params + 8 * (size_t)i;
+  // one trip for all of a CTA's inputs, which may be pinned host memory that
+  // changes between two replays of a graph: read through (ld.cv) and once
+  int seg = -1;
+  if (w == 1 && l < n) seg = __ldcv(a.item_seg + i);
+  if (w == 2 && l < n && a.term_x_dev) a.term_x_dev[i] = __ldcv(a.term_x + i);
+  for (int q = threadIdx.x; q < 8 * n; q += 128) s_p[q >> 3][q & 7] = __ldcv(a.params + 8 * (size_t)i0 + q);
+  __syncthreads();
+  const double *const p = s_p[l];
   ItemMix *const m = KIND == kPlanGrad ? &a.itemsgrad[l < n ? i : i0].m : a.itemsmix + (l < n ? i : i0);
   ItemF64 *const c64 = a.items64 + (l < n ? i : i0);
   if (w == 0) {
     for (int q = l; q < 2 * n; q += 32) {
       const int t = q >= n, j = t ? q - n : q;
-      const double *pj = a.params + 8 * (size_t)(i0 + j);
+      const double *pj = s_p[j];
       const double x = t ? 2. * pj[5] : pj[2];
       double s, c;
       sincos_tab(x, a.tw1024, &s, &c);
@@ -196,7 +204,6 @@ __global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
     if (l < n) {
       double v[8];
       int st = 0;
-      const int seg = a.item_seg[i];
 #pragma unroll
       for (int k = 0; k < 8; k++) {
         v[k] = p[k];
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
   for (int q = threadIdx.x; q < (KIND == kPlanF64 ? 2 : 8) * n; q += 128) {
     const int role = q / n, j = q - role * n;
     if (s_st[j]) continue;
-    const double *pj = a.params + 8 * (size_t)(i0 + j);
+    const double *pj = s_p[j];
     const double cth = pj[1], ci = pj[4], sth = s_sth[j];
     const double sph = s_sc[0][j].x, cph = s_sc[0][j].y, s2 = s_sc[1][j].x, c2 = s_sc[1][j].y;
     const double amp = scale_pow2(s_amp[j], -(32 - __clz(s_N[j])));  // amp / (2N), N a power of two
@@ -583,7 +590,7 @@ void fd_build_bank_tables(int format, double T, double fstar, int NFFT, int nseg
 cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWorkDev &work, int precision,
                             int nitems, const int *item_seg, const double *params, const double *term_x,
                             double *dlogl, double *term_y, double *hh, int *status, int n_fixed, int num_sms,
-                            cudaStream_t stream, int *nlaunch, double *term_ch) {
+                            cudaStream_t stream, int *nlaunch, double *term_ch, double *term_x_dev) {
   cudaError_t e;
   int launches = 0;
   const bool mix = precision == 1;
@@ -606,6 +613,8 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   pa.item_seg = item_seg;
   pa.params = params;
   pa.term_x = term_x;
+  pa.term_x_dev = term_x ? term_x_dev : nullptr;
+  if (pa.term_x_dev) term_x = pa.term_x_dev;  // what the later kernels read
   pa.seg_qmin = bank.qmin;
   pa.items64 = work.items64;
   pa.itemsmix = work.itemsmix;
@@ -687,14 +696,15 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
     a.fb_nscale = work.fb_nscale;
   }
   const bool perch = term_ch != nullptr;
-  // Inside a CUDA-graph capture, the re-evaluation (three launches, idle in
+  // Inside a CUDA-graph capture, the re-evaluation (two launches, idle in
   // batches with nothing listed) sits behind a conditional node that a
-  // one-thread kernel sets when something is listed; outside capture, or
-  // where the graph API refuses, it is launched unconditionally.
+  // one-thread kernel sets when something is listed; outside capture, where
+  // the graph API refuses, or for a batch so small that its two launches take
+  // less than the node, it is launched unconditionally.
   bool cond = false;
   cudaGraphConditionalHandle cond_h = 0;
   cudaGraph_t cap_graph = nullptr;
-  if (fallback) {
+  if (fallback && nitems > kSmallBatch) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamGetCaptureInfo(stream, &cs, nullptr, &cap_graph) == cudaSuccess &&
         cs == cudaStreamCaptureStatusActive &&

@@ -99,11 +99,18 @@ void fd_build_bank_tables(int format, double T, double fstar, int NFFT, int nseg
 cudaError_t fd_build_orbit_tables(FdTablesDev &tab, double T, double t0, cudaStream_t stream);
 
 // Enqueue plan + per-size kernels.  Returns the number of kernel launches
-// through *nlaunch.
+// through *nlaunch.  item_seg, params and term_x may be pinned host memory when
+// term_x_dev (room for nitems doubles on the device) is given, the outputs
+// always.
 cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWorkDev &work, int precision,
                             int nitems, const int *item_seg, const double *params, const double *term_x,
                             double *dlogl, double *term_y, double *hh, int *status, int n_fixed, int num_sms,
-                            cudaStream_t stream, int *nlaunch, double *term_ch = nullptr);
+                            cudaStream_t stream, int *nlaunch, double *term_ch = nullptr,
+                            double *term_x_dev = nullptr);
+// Batches of up to this many proposals: the host-pointer entry has the kernels
+// read and write pinned memory in place, and a graph holds the re-evaluation
+// unconditionally.
+constexpr int kSmallBatch = 256;
 
 // Bytes of series scratch a batch of nitems proposals on segments of NFFT bins
 // can need (every N is at most NFFT).

@@ -822,6 +822,7 @@ struct PlanArgs {
   const int *item_seg;
   const double *params;
   const double *term_x;
+  double *term_x_dev = nullptr;  // non-null: term_x (host memory) is copied there for the later kernels
   const int *seg_qmin;
   ItemF64 *items64 = nullptr;     // kPlanF64
   ItemMix *itemsmix = nullptr;    // kPlanMix

@@ -215,12 +215,14 @@ int glass_gpu_dlogl_batch(glass_gpu_ctx *ctx, int precision, int nitems, const i
  * host memory in place through the host's page tables (a coherent CPU-GPU
  * link), a gather kernel reads the caller's arrays and a scatter kernel
  * writes the results into them; otherwise the inputs go through one pinned
- * staging buffer of the context (one copy each way).  Either sequence for a
+ * staging buffer of the context (one copy each way); the kernels of a batch of
+ * up to 256 proposals, in either mode, read and write that buffer in place.
+ * Each sequence for a
  * batch shape (nitems, precision, term_x given or not) is recorded as a CUDA
  * graph on the first call and replayed on later calls of that shape; a new
  * bank, a new template size or larger buffers drop the recorded graphs.  Not
  * to be called while the context's stream is being captured.
- * In the in-place mode the GPU itself reads item_seg, params and term_x and
+ * In the in-place mode (above 256 proposals) the GPU itself reads item_seg, params and term_x and
  * writes dlogl, term_y, hh and status: every array must be valid, mapped
  * memory of this process for nitems elements until the call returns.  A bad
  * pointer is then a GPU memory fault, not a host crash, and it leaves the

@@ -96,3 +96,31 @@ def test_any_batch_gives_the_same(engine, n):
         _, ty, _, st = engine.dlogl_host((idx % 3).astype(np.int32), base[idx], precision=prec)
         assert (st == 0).all()
         np.testing.assert_allclose(ty, np.array(one)[idx], rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("n", [1, 5, 255, 256, 257])
+def test_host_calls_of_small_batches(engine, n):
+    """Up to 256 proposals the kernels read and write pinned memory in place: the
+    same bits as the device entry, whose kernels they are, for new arrays in every
+    call of one shape (the first records a graph), with and without term_x, and
+    for proposals that are skipped."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    f0s = np.array([1e-3, 4e-3, 1.1e-2])
+    engine.upload(_bank(rng, f0s))
+    dev = lambda x: torch.tensor(x, device="cuda")
+    for prec in (gg.PREC_FP64, gg.PREC_MIXED):
+        for k in range(4):
+            seg = (np.arange(n) % 3).astype(np.int32)
+            p = np.array([_source(rng, f0s[s], lnA=rng.uniform(-52, -49), costh=rng.uniform(-1, 1)) for s in seg])
+            if k == 2:
+                p[0, 1] = 1.5  # not a cosine: status 1
+                p[-1, 0] += 1e6  # outside its segment: status 4
+            tx = rng.normal(0, 5, n) if k % 2 else None
+            got = engine.dlogl_host(seg, p, term_x=tx, precision=prec)
+            out = [dev(np.zeros(n)) for _ in range(3)] + [dev(np.zeros(n, np.int32))]
+            engine.dlogl_device(dev(seg), dev(p), *out, None if tx is None else dev(tx), prec)
+            torch.cuda.synchronize()
+            for a, b in zip(got, out):
+                np.testing.assert_array_equal(a, b.cpu().numpy())
