@@ -701,11 +701,27 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
   a.status = status;
   if ((e = cudaEventRecord(work.fork, stream)) != cudaSuccess) return e;
   int nb = 0;
-  for (int b = 0; b < kNumBins; b++) {
+  while (nb < kNumBins && 32 << nb <= pa.NFFT) nb++;
+  // largest size first, on the caller's stream: its groups take whole SMs, and
+  // the smaller sizes fill in behind them as it ends (the other way round it
+  // waits for SMs to empty, and ends the call alone)
+  bool forked[kNumBins] = {};
+  auto join = [&] {
+    cudaError_t r = cudaSuccess;
+    for (int b = 0; b < nb; b++)
+      if (forked[b]) {
+        const cudaError_t rb = cudaStreamWaitEvent(stream, work.join[b], 0);
+        if (r == cudaSuccess) r = rb;
+      }
+    return r;
+  };
+  for (int b = nb - 1; b >= 0; b--) {
     const int N = 32 << b;
-    if (N > pa.NFFT) break;
-    cudaStream_t sb = work.side[b];
-    if ((e = cudaStreamWaitEvent(sb, work.fork, 0)) != cudaSuccess) return e;
+    cudaStream_t sb = b == nb - 1 ? stream : work.side[b];
+    if (sb != stream && (e = cudaStreamWaitEvent(sb, work.fork, 0)) != cudaSuccess) {
+      join();
+      return e;
+    }
     a.bin = b;
     a.bin_list = work.bin_list + (size_t)b * work.cap;
     a.tw = tab.tw32[b];
@@ -723,16 +739,17 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
     }
     launches++;
     // the branch is joined to the caller's stream even when its launch failed
-    const cudaError_t ej = cudaEventRecord(work.join[b], sb);
-    nb++;
-    if (e == cudaSuccess) e = ej;
+    if (sb != stream) {
+      const cudaError_t ej = cudaEventRecord(work.join[b], sb);
+      forked[b] = ej == cudaSuccess;
+      if (e == cudaSuccess) e = ej;
+    }
     if (e != cudaSuccess) {
-      for (int q = 0; q < nb; q++) cudaStreamWaitEvent(stream, work.join[q], 0);
+      join();
       return e;
     }
   }
-  for (int b = 0; b < nb; b++)
-    if ((e = cudaStreamWaitEvent(stream, work.join[b], 0)) != cudaSuccess) return e;
+  if ((e = join()) != cudaSuccess) return e;
   // leave the counts at zero for the next launch sequence
   if ((e = cudaMemsetAsync(work.bin_count, 0, sizeof(int) * (kNumBins + 1), stream)) != cudaSuccess) return e;
   work.counts_zero = true;
