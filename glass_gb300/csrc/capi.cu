@@ -1923,7 +1923,7 @@ static cudaError_t legacy_enqueue(LegacyThread &L, int fmt, double T, int BW, in
   if (e != cudaSuccess) return e;
   e = fd_waveform_launch(reinterpret_cast<const OrbitSample64 *>(L.d_in + LegacyThread::kPosOffset),
                          reinterpret_cast<const ItemF64 *>(L.d_in), BW, fmt, NI, T, fstar_of_orbit(), L.d_d6, L.d_out,
-                         L.tab.tw64[bin_index(BW)], L.tab.tw64[bin_index(kSincosTab)], s);
+                         L.tab.tt64[bin_index(BW)], L.tab.tw64[bin_index(kSincosTab)], s);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(L.h_out, L.d_out, sizeof(double) * nout, cudaMemcpyDeviceToHost, s);
 }
@@ -2202,6 +2202,7 @@ extern "C" int glass_gpu_wdm_by_layers_host(glass_gpu_ctx *ctx, int NF, int NT, 
   if (rc) return rc;
   std::vector<double2> tw((size_t)N);
   wdm_unit_roots((int)N, tw.data());
+  for (double2 &w : tw) w = tan_form(w.x, w.y);
   const size_t nwin = (size_t)NT / 2 + 1;
   const size_t bytes = sizeof(double2) * N + sizeof(double) * (N + nwin);
   void *mem = nullptr;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64_math.cuh"
+
 namespace glass {
 namespace {
 
@@ -62,12 +64,13 @@ __device__ __forceinline__ C mkc(decltype(C::x) x, decltype(C::x) y) {
 
 // In-place mixed-radix FFTs of nser series a[L], back to back, each held in
 // digit-reversed order; results in natural order.  tw[j * twmul] = e^{-2 pi i j /
-// L}; sign -1 forward, +1 inverse (unnormalised).  Whole CTA.  C = double2 or
-// float2.  In FP64 3.5 instructions per point and factor of two (28 per radix-4
-// butterfly), the first stage without its factors.
-template <typename C>
-__device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ tw, int twmul, int sign,
-                        int nser = 1) {
+// L}, in FP64 in tangent form (tan_form); SIGN -1 forward, +1 inverse
+// (unnormalised).  Whole CTA.  C = double2 or float2.  In FP64 3 instructions
+// per point and factor of two (24 per radix-4 butterfly), the first stage without
+// its factors.
+template <int SIGN, typename C>
+__device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ tw, int twmul, int nser = 1) {
+  constexpr int sign = SIGN;
   using R = decltype(C::x);
   constexpr bool kF64 = sizeof(R) == 8;
   int p = 1;
@@ -81,7 +84,22 @@ __device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ t
       if (Rd == 4) {
         C *const x2 = a + i0 + 2 * p, *const x3 = a + i0 + 3 * p;
         C v0 = *x0, v1 = *x1, v2 = *x2, v3 = *x3;
-        if (!kF64 || st > 0) {  // FP64: the first stage's factors are 1
+        if constexpr (kF64) {
+          if (st > 0) {
+            C w1 = tw[k * tstep], w2 = tw[2 * k * tstep];
+            if (sign > 0) {
+              w1.y = -w1.y;
+              w2.y = -w2.y;
+            }
+            tan_radix4<SIGN>(v0, v1, v2, v3, w1, w2);
+          } else {  // the first stage's factors are 1
+            plain_radix4<SIGN>(v0, v1, v2, v3);
+          }
+          *x0 = v0;
+          *x1 = v1;
+          *x2 = v2;
+          *x3 = v3;
+        } else {
           C w1 = tw[k * tstep], w2 = tw[2 * k * tstep], w3 = tw[3 * k * tstep];
           if (sign > 0) {
             w1.y = -w1.y;
@@ -91,21 +109,25 @@ __device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ t
           v1 = cmul(v1, w1);
           v2 = cmul(v2, w2);
           v3 = cmul(v3, w3);
+          const C t0 = mkc<C>(v0.x + v2.x, v0.y + v2.y), t1 = mkc<C>(v0.x - v2.x, v0.y - v2.y);
+          const C t2 = mkc<C>(v1.x + v3.x, v1.y + v3.y), t3 = mkc<C>(v1.x - v3.x, v1.y - v3.y);
+          const C t3r = sign < 0 ? mkc<C>(t3.y, -t3.x) : mkc<C>(-t3.y, t3.x);
+          *x0 = mkc<C>(t0.x + t2.x, t0.y + t2.y);
+          *x1 = mkc<C>(t1.x + t3r.x, t1.y + t3r.y);
+          *x2 = mkc<C>(t0.x - t2.x, t0.y - t2.y);
+          *x3 = mkc<C>(t1.x - t3r.x, t1.y - t3r.y);
         }
-        const C t0 = mkc<C>(v0.x + v2.x, v0.y + v2.y), t1 = mkc<C>(v0.x - v2.x, v0.y - v2.y);
-        const C t2 = mkc<C>(v1.x + v3.x, v1.y + v3.y), t3 = mkc<C>(v1.x - v3.x, v1.y - v3.y);
-        const C t3r = sign < 0 ? mkc<C>(t3.y, -t3.x) : mkc<C>(-t3.y, t3.x);
-        *x0 = mkc<C>(t0.x + t2.x, t0.y + t2.y);
-        *x1 = mkc<C>(t1.x + t3r.x, t1.y + t3r.y);
-        *x2 = mkc<C>(t0.x - t2.x, t0.y - t2.y);
-        *x3 = mkc<C>(t1.x - t3r.x, t1.y - t3r.y);
       } else if (Rd == 2) {
         C v0 = *x0, v1 = *x1;
         C w1 = tw[k * tstep];
         if (sign > 0) w1.y = -w1.y;
-        v1 = cmul(v1, w1);
-        *x0 = mkc<C>(v0.x + v1.x, v0.y + v1.y);
-        *x1 = mkc<C>(v0.x - v1.x, v0.y - v1.y);
+        if constexpr (kF64) {
+          tan_radix2(v0, v1, w1, *x0, *x1);
+        } else {
+          v1 = cmul(v1, w1);
+          *x0 = mkc<C>(v0.x + v1.x, v0.y + v1.y);
+          *x1 = mkc<C>(v0.x - v1.x, v0.y - v1.y);
+        }
       } else {
         C *const x2 = a + i0 + 2 * p;
         C v0 = *x0, v1 = *x1, v2 = *x2;
@@ -115,8 +137,13 @@ __device__ void dit_fft(C *a, int L, const RadixPlan &P, const C *__restrict__ t
             w1.y = -w1.y;
             w2.y = -w2.y;
           }
-          v1 = cmul(v1, w1);
-          v2 = cmul(v2, w2);
+          if constexpr (kF64) {
+            v1 = tan_mul(v1, w1);
+            v2 = tan_mul(v2, w2);
+          } else {
+            v1 = cmul(v1, w1);
+            v2 = cmul(v2, w2);
+          }
         }
         const R s3 = (R)0.86602540378443864676 * (R)sign;
         const C sm = mkc<C>(v1.x + v2.x, v1.y + v2.y), df = mkc<C>(v1.x - v2.x, v1.y - v2.y);

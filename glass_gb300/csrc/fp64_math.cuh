@@ -157,4 +157,45 @@ __device__ __forceinline__ float to_f32(double x) {
   return e - 903u >= 246u ? (float)x : f32_nearest(x);
 }
 
+// FFT factors in tangent form (Linzer and Feig, IEEE Trans. Signal Process. 41,
+// 1993): c + i y is kept as (c, t = y / c), so that a +- (c + i y) b = a +- c (b.x - t
+// b.y + i (b.y + t b.x)) takes 6 multiply-adds, where the product and the sums
+// take 8, and a radix-4 butterfly, as two levels of these with the factors w
+// and w^2, 24 where it takes 28 with w, w^2 and w^3.  The rounding of t is a
+// relative one of y, so no angle loses accuracy; at c = 0, c = 2^-60 stands in.
+__host__ __device__ inline double2 tan_form(double c, double y) {
+  if (fabs(c) < 1e-15) c = 1.0 / 1152921504606846976.0;
+  return make_double2(c, y / c);
+}
+__device__ __forceinline__ double2 tan_mul(double2 b, double2 w) {
+  return make_double2(w.x * fma(-w.y, b.y, b.x), w.x * fma(w.y, b.x, b.y));
+}
+// p, m = a +- w b
+__device__ __forceinline__ void tan_radix2(double2 a, double2 b, double2 w, double2 &p, double2 &m) {
+  const double u = fma(-w.y, b.y, b.x), v = fma(w.y, b.x, b.y);
+  p = make_double2(fma(w.x, u, a.x), fma(w.x, v, a.y));
+  m = make_double2(fma(-w.x, u, a.x), fma(-w.x, v, a.y));
+}
+// The 4-point DFT (sign -1: forward) of v0, w v1, w^2 v2, w^3 v3; w2 = w^2.
+template <int SIGN>
+__device__ __forceinline__ void tan_radix4(double2 &v0, double2 &v1, double2 &v2, double2 &v3, double2 w, double2 w2) {
+  double2 a, b, p, q;
+  tan_radix2(v0, v2, w2, a, b);
+  tan_radix2(v1, v3, w2, p, q);
+  tan_radix2(a, p, w, v0, v2);
+  const double u = w.x * SIGN, r = fma(-w.y, q.y, q.x), i = fma(w.y, q.x, q.y);  // b +- SIGN i w q
+  v1 = make_double2(fma(-u, i, b.x), fma(u, r, b.y));
+  v3 = make_double2(fma(u, i, b.x), fma(-u, r, b.y));
+}
+// The same with w = 1: 16 additions.
+template <int SIGN>
+__device__ __forceinline__ void plain_radix4(double2 &v0, double2 &v1, double2 &v2, double2 &v3) {
+  const double2 a = make_double2(v0.x + v2.x, v0.y + v2.y), b = make_double2(v0.x - v2.x, v0.y - v2.y);
+  const double2 p = make_double2(v1.x + v3.x, v1.y + v3.y), q = make_double2(v1.x - v3.x, v1.y - v3.y);
+  v0 = make_double2(a.x + p.x, a.y + p.y);
+  v2 = make_double2(a.x - p.x, a.y - p.y);
+  v1 = SIGN < 0 ? make_double2(b.x + q.y, b.y - q.x) : make_double2(b.x - q.y, b.y + q.x);
+  v3 = SIGN < 0 ? make_double2(b.x - q.y, b.y + q.x) : make_double2(b.x + q.y, b.y - q.x);
+}
+
 }  // namespace glass

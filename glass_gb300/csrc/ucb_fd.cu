@@ -477,6 +477,7 @@ __global__ void fd_orbit_table_kernel(FdTablesDev tab, double T, double t0) {
   double s, cth;
   sincospi(-2.0 * (double)n / (double)N, &s, &cth);
   tab.tw64[b][n] = make_double2(cth, s);
+  tab.tt64[b][n] = tan_form(cth, s);
   tab.tw32[b][n] = make_float2((float)cth, (float)s);
   if (tab.tw32x[b]) {
     const float ch = (float)cth, sh = (float)s;
@@ -490,7 +491,7 @@ cudaError_t fd_build_orbit_tables(FdTablesDev &tab, double T, double t0, cudaStr
     for (int b = 0; b < kNumBins; b++) {
       int N = 32 << b;
       total += (size_t)N * (sizeof(OrbitSample64) + sizeof(OrbitSampleMix) + 2 * sizeof(GeoSampleMix) +
-                            sizeof(float2) + sizeof(double2) + sizeof(float4));
+                            sizeof(float2) + 2 * sizeof(double2) + sizeof(float4));
     }
     cudaError_t e = cudaMalloc(&tab.base, total);
     if (e != cudaSuccess) return e;
@@ -506,6 +507,8 @@ cudaError_t fd_build_orbit_tables(FdTablesDev &tab, double T, double t0, cudaStr
       tab.geolo[b] = (GeoSampleMix *)p;
       p += (size_t)N * sizeof(GeoSampleMix);
       tab.tw64[b] = (double2 *)p;
+      p += (size_t)N * sizeof(double2);
+      tab.tt64[b] = (double2 *)p;
       p += (size_t)N * sizeof(double2);
       tab.tw32[b] = (float2 *)p;
       p += (size_t)N * sizeof(float2);
@@ -727,7 +730,7 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
       if ((e = cudaStreamWaitEvent(sb, work.fork, 0)) != cudaSuccess) return e;
       a.bin = b;
       a.bin_list = work.bin_list + (size_t)b * work.cap;
-      a.tw = mix ? (const void *)tab.tw32x[b] : (const void *)tab.tw64[b];
+      a.tw = mix ? (const void *)tab.tw32x[b] : (const void *)tab.tt64[b];
       e = mix ? fd_launch_spec_mixed(N, a, nitems, num_sms, sb, perch)
               : fd_launch_spec_fp64(N, a, nitems, num_sms, sb, perch);
       launches++;
@@ -745,7 +748,7 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
     A.nbins = nall;
     A.zero_counts = nb == 0 ? work.bin_count : nullptr;  // side kernels would still be reading them
     A.done = work.bin_count + kNumBins + 1;  // fb_count is at kNumBins
-    for (int b = 0; b < kSpecAllBins; b++) A.tw[b] = mix ? (const void *)tab.tw32x[b] : (const void *)tab.tw64[b];
+    for (int b = 0; b < kSpecAllBins; b++) A.tw[b] = mix ? (const void *)tab.tw32x[b] : (const void *)tab.tt64[b];
     e = mix ? fd_launch_spec_all_mixed(A, num_sms, stream, perch, work.tune.spec_ctas_per_sm)
             : fd_launch_spec_all_fp64(A, num_sms, stream, perch);
     launches++;

@@ -32,7 +32,8 @@ struct FdTablesDev {
   GeoSampleMix *geolo[kNumBins] = {};  // the same minus its float rounding (double-float slow part)
   float2 *tw32[kNumBins] = {};
   float4 *tw32x[kNumBins] = {};  // the same twiddles as hi + lo floats (mixed likelihood)
-  double2 *tw64[kNumBins] = {};
+  double2 *tw64[kNumBins] = {};  // 1024: the sine/cosine table too
+  double2 *tt64[kNumBins] = {};  // the same in tangent form (tan_form): the FP64 FFTs'
   void *base = nullptr;  // single allocation backing all of the above
 };
 
@@ -164,7 +165,7 @@ cudaError_t fs_finalize(const double *logl0, const int *pos, const double *scan,
 // pos: N orbit samples (device), item: the source's FP64 constants (device,
 // from source_geometry + make_item_f64), d6: 6 N complex scratch, out: 10*N
 // doubles (device) = X,Y,Z,A,E.  tw: the N-point FP64 twiddle table
-// (FdTablesDev::tw64 of the size), tw1024: the 1024-point one.
+// (FdTablesDev::tt64 of the size), tw1024: the 1024-point one.
 cudaError_t fd_waveform_launch(const OrbitSample64 *pos, const ItemF64 *item, int N, int format, int NI, double T,
                                double fstar, double2 *d6, double *out, const double2 *tw, const double2 *tw1024,
                                cudaStream_t stream);

@@ -69,7 +69,8 @@ __device__ __forceinline__ void group_bar(int g) {
 // with sub-transform size p reads x[i + m N/R], applies exp(-2 pi i m k/(pR)),
 // k = i mod p, and writes y[(i-k)R + k + m p].  Every thread holds its
 // butterflies' inputs in registers between the two barriers of a stage, which
-// lets the stage overwrite its own input.  CH series are processed per round to
+// lets the stage overwrite its own input.  tw: in tangent form (tan_form), 24 FP64
+// instructions per butterfly.  CH series are processed per round to
 // bound register use; rounds touch disjoint series, so a round's loads need no
 // barrier after the previous round's stores, only one at the end of the stage.
 // SYNC_CTA: the group is the whole CTA, which may be a partial warp; else the
@@ -92,14 +93,13 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane, int g =
     const int step = N / (4 * p);
     // the thread's butterfly twiddles, shared by every series (all 1 in the
     // first stage)
-    C w[B4][3];
+    C w[B4][2];
     if (st > 0) {
 #pragma unroll
       for (int b = 0; b < B4; ++b) {
         const int k = (lane + GT * b) & (p - 1);
         w[b][0] = tw[k * step];
         w[b][1] = tw[2 * k * step];
-        w[b][2] = tw[3 * k * step];
       }
     }
 #pragma unroll
@@ -120,17 +120,15 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane, int g =
         for (int b = 0; b < B4; ++b) {
           int i = lane + GT * b;
           int k = i & (p - 1);
-          C u0 = v[s][b][0];
-          C u1 = st > 0 ? cmul(v[s][b][1], w[b][0]) : v[s][b][1];
-          C u2 = st > 0 ? cmul(v[s][b][2], w[b][1]) : v[s][b][2];
-          C u3 = st > 0 ? cmul(v[s][b][3], w[b][2]) : v[s][b][3];
-          C a = cadd(u0, u2), bb = csub(u0, u2), c = cadd(u1, u3), d = cmi(csub(u1, u3));
+          C *u = v[s][b];
+          if (st > 0)
+            tan_radix4<-1>(u[0], u[1], u[2], u[3], w[b][0], w[b][1]);
+          else
+            plain_radix4<-1>(u[0], u[1], u[2], u[3]);
           int j = (i - k) * 4 + k;
           C *o = buf + (c0 + s) * N + j;
-          o[0] = cadd(a, c);
-          o[p] = cadd(bb, d);
-          o[2 * p] = csub(a, c);
-          o[3 * p] = csub(bb, d);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) o[m * p] = u[m];
         }
     }
     sync();
@@ -160,10 +158,9 @@ __device__ __forceinline__ void group_fft(C *buf, const C *tw, int lane, int g =
         for (int b = 0; b < B2; ++b) {
           int i = lane + GT * b;
           int k = i & (p - 1);
-          C u1 = cmul(v[s][b][1], w[b]);
           int j = (i - k) * 2 + k;
-          buf[(c0 + s) * N + j] = cadd(v[s][b][0], u1);
-          buf[(c0 + s) * N + j + p] = csub(v[s][b][0], u1);
+          C *o = buf + (c0 + s) * N + j;
+          tan_radix2(v[s][b][0], v[s][b][1], w[b], o[0], o[p]);
         }
     }
     sync();
@@ -1728,7 +1725,7 @@ struct SpecAllSmem {
 
 // In-place FFTs of four series of N = 2^ln points, back to back, by the CTA: radix-4
 // decimation in time from digit-reversed order (hp_rev) and a radix-2 stage when
-// log2 N is odd; results in natural order.  tw[j] = exp(-2 pi i j / N).
+// log2 N is odd; results in natural order.  tw[j] = exp(-2 pi i j / N) in tangent form.
 static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const double2 *tw) {
   int lp = 0;
   for (; lp + 2 <= ln; lp += 2) {
@@ -1737,16 +1734,14 @@ static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const doub
       const int k = t & (p - 1);
       double2 *const y = x + ((t - k) << 2) + k;
       double2 v0 = y[0], v1 = y[p], v2 = y[2 * p], v3 = y[3 * p];
-      if (lp > 0) {
-        v1 = cmul(v1, tw[k << lt]);
-        v2 = cmul(v2, tw[2 * k << lt]);
-        v3 = cmul(v3, tw[3 * k << lt]);
-      }
-      const double2 a = cadd(v0, v2), b = csub(v0, v2), c = cadd(v1, v3), e = csub(v1, v3);
-      y[0] = cadd(a, c);
-      y[p] = make_double2(b.x + e.y, b.y - e.x);
-      y[2 * p] = csub(a, c);
-      y[3 * p] = make_double2(b.x - e.y, b.y + e.x);
+      if (lp > 0)
+        tan_radix4<-1>(v0, v1, v2, v3, tw[k << lt], tw[2 * k << lt]);
+      else
+        plain_radix4<-1>(v0, v1, v2, v3);
+      y[0] = v0;
+      y[p] = v1;
+      y[2 * p] = v2;
+      y[3 * p] = v3;
     }
     __syncthreads();
   }
@@ -1755,9 +1750,7 @@ static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const doub
     for (int t = threadIdx.x; t < 2 << ln; t += blockDim.x) {
       const int k = t & (p - 1);
       double2 *const y = x + ((t - k) << 1) + k;
-      const double2 v0 = y[0], v1 = cmul(y[p], tw[k]);
-      y[0] = cadd(v0, v1);
-      y[p] = csub(v0, v1);
+      tan_radix2(y[0], y[p], tw[k], y[0], y[p]);
     }
     __syncthreads();
   }

@@ -43,6 +43,7 @@ static __device__ __align__(256) double2 na_g64[4 * (size_t)kNaMaxBins];
 static __device__ __align__(256) OrbitSample64 na_pos64[kTableSamples];
 static __device__ __align__(256) OrbitSampleMix na_mix[kTableSamples];
 static __device__ __align__(256) double2 na_tw64[kTableSamples];
+static __device__ __align__(256) double2 na_tt64[kTableSamples];
 static __device__ __align__(256) float2 na_tw32[kTableSamples];
 static __device__ __align__(256) ItemF64 na_items[kNaMaxItems];
 static __device__ __align__(256) int na_bin_count[kNumBins];
@@ -51,7 +52,7 @@ static __device__ __align__(256) double2 na_series[4 * (size_t)kNaMaxSamples];
 
 struct NaAddrs {
   bool ready = false;
-  double2 *w64, *g64, *tw64, *series;
+  double2 *w64, *g64, *tw64, *tt64, *series;
   OrbitSample64 *pos64;
   OrbitSampleMix *mix;
   float2 *tw32;
@@ -75,6 +76,7 @@ cudaError_t na_setup(int dev, NaAddrs *&out) {
     if ((e = cudaGetSymbolAddress((void **)&a.pos64, na_pos64)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress((void **)&a.mix, na_mix)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress((void **)&a.tw64, na_tw64)) != cudaSuccess) return e;
+    if ((e = cudaGetSymbolAddress((void **)&a.tt64, na_tt64)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress((void **)&a.tw32, na_tw32)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress((void **)&a.items, na_items)) != cudaSuccess) return e;
     if ((e = cudaGetSymbolAddress((void **)&a.bin_count, na_bin_count)) != cudaSuccess) return e;
@@ -165,6 +167,7 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
     tab.pos64[b] = na->pos64 + off;
     tab.mix[b] = na->mix + off;
     tab.tw64[b] = na->tw64 + off;
+    tab.tt64[b] = na->tt64 + off;
     tab.tw32[b] = na->tw32 + off;
     off += (size_t)32 << b;
   }
@@ -248,7 +251,7 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
     if (N > NFFT) break;
     a.bin = b;
     a.bin_list = na->bin_list + (size_t)b * kNaMaxItems;
-    a.tw = tab.tw64[b];
+    a.tw = tab.tt64[b];
     if ((e = fd_launch_spec_fp64(N, a, nitems, na->num_sms, s, false)) != cudaSuccess)
       return report_cuda_error(e, "dlogl_fp64_noalloc: spectral kernels");
   }

@@ -635,7 +635,7 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
       const int N = 16 << b;
       if (N > maxN || N > kMaxN) break;
       ca.bin = b;
-      ca.tw = b == 0 ? tab.tw64[0] : tab.tw64[b - 1];
+      ca.tw = b == 0 ? tab.tt64[0] : tab.tt64[b - 1];
       ca.tw_stride = b == 0 ? 2 : 1;
       switch (N) {
         case 16: e = fs_launch_spec<16>(ca, n, num_sms, stream); break;

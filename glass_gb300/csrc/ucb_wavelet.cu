@@ -479,11 +479,11 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
 constexpr int kLayerThreads = 256;
 
 // Bin idx (0 <= idx <= M) of the real spectrum from the packed spectrum zb, times
-// 2 w: 10 FP64 instructions.
+// 2 w; e: its factor in tangent form.  10 FP64 instructions.
 __device__ __forceinline__ double2 real_bin2(const double2 *zb, int M, int idx, double2 e, double w) {
   const double2 zk = zb[idx == M ? 0 : idx], zm = zb[idx == 0 ? 0 : M - idx];
   const double sx = zk.x + zm.x, sy = zk.y - zm.y, dx = zk.x - zm.x, dy = zk.y + zm.y;
-  return make_double2(w * fma(e.x, dy, fma(e.y, dx, sx)), w * fma(-e.x, dx, fma(e.y, dy, sy)));
+  return make_double2(w * fma(e.x, fma(e.y, dx, dy), sx), w * fma(e.x, fma(e.y, dy, -dx), sy));
 }
 
 // The layers jmin .. jmin + nl - 1 from the packed spectrum zb of their N = NT
@@ -524,7 +524,7 @@ __device__ void layers_from_spectrum(const double2 *zb, double2 *lb, int M, int 
         if (kp != k) lb[digit_rev(pp < 0 ? pp + NT : pp, PN)] = make_double2(ax + by, bx - ay);
       }
       __syncthreads();
-      dit_fft(lb, NT, PN, tw, nl + 1, +1);
+      dit_fft<+1>(lb, NT, PN, tw, nl + 1);
       for (int t = threadIdx.x; t < NT; t += blockDim.x) {
         const double2 v = lb[t];
         out[(size_t)t * nl + off] = (t & 2) ? -v.x : v.x;
@@ -541,7 +541,7 @@ __device__ void layers_from_spectrum(const double2 *zb, double2 *lb, int M, int 
         lb[digit_rev(t, PN)] = v;
       }
       __syncthreads();
-      dit_fft(lb, NT, PN, tw, nl + 1, +1);
+      dit_fft<+1>(lb, NT, PN, tw, nl + 1);
       for (int t = threadIdx.x; t < NT; t += blockDim.x) {
         const double2 v = lb[t];
         double o;
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kLayerThreads) wv_layers_kernel(WvGridDev g, i
   }
   __syncthreads();
   const double2 *tw = g.tw[nl];
-  dit_fft(zb, M, PM, tw, 2, -1);
+  dit_fft<-1>(zb, M, PM, tw, 2);
   layers_from_spectrum(zb, lb, M, NT, nl, S.jmin, g.NF, g.win[nl], tw, g.norm_sqrtNF / ((nl + 1.0) * NT),
                        coef + ((size_t)s * 3 + ch) * (kWvMaxLayers * (size_t)NT));
 }
@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(kLayerThreads) wdm_by_layers_kernel(int NF, in
   }
   __syncthreads();
   for (int i = threadIdx.x; i < Nds; i += blockDim.x) data[i] = 0.0;
-  dit_fft(zb, M, PM, tw, 2, -1);
+  dit_fft<-1>(zb, M, PM, tw, 2);
   layers_from_spectrum(zb, lb, M, NT, nl, jmin, NF, win, tw, sqrt((double)NF) / ((nl + 1.0) * NT), data);
 }
 
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kLayerThreads) wv_layers_mix_kernel(WvGridDev 
   }
   __syncthreads();
   const float2 *tw = g.tw32[nl];
-  dit_fft(zb, M, PM, tw, 2, -1);
+  dit_fft<-1>(zb, M, PM, tw, 2);
   const float norm = (float)(g.norm_sqrtNF / (nl + 1.0) / g.scale / NT);
   const float *win = g.win32[nl];
   float *out = coef + ((size_t)s * 3 + ch) * (kWvMaxLayers * (size_t)NT);
@@ -852,7 +852,7 @@ __global__ void __launch_bounds__(kLayerThreads) wv_layers_mix_kernel(WvGridDev 
       lb[digit_rev(t, PN)] = val;
     }
     __syncthreads();
-    dit_fft(lb, NT, PN, tw, nl + 1, +1);
+    dit_fft<+1>(lb, NT, PN, tw, nl + 1);
     for (int t = threadIdx.x; t < NT; t += blockDim.x) {
       const float re = lb[t].x * norm, im = lb[t].y * norm;
       float v;
@@ -1212,7 +1212,7 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
     for (int k = 0; k < Nds; k++) {
       double c, sn;
       unit_root(k, Nds, &c, &sn);
-      tw[nl][k] = make_double2(c, sn);
+      tw[nl][k] = tan_form(c, sn);
       tw32[nl][k] = make_float2((float)c, (float)sn);
     }
     win32[nl].assign(win[nl].begin(), win[nl].end());

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, doub
   const int c = blockIdx.x;
   for (int n1 = threadIdx.x; n1 < M1; n1 += blockDim.x) sm64[digit_rev(n1, P)] = src[(size_t)n1 * M2 + c];
   __syncthreads();
-  dit_fft(sm64, M1, P, tw1, 1, -1);
+  dit_fft<-1>(sm64, M1, P, tw1, 1);
   for (int k1 = threadIdx.x; k1 < M1; k1 += blockDim.x)
     dst[(size_t)k1 * M2 + c] = cmul(sm64[k1], root2(tlo, thi, (long long)c * k1, K, -1));
 }
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, d
     }
   }
   __syncthreads();
-  dit_fft(sm64, M1, P, tw1, 1, +1, two ? 2 : 1);
+  dit_fft<+1>(sm64, M1, P, tw1, 1, two ? 2 : 1);
   for (int t = threadIdx.x; t < (two ? 2 * M1 : M1); t += blockDim.x) {
     const int which = t >= M1, k1 = t - which * M1, col = which ? cm : c;
     dst[(size_t)k1 * M2 + col] = cmul(sm64[t], root2(mlo, mhi, (long long)col * k1, K, +1));
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, doub
   const int r = blockIdx.x;
   for (int t = threadIdx.x; t < M2; t += blockDim.x) sm64[digit_rev(t, P)] = src[(size_t)r * M2 + t];
   __syncthreads();
-  dit_fft(sm64, M2, P, tw2, 1, +1);
+  dit_fft<+1>(sm64, M2, P, tw2, 1);
   for (int k2 = threadIdx.x; k2 < M2; k2 += blockDim.x) dst[(size_t)r + (size_t)M1 * k2] = sm64[k2];
 }
 
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *sr
     sm64[which * M2 + digit_rev(k2, P)] = src[(size_t)(which ? rm : r) * M2 + k2];
   }
   __syncthreads();
-  dit_fft(sm64, M2, P, tw2, 1, -1, two ? 2 : 1);
+  dit_fft<-1>(sm64, M2, P, tw2, 1, two ? 2 : 1);
   const int bo = two ? M2 : 0;
   const int n = two ? M2 : r == 0 ? M2 / 2 + 1 : (M2 + 1) / 2;
   for (int k2 = threadIdx.x; k2 < n; k2 += blockDim.x) {
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, i
     if (pp != p) sm64[digit_rev(pp, P)] = make_double2(ax + by, bx - ay);
   }
   __syncthreads();
-  dit_fft(sm64, NT, P, twNT, 1, +1);
+  dit_fft<+1>(sm64, NT, P, twNT, 1);
   if (edge) {
     for (int n = 2 * threadIdx.x; n < NT; n += 2 * blockDim.x) {
       wdm[n] = sm64[n].x;
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, 
     sm64[digit_rev(n, P)] = v;
   }
   __syncthreads();
-  dit_fft(sm64, NT, P, twNT, 1, -1);
+  dit_fft<-1>(sm64, NT, P, twNT, 1);
   if (edge) {
     const double c = scale * 0.70710678118654752440;
     const long long M = (long long)NF * h;
@@ -733,6 +733,12 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   fill_roots(t1, P.M1);
   fill_roots(t2, P.M2);
   fill_roots(tn, NT);
+  if constexpr (sizeof(R) == 8) {  // dit_fft's; wdm_*_layer_kernel, for NT % 4 != 0, takes twNT as it is
+    for (C &w : t1) w = tan_form(w.x, w.y);
+    for (C &w : t2) w = tan_form(w.x, w.y);
+    if (NT % 4 == 0)
+      for (C &w : tn) w = tan_form(w.x, w.y);
+  }
   fill_two_level(mlo, mhi, M, P.K);
   fill_two_level(nlo, nhi, ND, P.K);
   std::vector<R> win(NT / 2 + 1);
