@@ -55,11 +55,12 @@ __device__ __forceinline__ void exp_tab_fill(double *t) {
 // sin x and cos x by table and short polynomials (the same method): x = k
 // 2 pi/1024 + r, |r| <= pi/1024, and the angle-sum formulas.  tw: the 1024-point
 // FFT twiddles exp(-2 pi i k/1024).  14 FP64 instructions (the library's take
-// about 25); within 1 ulp of 1 like theirs.  |x| >= 1e5 (where the reduction's
-// two-part 2 pi/1024 would lose accuracy) and non-finite x go to the library's.
+// about 25, and more beyond 1e5); within 1 ulp of 1 like theirs.  x - k (2 pi/1024),
+// with the constant's first 53 bits, is exact, and the next 53 leave 1e-17 up to
+// |x| = 1e7; larger and non-finite x go to the library's.
 constexpr int kSincosTab = 1024;
 __device__ __forceinline__ void sincos_tab(double x, const double2 *tw, double *s, double *c) {
-  if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) {
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x416312d0) {
     sincos(x, s, c);
     return;
   }
@@ -78,7 +79,7 @@ __device__ __forceinline__ void sincos_tab(double x, const double2 *tw, double *
 
 // cos x alone: 12 FP64 instructions.
 __device__ __forceinline__ double cos_tab(double x, const double2 *tw) {
-  if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) return cos(x);
+  if ((__double2hiint(x) & 0x7fffffff) >= 0x416312d0) return cos(x);
   constexpr double k2Pi = 6.283185307179586477, k2PiLo = 2.4492935982947064e-16;
   const double z = fma(x, kSincosTab / k2Pi, kRoundMagic);
   const double kd = z - kRoundMagic;

@@ -90,37 +90,69 @@ __device__ __forceinline__ int even_index(const EvenGrid &e, int n, double v) {
 // handles many value arrays at once: spline_rhs for node i (the forward sweep's
 // right-hand side, independent per node), spline_recurrence for one array on one
 // thread (the two sequential sweeps on z, which holds the right-hand sides on
-// entry and c2 on exit), spline_coeffs for node i (c1, c3).  Every value has the
-// same FP64 expression as in one sequential sweep, its divisions by div_by.
+// entry and c2 on exit), spline_coeffs for node i (c1, c3).  EXACT: every value
+// has the same FP64 expression as in one sequential sweep, its divisions by
+// div_by; the barycentre phase needs that (it reaches 1e6 rad, and the delayed
+// terms are second differences of it, so one coefficient's last bit shows at
+// 1e-9 in a channel).  Else quotients are products and sums are fused: 5
+// instead of 10, 3 instead of 7 and 8 instead of 17 FP64 instructions per node.
+template <bool EXACT>
 __device__ __forceinline__ double spline_rhs(const double *y, int i, int N, const double *fac) {
   const double *h = fac, *rh = fac + 3 * N;
-  return 3.0 * (div_by(y[i + 1] - y[i], h[i], rh[i]) - div_by(y[i] - y[i - 1], h[i - 1], rh[i - 1]));
+  const double d1 = y[i + 1] - y[i], d0 = y[i] - y[i - 1];
+  if (EXACT) return 3.0 * (div_by(d1, h[i], rh[i]) - div_by(d0, h[i - 1], rh[i - 1]));
+  return 3.0 * fma(d1, rh[i], -(d0 * rh[i - 1]));
 }
+template <bool EXACT>
 __device__ __forceinline__ void spline_recurrence(double *z, int N, const double *fac) {
   const double *h = fac, *l = fac + N, *mu = fac + 2 * N, *rl = fac + 4 * N;
   double zprev = 0.0;
   z[0] = 0.0;
   for (int i = 1; i < N - 1; i++) {
-    zprev = div_by(z[i] - h[i - 1] * zprev, l[i], rl[i]);
+    zprev = EXACT ? div_by(z[i] - h[i - 1] * zprev, l[i], rl[i]) : fma(-h[i - 1], zprev, z[i]) * rl[i];
     z[i] = zprev;
   }
-  z[N - 1] = 0.0;
-  for (int i = N - 2; i >= 0; i--) z[i] = z[i] - mu[i] * z[i + 1];
+  z[N - 1] = zprev = 0.0;
+  for (int i = N - 2; i >= 0; i--) z[i] = zprev = EXACT ? z[i] - mu[i] * zprev : fma(-mu[i], zprev, z[i]);
 }
+// The warp of a CTA that takes the sequential phases: each has one warp's work, at
+// 64 clocks per FP64 instruction of its sub-partition, so resident CTAs take
+// different ones.
+__device__ __forceinline__ int seq_thread() { return (int)threadIdx.x - 32 * ((blockIdx.x >> 7) & 3); }
 // c0..c3 ([4][N], out) of node i from the values y and c2 = z
+template <bool EXACT>
 __device__ __forceinline__ void spline_coeffs(const double *y, const double *z, int i, int N, const double *fac,
                                               double *out) {
   constexpr double third = 1.0 / 3.0;
   const double *h = fac, *rh = fac + 3 * N;
   out[i] = y[i];
   out[2 * N + i] = z[i];
-  if (i < N - 1) {
+  if (i == N - 1) {
+    out[N + i] = 0.0;
+    out[3 * N + i] = 0.0;
+  } else if (EXACT) {
     out[N + i] = div_by(y[i + 1] - y[i], h[i], rh[i]) - div_by(h[i] * (z[i + 1] + 2.0 * z[i]), 3.0, third);
     out[3 * N + i] = div_by(z[i + 1] - z[i], 3.0 * h[i], third * rh[i]);
   } else {
-    out[N + i] = 0.0;
-    out[3 * N + i] = 0.0;
+    out[N + i] = fma(y[i + 1] - y[i], rh[i], -(third * h[i]) * fma(2.0, z[i], z[i + 1]));
+    out[3 * N + i] = (z[i + 1] - z[i]) * (third * rh[i]);
   }
+}
+
+// atan2(y, x): FP32's estimate t, and the remaining angle (y cos t - x sin t) / (x
+// cos t + y sin t), below 1e-6, as its own arctangent to its cube: 27 FP64 instructions,
+// within 2 ulp of pi.  Arguments that FP32 cannot hold go to the library's.
+__device__ __forceinline__ double atan2_tab(double y, double x, const double2 *tw) {
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff, ey = (__double2hiint(y) >> 20) & 0x7ff;
+  const int e = max(ex, ey);
+  // the larger argument scaled by a power of two into [1, 2), the smaller with it
+  if (e < 200 || e > 1800 || e - min(ex, ey) > 60) return atan2(y, x);
+  const double xs = scale_pow2(x, 1023 - e), ys = scale_pow2(y, 1023 - e);
+  const double t = f64_of(atan2f(f32_nearest(ys), f32_nearest(xs)));
+  double s, c;
+  sincos_tab(t, tw, &s, &c);
+  const double d = fma(ys, c, -(xs * s)) * rcp_fast(fma(xs, c, ys * s));
+  return t + fma(d * d * d, -1.0 / 3.0, d);
 }
 
 // ------------------------------------------------------------ plan
@@ -221,13 +253,14 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
     const int c = q / norb, i = q - c * norb;
     if (!s_ok[c] || i == 0 || i == norb - 1) continue;
     double *ya = psm + (size_t)c * (4 * norb + 1), *yp = ya + norb, *za = ya + 2 * norb, *zp = ya + 3 * norb;
-    za[i] = spline_rhs(ya, i, norb, fac);
-    zp[i] = spline_rhs(yp, i, norb, fac);
+    za[i] = spline_rhs<true>(ya, i, norb, fac);
+    zp[i] = spline_rhs<true>(yp, i, norb, fac);
   }
   __syncthreads();
-  if ((int)threadIdx.x < 2 * nsrc) {
-    const int c = threadIdx.x >> 1;
-    if (s_ok[c]) spline_recurrence(psm + (size_t)c * (4 * norb + 1) + (2 + (threadIdx.x & 1)) * norb, norb, g.fac_orb);
+  const int st = seq_thread();
+  if (st >= 0 && st < 2 * nsrc) {
+    const int c = st >> 1;
+    if (s_ok[c]) spline_recurrence<true>(psm + (size_t)c * (4 * norb + 1) + (2 + (st & 1)) * norb, norb, g.fac_orb);
   }
   __syncthreads();
   for (int q = threadIdx.x; q < nsrc * norb; q += blockDim.x) {
@@ -235,31 +268,33 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
     if (!s_ok[c]) continue;
     const double *ya = psm + (size_t)c * (4 * norb + 1), *yp = ya + norb, *za = ya + 2 * norb, *zp = ya + 3 * norb;
     double *amp = ssb + (size_t)(base + c) * 8 * norb, *ph = amp + 4 * norb;
-    spline_coeffs(ya, za, i, norb, fac, amp);
-    spline_coeffs(yp, zp, i, norb, fac, ph);
+    spline_coeffs<true>(ya, za, i, norb, fac, amp);
+    spline_coeffs<true>(yp, zp, i, norb, fac, ph);
   }
 }
 
 // ------------------------------------------------------------ response
-// One (source, node): the barycentre splines, the four products of the
-// polarisation factors, and the arms' patterns over 1 -+ k.n.
+// One (source, node): the barycentre splines, and the arms' patterns over 1 + k.n
+// (p) and 1 - k.n (m) along the two quadratures of the polarisation.
 struct Pol {
-  double a, b, c, e;  // Ap c2p, Ac s2p, Ac c2p, Ap s2p
   const double *amp, *ph, *x;
   EvenGrid grid;
   const double2 *tw;
   int n;
-  double App[3], Apm[3], Acp[3], Acm[3];
+  double2 p[3], m[3];
 };
 
 // One delayed link term at time t: with h+ = A (a cos + b sin), hx = A (c sin -
-// e cos) of the barycentre amplitude A and phase, and their quadratures, the
-// term adds gp h+ + gc hx to M and the same of the quadratures to Mf, i.e. A (P
-// cos + Q sin) and A (Q cos - P sin) with P = a gp - e gc, Q = b gp + c gc.  The
-// phase keeps the reference's order (M and Mf are second differences of eight
-// terms, which amplify its rounding by up to 1e4): 43 FP64 instructions a term,
-// 1250 per (source, node), against 2360 with the reference's own expressions.
-__device__ __forceinline__ void link_term(const Pol &P, double t, double gp, double gc, double &m, double &mf) {
+// e cos) of the barycentre amplitude A and phase, and their quadratures, a pattern
+// (gp, gc) adds gp h+ + gc hx to M and the same of the quadratures to Mf, i.e. A (P
+// cos + Q sin) and A (Q cos - P sin) with P = a gp - e gc, Q = b gp + c gc; r:
+// (P, Q), linear in the patterns, so that the arms' differences are taken of
+// them.  sign -1 takes -r.  The phase keeps the reference's order (M and Mf are
+// second differences of eight terms, which amplify its rounding by up to 1e4):
+// 37 FP64 instructions a term, TIME_LT per (source, node), against 2360 with the
+// reference's own expressions.
+template <int sign>
+__device__ __forceinline__ void link_term(const Pol &P, double t, double2 r, double &m, double &mf) {
   const int j = even_index(P.grid, P.n, t);
   const double d = t - P.x[j];
   const double ph = spl_eval(P.ph, P.n, j, d), amp = spl_horner(P.amp, P.n, j, d);
@@ -267,9 +302,9 @@ __device__ __forceinline__ void link_term(const Pol &P, double t, double gp, dou
   sincos_tab(ph, P.tw, &sp, &cp);
   sp *= amp;
   cp *= amp;
-  const double p = fma(P.a, gp, -(P.e * gc)), q = fma(P.b, gp, P.c * gc);
-  m = fma(p, cp, fma(q, sp, m));
-  mf = fma(q, cp, fma(-p, sp, mf));
+  if (sign < 0) r = make_double2(-r.x, -r.y);
+  m = fma(r.x, cp, fma(r.y, sp, m));
+  mf = fma(r.y, cp, fma(-r.x, sp, mf));
 }
 
 // One Michelson channel (vertex a, arms b and c) from eight delayed link
@@ -277,15 +312,17 @@ __device__ __forceinline__ void link_term(const Pol &P, double t, double gp, dou
 template <int a, int b, int c>
 __device__ __forceinline__ void tdi_channel(const Pol &P, double tn, const double *kr, const double *L, double &m,
                                             double &mf) {
+  auto sub = [](double2 p, double2 q) { return make_double2(p.x - q.x, p.y - q.y); };
+  const double2 bb = sub(P.m[b], P.p[b]), cc = sub(P.p[c], P.m[c]);
   m = mf = 0.0;
-  link_term(P, tn - kr[a] - 2.0 * L[c] - 2.0 * L[b], P.Apm[b] - P.App[c], P.Acm[b] - P.Acp[c], m, mf);
-  link_term(P, tn - kr[b] - L[c] - 2.0 * L[b], P.App[c] - P.Apm[c], P.Acp[c] - P.Acm[c], m, mf);
-  link_term(P, tn - kr[c] - L[b] - 2.0 * L[c], P.App[b] - P.Apm[b], P.Acp[b] - P.Acm[b], m, mf);
-  link_term(P, tn - kr[a] - 2.0 * L[b], P.Apm[c] - P.Apm[b], P.Acm[c] - P.Acm[b], m, mf);
-  link_term(P, tn - kr[a] - 2.0 * L[c], P.App[c] - P.App[b], P.Acp[c] - P.Acp[b], m, mf);
-  link_term(P, tn - kr[c] - L[b], P.Apm[b] - P.App[b], P.Acm[b] - P.Acp[b], m, mf);
-  link_term(P, tn - kr[b] - L[c], P.Apm[c] - P.App[c], P.Acm[c] - P.Acp[c], m, mf);
-  link_term(P, tn - kr[a], P.App[b] - P.Apm[c], P.Acp[b] - P.Acm[c], m, mf);
+  link_term<1>(P, tn - kr[a] - 2.0 * L[c] - 2.0 * L[b], sub(P.m[b], P.p[c]), m, mf);
+  link_term<1>(P, tn - kr[b] - L[c] - 2.0 * L[b], cc, m, mf);
+  link_term<-1>(P, tn - kr[c] - L[b] - 2.0 * L[c], bb, m, mf);
+  link_term<1>(P, tn - kr[a] - 2.0 * L[b], sub(P.m[c], P.m[b]), m, mf);
+  link_term<1>(P, tn - kr[a] - 2.0 * L[c], sub(P.p[c], P.p[b]), m, mf);
+  link_term<1>(P, tn - kr[c] - L[b], bb, m, mf);
+  link_term<-1>(P, tn - kr[b] - L[c], cc, m, mf);
+  link_term<1>(P, tn - kr[a], sub(P.p[b], P.m[c]), m, mf);
 }
 
 // LISA_spline_response (utils/src/glass_lisa.c:920-1074) at one node, plus the
@@ -315,6 +352,7 @@ __global__ void wv_resp_kernel(WvGridDev g, int n, const WvSrc *srcs, const doub
     out[6 * norb + m] = spl_eval(ph, norb, j, tsc - g.orb_t[j]);
   }
   const double L[3] = {G[18], G[19], G[20]};
+  const double pa = S.Ap * S.c2p, pb = S.Ac * S.s2p, pc = S.Ac * S.c2p, pe = S.Ap * S.s2p;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     const double x = G[9 + 3 * i], y = G[10 + 3 * i], z = G[11 + 3 * i];
@@ -322,15 +360,10 @@ __global__ void wv_resp_kernel(WvGridDev g, int n, const WvSrc *srcs, const doub
     const double nu = fma(z, S.u[2], fma(y, S.u[1], x * S.u[0])), nv = fma(y, S.v[1], x * S.v[0]);
     const double dp = fma(nv, nv, -(nu * nu)), dc = 2.0 * nu * nv;
     const double rp = rcp_fast(1.0 + kn), rm = rcp_fast(1.0 - kn);
-    P.App[i] = dp * rp;
-    P.Apm[i] = dp * rm;
-    P.Acp[i] = dc * rp;
-    P.Acm[i] = dc * rm;
+    const double p = fma(pa, dp, -(pe * dc)), q = fma(pb, dp, pc * dc);
+    P.p[i] = make_double2(p * rp, q * rp);
+    P.m[i] = make_double2(p * rm, q * rm);
   }
-  P.a = S.Ap * S.c2p;
-  P.b = S.Ac * S.s2p;
-  P.c = S.Ac * S.c2p;
-  P.e = S.Ap * S.s2p;
   P.amp = amp;
   P.ph = ph;
   P.x = g.orb_t;
@@ -388,9 +421,13 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     As[i] = sqrt(M[i] * M[i] + Mf[i] * Mf[i]);
   }
   __syncthreads();
-  if ((int)threadIdx.x < nch && s_ok[threadIdx.x]) {
-    const int c = threadIdx.x;
+  const int st = seq_thread();
+  if (st >= 0 && st < nch && s_ok[st]) {
+    const int c = st;
     WV_TDI_PTRS
+    // not negative, so that their bits order them (a NaN, last there, flips nothing
+    // below)
+    auto less = [&](int p, int q) { return __double_as_longlong(As[p]) < __double_as_longlong(As[q]); };
     double *flip = za, *pj = zp;
     flip[0] = 1.0;
     pj[0] = 0.0;
@@ -398,7 +435,7 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     do {
       flip[i] = flip[i - 1];
       pj[i] = pj[i - 1];
-      if ((As[i] < As[i - 1]) && (As[i] < As[i + 1])) {
+      if (less(i, i - 1) && less(i, i + 1)) {
         const double d1 = As[i + 1] + As[i - 1] - 2.0 * As[i];
         const double d2 = -As[i + 1] + As[i - 1] - 2.0 * As[i];
         const double d3 = -As[i + 1] + As[i - 1] + 2.0 * As[i];
@@ -428,21 +465,19 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     const double nq = fma(phR[i], 1.0 / kPI2, kRoundMagic) - kRoundMagic;
     double v = fma(-nq, kPI2, phR[i]);
     if (fabs(v) > 0.5 * kPI2 || fabs(nq) > 1e15) v = remainder(phR[i], kPI2);
-    Q[i] = -atan2(Mf[i], M[i]) + zp[i] - v;
+    Q[i] = -atan2_tab(Mf[i], M[i], g.tw1024) + zp[i] - v;
   }
   __syncthreads();
-  if ((int)threadIdx.x < nch && s_ok[threadIdx.x]) {
-    const int c = threadIdx.x;
+  if (st >= 0 && st < nch && s_ok[st]) {
+    const int c = st;
     WV_TDI_PTRS
     double v = Q[0];
     for (int i = 0; i < N; i++) {
       double u = Q[i];
-      const double qq = rint(fabs(u - v) / (kPI2));
-      if (qq > 0.0) {
-        if (v > u)
-          u += qq * kPI2;
-        else
-          u -= qq * kPI2;
+      const double gap = u - v;
+      if ((__double_as_longlong(gap) & 0x7fffffffffffffffll) > __double_as_longlong(kPI)) {  // |gap| / 2 pi > 1/2
+        const double qq = rint(fabs(gap) / kPI2);
+        if (qq > 0.0) u = v > u ? u + qq * kPI2 : u - qq * kPI2;  // (not for a NaN)
       }
       v = u;
       Q[i] = u;
@@ -455,13 +490,13 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     const int c = q / N, i = q - c * N;
     if (!s_ok[c] || i == 0 || i == N - 1) continue;
     WV_TDI_PTRS
-    za[i] = spline_rhs(As, i, N, fac);
-    zp[i] = spline_rhs(Q, i, N, fac);
+    za[i] = spline_rhs<false>(As, i, N, fac);
+    zp[i] = spline_rhs<false>(Q, i, N, fac);
   }
   __syncthreads();
-  if ((int)threadIdx.x < 2 * nch && s_ok[threadIdx.x >> 1]) {
-    const int c = threadIdx.x >> 1;
-    spline_recurrence(tsm + (size_t)c * (4 * N + 1) + (2 + (threadIdx.x & 1)) * N, N, g.fac_ssb);
+  if (st >= 0 && st < 2 * nch && s_ok[st >> 1]) {
+    const int c = st >> 1;
+    spline_recurrence<false>(tsm + (size_t)c * (4 * N + 1) + (2 + (st & 1)) * N, N, g.fac_ssb);
   }
   __syncthreads();
   for (int q = threadIdx.x; q < nch * N; q += blockDim.x) {
@@ -469,8 +504,8 @@ __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const W
     if (!s_ok[c]) continue;
     WV_TDI_PTRS
     double *ca = tdi + ((size_t)s * 3 + ch) * 8 * N, *cp = ca + 4 * N;
-    spline_coeffs(As, za, i, N, fac, ca);
-    spline_coeffs(Q, zp, i, N, fac, cp);
+    spline_coeffs<false>(As, za, i, N, fac, ca);
+    spline_coeffs<false>(Q, zp, i, N, fac, cp);
   }
 #undef WV_TDI_PTRS
 }
@@ -1418,24 +1453,17 @@ __global__ void __launch_bounds__(kFisherThreads) wv_fisher_kernel(WvGridDev g, 
   if (threadIdx.x == 0 && status) status[s] = 0;
 }
 
-// Launches a tile kernel with C = 16, 4 or 1 items per CTA of 128 threads,
-// the largest whose shared memory (C x per bytes) fits 200 KB.
-template <typename K16, typename K4, typename K1, typename... Args>
-static cudaError_t wv_launch_tiles(K16 k16, K4 k4, K1 k1, size_t per, int items, cudaStream_t s, Args... args) {
-  const size_t cap = 200 * 1024;
-  cudaError_t e;
-  if (16 * per <= cap) {
-    if ((e = cudaFuncSetAttribute(k16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(16 * per))) != cudaSuccess)
-      return e;
-    k16<<<(items + 15) / 16, 128, 16 * per, s>>>(args...);
-  } else if (4 * per <= cap) {
-    if ((e = cudaFuncSetAttribute(k4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * per))) != cudaSuccess)
-      return e;
-    k4<<<(items + 3) / 4, 128, 4 * per, s>>>(args...);
-  } else {
-    if ((e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)per)) != cudaSuccess) return e;
-    k1<<<items, 128, per, s>>>(args...);
-  }
+// Launches a tile kernel with C = 16, 8, 4 or 1 items per CTA of 128 threads: the
+// largest of which four CTAs fit an SM (per bytes of shared memory an item), so
+// that four sequential phases run side by side, or that fits at all.
+template <typename K, typename... Args>
+static cudaError_t wv_launch_tiles(K const (&k)[4], size_t per, int items, cudaStream_t s, Args... args) {
+  constexpr int C[4] = {16, 8, 4, 1};
+  int q = 0;
+  while (q < 3 && C[q] * per > (size_t)(C[q] > 4 ? 55 : 200) * 1024) q++;
+  cudaError_t e = cudaFuncSetAttribute(k[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(C[q] * per));
+  if (e != cudaSuccess) return e;
+  k[q]<<<(items + C[q] - 1) / C[q], 128, C[q] * per, s>>>(args...);
   return cudaGetLastError();
 }
 
@@ -1448,16 +1476,17 @@ cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int preci
     // 4 norb doubles of shared memory per source; 16 sources per CTA where
     // they fit, fewer for long observations
     const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
-    if ((e = wv_launch_tiles(wv_plan_kernel<16>, wv_plan_kernel<4>, wv_plan_kernel<1>, per, n, s, g, n, params, w.src,
-                             w.ssb, status)) != cudaSuccess)
+    decltype(&wv_plan_kernel<1>) const k[4] = {wv_plan_kernel<16>, wv_plan_kernel<8>, wv_plan_kernel<4>,
+                                               wv_plan_kernel<1>};
+    if ((e = wv_launch_tiles(k, per, n, s, g, n, params, w.src, w.ssb, status)) != cudaSuccess)
       return e;
   }
   const long long nr = (long long)n * norb;
   wv_resp_kernel<<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(g, n, w.src, w.ssb, w.resp);
   {
     const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
-    if ((e = wv_launch_tiles(wv_tdi_kernel<16>, wv_tdi_kernel<4>, wv_tdi_kernel<1>, per, 3 * n, s, g, n, w.src, w.resp,
-                             w.tdi)) != cudaSuccess)
+    decltype(&wv_tdi_kernel<1>) const k[4] = {wv_tdi_kernel<16>, wv_tdi_kernel<8>, wv_tdi_kernel<4>, wv_tdi_kernel<1>};
+    if ((e = wv_launch_tiles(k, per, 3 * n, s, g, n, w.src, w.resp, w.tdi)) != cudaSuccess)
       return e;
   }
   if (precision == 1) {
