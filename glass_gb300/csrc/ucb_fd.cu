@@ -63,59 +63,18 @@ __device__ __noinline__ int snr_spread_fp64(const PlanArgs &a, double f0, double
   return pow2_above_dev(exp(lnA) * sqrt(a.T) * sf * (2.0 * a.L) / sqrt(sn4L2) - 1);
 }
 
-// The interval of (int)pow(2, (int)log2(v) + 1), within [Nmin, Nmax], for an FP32
-// estimate v good to 2e-5.
-__device__ __forceinline__ void pow2_above_f32(float v, int Nmin, int Nmax, int &lo, int &hi) {
-  lo = Nmin;
-  hi = Nmax;
-  if (isnan(v)) return;
-  const float v0 = v * 0.99998f, v1 = v * 1.00002f;
-  // the binary exponent of a v >= 1, plus 1 (at most 30 below infinity's)
-  const int e0 = min((__float_as_int(v0) >> 23) - 126, 30), e1 = min((__float_as_int(v1) >> 23) - 126, 30);
-  lo = max(min(v0 >= 1.f ? 1 << e0 : 1, Nmax), Nmin);
-  hi = max(min(v1 >= 1.f ? 1 << e1 : 1, Nmax), Nmin);
-}
-
 // The bandwidth rule of ucb/src/glass_ucb_waveform.c:698-725: N is always the
-// reference's.  FP32 estimates of the two spreads, good to 1e-5 over the range of
-// the test below (ln A rounded: 4e-6; the sine and cosine of f/f* <= 10: 2e-6); a
-// spread is evaluated in FP64 only where its estimate's interval leaves N open (or
-// the estimate overflows, or the input is outside that range), which one proposal
-// in 20,000 does; that lane runs 100 FP64 instructions, while its CTA waits.
+// reference's.  A spread is evaluated in FP64 only where its FP32 interval leaves
+// N open, which one proposal in 20,000 does; that lane runs 100 FP64
+// instructions, while its CTA waits.
 __device__ __forceinline__ int plan_size(const PlanArgs &a, const double *p, double f0) {
-  const int Nmin = 16, half = a.NFFT / 2;
-  const int Nmax = half >= 1 ? (1 << (31 - __clz(half))) : 0;
-  const float Tf = to_f32(a.T), f0f = to_f32(f0), lnA = to_f32(p[3]), p7 = to_f32(p[7]);
-  int D0 = Nmin, D1 = Nmax, S0 = Nmin, S1 = Nmax;
-  if (f0f > 1e-6f && f0f < 0.2f && fabsf(lnA) < 80.f && fabsf(p7) < 1e30f) {
-    // 1 - cos^2 in FP64, as it cancels at the poles
-    const float sinthf = sqrtf(fmaxf(0.f, to_f32(fma(-p[1], p[1], 1.0))));
-    const float bw = 2.f * Tf * (4.f + 6.2831853f * f0f * (float)(kAU / kCLIGHT) * sinthf) * (float)(1.0 / kYEAR) +
-                     2.f * fabsf(p7);
-    pow2_above_f32(bw - 1.f, Nmin, Nmax, D0, D1);
-    // AEnoise times (2L)^2 (AEnoise itself, ~1e-42, is below FP32's normal range)
-    float sx, cx;
-    sincosf(f0f * to_f32(a.invfstar), &sx, &cx);
-    const float c2x = 2.f * cx * cx - 1.f, rf = 1.f / f0f;
-    const float rw = rf * 0.15915494f, rw2 = rw * rw;
-    const float q1 = 2.0e-5f * rf, q2 = q1 * q1, q4 = q2 * q2, r1 = 1.0e-4f * rf;
-    const float red = 1.f + 16.f * (q4 * q4 * q2 + r1 * r1);
-    const float sn4L2 = (16.f / 3.f) * sx * sx *
-                        ((2.f + cx) * (float)(kSPS + kSLOC) +
-                         2.f * (3.f + 2.f * cx + c2x) * ((float)(kSLOC / 2.0) + (float)kSACC * (rw2 * rw2) * red));
-    // (at a zero of the sine its sign, and so the rule's outcome, is FP64's)
-    if (fabsf(sx) > 1e-3f)
-      pow2_above_f32(expf(lnA) * sqrtf(Tf) * sx * (2.f * to_f32(a.L)) * rsqrtf(sn4L2) - 1.f, Nmin, Nmax, S0, S1);
+  SpreadInterval s = spread_interval(a.T, a.invfstar, a.L, a.NFFT, f0, p[1], to_f32(p[3]), to_f32(p[7]));
+  if (s.open() && s.D0 != s.D1) {
+    const int D = doppler_spread_fp64(a.T, f0, div_by(p[7], a.T2, a.invT2), p[1]);
+    s.D0 = s.D1 = s.clamp(D);
   }
-  if (max(D0, S0) != max(D1, S1) && D0 != D1) {
-    D0 = doppler_spread_fp64(a.T, f0, div_by(p[7], a.T2, a.invT2), p[1]);
-    D0 = D1 = max(min(D0, Nmax), Nmin);
-  }
-  if (max(D0, S0) != max(D1, S1)) {
-    S0 = snr_spread_fp64(a, f0, p[3]);
-    S0 = max(min(S0, Nmax), Nmin);
-  }
-  return 2 * max(D0, S0);
+  if (s.open()) s.S0 = s.clamp(snr_spread_fp64(a, f0, p[3]));
+  return 2 * max(s.D0, s.S0);
 }
 
 // Warp-aggregated binning: one atomic per distinct size per warp, begun by

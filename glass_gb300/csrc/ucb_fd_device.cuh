@@ -428,6 +428,57 @@ static __device__ int bandwidth_dev(double L, double fstar, double f, double fdo
   return (DS > SS) ? DS : SS;
 }
 
+// The interval of (int)pow(2, (int)log2(v) + 1), within [Nmin, Nmax], for an FP32
+// estimate v good to 2e-5.
+__device__ __forceinline__ void pow2_above_f32(float v, int Nmin, int Nmax, int &lo, int &hi) {
+  lo = Nmin;
+  hi = Nmax;
+  if (isnan(v)) return;
+  const float v0 = v * 0.99998f, v1 = v * 1.00002f;
+  // the binary exponent of a v >= 1, plus 1 (at most 30 below infinity's)
+  const int e0 = min((__float_as_int(v0) >> 23) - 126, 30), e1 = min((__float_as_int(v1) >> 23) - 126, 30);
+  lo = max(min(v0 >= 1.f ? 1 << e0 : 1, Nmax), Nmin);
+  hi = max(min(v1 >= 1.f ? 1 << e1 : 1, Nmax), Nmin);
+}
+
+// FP32 intervals [D0, D1], [S0, S1] of the bandwidth rule's two spreads (ucb/src/
+// glass_ucb_waveform.c:708-722, with AEnoise, utils/src/glass_lisa.c:1188-1198), good
+// to 1e-5 over the range of the test below (ln A rounded: 4e-6; the sine and
+// cosine of f/f* <= 10: 2e-6); outside it everything is open.  fdT2: fdot T^2.
+struct SpreadInterval {
+  int Nmin, Nmax, D0, D1, S0, S1;
+  __device__ int clamp(int n) const { return max(min(n, Nmax), Nmin); }
+  __device__ bool open() const { return max(D0, S0) != max(D1, S1); }
+};
+__device__ __forceinline__ SpreadInterval spread_interval(double T, double invfstar, double L, int NFFT, double f0,
+                                                          double costh, float lnA, float fdT2) {
+  const int Nmin = 16, half = NFFT / 2;
+  const int Nmax = half >= 1 ? (1 << (31 - __clz(half))) : 0;
+  SpreadInterval s = {Nmin, Nmax, Nmin, Nmax, Nmin, Nmax};
+  const float Tf = to_f32(T), f0f = to_f32(f0);
+  if (f0f > 1e-6f && f0f < 0.2f && fabsf(lnA) < 80.f && fabsf(fdT2) < 1e30f) {
+    // 1 - cos^2 in FP64, as it cancels at the poles
+    const float sinthf = sqrtf(fmaxf(0.f, to_f32(fma(-costh, costh, 1.0))));
+    const float bw = 2.f * Tf * (4.f + 6.2831853f * f0f * (float)(kAU / kCLIGHT) * sinthf) * (float)(1.0 / kYEAR) +
+                     2.f * fabsf(fdT2);
+    pow2_above_f32(bw - 1.f, Nmin, Nmax, s.D0, s.D1);
+    // AEnoise times (2L)^2 (AEnoise itself, ~1e-42, is below FP32's normal range)
+    float sx, cx;
+    sincosf(f0f * to_f32(invfstar), &sx, &cx);
+    const float c2x = 2.f * cx * cx - 1.f, rf = 1.f / f0f;
+    const float rw = rf * 0.15915494f, rw2 = rw * rw;
+    const float q1 = 2.0e-5f * rf, q2 = q1 * q1, q4 = q2 * q2, r1 = 1.0e-4f * rf;
+    const float red = 1.f + 16.f * (q4 * q4 * q2 + r1 * r1);
+    const float sn4L2 = (16.f / 3.f) * sx * sx *
+                        ((2.f + cx) * (float)(kSPS + kSLOC) +
+                         2.f * (3.f + 2.f * cx + c2x) * ((float)(kSLOC / 2.0) + (float)kSACC * (rw2 * rw2) * red));
+    // (at a zero of the sine its sign, and so the rule's outcome, is FP64's)
+    if (fabsf(sx) > 1e-3f)
+      pow2_above_f32(expf(lnA) * sqrtf(Tf) * sx * (2.f * to_f32(L)) * rsqrtf(sn4L2) - 1.f, Nmin, Nmax, s.S0, s.S1);
+  }
+  return s;
+}
+
 // Source geometry shared by both precisions (ucb/src/glass_ucb_waveform.c:802-838,
 // utils/src/glass_lisa.c:1566-1596).
 struct SourceGeom {

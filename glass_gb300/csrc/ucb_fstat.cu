@@ -182,6 +182,7 @@ __device__ void fs_write(const FsPlanArgs &a, int i, const double *o, int st) {
 // (ucb/src/glass_ucb_fstatistic.c:241-344): f0 T, cos theta, phi, ln 2,
 // cos(pi/2), psi, phase (0, 0 for H), fdot T^2.
 __global__ void __launch_bounds__(128) fs_plan_kernel(FsPlanArgs a) {
+  grid_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int b = -1;
   if (i < a.ncells) {
@@ -196,7 +197,11 @@ __global__ void __launch_bounds__(128) fs_plan_kernel(FsPlanArgs a) {
       fs_write(a, i, o, GLASS_ITEM_NONFINITE);
     } else {
       const double costh = cos(theta);
-      const int N = bandwidth_dev(a.L, a.fstar, f0, fdot, costh, 1.e-22, a.T, a.NFFT);
+      // the rule at amplitude 1e-22, in FP64 only where its FP32 interval leaves it
+      // open (ln 1e-22 = -50.656872)
+      const SpreadInterval sp = spread_interval(a.T, 1.0 / a.fstar, a.L, a.NFFT, f0, costh, -50.656872f,
+                                                to_f32(fdot * (a.T * a.T)));
+      const int N = sp.open() ? bandwidth_dev(a.L, a.fstar, f0, fdot, costh, 1.e-22, a.T, a.NFFT) : max(sp.D0, sp.S0);
       const long long q = (long long)(f0 * a.T);
       const long long qq = q - (long long)a.seg_qmin[seg];
       // filter bin i sits at segment bin qq + i - N/2 (:378, :423); bins
@@ -259,6 +264,7 @@ __device__ __forceinline__ long long fs_bin_start(const int *bin_count, int bin)
 // glass_ucb_waveform.c:840-922 with real polarisation factors), combined to the
 // four A/E series each and stored at [cell][template][series][n].
 __global__ void __launch_bounds__(256) fs_slow_kernel(FsSlowArgs a) {
+  grid_begin();
   long long cs[kFsBins + 1];
   long long acc = 0;
 #pragma unroll
@@ -330,6 +336,7 @@ __global__ void __launch_bounds__(FsCfg<N>::CTA) fs_spec_kernel(FsSpecArgs a) {
   constexpr int GT = Cfg::GT, GPC = Cfg::GPC;
   constexpr int B = N / GT;  // bins per thread (4)
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  grid_begin();
   const int count = a.bin_count[a.bin];
   if (count == 0) return;
   double2 *tw = reinterpret_cast<double2 *>(smem_raw);
@@ -409,6 +416,7 @@ __global__ void __launch_bounds__(FsCfg<N>::CTA) fs_spec_kernel(FsSpecArgs a) {
 // ----------------------------------------------------------------- finish
 __global__ void __launch_bounds__(128) fs_finish_kernel(const FsCell *fc, int ncells, double *logl, double *fparams,
                                                         int *status) {
+  grid_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ncells || !fc[i].live) return;
   const double s = 4.0 * fc[i].it.amp_s, s2 = s * fc[i].it.amp_s;
@@ -447,8 +455,7 @@ cudaError_t fs_launch_spec(const FsSpecArgs &a, int ncells, int num_sms, cudaStr
   int grid = occ * num_sms;
   if (need < grid) grid = need;
   if (grid < 1) grid = 1;
-  fs_spec_kernel<N><<<grid, Cfg::CTA, Cfg::smem, stream>>>(a);
-  return cudaGetLastError();
+  return launch_chained(fs_spec_kernel<N>, grid, Cfg::CTA, Cfg::smem, stream, a);
 }
 
 
@@ -597,9 +604,9 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
     pa.logl = logl + off;
     pa.fparams = fparams ? fparams + 4 * (size_t)off : nullptr;
     pa.status = status ? status + off : nullptr;
-    fs_plan_kernel<<<(n + 127) / 128, 128, 0, stream>>>(pa);
+    e = launch_chained(fs_plan_kernel, (n + 127) / 128, 128, 0, stream, pa);
     launches++;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
 
     FsSlowArgs sa;
     sa.cap = w.cap;
@@ -616,9 +623,9 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
              return cudaOccupancyMaxActiveBlocksPerMultiprocessor(o, fs_slow_kernel, 256, 0);
            }, &occ)) != cudaSuccess)
         return e;
-      fs_slow_kernel<<<occ * num_sms, 256, 0, stream>>>(sa);
+      e = launch_chained(fs_slow_kernel, occ * num_sms, 256, 0, stream, sa);
       launches++;
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      if (e != cudaSuccess) return e;
     }
 
     FsSpecArgs ca;
@@ -651,9 +658,10 @@ cudaError_t fs_launch(const FdBankDev &bank, const FdTablesDev &tab, const doubl
       launches++;
       if (e != cudaSuccess) return e;
     }
-    fs_finish_kernel<<<(n + 127) / 128, 128, 0, stream>>>((const FsCell *)w.cells, n, pa.logl, pa.fparams, pa.status);
+    e = launch_chained(fs_finish_kernel, (n + 127) / 128, 128, 0, stream, (const FsCell *)w.cells, n, pa.logl,
+                       pa.fparams, pa.status);
     launches++;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
   }
   if (nlaunch) *nlaunch = launches;
   return cudaSuccess;

@@ -166,13 +166,14 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
                                                       double *ssb, int *status) {
   extern __shared__ __align__(16) double psm[];
   __shared__ int s_ok[C];
-  __shared__ double s_f0[C], s_phi0[C], s_fdot[C], s_A0[C];
+  __shared__ double s_f0[C], s_phi0[C], s_fdot[C], s_A0[C], s_dA[C];
   const int base = blockIdx.x * C;
   const int nsrc = min(C, n - base);
   const int norb = g.norb;
   const double Tobs = g.Tobs;
-  if ((int)threadIdx.x < nsrc) {
-    const int s = base + threadIdx.x;
+  const int st = seq_thread();
+  if (st >= 0 && st < nsrc) {
+    const int s = base + st;
     const double *p = params + 8 * (size_t)s;
     WvSrc S;
     bool ok = true;
@@ -210,7 +211,9 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
     }
     // geometry (LISA_polarization_tensor, utils/src/glass_lisa.c:1566-1596)
     const double costh = p[1], phi = p[2], cosi = p[4], psi = p[5];
-    const double sinth = sqrt(1.0 - costh * costh), cosph = cos(phi), sinph = sin(phi);
+    double cosph, sinph;
+    sincos(phi, &sinph, &cosph);
+    const double sinth = sqrt(1.0 - costh * costh);
     const double u[3] = {costh * cosph, costh * sinph, -sinth};
     const double v[3] = {sinph, -cosph, 0.};
     S.k[0] = -sinth * cosph;
@@ -220,19 +223,19 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
       S.u[i] = u[i];
       S.v[i] = v[i];
     }
-    S.c2p = cos(2. * psi);
-    S.s2p = sin(2. * psi);
+    sincos_tab(2. * psi, g.tw1024, &S.s2p, &S.c2p);
     S.Ap = 0.5 * (1. + cosi * cosi);
     S.Ac = -cosi;
     S.fhet = (S.jmin - 1) * g.wdf;
     S.pad = 0;
     srcs[s] = S;
     if (status) status[s] = S.status;
-    s_ok[threadIdx.x] = S.status == 0;
-    s_f0[threadIdx.x] = p[0] / Tobs;
-    s_phi0[threadIdx.x] = p[6];
-    s_fdot[threadIdx.x] = p[7] / Tobs / Tobs;
-    s_A0[threadIdx.x] = S.status == 0 ? exp(p[3]) : 0.0;
+    s_ok[st] = S.status == 0;
+    s_f0[st] = p[0] / Tobs;
+    s_phi0[st] = p[6];
+    s_fdot[st] = 0.5 * (p[7] / Tobs / Tobs);
+    s_A0[st] = S.status == 0 ? exp(p[3]) : 0.0;
+    s_dA[st] = 2.0 / 3.0 * (p[7] / Tobs / Tobs) / (p[0] / Tobs);
   }
   __syncthreads();
   // barycentre amplitude and phase on the orbit nodes (ucb_barycenter_waveform,
@@ -241,11 +244,9 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
     const int c = q / norb, i = q - c * norb;
     if (!s_ok[c]) continue;
     double *ya = psm + (size_t)c * (4 * norb + 1), *yp = ya + norb;
-    const double f0 = s_f0[c], phi0 = s_phi0[c], fdot = s_fdot[c], fddot = 0.0;
-    const double A0 = s_A0[c];
     const double t = g.orb_t[i];
-    yp[i] = -phi0 + kPI2 * (f0 * t + 0.5 * fdot * t * t + 1.0 / 6.0 * fddot * t * t * t);
-    ya[i] = A0 * (1.0 + 2.0 / 3.0 * fdot / f0 * t);
+    yp[i] = -s_phi0[c] + kPI2 * (s_f0[c] * t + s_fdot[c] * t * t);  // fddot = 0
+    ya[i] = s_A0[c] * (1.0 + s_dA[c] * t);
   }
   __syncthreads();
   const double *fac = g.fac_orb;
@@ -257,7 +258,6 @@ __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const 
     zp[i] = spline_rhs<true>(yp, i, norb, fac);
   }
   __syncthreads();
-  const int st = seq_thread();
   if (st >= 0 && st < 2 * nsrc) {
     const int c = st >> 1;
     if (s_ok[c]) spline_recurrence<true>(psm + (size_t)c * (4 * norb + 1) + (2 + (st & 1)) * norb, norb, g.fac_orb);
@@ -291,7 +291,7 @@ struct Pol {
 // (P, Q), linear in the patterns, so that the arms' differences are taken of
 // them.  sign -1 takes -r.  The phase keeps the reference's order (M and Mf are
 // second differences of eight terms, which amplify its rounding by up to 1e4):
-// 37 FP64 instructions a term, TIME_LT per (source, node), against 2360 with the
+// 37 FP64 instructions a term, 950 per (source, node), against 2360 with the
 // reference's own expressions.
 template <int sign>
 __device__ __forceinline__ void link_term(const Pol &P, double t, double2 r, double &m, double &mf) {
