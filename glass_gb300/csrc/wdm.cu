@@ -357,18 +357,43 @@ __global__ void wdm_pack_kernel(const C *X, long long M, const C *tlo, const C *
 }
 
 // ------------------------------------------------------------------ FP64
-// exp(sign 2 pi i p / P) from the two-level tables, in FP64.
-__device__ __forceinline__ double2 root2(const double2 *lo, const double2 *hi, long long p, int K, int sign) {
-  const double2 t = cmul(hi[p / K], lo[p % K]);
-  return make_double2(t.x, sign < 0 ? t.y : -t.y);
+// The passes' factors in tangent form, laid out as the passes read them (so that a
+// factor costs a coalesced load, where a product of two small tables costs 4 of a
+// point's 36 FP64 instructions): colf[c][k1] = e^{-2 pi i c k1/M} between the
+// four-step passes, packf[c][n1] and unpackf[r][k2] = e^{-2 pi i k/ND} of the bins k
+// = n1 M2 + c and r + M1 k2 where the inverse packs and the forward unpacks the real
+// spectrum.  32 bytes per complex point, kept with the plan.
+__device__ __forceinline__ double2 conj_tan(double2 w) { return make_double2(w.x, -w.y); }
+__device__ double2 tan_root(long long p, long long P) {  // e^{-2 pi i p / P}, 0 <= p < P
+  // quadrant and octant in integers: the angle taken is at most pi/4
+  const long long q = 4 * p / P, r = 4 * p - q * P;
+  const bool flip = 2 * r > P;
+  double s, c;
+  sincospi(0.5 * ((double)(flip ? P - r : r) / (double)P), &s, &c);
+  if (flip) {
+    const double t = s;
+    s = c;
+    c = t;
+  }
+  return q == 0 ? tan_form(c, -s) : q == 1 ? tan_form(-s, -c) : q == 2 ? tan_form(-c, s) : tan_form(s, c);
+}
+__global__ void wdm_roots64_kernel(double2 *colf, double2 *packf, double2 *unpackf, int M1, int M2) {
+  const long long M = (long long)M1 * M2, n1 = (long long)(M2 / 2 + 1) * M1, n2 = (long long)(M1 / 2 + 1) * M2;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M + n1 + n2; i += (long long)gridDim.x * blockDim.x) {
+    if (i < M)
+      colf[i] = tan_root((i / M1) * (i % M1), M);
+    else if (i < M + n1)
+      packf[i - M] = tan_root(((i - M) % M1) * M2 + (i - M) / M1, 2 * M);
+    else
+      unpackf[i - M - n1] = tan_root((i - M - n1) / M2 + (i - M - n1) % M2 * M1, 2 * M);
+  }
 }
 
 // Four-step pass 1, one column per CTA (16-byte accesses: two CTAs read each
 // sector, which L2 serves; the FP64 pipe is the bound, and 1024 CTAs balance
 // over 152 SMs where 256 of four columns leave a sixth of them idle).
 __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, double2 *dst, int M1, int M2,
-                                                        const double2 *tw1, const double2 *tlo, const double2 *thi,
-                                                        int K) {
+                                                        const double2 *tw1, const double2 *colf) {
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M1, P);
@@ -377,7 +402,7 @@ __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, doub
   __syncthreads();
   dit_fft<-1>(sm64, M1, P, tw1, 1);
   for (int k1 = threadIdx.x; k1 < M1; k1 += blockDim.x)
-    dst[(size_t)k1 * M2 + c] = cmul(sm64[k1], root2(tlo, thi, (long long)c * k1, K, -1));
+    dst[(size_t)k1 * M2 + c] = tan_mul(sm64[k1], colf[(size_t)c * M1 + k1]);
 }
 
 // The inverse's pass 1 on columns c and M2 - c, whose elements are bins k and M -
@@ -385,9 +410,8 @@ __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, doub
 // ignored as an inverse real FFT does): with s = X_k + X*_{M-k}, d = X_k - X*_{M-k}
 // and w = e^{2 pi i k/ND} d, the packed spectrum is Z_k = s + i w, Z_{M-k} = s* + i w*.
 __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, double2 *dst, int M1, int M2,
-                                                             const double2 *tw1, const double2 *mlo,
-                                                             const double2 *mhi, const double2 *nlo,
-                                                             const double2 *nhi, int K) {
+                                                             const double2 *tw1, const double2 *colf,
+                                                             const double2 *packf) {
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M1, P);
@@ -403,7 +427,7 @@ __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, d
     double2 xk = X[k], xm = X[M - k];
     if (k == 0) xk.y = xm.y = 0.0;
     const double2 s = make_double2(xk.x + xm.x, xk.y - xm.y), d = make_double2(xk.x - xm.x, xk.y + xm.y);
-    const double2 w = cmul(root2(nlo, nhi, k, K, +1), d);
+    const double2 w = tan_mul(d, conj_tan(packf[(size_t)c * M1 + n1]));
     sm64[digit_rev(n1, P)] = make_double2(s.x - w.y, s.y + w.x);
     if (k > 0) {
       const int nm = c == 0 ? M1 - n1 : M1 - 1 - n1;
@@ -414,7 +438,7 @@ __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, d
   dit_fft<+1>(sm64, M1, P, tw1, 1, two ? 2 : 1);
   for (int t = threadIdx.x; t < (two ? 2 * M1 : M1); t += blockDim.x) {
     const int which = t >= M1, k1 = t - which * M1, col = which ? cm : c;
-    dst[(size_t)k1 * M2 + col] = cmul(sm64[t], root2(mlo, mhi, (long long)col * k1, K, +1));
+    dst[(size_t)k1 * M2 + col] = tan_mul(sm64[t], conj_tan(colf[(size_t)col * M1 + k1]));
   }
 }
 
@@ -436,8 +460,7 @@ __global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, doub
 // with s = Z_k + Z*_{M-k}, d = Z_k - Z*_{M-k} and w = e^{-2 pi i k/ND} d, 2 X_k = s - i w
 // and 2 X_{M-k} = s* - i w*.
 __global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *src, double2 *X, int M1, int M2,
-                                                               const double2 *tw2, const double2 *nlo,
-                                                               const double2 *nhi, int K) {
+                                                               const double2 *tw2, const double2 *unpackf) {
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M2, P);
@@ -456,7 +479,7 @@ __global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *sr
     const long long k = (long long)r + (long long)M1 * k2;
     const double2 zk = sm64[k2], zm = sm64[bo + (r == 0 ? (k2 == 0 ? 0 : M2 - k2) : M2 - 1 - k2)];
     const double2 s = make_double2(zk.x + zm.x, zk.y - zm.y), d = make_double2(zk.x - zm.x, zk.y + zm.y);
-    const double2 w = cmul(root2(nlo, nhi, k, K, -1), d);
+    const double2 w = tan_mul(d, unpackf[(size_t)r * M2 + k2]);
     X[k] = make_double2(s.x + w.y, s.y - w.x);
     if (2 * k != M) X[M - k] = make_double2(s.x - w.y, -(s.y + w.x));
   }
@@ -745,10 +768,13 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   for (int i = 0; i <= NT / 2; i++) win[i] = (R)window[i];
   const size_t elem = sizeof(C);
   auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
-  const size_t sizes[12] = {elem * t1.size(), elem * t2.size(), elem * tn.size(), elem * mlo.size(),
+  // FP64: the passes' factors (wdm_roots64_kernel)
+  const size_t full = sizeof(R) == 8 ? elem : 0;
+  const size_t sizes[15] = {elem * t1.size(), elem * t2.size(), elem * tn.size(), elem * mlo.size(),
                             elem * mhi.size(), elem * nlo.size(), elem * nhi.size(), sizeof(R) * win.size(),
                             elem * (size_t)(M + 1), elem * (size_t)(M + 1), elem * (size_t)(M + 1),
-                            sizeof(double) * (size_t)ND};
+                            sizeof(double) * (size_t)ND,
+                            full * (size_t)M, full * (size_t)(P.M2 / 2 + 1) * P.M1, full * (size_t)(P.M1 / 2 + 1) * P.M2};
   size_t bytes = 0;
   for (size_t b : sizes) bytes += pad(b);
   cudaError_t e = cudaMalloc(&P.base, bytes);
@@ -756,9 +782,10 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
     P.base = nullptr;
     return e;
   }
-  void **slots[12] = {&P.tw1, &P.tw2, &P.twNT, &P.mlo, &P.mhi, &P.nlo, &P.nhi, &P.win, &P.bufA, &P.bufB, &P.bufX, &P.rbuf};
+  void **slots[15] = {&P.tw1, &P.tw2, &P.twNT, &P.mlo,  &P.mhi,  &P.nlo,   &P.nhi,    &P.win,
+                      &P.bufA, &P.bufB, &P.bufX, &P.rbuf, &P.colf, &P.packf, &P.unpackf};
   char *p = (char *)P.base;
-  for (int i = 0; i < 12; i++) {
+  for (int i = 0; i < 15; i++) {
     *slots[i] = p;
     p += pad(sizes[i]);
   }
@@ -770,6 +797,10 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   if ((e = upload(P.nlo, nlo, s)) != cudaSuccess) return e;
   if ((e = upload(P.nhi, nhi, s)) != cudaSuccess) return e;
   if ((e = upload(P.win, win, s)) != cudaSuccess) return e;
+  if constexpr (sizeof(R) == 8) {
+    wdm_roots64_kernel<<<1024, 256, 0, s>>>((double2 *)P.colf, (double2 *)P.packf, (double2 *)P.unpackf, P.M1, P.M2);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
   return cudaStreamSynchronize(s);  // the host vectors go out of scope
 }
 
@@ -830,11 +861,10 @@ static cudaError_t forward64(const WdmPlan &P, const double *time, double *wdm, 
     packed = reinterpret_cast<const double2 *>(P.rbuf);
   }
   if ((e = launch64(wdm_col64_kernel, P.M2, P.M1, 256, s, packed, (double2 *)P.bufB, P.M1, P.M2,
-                    (const double2 *)P.tw1, (const double2 *)P.mlo, (const double2 *)P.mhi, P.K)) != cudaSuccess)
+                    (const double2 *)P.tw1, (const double2 *)P.colf)) != cudaSuccess)
     return e;
   if ((e = launch64(wdm_row_unpack64_kernel, P.M1 / 2 + 1, 2 * P.M2, 512, s, (const double2 *)P.bufB,
-                    (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.nlo,
-                    (const double2 *)P.nhi, P.K)) != cudaSuccess)
+                    (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.unpackf)) != cudaSuccess)
     return e;
   return fwd_layers64(P, (const double2 *)P.bufX, 0.5, wdm, s);
 }
@@ -868,8 +898,8 @@ static cudaError_t inverse64(const WdmPlan &P, const double *wdm, double *time, 
   cudaError_t e;
   if ((e = inverse_layers64(P, wdm, 1.0 / (double)ND, s)) != cudaSuccess) return e;
   if ((e = launch64(wdm_pack_col64_kernel, P.M2 / 2 + 1, 2 * P.M1, 512, s, (const double2 *)P.bufX,
-                    (double2 *)P.bufB, P.M1, P.M2, (const double2 *)P.tw1, (const double2 *)P.mlo,
-                    (const double2 *)P.mhi, (const double2 *)P.nlo, (const double2 *)P.nhi, P.K)) != cudaSuccess)
+                    (double2 *)P.bufB, P.M1, P.M2, (const double2 *)P.tw1, (const double2 *)P.colf,
+                    (const double2 *)P.packf)) != cudaSuccess)
     return e;
   const bool direct = (uintptr_t)time % 16 == 0;
   double2 *dst = reinterpret_cast<double2 *>(direct ? (void *)time : P.rbuf);

@@ -14,6 +14,7 @@ struct WdmPlan {
   void *base = nullptr;
   void *tw1 = nullptr, *tw2 = nullptr, *twNT = nullptr;
   void *mlo = nullptr, *mhi = nullptr, *nlo = nullptr, *nhi = nullptr;
+  void *colf = nullptr, *packf = nullptr, *unpackf = nullptr;  // FP64: the passes' factors, one per point
   void *win = nullptr;
   void *bufA = nullptr, *bufB = nullptr, *bufX = nullptr;
   void *rbuf = nullptr;  // NF NT reals: staging for FP32 casts and unaligned FP64 input
