@@ -46,6 +46,7 @@
 #include <vector>
 
 #include "fft_dit.cuh"
+#include "glass_common.cuh"
 #include "wdm.cuh"
 
 namespace glass {
@@ -394,6 +395,7 @@ __global__ void wdm_roots64_kernel(double2 *colf, double2 *packf, double2 *unpac
 // over 152 SMs where 256 of four columns leave a sixth of them idle).
 __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, double2 *dst, int M1, int M2,
                                                         const double2 *tw1, const double2 *colf) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M1, P);
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(256) wdm_col64_kernel(const double2 *src, doub
 __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, double2 *dst, int M1, int M2,
                                                              const double2 *tw1, const double2 *colf,
                                                              const double2 *packf) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M1, P);
@@ -445,6 +448,7 @@ __global__ void __launch_bounds__(512) wdm_pack_col64_kernel(const double2 *X, d
 // The inverse's pass 2, one row per CTA: output index k1 + M1 k2.
 __global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, double2 *dst, int M1, int M2,
                                                         const double2 *tw2) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M2, P);
@@ -461,6 +465,7 @@ __global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, doub
 // and 2 X_{M-k} = s* - i w*.
 __global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *src, double2 *X, int M1, int M2,
                                                                const double2 *tw2, const double2 *unpackf) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M2, P);
@@ -495,6 +500,7 @@ __host__ __device__ __forceinline__ int layer_pairs(int NF) { return 1 + NF / 2;
 // they are (no shift).
 __global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, int NF, int NT, const double *phif,
                                                              const double2 *twNT, double scale, double *wdm) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(NT, P);
@@ -558,6 +564,7 @@ __global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, i
 __global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, int NF, int NT, int launch,
                                                              const double *phif, const double2 *twNT, double scale,
                                                              double2 *X) {
+  grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(NT, P);
@@ -833,8 +840,7 @@ template <typename K, typename... Args>
 static cudaError_t launch64(K kernel, int grid, int points, int most, cudaStream_t s, Args... args) {
   cudaError_t e;
   if (smem64(points) > 48 * 1024 && (e = set_smem((const void *)kernel, smem64(points))) != cudaSuccess) return e;
-  kernel<<<grid, threads64(points, most), smem64(points), s>>>(args...);
-  return cudaGetLastError();
+  return launch_chained(kernel, grid, threads64(points, most), smem64(points), s, args...);
 }
 
 // scale times the real spectrum X -> coefficients.
