@@ -39,6 +39,7 @@
 // the inverse's overlap-add runs in two launches (even, then odd layers: the
 // supports of same-parity layers are disjoint, so no atomics are needed and the
 // sum order is fixed).
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <mutex>
@@ -463,31 +464,41 @@ __global__ void __launch_bounds__(256) wdm_row64_kernel(const double2 *src, doub
 // M1 k2 and M - k of the packed spectrum Z, unpacked to twice the real spectrum:
 // with s = Z_k + Z*_{M-k}, d = Z_k - Z*_{M-k} and w = e^{-2 pi i k/ND} d, 2 X_k = s - i w
 // and 2 X_{M-k} = s* - i w*.
-__global__ void __launch_bounds__(512) wdm_row_unpack64_kernel(const double2 *src, double2 *X, int M1, int M2,
-                                                               const double2 *tw2, const double2 *unpackf) {
+//
+// A cluster of two CTAs per pair, a row each: 1026 CTAs balance over 152 SMs where
+// 513 leave a sixth of them idle (88 -> 77 us at 1024 x 1024 points).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) wdm_row_unpack64_kernel(const double2 *src, double2 *X,
+                                                                                        int M1, int M2,
+                                                                                        const double2 *tw2,
+                                                                                        const double2 *unpackf) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
   RadixPlan P;
   radix_plan(M2, P);
   const long long M = (long long)M1 * M2;
-  const int r = blockIdx.x, rm = r == 0 ? 0 : M1 - r;
+  const int h = (int)cluster.block_rank(), r = blockIdx.x >> 1, rm = r == 0 ? 0 : M1 - r;
   const bool two = rm != r;
-  for (int t = threadIdx.x; t < (two ? 2 * M2 : M2); t += blockDim.x) {
-    const int which = t >= M2, k2 = t - which * M2;
-    sm64[which * M2 + digit_rev(k2, P)] = src[(size_t)(which ? rm : r) * M2 + k2];
+  if (two || h == 0) {
+    for (int k2 = threadIdx.x; k2 < M2; k2 += blockDim.x)
+      sm64[digit_rev(k2, P)] = src[(size_t)(h ? rm : r) * M2 + k2];
+    __syncthreads();
+    dit_fft<-1>(sm64, M2, P, tw2, 1);
   }
-  __syncthreads();
-  dit_fft<-1>(sm64, M2, P, tw2, 1, two ? 2 : 1);
-  const int bo = two ? M2 : 0;
+  cluster.sync();  // both rows are transformed
+  const double2 *Z = cluster.map_shared_rank(sm64, 0), *Zm = cluster.map_shared_rank(sm64, two ? 1 : 0);
   const int n = two ? M2 : r == 0 ? M2 / 2 + 1 : (M2 + 1) / 2;
-  for (int k2 = threadIdx.x; k2 < n; k2 += blockDim.x) {
+  const int lo = h ? (n + 1) / 2 : 0, hi = h ? n : (n + 1) / 2;  // this CTA's part
+  for (int k2 = lo + threadIdx.x; k2 < hi; k2 += blockDim.x) {
     const long long k = (long long)r + (long long)M1 * k2;
-    const double2 zk = sm64[k2], zm = sm64[bo + (r == 0 ? (k2 == 0 ? 0 : M2 - k2) : M2 - 1 - k2)];
+    const double2 zk = Z[k2], zm = Zm[r == 0 ? (k2 == 0 ? 0 : M2 - k2) : M2 - 1 - k2];
     const double2 s = make_double2(zk.x + zm.x, zk.y - zm.y), d = make_double2(zk.x - zm.x, zk.y + zm.y);
     const double2 w = tan_mul(d, unpackf[(size_t)r * M2 + k2]);
     X[k] = make_double2(s.x + w.y, s.y - w.x);
     if (2 * k != M) X[M - k] = make_double2(s.x - w.y, -(s.y + w.x));
   }
+  cluster.sync();  // no CTA leaves while the other reads its row
 }
 
 // Layers of pair q: 0: the grid's first and last (0, NF); q >= 1: 2 q - 1 and 2 q
@@ -498,13 +509,21 @@ __host__ __device__ __forceinline__ int layer_pairs(int NF) { return 1 + NF / 2;
 // what the window must be multiplied with, 1/NT and the Hermitian parts' half
 // included).  The first and last layer use the real parts of even n alone, as
 // they are (no shift).
-__global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, int NF, int NT, const double *phif,
-                                                             const double2 *twNT, double scale, double *wdm) {
+//
+// A cluster of two CTAs per pair: CTA h takes the elements of parity h, half the
+// transform's length, and the last radix-2 stage, over half of the outputs each,
+// reads both halves (for 513 pairs 112 -> 102 us: 1026 CTAs balance over the SMs).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, int NF, int NT,
+                                                                                      const double *phif,
+                                                                                      const double2 *twNT, double scale,
+                                                                                      double *wdm) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
+  const int q = blockIdx.x >> 1, par = (int)cluster.block_rank(), h = NT / 2;
   RadixPlan P;
-  radix_plan(NT, P);
-  const int q = blockIdx.x, h = NT / 2;
+  radix_plan(h, P);
   const bool edge = q == 0;
   const int ma = edge ? 0 : 2 * q - 1, mb = edge ? NF : 2 * q;
   const bool has_b = edge || mb < NF;
@@ -520,7 +539,13 @@ __global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, i
     v = make_double2(v.x * w, v.y * w);
     return (!edge && (m & 1)) ? make_double2(-v.y, v.x) : v;
   };
-  for (int e = threadIdx.x; e <= h; e += blockDim.x) {
+  // e = 0 .. NT/2 gives the elements p and NT - p: of the layer pairs, p = e + 3 NT/4
+  // (mod NT) up to NT/4 and p = e above; of the edge layers, p = e.  Those of this
+  // CTA's parity: n1 up to NT/4, from e1, then the rest, from e2.
+  const int e1 = edge ? par : (par + 3 * (NT / 4)) & 1, n1 = e1 > NT / 4 ? 0 : (NT / 4 - e1) / 2 + 1;
+  const int e2 = NT / 4 + 1 + ((NT / 4 + 1 + par) & 1), n2 = e2 > h ? 0 : (h - e2) / 2 + 1;
+  for (int i = threadIdx.x; i < n1 + n2; i += blockDim.x) {
+    const int e = i < n1 ? e1 + 2 * i : e2 + 2 * (i - n1);
     int k, kp, p, pp;
     if (edge) {
       k = p = e;
@@ -534,23 +559,30 @@ __global__ void __launch_bounds__(256) wdm_fwd_pair64_kernel(const double2 *X, i
     const double2 zero = make_double2(0.0, 0.0);
     const double2 a0 = bin(ma, k), a1 = bin(ma, kp), b0 = has_b ? bin(mb, k) : zero, b1 = has_b ? bin(mb, kp) : zero;
     const double ax = a0.x + a1.x, ay = a0.y - a1.y, bx = b0.x + b1.x, by = b0.y - b1.y;
-    sm64[digit_rev(p, P)] = make_double2(ax - by, ay + bx);
-    if (pp != p) sm64[digit_rev(pp, P)] = make_double2(ax + by, bx - ay);
+    sm64[digit_rev(p >> 1, P)] = make_double2(ax - by, ay + bx);
+    if (pp != p) sm64[digit_rev(pp >> 1, P)] = make_double2(ax + by, bx - ay);
   }
   __syncthreads();
-  dit_fft<+1>(sm64, NT, P, twNT, 1);
-  if (edge) {
-    for (int n = 2 * threadIdx.x; n < NT; n += 2 * blockDim.x) {
-      wdm[n] = sm64[n].x;
-      wdm[n + 1] = sm64[n].y;
-    }
-  } else {
-    for (int n = threadIdx.x; n < NT; n += blockDim.x) {
-      const double2 v = sm64[n];
-      wdm[n + (size_t)NT * ma] = (n & 2) ? -v.x : v.x;
-      if (has_b) wdm[n + (size_t)NT * mb] = (n & 2) ? -v.y : v.y;
+  dit_fft<+1>(sm64, h, P, twNT, 2);
+  cluster.sync();  // both halves are transformed
+  const double2 *E = cluster.map_shared_rank(sm64, 0), *O = cluster.map_shared_rank(sm64, 1);
+  for (int k = par * (h / 2) + threadIdx.x; k < (par + 1) * (h / 2); k += blockDim.x) {
+    if (edge && (k & 1)) continue;  // even n alone
+    double2 v[2];
+    tan_radix2(E[k], O[k], conj_tan(twNT[k]), v[0], v[1]);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int n = k + u * h;
+      if (edge) {
+        wdm[n] = v[u].x;
+        wdm[n + 1] = v[u].y;
+      } else {
+        wdm[n + (size_t)NT * ma] = (n & 2) ? -v[u].x : v[u].x;
+        if (has_b) wdm[n + (size_t)NT * mb] = (n & 2) ? -v[u].y : v[u].y;
+      }
     }
   }
+  cluster.sync();  // no CTA leaves while the other reads its half
 }
 
 // Inverse layers, a pair per CTA: the FFT of u_a + i u_b, u a layer's coefficients
@@ -847,7 +879,7 @@ static cudaError_t launch64(K kernel, int grid, int points, int most, cudaStream
 static cudaError_t fwd_layers64(const WdmPlan &P, const double2 *X, double scale, double *wdm, cudaStream_t s) {
   const int NF = P.NF, NT = P.NT;
   if (NT % 4 == 0)
-    return launch64(wdm_fwd_pair64_kernel, layer_pairs(NF), NT, 256, s, X, NF, NT, (const double *)P.win,
+    return launch64(wdm_fwd_pair64_kernel, 2 * layer_pairs(NF), NT / 2, 256, s, X, NF, NT, (const double *)P.win,
                     (const double2 *)P.twNT, 0.5 * scale / NT, wdm);
   const size_t sm = fft_smem<double2>(NT, 1);
   const cudaError_t e = set_smem((const void *)wdm_fwd_layer_kernel<double2>, sm);
@@ -869,7 +901,7 @@ static cudaError_t forward64(const WdmPlan &P, const double *time, double *wdm, 
   if ((e = launch64(wdm_col64_kernel, P.M2, P.M1, 256, s, packed, (double2 *)P.bufB, P.M1, P.M2,
                     (const double2 *)P.tw1, (const double2 *)P.colf)) != cudaSuccess)
     return e;
-  if ((e = launch64(wdm_row_unpack64_kernel, P.M1 / 2 + 1, 2 * P.M2, 512, s, (const double2 *)P.bufB,
+  if ((e = launch64(wdm_row_unpack64_kernel, 2 * (P.M1 / 2 + 1), P.M2, 256, s, (const double2 *)P.bufB,
                     (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.unpackf)) != cudaSuccess)
     return e;
   return fwd_layers64(P, (const double2 *)P.bufX, 0.5, wdm, s);
