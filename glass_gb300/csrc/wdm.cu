@@ -593,20 +593,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256) wdm_fwd_pair64_
 // first layer adds in the second launch; the last stores in the first where the
 // pair below it is of even q, else adds in the second.  blockIdx: the launch's
 // pairs, then its edge layers (first, last).
-__global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, int NF, int NT, int launch,
-                                                             const double *phif, const double2 *twNT, double scale,
-                                                             double2 *X) {
+//
+// A cluster of four CTAs per unit: CTA r takes the elements n = r (mod 4), a
+// quarter of the transform's length, and the last radix-4 stage goes through
+// distributed shared memory, every fourth butterfly each; then each forms a quarter
+// of the bins (of 385 units 193 -> 159 us: 1540 CTAs balance over 152 SMs where
+// 385 leave a sixth of the pipes idle).
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, int NF, int NT,
+                                                                                      int launch, const double *phif,
+                                                                                      const double2 *twNT, double scale,
+                                                                                      double2 *X) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   grid_begin();
   extern __shared__ __align__(16) double2 sm64[];
+  const int r = (int)cluster.block_rank(), unit = blockIdx.x >> 2, L = NT / 4;
   RadixPlan P;
-  radix_plan(NT, P);
+  radix_plan(L, P);
   const int h = NT / 2, pairs = NF / 2, mine = launch == 0 ? (pairs + 1) / 2 : pairs / 2;
-  const bool edge = (int)blockIdx.x >= mine;
-  const int q = 2 * blockIdx.x + 1 + launch;
+  const bool edge = unit >= mine;
+  const int q = 2 * unit + 1 + launch;
   const int ma = 2 * q - 1, mb = 2 * q;
   const bool has_b = mb < NF;
-  const bool last = edge && (launch == 0 || (int)blockIdx.x > mine);  // the edge CTA's layer is NF
-  for (int n = threadIdx.x; n < NT; n += blockDim.x) {
+  const bool last = edge && (launch == 0 || unit > mine);  // the edge CTA's layer is NF
+  for (int n = r + 4 * threadIdx.x; n < NT; n += 4 * blockDim.x) {
     double2 v = make_double2(0.0, 0.0);
     if (edge) {
       v.x = wdm[(2 * n) % NT + last];
@@ -618,35 +628,53 @@ __global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, 
       if ((n + 1) & 2) v.x = -v.x;
       if (n & 2) v.y = -v.y;
     }
-    sm64[digit_rev(n, P)] = v;
+    sm64[digit_rev(n >> 2, P)] = v;
   }
   __syncthreads();
-  dit_fft<-1>(sm64, NT, P, twNT, 1);
+  dit_fft<-1>(sm64, L, P, twNT, 4);
+  cluster.sync();  // the four quarters are transformed
+  double2 *S[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) S[m] = cluster.map_shared_rank(sm64, (unsigned)m);
+  for (int k = r + 4 * threadIdx.x; k < L; k += 4 * blockDim.x) {
+    double2 v0 = S[0][k], v1 = S[1][k], v2 = S[2][k], v3 = S[3][k];
+    tan_radix4<-1>(v0, v1, v2, v3, twNT[k], twNT[2 * k]);
+    S[0][k] = v0;
+    S[1][k] = v1;
+    S[2][k] = v2;
+    S[3][k] = v3;
+  }
+  cluster.sync();  // bin k of the transform: S[k / L][k mod L]
+  auto bin = [&](int k) {
+    const int m = (k >= L) + (k >= 2 * L) + (k >= 3 * L);
+    return cluster.map_shared_rank(sm64, (unsigned)m)[k - m * L];
+  };
   if (edge) {
     const double c = scale * 0.70710678118654752440;
     const long long M = (long long)NF * h;
     // layer 0: bins 0 .. h - 1; layer NF: M - h .. M, bin M its own
-    for (int i = threadIdx.x; i < (last ? h + 1 : h); i += blockDim.x) {
+    for (int i = r * blockDim.x + threadIdx.x; i < (last ? h + 1 : h); i += 4 * blockDim.x) {
       const long long k = last ? M - i : i;
-      const double2 a = sm64[(int)((2 * k) % NT)];
+      const double2 a = bin((int)((2 * k) % NT));
       const double w = c * phif[i];
       if (last && (i == 0 || launch == 0))
         X[k] = make_double2(w * a.x, w * a.y);
       else
         X[k] = make_double2(fma(w, a.x, X[k].x), fma(w, a.y, X[k].y));
     }
+    cluster.sync();  // no CTA leaves while another reads its quarter
     return;
   }
   const double c = 0.5 * scale;
   // spectrum of layer a (real part's) or b at bin k of its own transform, twice
   auto part = [&](bool second, int k) {
-    const double2 f = sm64[k], g = sm64[k == 0 ? 0 : NT - k];
+    const double2 f = bin(k), g = bin(k == 0 ? 0 : NT - k);
     return second ? make_double2(f.y + g.y, g.x - f.x) : make_double2(f.x + g.x, f.y - g.y);
   };
   // bin i of layer m: R_m[i mod NT] = nu U_m[(i + NT/4) mod NT], nu = -i for layer a
   const int i0 = (q - 1) * NT, ca = ma * h, cb = ca + h;
   const int top = has_b ? NT : h;  // the upper layer's upper half
-  for (int t = threadIdx.x; t < top + h; t += blockDim.x) {
+  for (int t = r * blockDim.x + threadIdx.x; t < top + h; t += 4 * blockDim.x) {
     const int i = i0 + t, k = (t + NT / 4) % NT;  // i0 is a multiple of NT
     double2 v = make_double2(0.0, 0.0);
     if (t < NT) {
@@ -665,6 +693,7 @@ __global__ void __launch_bounds__(256) wdm_inv_pair64_kernel(const double *wdm, 
     }
     X[i] = v;
   }
+  cluster.sync();  // no CTA leaves while another reads its quarter
 }
 
 template <typename C>
@@ -918,10 +947,10 @@ static cudaError_t inverse_layers64(const WdmPlan &P, const double *wdm, double 
   if (NT % 4 == 0) {
     const int pairs = NF / 2;  // (1, 2), (3, 4), ...
     const bool last_first = pairs % 2 == 0;  // the last layer's place: see the kernel
-    if ((e = launch64(wdm_inv_pair64_kernel, (pairs + 1) / 2 + last_first, NT, 256, s, wdm, NF, NT, 0, win, tw, scale,
+    if ((e = launch64(wdm_inv_pair64_kernel, 4 * ((pairs + 1) / 2 + last_first), NT / 4, 256, s, wdm, NF, NT, 0, win, tw, scale,
                       X)) != cudaSuccess)
       return e;
-    return launch64(wdm_inv_pair64_kernel, pairs / 2 + 1 + !last_first, NT, 256, s, wdm, NF, NT, 1, win, tw, scale, X);
+    return launch64(wdm_inv_pair64_kernel, 4 * (pairs / 2 + 1 + !last_first), NT / 4, 256, s, wdm, NF, NT, 1, win, tw, scale, X);
   }
   wdm_zero_kernel<double2><<<blocks_for(P.M + 1), 256, 0, s>>>(X, P.M + 1);
   const size_t sm = fft_smem<double2>(NT, 1);
