@@ -702,9 +702,14 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
   if ((e = cudaEventRecord(work.fork, stream)) != cudaSuccess) return e;
   int nb = 0;
   while (nb < kNumBins && 32 << nb <= pa.NFFT) nb++;
-  // largest size first, on the caller's stream: its groups take whole SMs, and
-  // the smaller sizes fill in behind them as it ends (the other way round it
-  // waits for SMs to empty, and ends the call alone)
+  // In a stream, largest size first, on the caller's stream: its groups take whole
+  // SMs, and the smaller sizes fill in behind them as it ends (the other way round
+  // it waits for SMs to empty, and ends the call alone): 2500 proposals on
+  // 8192-bin segments 109 -> 102 us.  A graph starts its branches together, and
+  // there smallest first is the better order (101 against 118 us).
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if ((e = cudaStreamIsCapturing(stream, &capture)) != cudaSuccess) return e;
+  const bool graph = capture == cudaStreamCaptureStatusActive;
   bool forked[kNumBins] = {};
   auto join = [&] {
     cudaError_t r = cudaSuccess;
@@ -715,9 +720,10 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
       }
     return r;
   };
-  for (int b = nb - 1; b >= 0; b--) {
+  for (int q = 0; q < nb; q++) {
+    const int b = graph ? q : nb - 1 - q;
     const int N = 32 << b;
-    cudaStream_t sb = b == nb - 1 ? stream : work.side[b];
+    cudaStream_t sb = !graph && q == 0 ? stream : work.side[b];
     if (sb != stream && (e = cudaStreamWaitEvent(sb, work.fork, 0)) != cudaSuccess) {
       join();
       return e;

@@ -124,3 +124,53 @@ def test_host_calls_of_small_batches(engine, n):
             torch.cuda.synchronize()
             for a, b in zip(got, out):
                 np.testing.assert_array_equal(a, b.cpu().numpy())
+
+
+@pytest.mark.parametrize("NFFT", [1024, 4096])
+def test_chains_in_a_captured_graph(engine, NFFT):
+    """The chained launches under stream capture, with the size kernels' side branches
+    (banks beyond 1024 bins) and with and without the re-evaluation's conditional
+    node: a replay gives the direct call's bits, for new inputs in the same arrays."""
+    import torch
+
+    rng = np.random.default_rng(NFFT)
+    f0s = np.array([1e-3, 4e-3, 1.1e-2])
+    bank = _bank(rng, f0s)
+    if NFFT < 4096:
+        off = (4096 - NFFT) // 2
+        bank = wl.SegmentBank(T=T, NFFT=NFFT, qmin=(bank.qmin + off).astype(np.int32),
+                              **{k: np.ascontiguousarray(getattr(bank, k)[:, off:off + NFFT])
+                                 for k in ("dA", "dE", "invCA", "invCE")})
+    engine.upload(bank)
+    dev = lambda x: torch.tensor(x, device="cuda")
+    s = torch.cuda.Stream()
+    try:
+        for prec in (gg.PREC_FP64, gg.PREC_MIXED):
+            for n in (20, 700):
+                seg = (np.arange(n) % 3).astype(np.int32)
+                ps = [np.array([_source(rng, f0s[k], lnA=rng.uniform(-51, -48), costh=rng.uniform(-1, 1)) for k in seg])
+                      for _ in range(3)]
+                p, sg = dev(ps[0]), dev(seg)
+                out = [dev(np.zeros(n)) for _ in range(3)] + [dev(np.zeros(n, np.int32))]
+                ref = []
+                for q in ps:
+                    p.copy_(dev(q))
+                    engine.dlogl_device(sg, p, *out, None, prec)
+                    torch.cuda.synchronize()
+                    ref.append([o.clone() for o in out])
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=s):
+                    engine.set_stream(torch.cuda.current_stream().cuda_stream)
+                    engine.dlogl_device(sg, p, *out, None, prec)
+                engine.set_stream(None)
+                for q, r in zip(ps, ref):
+                    p.copy_(dev(q))
+                    for o in out:
+                        o.zero_()
+                    torch.cuda.synchronize()
+                    g.replay()
+                    torch.cuda.synchronize()
+                    for a, b in zip(out, r):
+                        assert torch.equal(a, b)
+    finally:
+        engine.set_stream(None)
