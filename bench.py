@@ -1425,7 +1425,7 @@ def run_ours(args):
     # dominant kernel of the mixed step: the longer of the slow-part and the
     # spectral kernel; its algorithmic flops per launch over its mean duration
     kern = {"fd_slow_kernel<1>": (phase_ms[1], flops_slow), "fd_spec_all_kernel<1, 0>": (phase_ms[2], flops_spec)}
-    phase_names = ("fd_planmix_kernel", "fd_slow_kernel<1>", "fd_spec_all_kernel<1, 0>", "re-evaluation")
+    phase_names = ("fd_plan_kernel<1>", "fd_slow_kernel<1>", "fd_spec_all_kernel<1, 0>", "re-evaluation")
     dom = max(kern, key=lambda k: kern[k][0])
     ms_dom, fl_dom = kern[dom]
     ach_dom = fl_dom / (ms_dom * 1e-3) / 1e12

@@ -35,11 +35,12 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompil
 # where a fused multiply-add would round differently by up to ~1e-10 rad) with
 # explicit round-to-nearest operations, so its translation units contract
 # freely.  The no-allocation entry point, the F-statistic, the wavelet-domain
-# waveform and the noise and sampler units keep contraction off: their
-# results follow the reference's operation order throughout.  So do the host
+# waveform and the noise and sampler units keep contraction off: what must
+# follow the reference's operation order is written in that order there, and
+# what may be fused uses fma explicitly.  Contraction is also off in the host
 # sums of the struct-based drop-ins (dropin_model.cu), which are bit-identical
-# to the reference's x86 build only without contraction (gcc on aarch64
-# contracts a * b + c by default).
+# to the reference's x86 build only without it (gcc on aarch64 contracts
+# a * b + c by default).
 PER_FILE_FLAGS = {"ucb_fd_noalloc.cu": ["-fmad=false"],
                   "wdm.cu": ["-Xcompiler", "-ffp-contract=off"],
                   "ucb_wavelet.cu": ["-fmad=false", "-Xcompiler", "-ffp-contract=off"],

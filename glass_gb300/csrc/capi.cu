@@ -128,6 +128,7 @@ struct glass_gpu_ctx {
   bool host_direct = false;     // in use
   HostIo *h_io = nullptr;
   std::map<long long, cudaGraphExec_t> host_graphs;
+  std::map<long long, int> host_launches;  // kernels of each graph (a conditional body not counted)
   int last_launches = 0;
   int n_fixed = 0;  // template size override (0: bandwidth rule)
   // mixed precision: proposals whose estimated delta-logL error exceeds this
@@ -892,7 +893,7 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
   auto it = ctx->host_graphs.find(key);
   if (it != ctx->host_graphs.end() && !ctx->work.phase_timing) {
     GLASS_CUDA(cudaGraphLaunch(it->second, s), "dlogl_batch_host graph launch");
-    ctx->last_launches = 3;
+    ctx->last_launches = small ? ctx->host_launches[key] : 3;
   } else {
     if ((rc = enqueue())) return rc;
     GLASS_CUDA(cudaStreamSynchronize(s), "dlogl_batch_host sync");
@@ -905,8 +906,10 @@ extern "C" int glass_gpu_dlogl_batch_host(glass_gpu_ctx *ctx, int precision, int
       if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
         const int rc2 = enqueue();
         const cudaError_t e2 = cudaStreamEndCapture(s, &g);
-        if (rc2 == GLASS_OK && e2 == cudaSuccess && cudaGraphInstantiate(&ge, g, 0) == cudaSuccess)
+        if (rc2 == GLASS_OK && e2 == cudaSuccess && cudaGraphInstantiate(&ge, g, 0) == cudaSuccess) {
           ctx->host_graphs[key] = ge;
+          ctx->host_launches[key] = nl;
+        }
         if (g) cudaGraphDestroy(g);
       }
       cudaGetLastError();

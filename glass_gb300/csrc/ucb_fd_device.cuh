@@ -624,7 +624,7 @@ __device__ __forceinline__ void fast_sincos(float x, float *s, float *c) {
 // is 87% busy): arm vectors from the sample table, antenna patterns from the
 // arms' projections on the polarisation axes, per-proposal constants instead of
 // divisions, sinc by series and sincos by table.  640 -> 320 FP64 instructions
-// per sample; 3072 proposals of 32..1024 samples 880 -> 393 us (the whole step 1169 -> 633,
+// per sample; 3072 proposals of 32..1024 samples 880 -> 393 us (the whole step 1169 -> 565,
 // with the spectral unit below).
 
 // kx / c, correctly rounded: the product with 1/c and one exact-residual step.

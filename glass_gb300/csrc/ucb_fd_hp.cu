@@ -230,8 +230,8 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // ping-pong buffers and a twiddle copy took 192 KB and left one CTA per SM); the
 // bank's entries of a thread's first bins are loaded before the transform, those
 // of each next bin and the twiddles of each next butterfly before the arithmetic of
-// the current one.  61 proposals of up to 1024 points 19.1 -> 16.5 us, 73 of up to
-// 2048 on 8192-bin segments 60.8 -> 38 us.
+// the current one.  61 proposals of up to 1024 points 19.1 -> 16 us, 73 of up to
+// 4096 on 8192-bin segments 60.8 -> 36 us.
 template <bool PERCH>
 __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;

@@ -11,7 +11,7 @@
 // memory and a stream; nothing else is needed.
 //
 // Consequences of the fixed arrays (also stated in include/glass_gb300.h):
-//  * every GPU that loads this library holds them (about 41 MB) until the
+//  * every GPU that loads this library holds them (about 43 MB) until the
 //    process exits;
 //  * every call on a device uses the same arrays, so calls that overlap on the
 //    GPU (two streams, or two host threads) race and corrupt each other;

@@ -34,10 +34,10 @@
 //           bins 0 < k < NFFT;
 //   finish  one thread per cell: the 4x4 solve, logL and the fit.
 // All four are bound by the FP64 pipe (85% busy by ncu).  Against four filters,
-// each with its own series, transforms and ten products, 1440 -> 340 FP64
-// instructions per sample in the slow part and 656 -> 235 in the spectral part;
+// each with its own series, transforms and ten products, 1440 -> 314 FP64
+// instructions per sample in the slow part and 656 -> 208 in the spectral part;
 // the solve, one lane of a warp per cell before, runs full warps.  51200 cells
-// of 64 samples: 13.43 -> 3.51 ms.
+// of 64 samples: 13.43 -> 3.27 ms.
 //
 // The A/E inner products of the reference weight both channels with the A
 // channel's noise C[0][0]; with templates and data whitened by their own

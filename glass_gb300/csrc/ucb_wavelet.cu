@@ -624,9 +624,9 @@ __global__ void __launch_bounds__(256) wv_carrier_kernel(WvGridDev g, const WvSr
 
 // Bound by the FP64 pipe: per sample 22 FP64 instructions for the channel's
 // amplitude and phase and a table cosine (the carrier is shared, its times and
-// intervals tabulated; 114 when each channel evaluated everything), 39 per point
+// intervals tabulated; 114 when each channel evaluated everything), 35 per point
 // of the packed FFT, and half a transform per layer.  4096 sources (three channels
-// of 6144 samples, two layers) 25.4 -> 10.3 ms (9.4, and 0.9 for the carrier kernel).
+// of 6144 samples, two layers) 25.4 -> 9.2 ms (8.3, and 0.9 for the carrier kernel).
 __global__ void __launch_bounds__(kLayerThreads) wv_layers_kernel(WvGridDev g, int n, const WvSrc *srcs,
                                                                   const double *carrier, const double *tdi,
                                                                   double *coef, const int *count, const int *list) {

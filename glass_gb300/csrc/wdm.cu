@@ -14,7 +14,8 @@
 //    (x[2n] + i x[2n+1]), done four-step as M1 x M2: FFTs down the M2 columns
 //    with the exp(-2 pi i n2 k1 / M) twiddle folded in, then FFTs along the M1
 //    rows;
-//  * one CTA per layer, or pair of layers, for the windowed NT-point transforms;
+//  * one CTA per layer, or a cluster per pair of layers, for the windowed NT-point
+//    transforms;
 //  * grids of the form 2^a 3^b, so NF = 1536 (the reference's default grid) works.
 //
 // FP64 (parity with the reference) is bound by the FP64 pipe, so FP64
@@ -30,9 +31,13 @@
 //    the Hermitian parts.  The inverse runs the same backwards;
 //  * the real spectrum is unpacked in the row pass and packed in the inverse's
 //    column pass, where both bins k and M - k are at hand (one product for the two).
-// 107 -> 66 FP64 instructions per sample forward, 104 -> 70 inverse.  2^21 samples
-// (1024 x 2048) forward 538 -> 333 us; 6.3 M samples (1536 x 4096) inverse 1787 ->
-// 1030 us.
+//  * the transforms' factors are in tangent form (fp64_math.cuh), those between
+//    the passes in full tables;
+//  * the pairs of layers and of rows are spread over clusters, as 385 or 513 equal
+//    units leave a sixth of 152 SMs idle in the last round.
+// 107 -> 57 FP64 instructions per sample forward, 104 -> 60 inverse.  2^21 samples
+// (1024 x 2048) forward 538 -> 245 us; 6.3 M samples (1536 x 4096) inverse 1787 ->
+// 755 us.
 //
 // FP32 (GLASS_PREC_MIXED), and in FP64 the layers of grids whose NT is not a
 // multiple of 4, run one layer per CTA on ping-pong Stockham transforms; there

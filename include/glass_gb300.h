@@ -683,7 +683,7 @@ int glass_gpu_mixed_reevaluated(glass_gpu_ctx *ctx, unsigned long long *count);
  * the layout of glass_gpu_bank_upload.
  *
  * Intermediate data live in fixed arrays compiled into the library (about
- * 41 MB of device memory, held by every GPU that loads the library until the
+ * 43 MB of device memory, held by every GPU that loads the library until the
  * process exits), which bounds the sizes:
  *   nitems <= GLASS_NOALLOC_MAX_ITEMS, nseg * NFFT <= GLASS_NOALLOC_MAX_BINS,
  *   nitems * min(NFFT, 4096) <= GLASS_NOALLOC_MAX_SAMPLES;

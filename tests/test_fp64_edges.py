@@ -63,10 +63,11 @@ def test_arm_phase_ranges(engine, port, f0):
     _check(engine, port, bank, np.arange(3, dtype=np.int32), src)
 
 
-def test_carrier_beyond_the_sine_table(engine, port):
-    # pi fdot t^2 reaches 3e5 rad: the library's sincos takes over inside a template
+@pytest.mark.parametrize("fdT2", [1e5, 4e6])
+def test_carrier_beyond_the_sine_table(engine, port, fdT2):
+    # pi fdot t^2 reaches 3e5 rad, and 1.3e7, where the library's sincos takes over inside a template
     rng = np.random.default_rng(3)
-    bank, src = _bank(rng, port, [5e-3] * 2, 1024, fdot=1e5 / T**2)
+    bank, src = _bank(rng, port, [5e-3] * 2, 1024, fdot=fdT2 / T**2)
     engine.upload(bank)
     _check(engine, port, bank, np.arange(2, dtype=np.int32), src)
 
