@@ -39,6 +39,7 @@ cudaError_t fd_launch_spec_mixed(int N, const SpecArgs &a, int nitems, int num_s
 cudaError_t fd_launch_spec_fp64(int N, const SpecArgs &a, int nitems, int num_sms, cudaStream_t stream, bool perch);
 cudaError_t fd_launch_spec_all_mixed(const SpecAllArgs &A, int num_sms, cudaStream_t stream, bool perch, int cap);
 cudaError_t fd_launch_spec_all_fp64(const SpecAllArgs &A, int num_sms, cudaStream_t stream, bool perch);
+cudaError_t fd_launch_spec_cluster_fp64(const SpecSmallArgs &A, cudaStream_t stream, bool perch);
 
 // ------------------------------------------------------------- plan kernel
 // The two spreads of the bandwidth rule (ucb/src/glass_ucb_waveform.c:708-722, with
@@ -680,7 +681,27 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   int nall = 0;
   while (nall < kSpecAllBins && (32 << nall) <= bank.NFFT) nall++;
   int nb = 0;
-  if (bank.NFFT > 1024) {
+  // a few FP64 proposals: a cluster of CTAs each, whatever the size (where the
+  // line lies: at fd_spec_cluster64_kernel)
+  const bool few = !mix && nall > 0 && nitems <= num_sms / 5;
+  if (few) {
+    SpecSmallArgs A;
+    A.a = a;
+    A.a.bin = 0;
+    A.a.bin_list = work.bin_list;
+    A.a.tw = nullptr;
+    A.nbins = 0;
+    for (int b = 0; b < kNumBins; b++) {
+      A.tw[b] = tab.tt64[b];
+      if (32 << b <= bank.NFFT) A.nbins = b + 1;
+    }
+    A.zero_counts = work.bin_count;
+    A.done = work.bin_count + kNumBins + 1;
+    e = fd_launch_spec_cluster_fp64(A, stream, perch);
+    launches++;
+    if (e != cudaSuccess) return e;
+  }
+  if (bank.NFFT > 1024 && !few) {
     if ((e = cudaEventRecord(work.fork, stream)) != cudaSuccess) return e;
     for (int b = kSpecAllBins; b < kNumBins; b++) {
       int N = 32 << b;
@@ -698,7 +719,7 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
       nb++;
     }
   }
-  if (nall > 0) {
+  if (nall > 0 && !few) {
     SpecAllArgs A;
     A.a = a;
     A.a.bin = 0;

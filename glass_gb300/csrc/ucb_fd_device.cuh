@@ -1774,14 +1774,15 @@ struct SpecAllSmem {
   static constexpr size_t bytes = sizeof(TW) * SN + sizeof(C) * 4 * SN + sizeof(double) * 96 * 4;
 };
 
-// In-place FFTs of four series of N = 2^ln points, back to back, by the CTA: radix-4
+// In-place FFTs of NSER series of N = 2^ln points, back to back, by the CTA: radix-4
 // decimation in time from digit-reversed order (hp_rev) and a radix-2 stage when
 // log2 N is odd; results in natural order.  tw[j] = exp(-2 pi i j / N) in tangent form.
-static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const double2 *tw) {
+template <int NSER = 4>
+__device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const double2 *tw) {
   int lp = 0;
   for (; lp + 2 <= ln; lp += 2) {
     const int p = 1 << lp, lt = ln - lp - 2;
-    for (int t = threadIdx.x; t < 1 << ln; t += blockDim.x) {  // butterflies of the four series in a row
+    for (int t = threadIdx.x; t < NSER << (ln - 2); t += blockDim.x) {  // butterflies of the series in a row
       const int k = t & (p - 1);
       double2 *const y = x + ((t - k) << 2) + k;
       double2 v0 = y[0], v1 = y[p], v2 = y[2 * p], v3 = y[3 * p];
@@ -1798,7 +1799,7 @@ static __device__ __forceinline__ void fft4_dit64(double2 *x, int ln, const doub
   }
   if (lp < ln) {
     const int p = 1 << lp;
-    for (int t = threadIdx.x; t < 2 << ln; t += blockDim.x) {
+    for (int t = threadIdx.x; t < NSER << (ln - 1); t += blockDim.x) {
       const int k = t & (p - 1);
       double2 *const y = x + ((t - k) << 1) + k;
       tan_radix2(y[0], y[p], tw[k], y[0], y[p]);
@@ -1882,6 +1883,15 @@ struct SpecAllArgs {
   int nbins;                     // sizes 32 << b for b < nbins
   int *zero_counts;              // non-null: the last CTA to finish zeroes the kNumBins counts there
   int *done = nullptr;           // CTA-done counter (zero between launches)
+};
+
+// The spectral stage of a few FP64 proposals (ucb_fd_fp64.cu).
+struct SpecSmallArgs {
+  SpecArgs a;                   // a.bin_list: all sizes' lists, stride cap; a.tw unused
+  const double2 *tw[kNumBins];  // factors per size
+  int nbins;                    // sizes 32 << b for b < nbins
+  int *zero_counts;             // left at zero (the size counts)
+  int *done;                    // CTA-done counter (zero between launches)
 };
 
 template <bool MIX, bool PERCH = false>

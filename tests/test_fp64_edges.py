@@ -121,16 +121,16 @@ def test_fstat_sizes_and_idle_groups(engine, port, fdot, n):
     assert np.minimum(d, np.abs(d - 2 * math.pi)).max() < 1e-7
 
 
-@pytest.mark.parametrize("N", [32, 64, 128, 256, 512, 1024])
+@pytest.mark.parametrize("N", [32, 64, 128, 256, 512, 1024, 2048, 4096])
 def test_small_batches(engine, port, N):
-    """Batches around the counts up to which a proposal has a CTA, and 32 samples one,
-    to themselves, against the packed form of a larger batch: 1e-12 of max(1, |h|^2)
+    """Batches around the counts up to which a proposal has a cluster or a CTA, and 32
+    samples a CTA, to themselves, against the packed form of a larger batch: 1e-12 of max(1, |h|^2)
     (sums of 2N products in another order: 1e-16 sqrt(2N) |w| |h|)."""
     import torch
 
     rng = np.random.default_rng(N)
-    bank, src = _bank(rng, port, [1e-3, 4e-3, 2e-2], 1024)
-    bank.qmin[1] += 500  # clipped by the segment's edge
+    bank, src = _bank(rng, port, [1e-3, 4e-3, 2e-2], max(1024, N))
+    bank.qmin[1] += max(1024, N) // 2 - 12  # clipped by the segment's edge
     engine.upload(bank)
     engine.set_template_size(N)
     try:
@@ -138,7 +138,7 @@ def test_small_batches(engine, port, N):
         _, ref, hh, st = engine.dlogl_host(seg, src[seg], precision=gg.PREC_FP64)
         assert (st[seg != 1] == 0).all()
         tol = 1e-12 * np.maximum(1.0, hh)
-        for n in (1, 2, 5, 9, 10, 19, 38, 76, 152, 153, 303, 304, 305):
+        for n in (1, 2, 5, 9, 10, 19, 30, 31, 38, 76, 152, 153, 303, 304, 305):
             _, ty, h, s2 = engine.dlogl_host(seg[:n], src[seg[:n]], precision=gg.PREC_FP64)
             assert (s2 == st[:n]).all()
             assert (np.abs(ty - ref[:n]) <= tol[:n]).all() and (np.abs(h - hh[:n]) <= tol[:n]).all()
