@@ -90,12 +90,12 @@ inline cudaError_t launch_setup(LaunchSetup &s, Init init, int *occ) {
 // start of each, the waiting CTAs take room from the running kernel's
 // neighbours, and the same batch takes 102 us.)
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*k)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args) {
+inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

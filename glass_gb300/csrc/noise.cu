@@ -323,6 +323,7 @@ __device__ __forceinline__ void noise_cell(const double *c, const double *P, dou
 // likelihood terms; the chunk's sum goes to partial[model][chunk].  Bound by
 // the FP64 pipe (see the top of the file).
 __global__ void __launch_bounds__(kNoiseThreads) noise_logl_kernel(NoiseArgs a) {
+  grid_begin();
   __shared__ double et[kExpTab];
   __shared__ NoiseModel M;
   const int chunk = blockIdx.x, p = blockIdx.y;
@@ -378,6 +379,7 @@ __global__ void __launch_bounds__(kNoiseThreads) noise_logl_kernel(NoiseArgs a) 
 // (noise/src/glass_noise_model.c:1104-1134).  sin^2(f/f*) is the table's
 // -8 sin^2 times -1/8 (exact).
 __global__ void __launch_bounds__(kNoiseThreads) noise_ch12_kernel(NoiseArgs a, int nch) {
+  grid_begin();
   __shared__ double et[kExpTab];
   __shared__ NoiseModel M;
   const int chunk = blockIdx.x, p = blockIdx.y;
@@ -424,6 +426,7 @@ __global__ void __launch_bounds__(kNoiseThreads) noise_ch12_kernel(NoiseArgs a, 
 
 // Per model: the chunks' sums in order, and the constant -3 N log(2 pi).
 __global__ void noise_finish_kernel(const double *partial, int nchunks, int nprop, double cst, double *logl) {
+  grid_begin();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nprop) return;
   double s = 0.0;
@@ -471,6 +474,7 @@ __device__ __forceinline__ double noise_wv_layer(const NoiseWvArgs &a, const Noi
 // layer's cells contribute -Q/2 (ixx Sxx + ... + 2 ixy Sxy ...) - Q/2 Ncoarse
 // log det with S the layer's sums of the cell statistics.  One CTA per model.
 __global__ void __launch_bounds__(kNoiseThreads) noise_wv_stationary_kernel(NoiseWvArgs a) {
+  grid_begin();
   __shared__ double et[kExpTab];
   __shared__ NoiseModel M;
   const int p = blockIdx.x;
@@ -507,6 +511,7 @@ __global__ void __launch_bounds__(kNoiseThreads) noise_wv_stationary_kernel(Nois
 // :1211-1241): 6 FP64 operations for its covariance, 26 in noise_cell.
 constexpr int kNoiseWvMaxLJ = 64;
 __global__ void __launch_bounds__(kNoiseThreads) noise_wv_dynamic_kernel(NoiseWvArgs a) {
+  grid_begin();
   __shared__ double et[kExpTab];
   __shared__ double lay[kNoiseWvMaxLJ][7];
   __shared__ NoiseModel M;
@@ -545,6 +550,7 @@ __global__ void __launch_bounds__(kNoiseThreads) noise_wv_dynamic_kernel(NoiseWv
 }
 
 __global__ void noise_wv_const_kernel(double *logl, int nprop, double cst) {
+  grid_begin();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p < nprop) logl[p] -= cst;
 }
@@ -869,9 +875,8 @@ cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const
       s.sgal = sgal ? sgal + 5 * (size_t)p0 : nullptr;
       s.sgwb = sgwb ? sgwb + 4 * (size_t)p0 : nullptr;
       s.out = logl + p0;
-      noise_wv_stationary_kernel<<<np, kNoiseThreads, 0, stream>>>(s);
       launches++;
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      if ((e = launch_chained(noise_wv_stationary_kernel, np, kNoiseThreads, 0, stream, s)) != cudaSuccess) return e;
     }
   } else {
     for (int p0 = 0; p0 < nprop; p0 += 65535) {
@@ -881,21 +886,19 @@ cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const
       s.sgal = sgal + 5 * (size_t)p0;
       s.sgwb = sgwb ? sgwb + 4 * (size_t)p0 : nullptr;
       s.out = w.partial + (size_t)p0 * a.nchunks;
-      noise_wv_dynamic_kernel<<<dim3(a.nchunks, np), kNoiseThreads, 0, stream>>>(s);
       launches++;
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      if ((e = launch_chained(noise_wv_dynamic_kernel, dim3(a.nchunks, np), kNoiseThreads, 0, stream, s)) != cudaSuccess)
+        return e;
     }
   }
   // my_noise_log_likelihood_wavelet_coarse's constant over the full pixel count (:1238-1240)
   const double cst = 0.5 * 3 * ((double)w.Nlayer * w.NT) * log(2 * M_PI);
-  if (mode == 2) {
-    noise_finish_kernel<<<(nprop + 255) / 256, 256, 0, stream>>>(w.partial, a.nchunks, nprop, cst, logl);
-  } else {
-    noise_wv_const_kernel<<<(nprop + 255) / 256, 256, 0, stream>>>(logl, nprop, cst);
-  }
   launches++;
   if (nlaunch) *nlaunch = launches;
-  return cudaGetLastError();
+  if (mode == 2)
+    return launch_chained(noise_finish_kernel, (nprop + 255) / 256, 256, 0, stream, (const double *)w.partial, a.nchunks,
+                          nprop, cst, logl);
+  return launch_chained(noise_wv_const_kernel, (nprop + 255) / 256, 256, 0, stream, logl, nprop, cst);
 }
 
 static int noise_bins_per_thread(int N, int nprop) {
@@ -964,19 +967,17 @@ cudaError_t noise_logl_launch(const NoiseDev &nd, int nprop, const double *inst,
     s.sgal = sgal ? sgal + 5 * (size_t)p0 : nullptr;
     s.sgwb = sgwb ? sgwb + 4 * (size_t)p0 : nullptr;
     s.partial = nd.partial + (size_t)p0 * a.nchunks;
-    if (nd.nch == 3)
-      noise_logl_kernel<<<dim3(a.nchunks, np), kNoiseThreads, 0, stream>>>(s);
-    else
-      noise_ch12_kernel<<<dim3(a.nchunks, np), kNoiseThreads, 0, stream>>>(s, nd.nch);
+    const cudaError_t e =
+        nd.nch == 3 ? launch_chained(noise_logl_kernel, dim3(a.nchunks, np), kNoiseThreads, 0, stream, s)
+                    : launch_chained(noise_ch12_kernel, dim3(a.nchunks, np), kNoiseThreads, 0, stream, s, nd.nch);
     launches++;
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   const double cst = nd.nch == 3 ? 3 * nd.N * log(2 * M_PI) : 0.0;
-  noise_finish_kernel<<<(nprop + 255) / 256, 256, 0, stream>>>(nd.partial, a.nchunks, nprop, cst, logl);
   launches++;
   if (nlaunch) *nlaunch = launches;
-  return cudaGetLastError();
+  return launch_chained(noise_finish_kernel, (nprop + 255) / 256, 256, 0, stream, (const double *)nd.partial, a.nchunks,
+                        nprop, cst, logl);
 }
 
 }  // namespace glass

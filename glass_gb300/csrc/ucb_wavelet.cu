@@ -164,6 +164,7 @@ __device__ __forceinline__ double atan2_tab(double y, double x, const double2 *t
 template <int C>
 __global__ void __launch_bounds__(128) wv_plan_kernel(WvGridDev g, int n, const double *params, WvSrc *srcs,
                                                       double *ssb, int *status) {
+  grid_begin();
   extern __shared__ __align__(16) double psm[];
   __shared__ int s_ok[C];
   __shared__ double s_f0[C], s_phi0[C], s_fdot[C], s_A0[C], s_dA[C];
@@ -328,6 +329,7 @@ __device__ __forceinline__ void tdi_channel(const Pol &P, double tn, const doubl
 // LISA_spline_response (utils/src/glass_lisa.c:920-1074) at one node, plus the
 // S/C-1 phase used as the reference phase (LISA_spacecraft_to_barycenter_time).
 __global__ void wv_resp_kernel(WvGridDev g, int n, const WvSrc *srcs, const double *ssb, double *resp) {
+  grid_begin();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int norb = g.norb;
   if (idx >= (long long)n * norb) return;
@@ -396,6 +398,7 @@ __global__ void wv_resp_kernel(WvGridDev g, int n, const WvSrc *srcs, const doub
 template <int C>
 __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const WvSrc *srcs, const double *resp,
                                                      double *tdi) {
+  grid_begin();
   extern __shared__ __align__(16) double tsm[];
   __shared__ int s_ok[C];
   const int base = blockIdx.x * C;
@@ -598,6 +601,7 @@ __device__ void layers_from_spectrum(const double2 *zb, double2 *lb, int M, int 
 constexpr int kCarrierSlices = 4;
 __global__ void __launch_bounds__(256) wv_carrier_kernel(WvGridDev g, const WvSrc *srcs, const double *ssb,
                                                          double *carrier, const int *count, const int *list) {
+  grid_begin();
   int s = blockIdx.y;
   if (list) {
     if (s >= *count) return;
@@ -630,6 +634,7 @@ __global__ void __launch_bounds__(256) wv_carrier_kernel(WvGridDev g, const WvSr
 __global__ void __launch_bounds__(kLayerThreads) wv_layers_kernel(WvGridDev g, int n, const WvSrc *srcs,
                                                                   const double *carrier, const double *tdi,
                                                                   double *coef, const int *count, const int *list) {
+  grid_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   int s = blockIdx.x / 3;
   const int ch = blockIdx.x - 3 * (blockIdx.x / 3);
@@ -699,6 +704,7 @@ __global__ void __launch_bounds__(kDloglThreads) wv_dlogl_kernel(WvGridDev g, in
                                                                  const double *coef, const double *term_x,
                                                                  double *dlogl, double *term_y, double *hh_out,
                                                                  int *status, const int *count, const int *list) {
+  grid_begin();
   int s = blockIdx.x;
   if (list) {
     if (s >= *count) return;
@@ -795,6 +801,7 @@ struct WvMixInterval {
 __global__ void __launch_bounds__(kLayerThreads) wv_layers_mix_kernel(WvGridDev g, int n, const WvSrc *srcs,
                                                                       const double *ssb, const double *tdi,
                                                                       float *coef) {
+  grid_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   const int s = blockIdx.x / 3, ch = blockIdx.x - 3 * (blockIdx.x / 3);
   const WvSrc &S = srcs[s];
@@ -913,6 +920,7 @@ __global__ void __launch_bounds__(kDloglThreads) wv_dlogl_mix_kernel(WvGridDev g
                                                                      double *dlogl, double *term_y, double *hh_out,
                                                                      int *status, double kest, int *count, int *list,
                                                                      unsigned long long *total) {
+  grid_begin();
   const int s = blockIdx.x;
   const WvSrc &S = srcs[s];
   __shared__ float2 red[2][kDloglThreads / 32];
@@ -1330,9 +1338,10 @@ static cudaError_t launch_layers64(const WvGridDev &g, const WvWorkDev &w, int n
   const size_t sm = sizeof(double2) * ((size_t)g.NT * (kWvMaxLayers + 1) / 2 + g.NT);
   const cudaError_t e = cudaFuncSetAttribute(wv_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  wv_carrier_kernel<<<dim3(kCarrierSlices, n), 256, 0, s>>>(g, w.src, w.ssb, w.carrier, count, list);
-  wv_layers_kernel<<<3 * n, kLayerThreads, sm, s>>>(g, n, w.src, w.carrier, w.tdi, w.coef, count, list);
-  return cudaGetLastError();
+  const cudaError_t ec = launch_chained(wv_carrier_kernel, dim3(kCarrierSlices, n), 256, 0, s, g, w.src, w.ssb, w.carrier,
+                                        count, list);
+  if (ec != cudaSuccess) return ec;
+  return launch_chained(wv_layers_kernel, 3 * n, kLayerThreads, sm, s, g, n, w.src, w.carrier, w.tdi, w.coef, count, list);
 }
 
 // ------------------------------------------------------------ Fisher matrix
@@ -1463,8 +1472,7 @@ static cudaError_t wv_launch_tiles(K const (&k)[4], size_t per, int items, cudaS
   while (q < 3 && C[q] * per > (size_t)(C[q] > 4 ? 55 : 200) * 1024) q++;
   cudaError_t e = cudaFuncSetAttribute(k[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(C[q] * per));
   if (e != cudaSuccess) return e;
-  k[q]<<<(items + C[q] - 1) / C[q], 128, C[q] * per, s>>>(args...);
-  return cudaGetLastError();
+  return launch_chained(k[q], (items + C[q] - 1) / C[q], 128, C[q] * per, s, args...);
 }
 
 cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int precision, int n, const double *params,
@@ -1473,8 +1481,7 @@ cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int preci
   const int norb = g.norb;
   cudaError_t e;
   {
-    // 4 norb doubles of shared memory per source; 16 sources per CTA where
-    // they fit, fewer for long observations
+    // 4 norb doubles of shared memory per source
     const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
     decltype(&wv_plan_kernel<1>) const k[4] = {wv_plan_kernel<16>, wv_plan_kernel<8>, wv_plan_kernel<4>,
                                                wv_plan_kernel<1>};
@@ -1482,7 +1489,9 @@ cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int preci
       return e;
   }
   const long long nr = (long long)n * norb;
-  wv_resp_kernel<<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(g, n, w.src, w.ssb, w.resp);
+  if ((e = launch_chained(wv_resp_kernel, dim3((unsigned)((nr + 127) / 128)), 128, 0, s, g, n, w.src, w.ssb, w.resp)) !=
+      cudaSuccess)
+    return e;
   {
     const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
     decltype(&wv_tdi_kernel<1>) const k[4] = {wv_tdi_kernel<16>, wv_tdi_kernel<8>, wv_tdi_kernel<4>, wv_tdi_kernel<1>};
@@ -1496,7 +1505,9 @@ cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int preci
                       std::max(sizeof(float2) * (size_t)g.NT, sizeof(WvMixInterval) * (size_t)norb + 16);
     e = cudaFuncSetAttribute(wv_layers_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    wv_layers_mix_kernel<<<3 * n, kLayerThreads, sm, s>>>(g, n, w.src, w.ssb, w.tdi, reinterpret_cast<float *>(w.coef));
+    if ((e = launch_chained(wv_layers_mix_kernel, 3 * n, kLayerThreads, sm, s, g, n, w.src, w.ssb, w.tdi,
+                            reinterpret_cast<float *>(w.coef))) != cudaSuccess)
+      return e;
   } else {
     if ((e = launch_layers64(g, w, n, nullptr, nullptr, s)) != cudaSuccess) return e;
   }
@@ -1524,23 +1535,24 @@ cudaError_t wv_dlogl_launch(const WvGridDev &g, const WvWorkDev &w, int precisio
     const double kest = tol > 0.0 ? kWvMixedErrK / tol : 0.0;
     cudaError_t e;
     if (kest > 0.0 && (e = cudaMemsetAsync(w.count, 0, sizeof(int), s)) != cudaSuccess) return e;
-    wv_dlogl_mix_kernel<<<n, kDloglThreads, 0, s>>>(g, n, w.src, reinterpret_cast<const float *>(w.coef), term_x,
-                                                    dlogl, term_y, hh, status, kest, w.count, w.list, w.total);
+    if ((e = launch_chained(wv_dlogl_mix_kernel, n, kDloglThreads, 0, s, g, n, w.src,
+                            reinterpret_cast<const float *>(w.coef), term_x, dlogl, term_y, hh, status, kest, w.count,
+                            w.list, w.total)) != cudaSuccess)
+      return e;
     if (nlaunch) *nlaunch += 1;
     if (kest > 0.0) {
       // the listed sources again in FP64: their layers (over the mixed
       // coefficients, which are no longer read) and their likelihood; the
       // grids cover every source and the CTAs past the list return at once
-      if ((e = cudaGetLastError()) != cudaSuccess) return e;
       if ((e = launch_layers64(g, w, n, w.count, w.list, s)) != cudaSuccess) return e;
-      wv_dlogl_kernel<<<n, kDloglThreads, 0, s>>>(g, n, w.src, w.coef, term_x, dlogl, term_y, hh, status, w.count,
-                                                  w.list);
       if (nlaunch) *nlaunch += 3;
+      return launch_chained(wv_dlogl_kernel, n, kDloglThreads, 0, s, g, n, w.src, w.coef, term_x, dlogl, term_y, hh, status,
+                            w.count, w.list);
     }
   } else {
-    wv_dlogl_kernel<<<n, kDloglThreads, 0, s>>>(g, n, w.src, w.coef, term_x, dlogl, term_y, hh, status, nullptr,
-                                                nullptr);
     if (nlaunch) *nlaunch += 1;
+    return launch_chained(wv_dlogl_kernel, n, kDloglThreads, 0, s, g, n, w.src, w.coef, term_x, dlogl, term_y, hh, status,
+                          nullptr, nullptr);
   }
   return cudaGetLastError();
 }
