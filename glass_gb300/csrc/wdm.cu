@@ -34,7 +34,7 @@
 //  * the transforms' factors are in tangent form (fp64_math.cuh), those between
 //    the passes in full tables;
 //  * the pairs of layers and of rows are spread over clusters, as 385 or 513 equal
-//    units leave a sixth of 152 SMs idle in the last round.
+//    units leave a sixth of 152 SMs idle in the last wave.
 // 107 -> 57 FP64 instructions per sample forward, 104 -> 60 inverse.  2^21 samples
 // (1024 x 2048) forward 538 -> 245 us; 6.3 M samples (1536 x 4096) inverse 1787 ->
 // 755 us.
