@@ -78,6 +78,19 @@ inline cudaError_t launch_setup(LaunchSetup &s, Init init, int *occ) {
   return cudaSuccess;
 }
 
+// Raises kernel K's dynamic shared-memory limit to `most`, the largest any call
+// asks of it, once per device.  (Set to a call's own size before its launch, the limit
+// would be lowered under the launch of a larger one by another thread.)
+template <auto K>
+inline cudaError_t smem_limit(size_t most) {
+  static LaunchSetup setup;
+  int done = 0;
+  return launch_setup(setup, [&](int *o) {
+    *o = 1;
+    return cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  }, &done);
+}
+
 // Launch of a kernel of a chain, its start overlapped with the end of the one
 // before it in the stream (programmatic dependent launch): its CTAs are placed as
 // that one's leave, and each begins with grid_begin(), which waits until every

@@ -1139,7 +1139,7 @@ static void unit_root(long long j, long long P, double *c, double *s) {
 cudaError_t wdm_by_layers_launch(int NF, int NT, int jmin, int nl, const double *d_win, const double2 *d_tw,
                                  double *d_data, cudaStream_t s) {
   const size_t sm = sizeof(double2) * ((size_t)NT * (nl + 1) / 2 + NT);
-  cudaError_t e = cudaFuncSetAttribute(wdm_by_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = smem_limit<wdm_by_layers_kernel>((size_t)227 << 10);  // the entry point's bound
   if (e != cudaSuccess) return e;
   wdm_by_layers_kernel<<<1, kLayerThreads, sm, s>>>(NF, NT, jmin, nl, d_win, d_tw, d_data);
   return cudaGetLastError();
@@ -1336,7 +1336,8 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
 static cudaError_t launch_layers64(const WvGridDev &g, const WvWorkDev &w, int n, const int *count, const int *list,
                                    cudaStream_t s) {
   const size_t sm = sizeof(double2) * ((size_t)g.NT * (kWvMaxLayers + 1) / 2 + g.NT);
-  const cudaError_t e = cudaFuncSetAttribute(wv_layers_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  constexpr size_t most = sizeof(double2) * ((size_t)kWvMaxNT * (kWvMaxLayers + 1) / 2 + kWvMaxNT);
+  const cudaError_t e = smem_limit<wv_layers_kernel>(most);
   if (e != cudaSuccess) return e;
   const cudaError_t ec = launch_chained(wv_carrier_kernel, dim3(kCarrierSlices, n), 256, 0, s, g, w.src, w.ssb, w.carrier,
                                         count, list);
@@ -1463,16 +1464,24 @@ __global__ void __launch_bounds__(kFisherThreads) wv_fisher_kernel(WvGridDev g, 
 }
 
 // Launches a tile kernel with C = 16, 8, 4 or 1 items per CTA of 128 threads: the
-// largest of which four CTAs fit an SM (per bytes of shared memory an item), so
-// that four sequential phases run side by side, or that fits at all.
-template <typename K, typename... Args>
-static cudaError_t wv_launch_tiles(K const (&k)[4], size_t per, int items, cudaStream_t s, Args... args) {
-  constexpr int C[4] = {16, 8, 4, 1};
-  int q = 0;
-  while (q < 3 && C[q] * per > (size_t)(C[q] > 4 ? 55 : 200) * 1024) q++;
-  cudaError_t e = cudaFuncSetAttribute(k[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(C[q] * per));
+// largest of which four CTAs fit an SM (4 norb + 1 doubles of shared memory an item),
+// so that four sequential phases run side by side, or that fits at all.
+template <int C, auto K, typename... Args>
+static cudaError_t wv_launch_tile(size_t most, size_t per, int items, cudaStream_t s, Args... args) {
+  const cudaError_t e = smem_limit<K>(most);
   if (e != cudaSuccess) return e;
-  return launch_chained(k[q], (items + C[q] - 1) / C[q], 128, C[q] * per, s, args...);
+  return launch_chained(K, (items + C - 1) / C, 128, C * per, s, args...);
+}
+template <auto K16, auto K8, auto K4, auto K1, typename... Args>
+static cudaError_t wv_launch_tiles(int norb, int items, cudaStream_t s, Args... args) {
+  constexpr size_t kFour = (size_t)55 << 10, kOne = (size_t)200 << 10;
+  constexpr size_t kMost = sizeof(double) * (4 * (size_t)kWvMaxOrb + 1);
+  static_assert(kMost <= kOne, "one item fits");
+  const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
+  if (16 * per <= kFour) return wv_launch_tile<16, K16>(kFour, per, items, s, args...);
+  if (8 * per <= kFour) return wv_launch_tile<8, K8>(kFour, per, items, s, args...);
+  if (4 * per <= kOne) return wv_launch_tile<4, K4>(kOne, per, items, s, args...);
+  return wv_launch_tile<1, K1>(kMost, per, items, s, args...);
 }
 
 cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int precision, int n, const double *params,
@@ -1480,31 +1489,25 @@ cudaError_t wv_waveform_launch(const WvGridDev &g, const WvWorkDev &w, int preci
   if (n <= 0) return cudaSuccess;
   const int norb = g.norb;
   cudaError_t e;
-  {
-    // 4 norb doubles of shared memory per source
-    const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
-    decltype(&wv_plan_kernel<1>) const k[4] = {wv_plan_kernel<16>, wv_plan_kernel<8>, wv_plan_kernel<4>,
-                                               wv_plan_kernel<1>};
-    if ((e = wv_launch_tiles(k, per, n, s, g, n, params, w.src, w.ssb, status)) != cudaSuccess)
-      return e;
-  }
+  if ((e = wv_launch_tiles<wv_plan_kernel<16>, wv_plan_kernel<8>, wv_plan_kernel<4>, wv_plan_kernel<1>>(
+           norb, n, s, g, n, params, w.src, w.ssb, status)) != cudaSuccess)
+    return e;
   const long long nr = (long long)n * norb;
   if ((e = launch_chained(wv_resp_kernel, dim3((unsigned)((nr + 127) / 128)), 128, 0, s, g, n, w.src, w.ssb, w.resp)) !=
       cudaSuccess)
     return e;
-  {
-    const size_t per = sizeof(double) * (4 * (size_t)norb + 1);
-    decltype(&wv_tdi_kernel<1>) const k[4] = {wv_tdi_kernel<16>, wv_tdi_kernel<8>, wv_tdi_kernel<4>, wv_tdi_kernel<1>};
-    if ((e = wv_launch_tiles(k, per, 3 * n, s, g, n, w.src, w.resp, w.tdi)) != cudaSuccess)
-      return e;
-  }
+  if ((e = wv_launch_tiles<wv_tdi_kernel<16>, wv_tdi_kernel<8>, wv_tdi_kernel<4>, wv_tdi_kernel<1>>(
+           norb, 3 * n, s, g, n, w.src, w.resp, w.tdi)) != cudaSuccess)
+    return e;
   if (precision == 1) {
     // float2 samples and layer buffer; the interval table shares the layer
     // buffer's place and may be larger than it
-    const size_t sm = sizeof(float2) * (size_t)g.NT * (kWvMaxLayers + 1) / 2 +
-                      std::max(sizeof(float2) * (size_t)g.NT, sizeof(WvMixInterval) * (size_t)norb + 16);
-    e = cudaFuncSetAttribute(wv_layers_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
+    auto bytes = [](size_t NT, size_t nodes) {
+      return sizeof(float2) * NT * (kWvMaxLayers + 1) / 2 +
+             std::max(sizeof(float2) * NT, sizeof(WvMixInterval) * nodes + 16);
+    };
+    const size_t sm = bytes(g.NT, norb);
+    if ((e = smem_limit<wv_layers_mix_kernel>(bytes(kWvMaxNT, kWvMaxOrb))) != cudaSuccess) return e;
     if ((e = launch_chained(wv_layers_mix_kernel, 3 * n, kLayerThreads, sm, s, g, n, w.src, w.ssb, w.tdi,
                             reinterpret_cast<float *>(w.coef))) != cudaSuccess)
       return e;

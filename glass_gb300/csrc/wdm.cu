@@ -751,16 +751,16 @@ static size_t fft_smem(int L, int nser) {
   return sizeof(C) * ((size_t)L + 2 * (size_t)nser * L);
 }
 
+constexpr int kMaxLine = 4096;                 // points of a row, column or layer
+constexpr size_t kPassSmem = (size_t)200 << 10;  // of a pass of several series per CTA
+
 // series per CTA for a pass over `count` series of length L
 template <typename C>
 static int pick_batch(int L, int count) {
+  static_assert(sizeof(C) * 3 * kMaxLine <= kPassSmem, "one series fits");
   for (int n = 8; n > 1; n /= 2)
-    if (count % n == 0 && fft_smem<C>(L, n) <= 200 * 1024) return n;
+    if (count % n == 0 && fft_smem<C>(L, n) <= kPassSmem) return n;
   return 1;
-}
-
-static cudaError_t set_smem(const void *fn, size_t bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // e^{-2 pi i j / P}: the angle is reduced to [0, pi] by conjugate symmetry
@@ -821,7 +821,7 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   P.NF = NF;
   P.NT = NT;
   P.M = M;
-  P.M1 = split_factor(M, 4096);
+  P.M1 = split_factor(M, kMaxLine);
   if (!P.M1) return cudaErrorInvalidValue;
   P.M2 = (int)(M / P.M1);
   P.K = 1024;
@@ -885,8 +885,8 @@ static cudaError_t four_step(const WdmPlan &P, const C *src, C *tmp, C *dst, int
   const int nc = pick_batch<C>(M1, M2), nr = pick_batch<C>(M2, M1);
   const size_t sm1 = fft_smem<C>(M1, nc), sm2 = fft_smem<C>(M2, nr);
   cudaError_t e;
-  if ((e = set_smem((const void *)wdm_col_kernel<C>, sm1)) != cudaSuccess) return e;
-  if ((e = set_smem((const void *)wdm_row_kernel<C>, sm2)) != cudaSuccess) return e;
+  if ((e = smem_limit<wdm_col_kernel<C>>(kPassSmem)) != cudaSuccess) return e;
+  if ((e = smem_limit<wdm_row_kernel<C>>(kPassSmem)) != cudaSuccess) return e;
   wdm_col_kernel<C><<<M2 / nc, 256, sm1, s>>>(src, tmp, M1, M2, nc, (const C *)P.tw1, (const C *)P.mlo,
                                                (const C *)P.mhi, P.K, sign);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -902,21 +902,22 @@ static int threads64(int points, int most) {  // one radix-4 butterfly per threa
   int t = (points / 4 + 31) / 32 * 32;
   return t < 32 ? 32 : t > most ? most : t;
 }
-template <typename K, typename... Args>
-static cudaError_t launch64(K kernel, int grid, int points, int most, cudaStream_t s, Args... args) {
+// most_points, most_threads: the most that any grid takes of the kernel.
+template <auto K, typename... Args>
+static cudaError_t launch64(int grid, int points, int most_points, int most_threads, cudaStream_t s, Args... args) {
   cudaError_t e;
-  if (smem64(points) > 48 * 1024 && (e = set_smem((const void *)kernel, smem64(points))) != cudaSuccess) return e;
-  return launch_chained(kernel, grid, threads64(points, most), smem64(points), s, args...);
+  if (smem64(most_points) > 48 * 1024 && (e = smem_limit<K>(smem64(most_points))) != cudaSuccess) return e;
+  return launch_chained(K, grid, threads64(points, most_threads), smem64(points), s, args...);
 }
 
 // scale times the real spectrum X -> coefficients.
 static cudaError_t fwd_layers64(const WdmPlan &P, const double2 *X, double scale, double *wdm, cudaStream_t s) {
   const int NF = P.NF, NT = P.NT;
   if (NT % 4 == 0)
-    return launch64(wdm_fwd_pair64_kernel, 2 * layer_pairs(NF), NT / 2, 256, s, X, NF, NT, (const double *)P.win,
+    return launch64<wdm_fwd_pair64_kernel>(2 * layer_pairs(NF), NT / 2, kMaxLine / 2, 256, s, X, NF, NT, (const double *)P.win,
                     (const double2 *)P.twNT, 0.5 * scale / NT, wdm);
   const size_t sm = fft_smem<double2>(NT, 1);
-  const cudaError_t e = set_smem((const void *)wdm_fwd_layer_kernel<double2>, sm);
+  const cudaError_t e = smem_limit<wdm_fwd_layer_kernel<double2>>(fft_smem<double2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
   wdm_fwd_layer_kernel<double2><<<NF + 1, 256, sm, s>>>(nullptr, X, P.M, NF, NT, (const double *)P.win,
                                                         (const double2 *)P.twNT, (const double2 *)P.nlo,
@@ -932,10 +933,10 @@ static cudaError_t forward64(const WdmPlan &P, const double *time, double *wdm, 
     if ((e = cudaMemcpyAsync(P.rbuf, time, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
     packed = reinterpret_cast<const double2 *>(P.rbuf);
   }
-  if ((e = launch64(wdm_col64_kernel, P.M2, P.M1, 256, s, packed, (double2 *)P.bufB, P.M1, P.M2,
+  if ((e = launch64<wdm_col64_kernel>(P.M2, P.M1, kMaxLine, 256, s, packed, (double2 *)P.bufB, P.M1, P.M2,
                     (const double2 *)P.tw1, (const double2 *)P.colf)) != cudaSuccess)
     return e;
-  if ((e = launch64(wdm_row_unpack64_kernel, 2 * (P.M1 / 2 + 1), P.M2, 256, s, (const double2 *)P.bufB,
+  if ((e = launch64<wdm_row_unpack64_kernel>(2 * (P.M1 / 2 + 1), P.M2, kMaxLine, 256, s, (const double2 *)P.bufB,
                     (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.unpackf)) != cudaSuccess)
     return e;
   return fwd_layers64(P, (const double2 *)P.bufX, 0.5, wdm, s);
@@ -952,14 +953,15 @@ static cudaError_t inverse_layers64(const WdmPlan &P, const double *wdm, double 
   if (NT % 4 == 0) {
     const int pairs = NF / 2;  // (1, 2), (3, 4), ...
     const bool last_first = pairs % 2 == 0;  // the last layer's place: see the kernel
-    if ((e = launch64(wdm_inv_pair64_kernel, 4 * ((pairs + 1) / 2 + last_first), NT / 4, 256, s, wdm, NF, NT, 0, win, tw, scale,
-                      X)) != cudaSuccess)
+    if ((e = launch64<wdm_inv_pair64_kernel>(4 * ((pairs + 1) / 2 + last_first), NT / 4, kMaxLine / 4, 256, s, wdm, NF, NT, 0, win,
+                                             tw, scale, X)) != cudaSuccess)
       return e;
-    return launch64(wdm_inv_pair64_kernel, 4 * (pairs / 2 + 1 + !last_first), NT / 4, 256, s, wdm, NF, NT, 1, win, tw, scale, X);
+    return launch64<wdm_inv_pair64_kernel>(4 * (pairs / 2 + 1 + !last_first), NT / 4, kMaxLine / 4, 256, s, wdm, NF, NT, 1, win,
+                                           tw, scale, X);
   }
   wdm_zero_kernel<double2><<<blocks_for(P.M + 1), 256, 0, s>>>(X, P.M + 1);
   const size_t sm = fft_smem<double2>(NT, 1);
-  if ((e = set_smem((const void *)wdm_inv_layer_kernel<double2>, sm)) != cudaSuccess) return e;
+  if ((e = smem_limit<wdm_inv_layer_kernel<double2>>(fft_smem<double2>(kMaxLine, 1))) != cudaSuccess) return e;
   for (int parity = 0; parity < 2; parity++)
     wdm_inv_layer_kernel<double2><<<(NF - parity) / 2 + 1, 256, sm, s>>>(wdm, NF, NT, parity, win, tw, scale, X);
   return cudaGetLastError();
@@ -969,13 +971,13 @@ static cudaError_t inverse64(const WdmPlan &P, const double *wdm, double *time, 
   const long long ND = (long long)P.NF * P.NT;
   cudaError_t e;
   if ((e = inverse_layers64(P, wdm, 1.0 / (double)ND, s)) != cudaSuccess) return e;
-  if ((e = launch64(wdm_pack_col64_kernel, P.M2 / 2 + 1, 2 * P.M1, 512, s, (const double2 *)P.bufX,
+  if ((e = launch64<wdm_pack_col64_kernel>(P.M2 / 2 + 1, 2 * P.M1, 2 * kMaxLine, 512, s, (const double2 *)P.bufX,
                     (double2 *)P.bufB, P.M1, P.M2, (const double2 *)P.tw1, (const double2 *)P.colf,
                     (const double2 *)P.packf)) != cudaSuccess)
     return e;
   const bool direct = (uintptr_t)time % 16 == 0;
   double2 *dst = reinterpret_cast<double2 *>(direct ? (void *)time : P.rbuf);
-  if ((e = launch64(wdm_row64_kernel, P.M1, P.M2, 256, s, (const double2 *)P.bufB, dst, P.M1, P.M2,
+  if ((e = launch64<wdm_row64_kernel>(P.M1, P.M2, kMaxLine, 256, s, (const double2 *)P.bufB, dst, P.M1, P.M2,
                     (const double2 *)P.tw2)) != cudaSuccess)
     return e;
   if (!direct) return cudaMemcpyAsync(time, P.rbuf, sizeof(double) * ND, cudaMemcpyDeviceToDevice, s);
@@ -1010,7 +1012,7 @@ static cudaError_t forward32(const WdmPlan &P, const double *time, double *wdm, 
   if ((e = four_step<float2>(P, (const float2 *)P.rbuf, (float2 *)P.bufB, (float2 *)P.bufA, -1, 1.f, s)) != cudaSuccess)
     return e;
   const size_t sm = fft_smem<float2>(P.NT, 1);
-  if ((e = set_smem((const void *)wdm_fwd_layer_kernel<float2>, sm)) != cudaSuccess) return e;
+  if ((e = smem_limit<wdm_fwd_layer_kernel<float2>>(fft_smem<float2>(kMaxLine, 1))) != cudaSuccess) return e;
   wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>((const float2 *)P.bufA, nullptr, P.M, P.NF, P.NT,
                                                          (const float *)P.win, (const float2 *)P.twNT,
                                                          (const float2 *)P.nlo, (const float2 *)P.nhi, P.K, 1.f, out);
@@ -1026,7 +1028,7 @@ static cudaError_t inverse_layers32(const WdmPlan &P, const double *wdm, cudaStr
   wdm_cast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>(wdm, (float *)P.rbuf, ND);
   wdm_zero_kernel<float2><<<blocks_for(P.M + 1), 256, 0, s>>>((float2 *)P.bufX, P.M + 1);
   const size_t sm = fft_smem<float2>(NT, 1);
-  const cudaError_t e = set_smem((const void *)wdm_inv_layer_kernel<float2>, sm);
+  const cudaError_t e = smem_limit<wdm_inv_layer_kernel<float2>>(fft_smem<float2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
   // even layers, then odd: same-parity layers have disjoint supports
   for (int parity = 0; parity < 2; parity++)
@@ -1061,7 +1063,7 @@ static cudaError_t from_freq32(const WdmPlan &P, const double *freq, double *wdm
   const long long ND = (long long)P.NF * P.NT, n = 2 * (P.M + 1);
   wdm_cast_kernel<float2><<<blocks_for(n), 256, 0, s>>>(freq, (float *)P.bufX, n);
   const size_t sm = fft_smem<float2>(P.NT, 1);
-  cudaError_t e = set_smem((const void *)wdm_fwd_layer_kernel<float2>, sm);
+  cudaError_t e = smem_limit<wdm_fwd_layer_kernel<float2>>(fft_smem<float2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
   wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>(nullptr, (const float2 *)P.bufX, P.M, P.NF, P.NT,
                                                          (const float *)P.win, (const float2 *)P.twNT,
@@ -1073,9 +1075,9 @@ static cudaError_t from_freq32(const WdmPlan &P, const double *freq, double *wdm
 }
 
 bool wdm_grid_supported(int NF, int NT) {
-  if (NF < 2 || NT < 8 || NT > 4096 || NT % 2 || !smooth23(NT)) return false;
+  if (NF < 2 || NT < 8 || NT > kMaxLine || NT % 2 || !smooth23(NT)) return false;
   const long long M = (long long)NF * NT / 2;
-  return split_factor(M, 4096) != 0;
+  return split_factor(M, kMaxLine) != 0;
 }
 
 cudaError_t wdm_prepare(WdmPlan &P, int precision, int NF, int NT, const double *window, cudaStream_t s) {
