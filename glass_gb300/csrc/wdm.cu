@@ -28,7 +28,13 @@
 //    real or the imaginary part; multiplied by (-i)^n (a shift of the spectrum by
 //    NT/4) those are the real part, up to a sign s(n) of period four, so layers a
 //    and b are the real and imaginary part of the inverse FFT of H_a + i H_b, H
-//    the Hermitian parts.  The inverse runs the same backwards;
+//    the Hermitian parts.  The inverse runs the same backwards.  Only between a
+//    series and its coefficients, where every value depends on all others: to and
+//    from a spectrum a layer belongs to its own bins, and a transform shared with a
+//    neighbour would give it rounding of that one's size, and its NaNs (a layer
+//    beside one of 1e12 times its size lost all but four digits).  One layer per
+//    transform there: 1024 x 2048 from a spectrum 192 us where pairs take 100,
+//    1536 x 4096 to one 865 us where they take 331;
 //  * the real spectrum is unpacked in the row pass and packed in the inverse's
 //    column pass, where both bins k and M - k are at hand (one product for the two).
 //  * the transforms' factors are in tangent form (fp64_math.cuh), those between
@@ -39,9 +45,9 @@
 // (1024 x 2048) forward 538 -> 245 us; 6.3 M samples (1536 x 4096) inverse 1787 ->
 // 755 us.
 //
-// FP32 (GLASS_PREC_MIXED), and in FP64 the layers of grids whose NT is not a
-// multiple of 4, run one layer per CTA on ping-pong Stockham transforms; there
-// the inverse's overlap-add runs in two launches (even, then odd layers: the
+// FP32 (GLASS_PREC_MIXED), and in FP64 the layers of the spectrum forms and of grids
+// whose NT is not a multiple of 4, run one layer per CTA on ping-pong Stockham
+// transforms; there the inverse's overlap-add runs in two launches (even, then odd layers: the
 // supports of same-parity layers are disjoint, so no atomics are needed and the
 // sum order is fixed).
 #include <cooperative_groups.h>
@@ -829,11 +835,11 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   fill_roots(t1, P.M1);
   fill_roots(t2, P.M2);
   fill_roots(tn, NT);
-  if constexpr (sizeof(R) == 8) {  // dit_fft's; wdm_*_layer_kernel, for NT % 4 != 0, takes twNT as it is
+  std::vector<C> ttn;
+  if constexpr (sizeof(R) == 8) {  // dit_fft's; the wdm_*_layer_kernels take twNT as it is
     for (C &w : t1) w = tan_form(w.x, w.y);
     for (C &w : t2) w = tan_form(w.x, w.y);
-    if (NT % 4 == 0)
-      for (C &w : tn) w = tan_form(w.x, w.y);
+    for (C w : tn) ttn.push_back(tan_form(w.x, w.y));
   }
   fill_two_level(mlo, mhi, M, P.K);
   fill_two_level(nlo, nhi, ND, P.K);
@@ -843,11 +849,12 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
   // FP64: the passes' factors (wdm_roots64_kernel)
   const size_t full = sizeof(R) == 8 ? elem : 0;
-  const size_t sizes[15] = {elem * t1.size(), elem * t2.size(), elem * tn.size(), elem * mlo.size(),
+  const size_t sizes[16] = {elem * t1.size(), elem * t2.size(), elem * tn.size(), elem * mlo.size(),
                             elem * mhi.size(), elem * nlo.size(), elem * nhi.size(), sizeof(R) * win.size(),
                             elem * (size_t)(M + 1), elem * (size_t)(M + 1), elem * (size_t)(M + 1),
                             sizeof(double) * (size_t)ND,
-                            full * (size_t)M, full * (size_t)(P.M2 / 2 + 1) * P.M1, full * (size_t)(P.M1 / 2 + 1) * P.M2};
+                            full * (size_t)M, full * (size_t)(P.M2 / 2 + 1) * P.M1, full * (size_t)(P.M1 / 2 + 1) * P.M2,
+                            elem * ttn.size()};
   size_t bytes = 0;
   for (size_t b : sizes) bytes += pad(b);
   cudaError_t e = cudaMalloc(&P.base, bytes);
@@ -855,10 +862,11 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
     P.base = nullptr;
     return e;
   }
-  void **slots[15] = {&P.tw1, &P.tw2, &P.twNT, &P.mlo,  &P.mhi,  &P.nlo,   &P.nhi,    &P.win,
-                      &P.bufA, &P.bufB, &P.bufX, &P.rbuf, &P.colf, &P.packf, &P.unpackf};
+  void **slots[16] = {&P.tw1, &P.tw2, &P.twNT, &P.mlo,  &P.mhi,  &P.nlo,   &P.nhi,    &P.win,
+                      &P.bufA, &P.bufB, &P.bufX, &P.rbuf, &P.colf, &P.packf, &P.unpackf,
+                      &P.ttNT};
   char *p = (char *)P.base;
-  for (int i = 0; i < 15; i++) {
+  for (int i = 0; i < 16; i++) {
     *slots[i] = p;
     p += pad(sizes[i]);
   }
@@ -871,6 +879,7 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   if ((e = upload(P.nhi, nhi, s)) != cudaSuccess) return e;
   if ((e = upload(P.win, win, s)) != cudaSuccess) return e;
   if constexpr (sizeof(R) == 8) {
+    if ((e = upload(P.ttNT, ttn, s)) != cudaSuccess) return e;
     wdm_roots64_kernel<<<1024, 256, 0, s>>>((double2 *)P.colf, (double2 *)P.packf, (double2 *)P.unpackf, P.M1, P.M2);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -910,12 +919,17 @@ static cudaError_t launch64(int grid, int points, int most_points, int most_thre
   return launch_chained(K, grid, threads64(points, most_threads), smem64(points), s, args...);
 }
 
+// Two layers to a transform: where all values depend on each other, and NT is a
+// multiple of 4.
+enum class Layers { kPaired, kSeparate };
+
 // scale times the real spectrum X -> coefficients.
-static cudaError_t fwd_layers64(const WdmPlan &P, const double2 *X, double scale, double *wdm, cudaStream_t s) {
+static cudaError_t fwd_layers64(const WdmPlan &P, Layers how, const double2 *X, double scale, double *wdm,
+                                cudaStream_t s) {
   const int NF = P.NF, NT = P.NT;
-  if (NT % 4 == 0)
+  if (how == Layers::kPaired && NT % 4 == 0)
     return launch64<wdm_fwd_pair64_kernel>(2 * layer_pairs(NF), NT / 2, kMaxLine / 2, 256, s, X, NF, NT, (const double *)P.win,
-                    (const double2 *)P.twNT, 0.5 * scale / NT, wdm);
+                    (const double2 *)P.ttNT, 0.5 * scale / NT, wdm);
   const size_t sm = fft_smem<double2>(NT, 1);
   const cudaError_t e = smem_limit<wdm_fwd_layer_kernel<double2>>(fft_smem<double2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
@@ -939,18 +953,18 @@ static cudaError_t forward64(const WdmPlan &P, const double *time, double *wdm, 
   if ((e = launch64<wdm_row_unpack64_kernel>(2 * (P.M1 / 2 + 1), P.M2, kMaxLine, 256, s, (const double2 *)P.bufB,
                     (double2 *)P.bufX, P.M1, P.M2, (const double2 *)P.tw2, (const double2 *)P.unpackf)) != cudaSuccess)
     return e;
-  return fwd_layers64(P, (const double2 *)P.bufX, 0.5, wdm, s);
+  return fwd_layers64(P, Layers::kPaired, (const double2 *)P.bufX, 0.5, wdm, s);
 }
 
 // WDM -> scale times the spectrum, bins 0..M of P.bufX.
-static cudaError_t inverse_layers64(const WdmPlan &P, const double *wdm, double scale, cudaStream_t s) {
+static cudaError_t inverse_layers64(const WdmPlan &P, Layers how, const double *wdm, double scale, cudaStream_t s) {
   const int NF = P.NF, NT = P.NT;
   const double *win = (const double *)P.win;
-  const double2 *tw = (const double2 *)P.twNT;
   double2 *X = (double2 *)P.bufX;
   cudaError_t e;
   scale *= 0.5 * NF;
-  if (NT % 4 == 0) {
+  if (how == Layers::kPaired && NT % 4 == 0) {
+    const double2 *tw = (const double2 *)P.ttNT;
     const int pairs = NF / 2;  // (1, 2), (3, 4), ...
     const bool last_first = pairs % 2 == 0;  // the last layer's place: see the kernel
     if ((e = launch64<wdm_inv_pair64_kernel>(4 * ((pairs + 1) / 2 + last_first), NT / 4, kMaxLine / 4, 256, s, wdm, NF, NT, 0, win,
@@ -963,14 +977,15 @@ static cudaError_t inverse_layers64(const WdmPlan &P, const double *wdm, double 
   const size_t sm = fft_smem<double2>(NT, 1);
   if ((e = smem_limit<wdm_inv_layer_kernel<double2>>(fft_smem<double2>(kMaxLine, 1))) != cudaSuccess) return e;
   for (int parity = 0; parity < 2; parity++)
-    wdm_inv_layer_kernel<double2><<<(NF - parity) / 2 + 1, 256, sm, s>>>(wdm, NF, NT, parity, win, tw, scale, X);
+    wdm_inv_layer_kernel<double2><<<(NF - parity) / 2 + 1, 256, sm, s>>>(wdm, NF, NT, parity, win, (const double2 *)P.twNT,
+                                                                         scale, X);
   return cudaGetLastError();
 }
 
 static cudaError_t inverse64(const WdmPlan &P, const double *wdm, double *time, cudaStream_t s) {
   const long long ND = (long long)P.NF * P.NT;
   cudaError_t e;
-  if ((e = inverse_layers64(P, wdm, 1.0 / (double)ND, s)) != cudaSuccess) return e;
+  if ((e = inverse_layers64(P, Layers::kPaired, wdm, 1.0 / (double)ND, s)) != cudaSuccess) return e;
   if ((e = launch64<wdm_pack_col64_kernel>(P.M2 / 2 + 1, 2 * P.M1, 2 * kMaxLine, 512, s, (const double2 *)P.bufX,
                     (double2 *)P.bufB, P.M1, P.M2, (const double2 *)P.tw1, (const double2 *)P.colf,
                     (const double2 *)P.packf)) != cudaSuccess)
@@ -986,7 +1001,7 @@ static cudaError_t inverse64(const WdmPlan &P, const double *wdm, double *time, 
 
 // wdm -> ND/2 + 1 complex bins (ND + 2 doubles), wavelet_transform_inverse_freq
 static cudaError_t to_freq64(const WdmPlan &P, const double *wdm, double *freq, cudaStream_t s) {
-  const cudaError_t e = inverse_layers64(P, wdm, 1.0, s);
+  const cudaError_t e = inverse_layers64(P, Layers::kSeparate, wdm, 1.0, s);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(freq, P.bufX, sizeof(double2) * (size_t)(P.M + 1), cudaMemcpyDeviceToDevice, s);
 }
@@ -1000,7 +1015,7 @@ static cudaError_t from_freq64(const WdmPlan &P, const double *freq, double *wdm
     if (e != cudaSuccess) return e;
     X = (const double2 *)P.bufX;
   }
-  return fwd_layers64(P, X, 1.0, wdm, s);
+  return fwd_layers64(P, Layers::kSeparate, X, 1.0, wdm, s);
 }
 
 // ---- FP32 (double at the boundary)

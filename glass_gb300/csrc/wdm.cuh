@@ -13,6 +13,7 @@ struct WdmPlan {
   int M1 = 0, M2 = 0, K = 0;
   void *base = nullptr;
   void *tw1 = nullptr, *tw2 = nullptr, *twNT = nullptr;
+  void *ttNT = nullptr;  // FP64: twNT in tangent form
   void *mlo = nullptr, *mhi = nullptr, *nlo = nullptr, *nhi = nullptr;
   void *colf = nullptr, *packf = nullptr, *unpackf = nullptr;  // FP64: the passes' factors, one per point
   void *win = nullptr;
