@@ -47,9 +47,9 @@
 //
 // FP32 (GLASS_PREC_MIXED), and in FP64 the layers of the spectrum forms and of grids
 // whose NT is not a multiple of 4, run one layer per CTA on ping-pong Stockham
-// transforms; there the inverse's overlap-add runs in two launches (even, then odd layers: the
-// supports of same-parity layers are disjoint, so no atomics are needed and the
-// sum order is fixed).
+// transforms; there the inverse's overlap-add runs in two launches (even, then odd
+// layers: the supports of same-parity layers are disjoint, so no atomics are needed
+// and the sum order is fixed).
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -259,11 +259,11 @@ __device__ __forceinline__ C real_bin(const C *Z, long long M, long long k, cons
   return mk<C>((R)0.5 * (s.x + ed.y), (R)0.5 * (s.y - ed.x));
 }
 
-// Forward layers: one CTA per layer m in [0, NF].  The spectrum is either X
-// (bins 0..M given, times scale) or unpacked on the fly from Z, the FFT of the
-// packed samples.
-template <typename C>
-__global__ void wdm_fwd_layer_kernel(const C *Z, const C *X, long long M, int NF, int NT,
+// Forward layers: one CTA per layer m in [0, NF].  X: the spectrum's bins 0..M times
+// scale, or (PACKED) the FFT of the packed samples, unpacked on the fly with the
+// tables tlo and thi.
+template <typename C, bool PACKED>
+__global__ void wdm_fwd_layer_kernel(const C *X, long long M, int NF, int NT,
                                      const decltype(C().x) *phif, const C *twNT, const C *tlo, const C *thi, int K,
                                      decltype(C().x) scale, decltype(C().x) *wdm) {
   using R = decltype(C().x);
@@ -284,7 +284,10 @@ __global__ void wdm_fwd_layer_kernel(const C *Z, const C *X, long long M, int NF
     if (ok) {
       R w = phif[j < 0 ? -j : j];
       if (j == 0 && (m == 0 || m == NF)) w *= (R)0.5;
-      v = csc(X ? X[idx] : real_bin(Z, M, (long long)idx, tlo, thi, K), w);
+      if constexpr (PACKED)
+        v = csc(real_bin(X, M, (long long)idx, tlo, thi, K), w);
+      else
+        v = csc(X[idx], w);
     }
     a[t] = v;
   }
@@ -841,8 +844,12 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
     for (C &w : t2) w = tan_form(w.x, w.y);
     for (C w : tn) ttn.push_back(tan_form(w.x, w.y));
   }
-  fill_two_level(mlo, mhi, M, P.K);
-  fill_two_level(nlo, nhi, ND, P.K);
+  // FP32: two-level tables, and the four-step passes' and packed spectrum's buffer
+  const size_t f32 = sizeof(R) == 4 ? sizeof(C) : 0;
+  if (f32) {
+    fill_two_level(mlo, mhi, M, P.K);
+    fill_two_level(nlo, nhi, ND, P.K);
+  }
   std::vector<R> win(NT / 2 + 1);
   for (int i = 0; i <= NT / 2; i++) win[i] = (R)window[i];
   const size_t elem = sizeof(C);
@@ -851,7 +858,7 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   const size_t full = sizeof(R) == 8 ? elem : 0;
   const size_t sizes[16] = {elem * t1.size(), elem * t2.size(), elem * tn.size(), elem * mlo.size(),
                             elem * mhi.size(), elem * nlo.size(), elem * nhi.size(), sizeof(R) * win.size(),
-                            elem * (size_t)(M + 1), elem * (size_t)(M + 1), elem * (size_t)(M + 1),
+                            f32 * (size_t)(M + 1), elem * (size_t)(M + 1), elem * (size_t)(M + 1),
                             sizeof(double) * (size_t)ND,
                             full * (size_t)M, full * (size_t)(P.M2 / 2 + 1) * P.M1, full * (size_t)(P.M1 / 2 + 1) * P.M2,
                             elem * ttn.size()};
@@ -873,12 +880,13 @@ static cudaError_t prepare_t(WdmPlan &P, int NF, int NT, const double *window, c
   if ((e = upload(P.tw1, t1, s)) != cudaSuccess) return e;
   if ((e = upload(P.tw2, t2, s)) != cudaSuccess) return e;
   if ((e = upload(P.twNT, tn, s)) != cudaSuccess) return e;
-  if ((e = upload(P.mlo, mlo, s)) != cudaSuccess) return e;
-  if ((e = upload(P.mhi, mhi, s)) != cudaSuccess) return e;
-  if ((e = upload(P.nlo, nlo, s)) != cudaSuccess) return e;
-  if ((e = upload(P.nhi, nhi, s)) != cudaSuccess) return e;
   if ((e = upload(P.win, win, s)) != cudaSuccess) return e;
-  if constexpr (sizeof(R) == 8) {
+  if constexpr (sizeof(R) == 4) {
+    if ((e = upload(P.mlo, mlo, s)) != cudaSuccess) return e;
+    if ((e = upload(P.mhi, mhi, s)) != cudaSuccess) return e;
+    if ((e = upload(P.nlo, nlo, s)) != cudaSuccess) return e;
+    if ((e = upload(P.nhi, nhi, s)) != cudaSuccess) return e;
+  } else {
     if ((e = upload(P.ttNT, ttn, s)) != cudaSuccess) return e;
     wdm_roots64_kernel<<<1024, 256, 0, s>>>((double2 *)P.colf, (double2 *)P.packf, (double2 *)P.unpackf, P.M1, P.M2);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -931,11 +939,10 @@ static cudaError_t fwd_layers64(const WdmPlan &P, Layers how, const double2 *X, 
     return launch64<wdm_fwd_pair64_kernel>(2 * layer_pairs(NF), NT / 2, kMaxLine / 2, 256, s, X, NF, NT, (const double *)P.win,
                     (const double2 *)P.ttNT, 0.5 * scale / NT, wdm);
   const size_t sm = fft_smem<double2>(NT, 1);
-  const cudaError_t e = smem_limit<wdm_fwd_layer_kernel<double2>>(fft_smem<double2>(kMaxLine, 1));
+  const cudaError_t e = smem_limit<wdm_fwd_layer_kernel<double2, false>>(fft_smem<double2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
-  wdm_fwd_layer_kernel<double2><<<NF + 1, 256, sm, s>>>(nullptr, X, P.M, NF, NT, (const double *)P.win,
-                                                        (const double2 *)P.twNT, (const double2 *)P.nlo,
-                                                        (const double2 *)P.nhi, P.K, scale, wdm);
+  wdm_fwd_layer_kernel<double2, false><<<NF + 1, 256, sm, s>>>(
+      X, P.M, NF, NT, (const double *)P.win, (const double2 *)P.twNT, nullptr, nullptr, 0, scale, wdm);
   return cudaGetLastError();
 }
 
@@ -1027,10 +1034,10 @@ static cudaError_t forward32(const WdmPlan &P, const double *time, double *wdm, 
   if ((e = four_step<float2>(P, (const float2 *)P.rbuf, (float2 *)P.bufB, (float2 *)P.bufA, -1, 1.f, s)) != cudaSuccess)
     return e;
   const size_t sm = fft_smem<float2>(P.NT, 1);
-  if ((e = smem_limit<wdm_fwd_layer_kernel<float2>>(fft_smem<float2>(kMaxLine, 1))) != cudaSuccess) return e;
-  wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>((const float2 *)P.bufA, nullptr, P.M, P.NF, P.NT,
-                                                         (const float *)P.win, (const float2 *)P.twNT,
-                                                         (const float2 *)P.nlo, (const float2 *)P.nhi, P.K, 1.f, out);
+  if ((e = smem_limit<wdm_fwd_layer_kernel<float2, true>>(fft_smem<float2>(kMaxLine, 1))) != cudaSuccess) return e;
+  wdm_fwd_layer_kernel<float2, true><<<P.NF + 1, 256, sm, s>>>(
+      (const float2 *)P.bufA, P.M, P.NF, P.NT, (const float *)P.win, (const float2 *)P.twNT, (const float2 *)P.nlo,
+      (const float2 *)P.nhi, P.K, 1.f, out);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   wdm_uncast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>(out, wdm, ND);
   return cudaGetLastError();
@@ -1078,12 +1085,11 @@ static cudaError_t from_freq32(const WdmPlan &P, const double *freq, double *wdm
   const long long ND = (long long)P.NF * P.NT, n = 2 * (P.M + 1);
   wdm_cast_kernel<float2><<<blocks_for(n), 256, 0, s>>>(freq, (float *)P.bufX, n);
   const size_t sm = fft_smem<float2>(P.NT, 1);
-  cudaError_t e = smem_limit<wdm_fwd_layer_kernel<float2>>(fft_smem<float2>(kMaxLine, 1));
+  cudaError_t e = smem_limit<wdm_fwd_layer_kernel<float2, false>>(fft_smem<float2>(kMaxLine, 1));
   if (e != cudaSuccess) return e;
-  wdm_fwd_layer_kernel<float2><<<P.NF + 1, 256, sm, s>>>(nullptr, (const float2 *)P.bufX, P.M, P.NF, P.NT,
-                                                         (const float *)P.win, (const float2 *)P.twNT,
-                                                         (const float2 *)P.nlo, (const float2 *)P.nhi, P.K, 1.f,
-                                                         (float *)P.rbuf);
+  wdm_fwd_layer_kernel<float2, false><<<P.NF + 1, 256, sm, s>>>((const float2 *)P.bufX, P.M, P.NF, P.NT,
+                                                                (const float *)P.win, (const float2 *)P.twNT, nullptr,
+                                                                nullptr, 0, 1.f, (float *)P.rbuf);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   wdm_uncast_kernel<float2><<<blocks_for(ND), 256, 0, s>>>((const float *)P.rbuf, wdm, ND);
   return cudaGetLastError();

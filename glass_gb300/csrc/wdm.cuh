@@ -14,7 +14,7 @@ struct WdmPlan {
   void *base = nullptr;
   void *tw1 = nullptr, *tw2 = nullptr, *twNT = nullptr;
   void *ttNT = nullptr;  // FP64: twNT in tangent form
-  void *mlo = nullptr, *mhi = nullptr, *nlo = nullptr, *nhi = nullptr;
+  void *mlo = nullptr, *mhi = nullptr, *nlo = nullptr, *nhi = nullptr;  // FP32
   void *colf = nullptr, *packf = nullptr, *unpackf = nullptr;  // FP64: the passes' factors, one per point
   void *win = nullptr;
   void *bufA = nullptr, *bufB = nullptr, *bufX = nullptr;
