@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(128) fd_plan_kernel(PlanArgs a) {
   const int i0 = blockIdx.x * P, n = min(P, a.nitems - i0);
   const int i = i0 + l;
   // one trip for all of a CTA's inputs, which may be pinned host memory that
-  // changes between two replays of a graph: read through (ld.cv) and once
+  // changes between two replays of a graph: read through (ld.cv)
   int seg = -1;
   if (w == 1 && l < n) seg = __ldcv(a.item_seg + i);
   if (w == 2 && l < n && a.term_x_dev) a.term_x_dev[i] = __ldcv(a.term_x + i);

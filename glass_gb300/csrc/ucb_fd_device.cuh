@@ -886,9 +886,10 @@ cudaError_t fd_launch_plan(PlanKind kind, PlanArgs a, const FdTablesDev &tab, in
                            cudaStream_t stream);
 
 // Outputs of a proposal that is not evaluated (bad input, or a template
-// entirely outside its segment).
+// entirely outside its segment).  term_x may be pinned host memory, as the other
+// inputs of the plan: read through.
 __device__ __forceinline__ void plan_write_skipped(const PlanArgs &a, int i, int st) {
-  const double tx = a.term_x ? a.term_x[i] : 0.0;
+  const double tx = a.term_x ? __ldcv(a.term_x + i) : 0.0;
   if (st & 3) {
     const double nan = __longlong_as_double(0x7ff8000000000000ULL);
     a.dlogl[i] = nan;
