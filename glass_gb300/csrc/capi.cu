@@ -1376,11 +1376,13 @@ extern "C" int glass_gpu_noise_logl_batch_sgwb(glass_gpu_ctx *ctx, int nprop, co
     cudaFree(nd.partial);
     nd.partial = nullptr;
     nd.partial_models = 0;
-    GLASS_CUDA(cudaMalloc(&nd.partial, sizeof(double) * noise_partials(nd.N, want)), "cudaMalloc(noise partial)");
+    GLASS_CUDA(cudaMalloc(&nd.partial, sizeof(double) * noise_partials(nd.N, want, ctx->num_sms)),
+               "cudaMalloc(noise partial)");
     nd.partial_models = want;
   }
   int nl = 0;
-  cudaError_t e = noise_logl_launch(nd, nprop, inst, sgal, ctx->sgwb_type, sgwb, logl, ctx->stream, &nl);
+  cudaError_t e = noise_logl_launch(nd, nprop, inst, sgal, ctx->sgwb_type, sgwb, logl, ctx->num_sms, ctx->stream,
+                                    &nl);
   ctx->last_launches = nl;
   if (e != cudaSuccess) return cuda_err(e, "noise_logl_batch launch");
   return GLASS_OK;
@@ -1568,11 +1570,13 @@ extern "C" int glass_gpu_noise_wavelet_logl_batch_sgwb(glass_gpu_ctx *ctx, int m
     cudaFree(w.partial);
     w.partial = nullptr;
     w.partial_models = 0;
-    GLASS_CUDA(cudaMalloc(&w.partial, sizeof(double) * noise_wv_partials(w, want)), "cudaMalloc(noise wv partial)");
+    GLASS_CUDA(cudaMalloc(&w.partial, sizeof(double) * noise_wv_partials(w.Nlayer, w.Ncoarse, want, ctx->num_sms)),
+               "cudaMalloc(noise wv partial)");
     w.partial_models = want;
   }
   int nl = 0;
-  cudaError_t e = noise_wv_logl_launch(w, mode, nprop, inst, sgal, ctx->sgwb_type, sgwb, logl, ctx->stream, &nl);
+  cudaError_t e = noise_wv_logl_launch(w, mode, nprop, inst, sgal, ctx->sgwb_type, sgwb, logl, ctx->num_sms, ctx->stream,
+                                       &nl);
   ctx->last_launches = nl;
   if (e != cudaSuccess) return cuda_err(e, "noise_wavelet_logl_batch launch");
   return GLASS_OK;

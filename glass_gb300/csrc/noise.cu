@@ -55,7 +55,7 @@ constexpr int kNoiseThreads = 128;
 // SM take 16x what they take on 16); at the most, a CTA's model constants and
 // its reduction are 2% of its work.
 constexpr int kNoiseMaxBins = 16;
-constexpr int kNoiseTargetCtas = 608;  // 4 per SM of a 152-SM GPU
+constexpr int kNoiseCtasPerSm = 4;  // (608 on 152 SMs)
 
 struct NoiseArgs {
   int N, nchunks, nprop, R;  // R bins per thread
@@ -834,26 +834,30 @@ int noise_sgwb_rows(int nresp, const double *resp, int N, const double *f, doubl
 // Layers per CTA of the modulated form: about 4096 cells, fewer where the
 // batch is too small to give every SM a few CTAs (a CTA's model constants and
 // layer covariances cost about as much as 300 cells).
-static int noise_wv_lj(const NoiseWvDev &w, int nprop) {
-  int lj = 4096 / (w.Ncoarse > 0 ? w.Ncoarse : 1);
+int noise_wv_layers_per_cta(int Nlayer, int Ncoarse, int nprop, int num_sms) {
+  int lj = 4096 / (Ncoarse > 0 ? Ncoarse : 1);
   if (lj < 1) lj = 1;
   if (lj > kNoiseWvMaxLJ) lj = kNoiseWvMaxLJ;
-  while (lj > 1 && (long long)((w.Nlayer + lj - 1) / lj) * nprop < kNoiseTargetCtas) lj = (lj + 1) / 2;
+  while (lj > 1 && (long long)((Nlayer + lj - 1) / lj) * nprop < (long long)kNoiseCtasPerSm * num_sms) lj = (lj + 1) / 2;
   return lj;
 }
 
-size_t noise_wv_partials(const NoiseWvDev &w, int nprop) {
-  const size_t most = (size_t)nprop * ((w.Nlayer + noise_wv_lj(w, 1 << 30) - 1) / noise_wv_lj(w, 1 << 30));
-  return most > 4 * (size_t)kNoiseTargetCtas + 4 * (size_t)nprop ? most : 4 * (size_t)kNoiseTargetCtas + 4 * (size_t)nprop;
+// As noise_partials.
+size_t noise_wv_partials(int Nlayer, int Ncoarse, int nprop, int num_sms) {
+  const int lj = noise_wv_layers_per_cta(Nlayer, Ncoarse, 1 << 30, num_sms);
+  const size_t most = (size_t)nprop * ((Nlayer + lj - 1) / lj);
+  const size_t few = 2 * (size_t)kNoiseCtasPerSm * num_sms + 2 * (size_t)nprop;
+  return most > few ? most : few;
 }
 
 cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const double *inst, const double *sgal,
-                                 int sg_type, const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch) {
+                                 int sg_type, const double *sgwb, double *logl, int num_sms, cudaStream_t stream,
+                                 int *nlaunch) {
   NoiseWvArgs a;
   a.Nlayer = w.Nlayer;
   a.Ncoarse = w.Ncoarse;
   a.Q = w.Q;
-  a.LJ = noise_wv_lj(w, nprop);
+  a.LJ = noise_wv_layers_per_cta(w.Nlayer, w.Ncoarse, nprop, num_sms);
   a.nchunks = (w.Nlayer + a.LJ - 1) / a.LJ;
   a.mode = mode;
   a.inv_ND = 1.0 / (double)((long long)w.NF * w.NT);
@@ -901,18 +905,20 @@ cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const
   return launch_chained(noise_wv_const_kernel, (nprop + 255) / 256, 256, 0, stream, logl, nprop, cst);
 }
 
-static int noise_bins_per_thread(int N, int nprop) {
+int noise_bins_per_thread(int N, int nprop, int num_sms) {
   int R = kNoiseMaxBins;
-  while (R > 1 && (long long)((N + kNoiseThreads * R - 1) / (kNoiseThreads * R)) * nprop < kNoiseTargetCtas) R /= 2;
+  while (R > 1 && (long long)((N + kNoiseThreads * R - 1) / (kNoiseThreads * R)) * nprop <
+                      (long long)kNoiseCtasPerSm * num_sms)
+    R /= 2;
   return R;
 }
 
 // What any batch of at most nprop models needs: below the largest chunk the
 // rule stops at the first size that reaches the target, at most twice it.
-size_t noise_partials(int N, int nprop) {
+size_t noise_partials(int N, int nprop, int num_sms) {
   const int chunk = kNoiseThreads * kNoiseMaxBins;
   const size_t most = (size_t)nprop * ((N + chunk - 1) / chunk);
-  const size_t few = 2 * (size_t)kNoiseTargetCtas + 2 * (size_t)nprop;
+  const size_t few = 2 * (size_t)kNoiseCtasPerSm * num_sms + 2 * (size_t)nprop;
   return most > few ? most : few;
 }
 
@@ -943,10 +949,10 @@ cudaError_t spline_noise_launch(const SplineNoiseDev &s, int nprop, int kmax, co
 }
 
 cudaError_t noise_logl_launch(const NoiseDev &nd, int nprop, const double *inst, const double *sgal, int sg_type,
-                              const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch) {
+                              const double *sgwb, double *logl, int num_sms, cudaStream_t stream, int *nlaunch) {
   NoiseArgs a;
   a.N = nd.N;
-  a.R = noise_bins_per_thread(nd.N, nprop);
+  a.R = noise_bins_per_thread(nd.N, nprop, num_sms);
   a.nchunks = (nd.N + kNoiseThreads * a.R - 1) / (kNoiseThreads * a.R);
   a.fstep = kNoiseThreads / nd.T;
   a.nprop = nprop;

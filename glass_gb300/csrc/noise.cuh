@@ -54,13 +54,16 @@ struct NoiseWvDev {
 // kTabXX .. kTabYZ).
 void noise_wv_build(int NT, double df, int lmin, int Nlayer, int Q, const double *X, const double *Y, const double *Z,
                     double *tab, double *P);
-// doubles that w.partial needs for any batch of at most nprop models
-size_t noise_wv_partials(const NoiseWvDev &w, int nprop);
+// Layers per CTA of the modulated form for nprop models, and the doubles that
+// w.partial needs for any batch of at most nprop models.
+int noise_wv_layers_per_cta(int Nlayer, int Ncoarse, int nprop, int num_sms);
+size_t noise_wv_partials(int Nlayer, int Ncoarse, int nprop, int num_sms);
 // mode 0 instrument, 1 stationary foreground, 2 modulated foreground; plus,
 // with sgwb (4 per model, template sg_type), the stochastic background;
-// w.partial must hold noise_wv_partials(w, nprop) (mode 2).
+// w.partial must hold noise_wv_partials for nprop models (mode 2).
 cudaError_t noise_wv_logl_launch(const NoiseWvDev &w, int mode, int nprop, const double *inst, const double *sgal,
-                                 int sg_type, const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch);
+                                 int sg_type, const double *sgwb, double *logl, int num_sms, cudaStream_t stream,
+                                 int *nlaunch);
 
 // SGWB templates (SGWB_t, noise/src/glass_noise_model.h:99-108) and their
 // parameter counts
@@ -83,14 +86,16 @@ struct SplineNoiseDev {
 // knot_C[(p nch + c) kmax ..] (device pointers)
 cudaError_t spline_noise_launch(const SplineNoiseDev &s, int nprop, int kmax, const int *nknots, const double *knot_f,
                                 const double *knot_C, double *logl, cudaStream_t stream, int *nlaunch);
-// doubles that nd.partial needs for any batch of at most nprop models
-size_t noise_partials(int N, int nprop);
+// Bins per thread (of 128 per CTA) for nprop models, and the doubles that
+// nd.partial needs for any batch of at most nprop models.
+int noise_bins_per_thread(int N, int nprop, int num_sms);
+size_t noise_partials(int N, int nprop, int num_sms);
 // logl[p] for noise models inst[12 p ..] (sacc[6], soms[6]) and sgal[5 p ..]
 // (or null: instrument only), plus, with sgwb[4 p ..] (or null), the SGWB of
 // template sg_type (three channels only); nd.partial must hold
-// noise_partials(N, nprop).  Three channels: my_noise_log_likelihood; one or two:
+// noise_partials for nprop models.  Three channels: my_noise_log_likelihood; one or two:
 // noise_log_likelihood (no 2 pi constant), link levels sacc[0], soms[0].
 cudaError_t noise_logl_launch(const NoiseDev &nd, int nprop, const double *inst, const double *sgal, int sg_type,
-                              const double *sgwb, double *logl, cudaStream_t stream, int *nlaunch);
+                              const double *sgwb, double *logl, int num_sms, cudaStream_t stream, int *nlaunch);
 
 }  // namespace glass
