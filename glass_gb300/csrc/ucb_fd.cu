@@ -568,7 +568,6 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   pa.nseg = bank.nseg;
   pa.NFFT = bank.NFFT;
   pa.cap = work.cap;
-  pa.precision = precision;
   pa.n_fixed = n_fixed;
   pa.T = bank.T;
   pa.fstar = bank.fstar;
@@ -599,9 +598,6 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
   SlowArgs sa;
   sa.cap = work.cap;
   sa.NFFT = bank.NFFT;
-  sa.fstar = bank.fstar;
-  sa.L = kLARM;
-  sa.Rf = (float)(kAU * (kLARM / (2.0 * kSQ3 * kAU)));
   sa.invLf = (float)(1.0 / kLARM);
   sa.AUcf = (float)(kAU / kCLIGHT);
   sa.invTf = (float)(1.0 / bank.T);

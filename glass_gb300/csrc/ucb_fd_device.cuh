@@ -482,8 +482,8 @@ __device__ __forceinline__ SpreadInterval spread_interval(double T, double invfs
 // Source geometry shared by both precisions (ucb/src/glass_ucb_waveform.c:802-838,
 // utils/src/glass_lisa.c:1566-1596).
 struct SourceGeom {
-  double f0, fdot, phi0, amp, eps, dfq;
-  double k[3], u[3], v[3], ep[6], ec[6];
+  double f0, fdot, phi0, amp, dfq;
+  double k[3], u[3], v[3];
   double DPr, DPi, DCr, DCi;
 };
 
@@ -493,9 +493,7 @@ static __host__ __device__ void source_geometry(const double *p, int NP, double 
   g.amp = exp(p[3]);
   g.phi0 = p[6];
   g.fdot = NP > 7 ? p[7] / (T * T) : 0.0;
-  double fT = f0 * T;
-  long long q = (long long)fT;
-  g.eps = fT - (double)q;
+  long long q = (long long)(f0 * T);
   g.dfq = kPI2 * (((double)q) / T);
   double sinps, cosps;
   sincos(2. * psi, &sinps, &cosps);
@@ -516,12 +514,6 @@ static __host__ __device__ void source_geometry(const double *p, int NP, double 
   g.k[0] = -sinth * cosph;
   g.k[1] = -sinth * sinph;
   g.k[2] = -costh;
-  int idx = 0;
-  for (int i = 0; i < 3; i++)
-    for (int j = i; j < 3; j++, idx++) {
-      g.ep[idx] = v[i] * v[j] - u[i] * u[j];
-      g.ec[idx] = u[i] * v[j] + v[i] * u[j];
-    }
 }
 
 static __host__ __device__ void make_item_f64(const SourceGeom &g, int N, double fstar, ItemF64 &c) {
@@ -546,12 +538,6 @@ static __host__ __device__ void make_item_f64(const SourceGeom &g, int N, double
 }
 
 // ----------------------------------------------------------------- slow part
-// Symmetric 3x3 quadratic form r^T E r, E stored as xx, xy, xz, yy, yz, zz.
-template <typename R>
-__device__ __forceinline__ R quad(const R *e, R x, R y, R z) {
-  return e[0] * x * x + e[3] * y * y + e[5] * z * z + (R)2 * (e[1] * x * y + e[2] * x * z + e[4] * y * z);
-}
-
 // sin(x)/x: Taylor series through x^12 for |x| <= 1 (truncation < 1e-12).
 // sinc(x) - 1, so that a product with sinc(x) ~ 1 need not round it near 1
 // (as 1 + small it would round to the same float over many samples of a
@@ -861,7 +847,7 @@ __device__ __forceinline__ void ae_combos64(const double2 d[6], double2 out[4]) 
 
 // ------------------------------------------------------------- kernel args
 struct PlanArgs {
-  int nitems, nseg, NFFT, cap, precision;
+  int nitems, nseg, NFFT, cap;
   int n_fixed;  // 0: bandwidth rule
   int per_cta = 16;  // proposals per CTA (8 .. 32)
   double T, fstar, L;
@@ -913,8 +899,7 @@ __device__ __forceinline__ void plan_write_skipped(const PlanArgs &a, int i, int
 // four arm-combination series of each proposal.
 struct SlowArgs {
   int cap, NFFT;
-  double fstar, L;
-  float Rf, invLf, AUcf, invTf;  // orbit radius, 1/L, AU/c, 1/T for the FP32 path
+  float invLf, AUcf, invTf;  // 1/L, AU/c, 1/T for the FP32 path
   const int *bin_count, *bin_list;
   const ItemF64 *items64;
   const ItemMix *itemsmix;

@@ -32,7 +32,6 @@ __device__ __forceinline__ df df_sq_sum(dc a) { return df_mul2_add(a.re, a.re, a
 __device__ __forceinline__ dc dc_scale2(dc a, float p2) {
   return {{a.re.hi * p2, a.re.lo * p2}, {a.im.hi * p2, a.im.lo * p2}};
 }
-__device__ __forceinline__ dc dc_scale(dc a, df s) { return {df_mul(a.re, s), df_mul(a.im, s)}; }
 
 // Double-float division (one Newton correction of the float quotient).
 __device__ __forceinline__ df df_div(df a, df b) {
@@ -80,25 +79,6 @@ __device__ __forceinline__ df df_alt_series(df x2) {
     p = df_add(df_mul(p, x2), c);
   }
   return p;
-}
-
-// sin and cos of a double-float angle of at most a few tens of radians:
-// reduction by pi/2 (three-part constant, exact products of the quadrant
-// count), then the Taylor series of sin (through r^17) and cos (through
-// r^16) on r in [-pi/4, pi/4] (truncation below 1e-16).
-__device__ __forceinline__ void df_sincos(df x, df *s, df *c) {
-  const float q = rintf(x.hi * 0.63661977236758134f);
-  df r = df_add(x, df_neg(two_prod(q, 1.5707963705062866f)));
-  r = df_add(r, df_neg(two_prod(q, -4.371138828673793e-08f)));
-  r = df_add(r, df{q * 1.7151245100058819e-15f, 0.f});
-  const df r2 = df_mul(r, r);
-  const df sr = df_mul(r, df_alt_series<1, 9>(r2));
-  const df cr = df_alt_series<0, 9>(r2);
-  const int qi = ((int)q) & 3;
-  const df ss = (qi & 1) ? cr : sr;
-  const df cc = (qi & 1) ? sr : cr;
-  *s = (qi & 2) ? df_neg(ss) : ss;
-  *c = ((qi + 1) & 2) ? df_neg(cc) : cc;
 }
 
 // sin and cos of a double-float angle with a table: tab[k] = (sin, cos) of

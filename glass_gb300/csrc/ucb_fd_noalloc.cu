@@ -183,7 +183,6 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
   pa.nseg = nseg;
   pa.NFFT = NFFT;
   pa.cap = kNaMaxItems;
-  pa.precision = 0;
   pa.n_fixed = 0;
   pa.T = T;
   pa.fstar = fstar;
@@ -204,9 +203,6 @@ extern "C" int glass_gpu_dlogl_fp64_noalloc(void *stream, int format, double T, 
   SlowArgs sa;
   sa.cap = kNaMaxItems;
   sa.NFFT = NFFT;
-  sa.fstar = fstar;
-  sa.L = kLARM;
-  sa.Rf = (float)(kAU * (kLARM / (2.0 * kSQ3 * kAU)));
   sa.invLf = (float)(1.0 / kLARM);
   sa.AUcf = (float)(kAU / kCLIGHT);
   sa.invTf = (float)(1.0 / T);

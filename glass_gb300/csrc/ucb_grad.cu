@@ -656,7 +656,6 @@ cudaError_t fd_grad_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWork
   pa.nseg = bank.nseg;
   pa.NFFT = bank.NFFT;
   pa.cap = work.cap;
-  pa.precision = 1;
   pa.n_fixed = N_fixed;
   pa.T = bank.T;
   pa.fstar = bank.fstar;

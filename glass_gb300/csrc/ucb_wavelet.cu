@@ -770,12 +770,6 @@ __global__ void __launch_bounds__(kDloglThreads) wv_dlogl_kernel(WvGridDev g, in
 }
 
 // ------------------------------------------------------------ mixed precision
-// Spline value in FP32 (Horner) from FP64 coefficients (the channel amplitude,
-// O(1e-22)).
-__device__ __forceinline__ float spl_eval_f(const double *c, int n, int j, float d) {
-  return (float)c[j] + d * ((float)c[n + j] + d * ((float)c[2 * n + j] + d * (float)c[3 * n + j]));
-}
-
 // Per spline interval j of one (source, channel), the constants the mixed
 // sampler needs, built in FP64 and stored as floats / double-floats:
 //   carrier (barycentre phase spline on the orbit grid x, heterodyne folded in)
