@@ -18,8 +18,10 @@ __device__ __forceinline__ double rcp_fast(double x) {
   return fma(r, fma(e, e, e), r);
 }
 
-// a / b, correctly rounded, from rb = 1/b: the product and one exact-residual
-// step (3 FP64 instructions instead of about 9).
+// a / b from rb = 1/b: the product and one exact-residual step (3 FP64 instructions
+// instead of about 9).  Before its rounding the result is within 2^-104 of the
+// quotient, relatively (2^-102 where rb is good to a few ulp only): the last bit can
+// differ from the quotient's where that lies so close to the middle of two doubles.
 __device__ __forceinline__ double div_by(double a, double b, double rb) {
   const double q = a * rb;
   return fma(fma(-q, b, a), rb, q);

@@ -12,15 +12,17 @@
 // amplitude/phase splines, samples the heterodyned signal at NT (nl + 1)
 // points and applies the per-layer WDM transform
 // (utils/src/glass_wavelet.c:544-611).  The GPU version splits that into:
-//  * wv_plan_kernel    one thread per source: layers, geometry, the two
-//                      barycentre splines (Thomas sweeps; the grid's own
-//                      factors are precomputed, only the data sweeps remain);
+//  * wv_plan_kernel    a CTA per 16 (8 for a year's nodes) sources: layers and
+//                      geometry on a thread each, the two barycentre splines over
+//                      all threads but for the Thomas sweeps, a thread each (the
+//                      grid's own factors are precomputed, only the data sweeps
+//                      remain);
 //  * wv_resp_kernel    one thread per (source, orbit node): light-time shift
 //                      and the X, Y, Z responses M, Mf;
-//  * wv_tdi_kernel     one thread per (source, channel): amplitude sign flips,
-//                      phase extraction and unwrapping (sequential scans as in
-//                      utils/src/glass_math.c:1034-1052, 1244-1308), and the
-//                      two channel splines;
+//  * wv_tdi_kernel     a CTA per 16 or 8 (source, channel) pairs: amplitude sign
+//                      flips, phase extraction and unwrapping (the sequential scans
+//                      of utils/src/glass_math.c:1034-1052, 1244-1308 on a thread
+//                      each), and the two channel splines;
 //  * wv_carrier_kernel one thread per (source, sample): the barycentre phase
 //                      at the light-time-shifted time, which the three channels
 //                      share;
@@ -91,8 +93,9 @@ __device__ __forceinline__ int even_index(const EvenGrid &e, int n, double v) {
 // right-hand side, independent per node), spline_recurrence for one array on one
 // thread (the two sequential sweeps on z, which holds the right-hand sides on
 // entry and c2 on exit), spline_coeffs for node i (c1, c3).  EXACT: every value
-// has the same FP64 expression as in one sequential sweep, its divisions by
-// div_by; the barycentre phase needs that (it reaches 1e6 rad, and the delayed
+// has the same FP64 expression as in one sequential sweep, its quotients to the
+// last bit by div_by (but one in ~2^50: c3's reciprocal, of 3 h, is a third of the
+// tabulated 1/h); the barycentre phase needs that (it reaches 1e6 rad, and the delayed
 // terms are second differences of it, so one coefficient's last bit shows at
 // 1e-9 in a channel).  Else quotients are products and sums are fused: 5
 // instead of 10, 3 instead of 7 and 8 instead of 17 FP64 instructions per node.
@@ -385,16 +388,17 @@ __global__ void wv_resp_kernel(WvGridDev g, int n, const WvSrc *srcs, const doub
 
 // ------------------------------------------------------------ TDI splines
 // extract_amplitude_and_phase + unwrap_phase (utils/src/glass_math.c:1244-1308,
-// 1034-1052) and the channel's amplitude / phase splines; one thread per
-// (source, channel).  The flip and phase-jump arrays live in the slots of
-// the spline's c1 and c2 coefficients until the sweeps overwrite them.
+// 1034-1052) and the channel's amplitude / phase splines.
 // C (source, channel) pairs per CTA of 128 threads, 4 norb doubles of shared
 // memory per pair: the per-node work (|M + i Mf|, atan2, remainder, the spline
 // right-hand sides and coefficients) over all threads (node-parallel); the
 // flip scan, the unwrapping scan and the spline recurrences on one thread per
 // pair (per array for the recurrences).  The flip and phase-jump arrays use
-// the slots of the two right-hand-side arrays until those are formed.  Every
-// value has the same FP64 expression as in one sequential pass.
+// the slots of the two right-hand-side arrays until those are formed.  The scans
+// and their decisions are the reference's; atan2 is atan2_tab (2 ulp of pi), the
+// remainder an exact residual, and the splines, of a phase of a few radians after
+// the carrier is taken out, use reciprocals and fused sums: a few 1e-15 of a
+// channel's largest value against one sequential pass.
 template <int C>
 __global__ void __launch_bounds__(128) wv_tdi_kernel(WvGridDev g, int n, const WvSrc *srcs, const double *resp,
                                                      double *tdi) {
@@ -1054,8 +1058,9 @@ void wv_analytic_orbit(double Tobs, double t0, std::vector<double> &t, std::vect
 
 namespace {
 
-// Host copy of the cubic spline (same arithmetic as warp_spline_pair plus the
-// grid factors), evaluated with the binary-search lookup.
+// Host copy of the cubic spline (the expressions of spline_rhs<true>,
+// spline_recurrence<true> and spline_coeffs<true>, with divisions), evaluated
+// with the binary-search lookup.
 struct HostSpline {
   int n = 0;
   const double *x = nullptr;

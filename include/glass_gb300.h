@@ -789,7 +789,11 @@ int glass_gpu_wdm_by_layers_host(glass_gpu_ctx *ctx, int NF, int NT, int jmin, i
  * arrays struct Orbit holds, utils/src/glass_lisa.h:60-109), or, with both
  * NULL, is initialize_interpolated_analytic_orbits (utils/src/glass_lisa.c:271).
  * Limits: NT even, of the form 2^a 3^b, 8 <= NT <= 4096; 20 <= norb <= 2048.
- * Host pointers; synchronous; allocates the grid tables and a work area.
+ * Host pointers; synchronous; allocates the grid tables and a work area for 4096
+ * sources at a time, about 4096 (104 NT + 312 norb) bytes whatever the precision
+ * used later: 1.1 GB at NT = 2048 and 200 nodes, 2.0 GB at NT = 4096.  Of these
+ * 32 NT bytes per source hold the samples' carrier phases, which FP64 calls and the
+ * FP64 re-evaluation of mixed ones use.
  */
 int glass_gpu_wavelet_setup(glass_gpu_ctx *ctx, double Tobs, double t0, int NF, int NT, double wdt, double wdf,
                             double A, double nx, int kmin, int kmax, int norb, const double *orbit_t,
