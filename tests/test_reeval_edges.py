@@ -1,6 +1,6 @@
-"""The double-float re-evaluation at every template size, on banks where a series has
-one CTA and where it has two, for one proposal and for more than a launch holds at
-once, clipped by the segment's edges and per channel.
+"""The double-float re-evaluation at every template size, on banks of 512 to 8192 bins
+(whose width sets the launch's shared memory), for one proposal and for more than a
+launch holds at once, clipped by the segment's edges and per channel.
 
 Tolerance 1e-10 of max(1, |h|^2): double-float rounding is 4e-15 of the sums, whose
 scale is |h| |r|, and the carrier phase of both forms is good to 1e-11 rad.
