@@ -22,7 +22,8 @@
 //     whitened template per bin from their own spectrum and their partner's
 //     (read through distributed shared memory), each over half of the bins,
 //     and sum the residual power and the template power; CTA 0 gathers the
-//     four partial sums and writes the results over the mixed ones.
+//     four partial sums and writes the results over the mixed ones.  Proposals of
+//     up to 256 points take one CTA each, with the same sums.
 // What is left is of order 1e-12 of the same scale.
 #include <math.h>
 
@@ -184,6 +185,10 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
   }
 }
 
+// Proposals of up to this many points take one CTA each.
+constexpr int kHpSmallBins = 4;  // N = 32 << b, b < 4
+constexpr int kHpSmallN = 32 << (kHpSmallBins - 1);
+
 // ------------------------------------------------------- spectral stage, df
 // The proposal of entry k (largest sizes first, so that the long ones start
 // early): item, size, segment, placement, size bin and series offset (float4
@@ -232,6 +237,14 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // of each next bin and the twiddles of each next butterfly before the arithmetic of
 // the current one.  61 proposals of up to 1024 points 19.1 -> 16 us, 73 of up to
 // 4096 on 8192-bin segments 60.8 -> 36 us.
+//
+// The registers that takes leave 74 clusters resident.  Up to 256 points one CTA
+// holds a proposal's four series and has a butterfly of a stage per thread, as
+// a cluster has, without its barriers: 296 at once (series and transform of 3000
+// proposals of 32 points 217 -> 66 us, of 600 of 128 points 72 -> 39; with ping-pong
+// buffers and 114 clusters resident they took 143 and 59).  The sums keep the
+// clusters' order: a partial one per channel and half of the bins, bins over
+// lanes, lanes by halving distances, then warps in turn.
 template <bool PERCH>
 __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;
@@ -240,6 +253,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 red[32];
   __shared__ float4 s_part[2];  // this CTA's {rr hi, rr lo, hw hi, hw lo}, by turns
+  __shared__ float4 s_small[4 * kHpSmallN / 64];  // a small proposal's, per part and warp
   const int NFFT = a.NFFT;
   dc *S = reinterpret_cast<dc *>(smem_raw);
   const int r = (int)cluster.block_rank(), ch = r >> 1;
@@ -252,8 +266,30 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     if ((32 << b) <= NFFT) total += a.bin_count[b];
   }
   if (total == 0) return;  // nothing listed: the counters are zero already
+  // the bank's entries of bin q of channel c
+  struct Bin {
+    float4 gh, gl, wh, wl;
+  };
+  auto load_bin = [&](const HpEntry &e, int N, int c, int q, Bin &t) {
+    const int j = e.imin + ((q + (N >> 1)) & (N - 1));  // fftshift
+    if (j < 0 || j >= NFFT) return false;
+    const size_t sj = (size_t)e.seg * NFFT + j;
+    t = {a.g32[2 * sj + c], a.g32lo[2 * sj + c], a.w32[sj], a.w32lo[sj]};
+    return true;
+  };
+  // residual and template power of a bin from the channel's two spectra there
+  auto add_bin = [&](const HpEntry &e, const Bin &t, int c, dc s0, dc s1, df &rr, df &hw) {
+    dc h = dc_add(dc_mul(s0, dc_from(make_float2(t.gh.x, t.gh.y), make_float2(t.gl.x, t.gl.y))),
+                  dc_mul(s1, dc_from(make_float2(t.gh.z, t.gh.w), make_float2(t.gl.z, t.gl.w))));
+    h = dc_scale2(h, e.amp_p2);
+    const dc w = c == 0 ? dc_from(make_float2(t.wh.x, t.wh.y), make_float2(t.wl.x, t.wl.y))
+                        : dc_from(make_float2(t.wh.z, t.wh.w), make_float2(t.wl.z, t.wl.w));
+    rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
+    hw = df_add(hw, df_sq_sum(h));
+  };
+  const int nbig = cs[kHpSmallBins - 1];  // entries of more than kHpSmallN points come first
   int turn = 0;
-  for (int k = (int)(blockIdx.x >> 2); k < total; k += ncl, turn ^= 1) {
+  for (int k = (int)(blockIdx.x >> 2); k < nbig; k += ncl, turn ^= 1) {
     const HpEntry e = hp_entry(a, k, cs);
     const int N = e.N, ln = e.bin + 5;
     const float4 *src = a.series + e.off + (long long)r * N;
@@ -266,20 +302,10 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
       for (int u = 0; u < 4; u++)
         if (n0 + u * kHpThreads < N) S[hp_at(hp_rev(n0 + u * kHpThreads, ln))] = dc_from(v[u]);
     }
-    // the bank's entries of bin q of this CTA's half
+    // bins of this CTA's half
     const int half = N >> 1, q0 = (r & 1) * half;
-    struct Bin {
-      float4 gh, gl, wh, wl;
-    };
-    auto load_bin = [&](int q, Bin &t) {
-      const int j = e.imin + ((q + half) & (N - 1));  // fftshift
-      if (q >= q0 + half || j < 0 || j >= NFFT) return false;
-      const size_t sj = (size_t)e.seg * NFFT + j;
-      t = {a.g32[2 * sj + ch], a.g32lo[2 * sj + ch], a.w32[sj], a.w32lo[sj]};
-      return true;
-    };
     Bin t;
-    bool has = load_bin(q0 + (int)threadIdx.x, t);
+    bool has = (int)threadIdx.x < half && load_bin(e, N, ch, q0 + (int)threadIdx.x, t);
     __syncthreads();
     hp_fft(S, ln, a.tw32x[e.bin]);
     cluster.sync();  // every spectrum of the proposal is complete
@@ -288,17 +314,8 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     df rr = {0.f, 0.f}, hw = {0.f, 0.f};
     for (int q = q0 + threadIdx.x; q < q0 + half; q += blockDim.x) {
       Bin next;
-      const bool has_next = load_bin(q + kHpThreads, next);
-      if (has) {
-        const int qs = hp_at(q);
-        dc h = dc_add(dc_mul(S0[qs], dc_from(make_float2(t.gh.x, t.gh.y), make_float2(t.gl.x, t.gl.y))),
-                      dc_mul(S1[qs], dc_from(make_float2(t.gh.z, t.gh.w), make_float2(t.gl.z, t.gl.w))));
-        h = dc_scale2(h, e.amp_p2);
-        const dc w = ch == 0 ? dc_from(make_float2(t.wh.x, t.wh.y), make_float2(t.wl.x, t.wl.y))
-                             : dc_from(make_float2(t.wh.z, t.wh.w), make_float2(t.wl.z, t.wl.w));
-        rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
-        hw = df_add(hw, df_sq_sum(h));
-      }
+      const bool has_next = q + kHpThreads < q0 + half && load_bin(e, N, ch, q + kHpThreads, next);
+      if (has) add_bin(e, t, ch, S0[hp_at(q)], S1[hp_at(q)], rr, hw);
       t = next;
       has = has_next;
     }
@@ -319,8 +336,58 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     // the next proposal's sums go to the other s_part, the one after it follows
     // two more cluster barriers
   }
-  cluster.sync();  // no CTA leaves while CTA 0 may be reading its s_part
+  if ((int)(blockIdx.x >> 2) < nbig) cluster.sync();  // CTA 0 has read every s_part
+  // small proposals, first on the CTAs that had no large one
+  for (int k = nbig + (int)(gridDim.x - 1 - blockIdx.x); k < total; k += (int)gridDim.x) {
+    const HpEntry e = hp_entry(a, k, cs);
+    const int N = e.N, ln = e.bin + 5, half = N >> 1, tid = threadIdx.x;
+    const float4 *src = a.series + e.off;
+    for (int n = tid; n < 4 * N; n += kHpThreads)
+      S[hp_at((n & ~(N - 1)) + hp_rev(n & (N - 1), ln))] = dc_from(src[n]);
+    // part (channel, half of the bins) and bin of item i
+    auto part = [&](int i) { return i >> (ln - 1); };
+    auto bin = [&](int i) { return i & (N - 1); };
+    Bin t;
+    bool has = tid < 2 * N && load_bin(e, N, part(tid) >> 1, bin(tid), t);
+    __syncthreads();
+    hp_fft4(S, ln, a.tw32x[e.bin]);
+    const int g = half < 32 ? half : 32;  // lanes of a part's partial sum
+    for (int i = tid; i < 2 * N; i += kHpThreads) {  // whole warps
+      Bin next;
+      const bool has_next = i + kHpThreads < 2 * N && load_bin(e, N, part(i + kHpThreads) >> 1, bin(i + kHpThreads), next);
+      const int c = part(i) >> 1, q = bin(i);
+      df rr = {0.f, 0.f}, hw = {0.f, 0.f};
+      if (has) add_bin(e, t, c, S[hp_at(2 * c * N + q)], S[hp_at((2 * c + 1) * N + q)], rr, hw);
+      for (int off = g >> 1; off > 0; off >>= 1) {
+        const df ro = {__shfl_xor_sync(0xffffffffu, rr.hi, off), __shfl_xor_sync(0xffffffffu, rr.lo, off)};
+        const df ho = {__shfl_xor_sync(0xffffffffu, hw.hi, off), __shfl_xor_sync(0xffffffffu, hw.lo, off)};
+        rr = df_add(rr, ro);
+        hw = df_add(hw, ho);
+      }
+      if ((i & (g - 1)) == 0) s_small[i / g] = make_float4(rr.hi, rr.lo, hw.hi, hw.lo);
+      t = next;
+      has = has_next;
+    }
+    __syncthreads();  // the sums are published, and S is free
+    if (tid == 0 && e.ok) {
+      const int nw = half / g;
+      df s[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+      for (int p = 0; p < 4; p++) {
+        df rr = {0.f, 0.f}, hw = {0.f, 0.f};
+        for (int w = 0; w < nw; w++) {
+          const float4 o = s_small[p * nw + w];
+          rr = df_add(rr, df{o.x, o.y});
+          hw = df_add(hw, df{o.z, o.w});
+        }
+        s[p >> 1] = df_add(s[p >> 1], rr);
+        s[2] = df_add(s[2], hw);
+      }
+      hp_write(e.item, N, e.seg, e.imin, NFFT, s, a.Q, a.QA, PERCH, a.term_x, a.dlogl, a.term_y, a.hh, a.term_ch,
+               a.status);
+    }
+  }
   // the last CTA leaves the counters it was given at zero
+  __syncthreads();  // this one has read them
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(a.done, 1) == (int)gridDim.x - 1) {
@@ -330,7 +397,9 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   }
 }
 
-static size_t hp_smem_bytes(int nmax) { return (size_t)nmax * sizeof(dc); }
+static size_t hp_smem_bytes(int nmax) {
+  return (size_t)(nmax > 4 * kHpSmallN ? nmax : 4 * kHpSmallN) * sizeof(dc);
+}
 
 template <bool PERCH>
 static cudaError_t launch_hp(const HpArgs &a, int num_sms, cudaStream_t stream) {

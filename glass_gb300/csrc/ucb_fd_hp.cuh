@@ -133,6 +133,20 @@ __device__ __forceinline__ int hp_rev(int n, int ln) {
   const unsigned r = __brev((unsigned)m) >> (32 - l4);
   return top + (int)(((r & 0x55555555u) << 1) | ((r >> 1) & 0x55555555u));
 }
+// A radix-4 butterfly (w1, w2, w3: its factors, where it has any).
+__device__ __forceinline__ void hp_radix4(dc *x0, dc *x1, dc *x2, dc *x3, dc u0, dc u1, dc u2, dc u3, bool factors,
+                                          float4 w1, float4 w2, float4 w3) {
+  if (factors) {
+    u1 = dc_mul(u1, dc_from(w1));
+    u2 = dc_mul(u2, dc_from(w2));
+    u3 = dc_mul(u3, dc_from(w3));
+  }
+  const dc a = dc_add(u0, u2), b = dc_sub(u0, u2), c = dc_add(u1, u3), d = dc_mi(dc_sub(u1, u3));
+  *x0 = dc_add(a, c);
+  *x1 = dc_add(b, d);
+  *x2 = dc_sub(a, c);
+  *x3 = dc_sub(b, d);
+}
 // The twiddles of a thread's next butterfly (of its next stage, after the last of
 // one) are loaded before the arithmetic of the current one: each is used once per
 // series, so every load is a trip to L2.
@@ -160,16 +174,7 @@ __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__
       } else if (lq < ln) {
         w[0] = tw[in];  // the radix-2 stage's first
       }
-      if (lp > 0) {
-        u1 = dc_mul(u1, dc_from(w1));
-        u2 = dc_mul(u2, dc_from(w2));
-        u3 = dc_mul(u3, dc_from(w3));
-      }
-      const dc a = dc_add(u0, u2), b = dc_sub(u0, u2), c = dc_add(u1, u3), d = dc_mi(dc_sub(u1, u3));
-      *x0 = dc_add(a, c);
-      *x1 = dc_add(b, d);
-      *x2 = dc_sub(a, c);
-      *x3 = dc_sub(b, d);
+      hp_radix4(x0, x1, x2, x3, u0, u1, u2, u3, lp > 0, w1, w2, w3);
     }
     __syncthreads();
   }
@@ -180,6 +185,44 @@ __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__
       const float4 w1 = w[0];
       if (k + (int)blockDim.x < N / 2) w[0] = tw[k + blockDim.x];
       const dc a = *x0, b = dc_mul(*x1, dc_from(w1));
+      *x0 = dc_add(a, b);
+      *x1 = dc_sub(a, b);
+    }
+    __syncthreads();
+  }
+}
+
+// The same of four series of N = 2^ln points, back to back (element n of series s at
+// hp_at(s N + hp_rev(n, ln))), N at most the CTA's threads: one butterfly per thread
+// and stage.
+__device__ __forceinline__ void hp_fft4(dc *x, int ln, const float4 *__restrict__ tw) {
+  const int N = 1 << ln, t = threadIdx.x, i = t & (N / 4 - 1), base = (t - i) << 2;
+  const bool odd = ln & 1;
+  float4 w[3] = {}, wl = {};
+  if (odd && t < 2 * N) wl = tw[t & (N / 2 - 1)];  // the radix-2 stage's
+  int lp = 0;
+  for (; lp + 2 <= ln; lp += 2) {
+    if (t < N) {
+      const int p = 1 << lp, k = i & (p - 1), j = base + ((i - k) << 2) + k;
+      dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + p), *const x2 = x + hp_at(j + 2 * p),
+               *const x3 = x + hp_at(j + 3 * p);
+      const dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
+      const float4 w1 = w[0], w2 = w[1], w3 = w[2];
+      if (lp + 4 <= ln) {
+        const int kn = (i & (4 * p - 1)) << (ln - lp - 4);
+        w[0] = tw[kn];
+        w[1] = tw[2 * kn];
+        w[2] = tw[3 * kn];
+      }
+      hp_radix4(x0, x1, x2, x3, u0, u1, u2, u3, lp > 0, w1, w2, w3);
+    }
+    __syncthreads();
+  }
+  if (odd) {
+    if (t < 2 * N) {
+      const int k = t & (N / 2 - 1), j = 2 * (t - k) + k;
+      dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + N / 2);
+      const dc a = *x0, b = dc_mul(*x1, dc_from(wl));
       *x0 = dc_add(a, b);
       *x1 = dc_sub(a, b);
     }
