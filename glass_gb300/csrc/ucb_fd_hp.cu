@@ -23,7 +23,8 @@
 //     (read through distributed shared memory), each over half of the bins,
 //     and sum the residual power and the template power; CTA 0 gathers the
 //     four partial sums and writes the results over the mixed ones.  Proposals of
-//     up to 256 points take one CTA each, with the same sums.
+//     up to 256 points, and of 512 where clusters would queue, take one CTA each,
+//     with the same sums.
 // What is left is of order 1e-12 of the same scale.
 #include <math.h>
 
@@ -185,9 +186,10 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
   }
 }
 
-// Proposals of up to this many points take one CTA each.
-constexpr int kHpSmallBins = 4;  // N = 32 << b, b < 4
-constexpr int kHpSmallN = 32 << (kHpSmallBins - 1);
+// Proposals of up to 256 points (sizes b < kHpSmallBins, 32 << b) take one CTA each,
+// those of 512 too where more of 512 points and above are listed than clusters.
+constexpr int kHpSmallBins = 4;
+constexpr int kHpSmallMax = 32 << kHpSmallBins;
 
 // ------------------------------------------------------- spectral stage, df
 // The proposal of entry k (largest sizes first, so that the long ones start
@@ -242,8 +244,11 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // holds a proposal's four series and has a butterfly of a stage per thread, as
 // a cluster has, without its barriers: 296 at once (series and transform of 3000
 // proposals of 32 points 217 -> 66 us, of 600 of 128 points 72 -> 39; with ping-pong
-// buffers and 114 clusters resident they took 143 and 59).  The sums keep the
-// clusters' order: a partial one per channel and half of the bins, bins over
+// buffers and 114 clusters resident they took 143 and 59).  At 512 points a CTA takes
+// two butterflies per thread and stage: longer for one proposal, but without the
+// clusters' idle half and waits more of them in a given time, so these take
+// CTAs where more are listed than clusters fit (3000: 618 -> 485 us, 100: 34.8 ->
+// 32.8; 60 stay at 24.6).  The sums keep the clusters' order: a partial one per channel and half of the bins, bins over
 // lanes, lanes by halving distances, then warps in turn.
 template <bool PERCH>
 __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 red[32];
   __shared__ float4 s_part[2];  // this CTA's {rr hi, rr lo, hw hi, hw lo}, by turns
-  __shared__ float4 s_small[4 * kHpSmallN / 64];  // a small proposal's, per part and warp
+  __shared__ float4 s_small[4 * kHpSmallMax / 64];  // a small proposal's, per part and warp
   const int NFFT = a.NFFT;
   dc *S = reinterpret_cast<dc *>(smem_raw);
   const int r = (int)cluster.block_rank(), ch = r >> 1;
@@ -287,7 +292,8 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     rr = df_add(rr, df_sq_sum(dc_sub(w, h)));
     hw = df_add(hw, df_sq_sum(h));
   };
-  const int nbig = cs[kHpSmallBins - 1];  // entries of more than kHpSmallN points come first
+  // the large entries come first
+  const int nbig = cs[kHpSmallBins - 1] > ncl ? cs[kHpSmallBins] : cs[kHpSmallBins - 1];
   int turn = 0;
   for (int k = (int)(blockIdx.x >> 2); k < nbig; k += ncl, turn ^= 1) {
     const HpEntry e = hp_entry(a, k, cs);
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     Bin t;
     bool has = tid < 2 * N && load_bin(e, N, part(tid) >> 1, bin(tid), t);
     __syncthreads();
-    hp_fft4(S, ln, a.tw32x[e.bin]);
+    hp_fft<4>(S, ln, a.tw32x[e.bin]);
     const int g = half < 32 ? half : 32;  // lanes of a part's partial sum
     for (int i = tid; i < 2 * N; i += kHpThreads) {  // whole warps
       Bin next;
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
 }
 
 static size_t hp_smem_bytes(int nmax) {
-  return (size_t)(nmax > 4 * kHpSmallN ? nmax : 4 * kHpSmallN) * sizeof(dc);
+  return (size_t)(nmax > 4 * kHpSmallMax ? nmax : 4 * kHpSmallMax) * sizeof(dc);
 }
 
 template <bool PERCH>

@@ -111,10 +111,11 @@ __device__ __forceinline__ df df_sinc(df x, const float4 *tab) {
   return df_div(s, x);
 }
 
-// In-place FFT of one series of N = 2^ln double-floats by the CTA: decimation in
-// time from digit-reversed order (element n at hp_at(hp_rev(n, ln))), radix-4
-// stages (sub-transform size p: butterfly i < N/4, k = i mod p, on x[4 (i - k) + k
-// + m p] times exp(-2 pi i m k / (4p)), m = 0..3) and a final radix-2 stage when
+// In-place FFT of NSER series of N = 2^ln double-floats, back to back, by the CTA:
+// decimation in time from digit-reversed order (element n of series s at hp_at(s N +
+// hp_rev(n, ln))), radix-4 stages (sub-transform size p: butterfly i < NSER N/4, k =
+// i mod p, on x[4 (i - k) + k + m p] times exp(-2 pi i m k / (4p)), m = 0..3) and a
+// final radix-2 stage when
 // log2 N is odd; results in natural order at hp_at.  tw[j] = exp(-2 pi i j / N) as
 // hi + lo floats, read from global memory (L1 after the first touch): 16 bytes of
 // shared memory per point.
@@ -150,19 +151,20 @@ __device__ __forceinline__ void hp_radix4(dc *x0, dc *x1, dc *x2, dc *x3, dc u0,
 // The twiddles of a thread's next butterfly (of its next stage, after the last of
 // one) are loaded before the arithmetic of the current one: each is used once per
 // series, so every load is a trip to L2.
+template <int NSER = 1>
 __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__ tw) {
-  const int N = 1 << ln;
+  const int N = 1 << ln, Q = NSER * N / 4;  // Q radix-4 butterflies a stage
   float4 w[3] = {};
   int lp = 0;
   for (; lp + 2 <= ln; lp += 2) {
     const int p = 1 << lp;
-    for (int i = threadIdx.x; i < N / 4; i += blockDim.x) {
+    for (int i = threadIdx.x; i < Q; i += blockDim.x) {
       const int k = i & (p - 1), j = ((i - k) << 2) + k;
       dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + p), *const x2 = x + hp_at(j + 2 * p),
                *const x3 = x + hp_at(j + 3 * p);
-      dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
+      const dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
       const float4 w1 = w[0], w2 = w[1], w3 = w[2];
-      const bool last = i + (int)blockDim.x >= N / 4;
+      const bool last = i + (int)blockDim.x >= Q;
       const int lq = last ? lp + 2 : lp, in = last ? (int)threadIdx.x : i + (int)blockDim.x;
       if (lq + 2 <= ln) {
         const int kn = (in & ((1 << lq) - 1)) << (ln - lq - 2);
@@ -172,57 +174,20 @@ __device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__
           w[2] = tw[3 * kn];
         }
       } else if (lq < ln) {
-        w[0] = tw[in];  // the radix-2 stage's first
+        w[0] = tw[in & (N / 2 - 1)];  // the radix-2 stage's first
       }
       hp_radix4(x0, x1, x2, x3, u0, u1, u2, u3, lp > 0, w1, w2, w3);
     }
     __syncthreads();
   }
   if (lp < ln) {  // log2 N odd: one radix-2 stage, p = N/2
-    if ((int)threadIdx.x >= N / 4 && (int)threadIdx.x < N / 2) w[0] = tw[threadIdx.x];
-    for (int k = threadIdx.x; k < N / 2; k += blockDim.x) {
-      dc *const x0 = x + hp_at(k), *const x1 = x + hp_at(k + N / 2);
-      const float4 w1 = w[0];
-      if (k + (int)blockDim.x < N / 2) w[0] = tw[k + blockDim.x];
-      const dc a = *x0, b = dc_mul(*x1, dc_from(w1));
-      *x0 = dc_add(a, b);
-      *x1 = dc_sub(a, b);
-    }
-    __syncthreads();
-  }
-}
-
-// The same of four series of N = 2^ln points, back to back (element n of series s at
-// hp_at(s N + hp_rev(n, ln))), N at most the CTA's threads: one butterfly per thread
-// and stage.
-__device__ __forceinline__ void hp_fft4(dc *x, int ln, const float4 *__restrict__ tw) {
-  const int N = 1 << ln, t = threadIdx.x, i = t & (N / 4 - 1), base = (t - i) << 2;
-  const bool odd = ln & 1;
-  float4 w[3] = {}, wl = {};
-  if (odd && t < 2 * N) wl = tw[t & (N / 2 - 1)];  // the radix-2 stage's
-  int lp = 0;
-  for (; lp + 2 <= ln; lp += 2) {
-    if (t < N) {
-      const int p = 1 << lp, k = i & (p - 1), j = base + ((i - k) << 2) + k;
-      dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + p), *const x2 = x + hp_at(j + 2 * p),
-               *const x3 = x + hp_at(j + 3 * p);
-      const dc u0 = *x0, u1 = *x1, u2 = *x2, u3 = *x3;
-      const float4 w1 = w[0], w2 = w[1], w3 = w[2];
-      if (lp + 4 <= ln) {
-        const int kn = (i & (4 * p - 1)) << (ln - lp - 4);
-        w[0] = tw[kn];
-        w[1] = tw[2 * kn];
-        w[2] = tw[3 * kn];
-      }
-      hp_radix4(x0, x1, x2, x3, u0, u1, u2, u3, lp > 0, w1, w2, w3);
-    }
-    __syncthreads();
-  }
-  if (odd) {
-    if (t < 2 * N) {
-      const int k = t & (N / 2 - 1), j = 2 * (t - k) + k;
+    if ((int)threadIdx.x >= Q && (int)threadIdx.x < 2 * Q) w[0] = tw[threadIdx.x & (N / 2 - 1)];
+    for (int i = threadIdx.x; i < 2 * Q; i += blockDim.x) {
+      const int k = i & (N / 2 - 1), j = ((i - k) << 1) + k;
       dc *const x0 = x + hp_at(j), *const x1 = x + hp_at(j + N / 2);
-      const dc a = *x0, b = dc_mul(*x1, dc_from(wl));
+      const float4 w1 = w[0];
+      if (i + (int)blockDim.x < 2 * Q) w[0] = tw[(i + blockDim.x) & (N / 2 - 1)];
+      const dc a = *x0, b = dc_mul(*x1, dc_from(w1));
       *x0 = dc_add(a, b);
       *x1 = dc_sub(a, b);
     }

@@ -1,5 +1,6 @@
 """The double-float re-evaluation of more proposals than are resident at once: small
-ones (a CTA each) and large ones (a cluster each) of one batch, per channel, clipped
+ones (a CTA each, at 512 points where clusters would queue) and large ones (a cluster
+each) of one batch, per channel, clipped
 by the segment's edges; and how its time grows with their number.  A proposal's
 results are the same bits as alone (whose accuracy the re-evaluation's edge tests
 check at every size).
@@ -70,16 +71,17 @@ def test_mixed_sizes(engine, NFFT):
         engine.set_mixed_tolerance(1e-3)
 
 
-def test_time_of_many_small_ones(engine):
-    """3000 templates of 32 points: 4 times the time of 60, which are resident at once;
-    12 times where each takes a cluster of its own (7 with 114 clusters resident
-    instead of 74)."""
+@pytest.mark.parametrize("N,most", [(32, 6.5), (512, 22.5)])
+def test_time_of_many(engine, N, most):
+    """3000 templates against 60, which are resident at once, of 32 and 512 points: 4 and
+    20 times the time; 12 and 25 times where each takes a cluster (7 and 21 with
+    114 clusters resident instead of 74)."""
     rng = np.random.default_rng(1)
     _upload(engine, rng, 1024)
     dev = lambda x: torch.tensor(x, device="cuda")
     us = {}
     try:
-        engine.set_template_size(32)
+        engine.set_template_size(N)
         engine.set_mixed_tolerance(1e-15)
         engine.set_phase_timing(True)
         for n in (60, 3000):
@@ -96,4 +98,4 @@ def test_time_of_many_small_ones(engine):
         engine.set_phase_timing(False)
         engine.set_mixed_tolerance(1e-3)
         engine.set_template_size(0)
-    assert us[3000] < 6.5 * us[60], us
+    assert us[3000] < most * us[60], us
