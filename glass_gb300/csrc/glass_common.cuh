@@ -104,7 +104,8 @@ inline cudaError_t smem_limit(size_t most) {
 // start of each, the waiting CTAs take room from the running kernel's
 // neighbours, and a batch that took 89 us without chaining took 102.)
 template <typename... P, typename... A>
-inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A... args) {
+inline cudaError_t launch_after(bool chained, void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream,
+                                A... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -114,8 +115,12 @@ inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, int block, size_t 
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, k, args...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, int block, size_t smem, cudaStream_t stream, A... args) {
+  return launch_after(true, k, grid, block, smem, stream, args...);
 }
 __device__ __forceinline__ void grid_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -724,6 +724,16 @@ cudaError_t fd_dlogl_launch(const FdBankDev &bank, const FdTablesDev &tab, FdWor
     A.nbins = nall;
     A.zero_counts = nb == 0 ? work.bin_count : nullptr;  // side kernels would still be reading them
     A.done = work.bin_count + kNumBins + 1;  // fb_count is at kNumBins
+    // In a graph a chained launch starts ahead of the size kernels on its side
+    // branches, which suits a light batch (1000 proposals of at most 1024 points on
+    // 2048 bins 35 -> 29 us) but not a large one whose size kernels end it, as with the
+    // re-evaluation off: 10000 of up to 2048 points 1063 us after an ordinary launch,
+    // 1115 chained, 3000 343 and 361; 3000 light ones 45.6 and 43.5.
+    if (nb > 0 && mix && !fallback && nitems > 1024) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      if ((e = cudaStreamIsCapturing(stream, &cs)) != cudaSuccess) return e;
+      A.chained = cs != cudaStreamCaptureStatusActive;
+    }
     for (int b = 0; b < kSpecAllBins; b++) A.tw[b] = mix ? (const void *)tab.tw32x[b] : (const void *)tab.tt64[b];
     e = mix ? fd_launch_spec_all_mixed(A, num_sms, stream, perch, work.tune.spec_ctas_per_sm)
             : fd_launch_spec_all_fp64(A, num_sms, stream, perch);

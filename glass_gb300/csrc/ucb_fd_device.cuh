@@ -1869,6 +1869,7 @@ struct SpecAllArgs {
   int nbins;                     // sizes 32 << b for b < nbins
   int *zero_counts;              // non-null: the last CTA to finish zeroes the kNumBins counts there
   int *done = nullptr;           // CTA-done counter (zero between launches)
+  bool chained = true;           // launched as launch_chained does
 };
 
 // The spectral stage of a few FP64 proposals (ucb_fd_fp64.cu).
@@ -1994,8 +1995,8 @@ static cudaError_t launch_spec_all(const SpecAllArgs &A, int num_sms, cudaStream
   }, &occ);
   if (e != cudaSuccess) return e;
   if (cap > 0 && cap < occ) occ = cap;
-  return launch_chained(fd_spec_all_kernel<MIX, PERCH>, grid_for(occ * num_sms, A.a.nitems), kSpecAllThreads, smem,
-                        stream, A);
+  return launch_after(A.chained, fd_spec_all_kernel<MIX, PERCH>, grid_for(occ * num_sms, A.a.nitems), kSpecAllThreads,
+                      smem, stream, A);
 }
 
 // Launch of one size's kernel with a grid bounded by the SM count times the
