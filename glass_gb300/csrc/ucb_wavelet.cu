@@ -41,6 +41,7 @@
 // spline systems' factorisations) is built once per grid on the host.
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <algorithm>
 
@@ -1111,11 +1112,15 @@ static int node_below(const double *x, int n, double v) {
   return (int)(std::upper_bound(x, x + n, v) - x) - 1;
 }
 
-static double host_eval(const HostSpline &sp, double v) {
+// The same for a v near the last one, whose node j holds.
+static int node_near(const double *x, int n, double v, int &j) {
+  if (!(j + 1 < n && x[j] <= v && v < x[j + 1])) j = node_below(x, n, v);
+  return j;
+}
+
+// The spline at x[j] + d (splines of the same nodes share the search for j).
+static double host_eval(const HostSpline &sp, int j, double d) {
   const int n = sp.n;
-  const double *x = sp.x;
-  const int j = node_below(x, n, v);
-  const double d = v - x[j];
   const double *c = sp.c.data();
   return c[j] + c[n + j] * d + c[2 * n + j] * d * d + c[3 * n + j] * d * d * d;
 }
@@ -1200,8 +1205,9 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
   std::vector<double> geo(21 * (size_t)norb);
   for (int m = 0; m < norb; m++) {
     double x[3][3], nv[3][3], L[3];
+    const int j = node_below(h.orb_t.data(), norb, tssb[m]);
     for (int i = 0; i < 3; i++)
-      for (int d = 0; d < 3; d++) x[i][d] = host_eval(pos[3 * i + d], tssb[m]) / kCLIGHT;
+      for (int d = 0; d < 3; d++) x[i][d] = host_eval(pos[3 * i + d], j, tssb[m] - h.orb_t[j]) / kCLIGHT;
     for (int d = 0; d < 3; d++) {
       nv[0][d] = x[1][d] - x[2][d];
       nv[1][d] = x[2][d] - x[0][d];
@@ -1234,15 +1240,16 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
   for (int nl = 1; nl <= kWvMaxLayers; nl++) {
     const int Nds = NT * (nl + 1);
     const double dtds = h.wdt / (double)(nl + 1);
+    int j = 0, jb = 0;  // intervals of the orbit's and of the TDI splines (their binary_search's)
     r0[nl].resize(3 * (size_t)Nds);
     tds[nl].resize(Nds);
     dds[nl].resize(Nds);
     jds[nl].resize(Nds);
     for (int i = 0; i < Nds; i++) {
       const double t = h.t0 + i * dtds;
-      for (int d = 0; d < 3; d++) r0[nl][3 * (size_t)i + d] = host_eval(pos[d], t) / kCLIGHT;
-      // the TDI splines' interval, as their binary_search finds it
-      const int jb = node_below(tssb.data(), norb, t);
+      node_near(h.orb_t.data(), norb, t, j);
+      for (int d = 0; d < 3; d++) r0[nl][3 * (size_t)i + d] = host_eval(pos[d], j, t - h.orb_t[j]) / kCLIGHT;
+      node_near(tssb.data(), norb, t, jb);
       tds[nl][i] = t;
       dds[nl][i] = t - tssb[jb];
       jds[nl][i] = jb;
@@ -1277,11 +1284,13 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
   cudaError_t e = cudaMalloc((void **)&base, bytes);
   if (e != cudaSuccess) return e;
   *mem = base;
-  char *p = base;
+  // the tables side by side on the host, for one copy
+  std::vector<char> host(bytes);
+  size_t at = 0;
   auto put = [&](const void *src, size_t b) -> const void * {
-    void *dst = p;
-    p += pad(b);
-    e = e != cudaSuccess ? e : cudaMemcpyAsync(dst, src, b, cudaMemcpyHostToDevice, s);
+    memcpy(host.data() + at, src, b);
+    void *dst = base + at;
+    at += pad(b);
     return dst;
   };
   g->orb_t = (const double *)put(h.orb_t.data(), 8 * (size_t)norb);
@@ -1313,7 +1322,7 @@ cudaError_t wv_build_grid(const WvGridHost &h, WvGridDev *g, void **mem, cudaStr
     g->dds[nl] = (const double *)put(dds[nl].data(), 8 * dds[nl].size());
     g->jds[nl] = (const int *)put(jds[nl].data(), 4 * jds[nl].size());
   }
-  if (e != cudaSuccess) return e;
+  if ((e = cudaMemcpyAsync(base, host.data(), bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
   g->NF = h.NF;
   g->NT = NT;
   g->norb = norb;
