@@ -243,13 +243,14 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // The registers that takes leave 74 clusters resident.  Up to 256 points one CTA
 // holds a proposal's four series and has a butterfly of a stage per thread, as
 // a cluster has, without its barriers: 296 at once (series and transform of 3000
-// proposals of 32 points 217 -> 66 us, of 600 of 128 points 72 -> 39; with ping-pong
+// proposals of 32 points 217 -> 72 us, of 600 of 128 points 72 -> 41; with ping-pong
 // buffers and 114 clusters resident they took 143 and 59).  At 512 points a CTA takes
 // two butterflies per thread and stage: longer for one proposal, but without the
 // clusters' idle half and waits more of them in a given time, so these take
-// CTAs where more are listed than clusters fit (3000: 618 -> 485 us, 100: 34.8 ->
-// 32.8; 60 stay at 24.6).  The sums keep the clusters' order: a partial one per channel and half of the bins, bins over
-// lanes, lanes by halving distances, then warps in turn.
+// CTAs where more are listed than clusters fit (3000: 618 -> 495 us, 100: 34.8 ->
+// 32.8; 60 stay at 24.6).  The sums keep the clusters' order: a partial one per
+// channel and half of the bins, bins over lanes, lanes by halving distances, then
+// warps in turn.
 template <bool PERCH>
 __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
   namespace cg = cooperative_groups;
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     Bin t;
     bool has = (int)threadIdx.x < half && load_bin(e, N, ch, q0 + (int)threadIdx.x, t);
     __syncthreads();
-    hp_fft(S, ln, a.tw32x[e.bin]);
+    hp_fft(S, ln, 1, a.tw32x[e.bin]);
     cluster.sync();  // every spectrum of the proposal is complete
     const dc *Sp = cluster.map_shared_rank(S, (unsigned)(r ^ 1));
     const dc *S0 = (r & 1) ? Sp : S, *S1 = (r & 1) ? S : Sp;  // the channel's series 2c, 2c + 1
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     Bin t;
     bool has = tid < 2 * N && load_bin(e, N, part(tid) >> 1, bin(tid), t);
     __syncthreads();
-    hp_fft<4>(S, ln, a.tw32x[e.bin]);
+    hp_fft(S, ln, 4, a.tw32x[e.bin]);
     const int g = half < 32 ? half : 32;  // lanes of a part's partial sum
     for (int i = tid; i < 2 * N; i += kHpThreads) {  // whole warps
       Bin next;

@@ -111,14 +111,13 @@ __device__ __forceinline__ df df_sinc(df x, const float4 *tab) {
   return df_div(s, x);
 }
 
-// In-place FFT of NSER series of N = 2^ln double-floats, back to back, by the CTA:
+// In-place FFT of nser series of N = 2^ln double-floats, back to back, by the CTA:
 // decimation in time from digit-reversed order (element n of series s at hp_at(s N +
-// hp_rev(n, ln))), radix-4 stages (sub-transform size p: butterfly i < NSER N/4, k =
+// hp_rev(n, ln))), radix-4 stages (sub-transform size p: butterfly i < nser N/4, k =
 // i mod p, on x[4 (i - k) + k + m p] times exp(-2 pi i m k / (4p)), m = 0..3) and a
-// final radix-2 stage when
-// log2 N is odd; results in natural order at hp_at.  tw[j] = exp(-2 pi i j / N) as
-// hi + lo floats, read from global memory (L1 after the first touch): 16 bytes of
-// shared memory per point.
+// final radix-2 stage when log2 N is odd; results in natural order at hp_at.  tw[j] =
+// exp(-2 pi i j / N) as hi + lo floats, read from global memory (L1 after the first
+// touch): 16 bytes of shared memory per point.
 //
 // hp_at: a 16-byte access serves 8 lanes at a time, one per 16-byte column; the
 // permutation within each run of 8 elements puts the strides of the first stages
@@ -150,10 +149,11 @@ __device__ __forceinline__ void hp_radix4(dc *x0, dc *x1, dc *x2, dc *x3, dc u0,
 }
 // The twiddles of a thread's next butterfly (of its next stage, after the last of
 // one) are loaded before the arithmetic of the current one: each is used once per
-// series, so every load is a trip to L2.
-template <int NSER = 1>
-__device__ __forceinline__ void hp_fft(dc *x, int ln, const float4 *__restrict__ tw) {
-  const int N = 1 << ln, Q = NSER * N / 4;  // Q radix-4 butterflies a stage
+// series, so every load is a trip to L2.  One copy for clusters and single CTAs: with
+// a copy each, fetching the kernel's instructions cost a step that starts with cold
+// caches 0.9 us.
+static __device__ __noinline__ void hp_fft(dc *x, int ln, int nser, const float4 *__restrict__ tw) {
+  const int N = 1 << ln, Q = nser * N / 4;  // Q radix-4 butterflies a stage
   float4 w[3] = {};
   int lp = 0;
   for (; lp + 2 <= ln; lp += 2) {
