@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(96) fd_slow_hp_kernel(SlowArgs a) {
 }
 
 // Proposals of up to 256 points (sizes b < kHpSmallBins, 32 << b) take one CTA each,
-// those of 512 too where more of 512 points and above are listed than clusters.
+// those of 512 too where the clusters are too few and either every one finds a CTA
+// beside the larger ones' clusters or the batch is several waves long.
 constexpr int kHpSmallBins = 4;
 constexpr int kHpSmallMax = 32 << kHpSmallBins;
 
@@ -248,7 +249,9 @@ __device__ __forceinline__ HpEntry hp_entry(const HpArgs &a, int k, const int *c
 // two butterflies per thread and stage: longer for one proposal, but without the
 // clusters' idle half and waits more of them in a given time, so these take
 // CTAs where more are listed than clusters fit (3000: 618 -> 495 us, 100: 34.8 ->
-// 32.8; 60 stay at 24.6).  The sums keep the clusters' order: a partial one per
+// 32.8; 60 stay at 24.6), unless they would come after larger ones on the same SMs (70 of
+// 1024 points and 23 of 512: 44.7 us as clusters, 51.2 as CTAs; 53 and 40: 42.9 and 40.5) and are
+// too few to make up for their length.  The sums keep the clusters' order: a partial one per
 // channel and half of the bins, bins over lanes, lanes by halving distances, then
 // warps in turn.
 template <bool PERCH>
@@ -294,7 +297,9 @@ __global__ void __launch_bounds__(kHpThreads, 2) fd_hp_kernel(HpArgs a) {
     hw = df_add(hw, df_sq_sum(h));
   };
   // the large entries come first
-  const int nbig = cs[kHpSmallBins - 1] > ncl ? cs[kHpSmallBins] : cs[kHpSmallBins - 1];
+  const int nlarge = cs[kHpSmallBins], n512 = cs[kHpSmallBins - 1] - nlarge;
+  const bool cta512 = nlarge + n512 > ncl && (4 * nlarge + n512 <= 4 * ncl || nlarge + n512 > 4 * ncl);
+  const int nbig = cta512 ? nlarge : nlarge + n512;
   int turn = 0;
   for (int k = (int)(blockIdx.x >> 2); k < nbig; k += ncl, turn ^= 1) {
     const HpEntry e = hp_entry(a, k, cs);

@@ -1,9 +1,8 @@
 """The double-float re-evaluation of more proposals than are resident at once: small
-ones (a CTA each, at 512 points where clusters would queue) and large ones (a cluster
-each) of one batch, per channel, clipped
-by the segment's edges; and how its time grows with their number.  A proposal's
-results are the same bits as alone (whose accuracy the re-evaluation's edge tests
-check at every size).
+ones (a CTA each, at 512 points by number) and large ones (a cluster each) of one batch,
+per channel, clipped by the segment's edges; and how its time grows with their number.
+A proposal's results are the same bits as alone (whose accuracy the re-evaluation's edge
+tests check at every size).
 """
 import numpy as np
 import pytest
@@ -99,3 +98,39 @@ def test_time_of_many(engine, N, most):
         engine.set_mixed_tolerance(1e-3)
         engine.set_template_size(0)
     assert us[3000] < most * us[60], us
+
+
+@pytest.mark.parametrize("n1024,n512,most", [(70, 23, 1.3), (74, 40, 1.41)])
+def test_time_past_one_wave(engine, n1024, n512, most):
+    """Templates of 1024 points that take most clusters, and some of 512, against the
+    larger ones alone: 1.21 and 1.33 times the time where the 512-point ones follow as
+    clusters, 1.39 and 1.49 where a CTA takes one after its share of a larger one."""
+    rng = np.random.default_rng(2)
+    _upload(engine, rng, 1024)
+    dev = lambda x: torch.tensor(x, device="cuda")
+    p, seg = {512: [], 1024: []}, {512: [], 1024: []}
+    while len(p[512]) < n512 or len(p[1024]) < n1024:
+        s = int(rng.integers(3))
+        x = wl.draw_source(rng, F0[s], 10 ** rng.uniform(-23, -20), 1e-17)
+        N = 2 * gg.ucb_bandwidth(wl.LARM, wl.FSTAR, x[0] / T, x[7] / T / T, x[1], np.exp(x[3]), T, 1024)
+        if N in p:
+            p[N].append(x), seg[N].append(s)
+    us = {}
+    try:
+        engine.set_mixed_tolerance(1e-15)
+        engine.set_phase_timing(True)
+        for n in (n1024, n1024 + n512):
+            k = n - n1024
+            ds = dev(np.array(seg[1024][:n1024] + seg[512][:k], np.int32))
+            dp = dev(np.array(p[1024][:n1024] + p[512][:k]))
+            out = [dev(np.zeros(n)) for _ in range(3)] + [dev(np.zeros(n, np.int32))]
+            t = []
+            for _ in range(100):
+                engine.dlogl_device(ds, dp, *out, None, gg.PREC_MIXED)
+                torch.cuda.synchronize()
+                t.append(engine.last_phase_ms()[3])
+            us[n] = np.mean(sorted(t[10:])[:70])
+    finally:
+        engine.set_phase_timing(False)
+        engine.set_mixed_tolerance(1e-3)
+    assert us[n1024 + n512] < most * us[n1024], us
