@@ -134,9 +134,30 @@ __constant__ unsigned char kLevelIdx[15][4] = {
     {5, 3, 12, 12}, {1, 5, 12, 12}, {3, 0, 12, 12},  {4, 2, 12, 12}, {6, 7, 12, 12},
     {10, 11, 12, 12}, {9, 8, 12, 12}, {0, 1, 12, 12}, {4, 5, 12, 12}, {3, 2, 12, 12}};
 
-// By the CTA's first warp; the caller synchronises.  fstep: the frequency step
-// between a thread's bins.
-//
+// By the CTA's first warp, the foreground by its second; the caller synchronises.
+// fstep: the frequency step between a thread's bins.
+__device__ __forceinline__ void noise_foreground_load(NoiseModel &M, const double *sg, double fstep) {
+  const int lane = threadIdx.x & 31;
+  const double v = lane < 5 ? sg[lane] : 0.0, x = lane == 2 ? 0.0 : v;
+  const double e = exp(x);
+  const double f2 = __shfl_sync(0xffffffffu, e, 4);
+  if (lane == 0) M.Amp = e;
+  if (lane == 1) {
+    M.l1 = v;
+    M.f10 = e * 10;
+  }
+  if (lane == 2) M.alpha = v;
+  if (lane == 3) M.fk = e;
+  if (lane == 4) {
+    // a step of the sequence by more than e^1 could leave the exponent range
+    // within a thread's bins and not come back
+    const double st = 2.0 * fstep / f2;
+    M.i2 = 2.0 / f2;
+    M.estep = exp(st);
+    M.chain = st < 1.0;
+  }
+}
+
 // At low frequencies the acceleration noise of X + Y + Z cancels to (1 - cos)^2 ~ 1e-7
 // of its terms, for a (12 + 13, 23 + 21, 31 + 32), b (21 + 31, 32 + 12, 13 + 23) and
 // s = q / 2 (12 + 21, 13 + 31, 23 + 32) that obey a_x + b_x = s_xy + s_xz and so on.
@@ -146,8 +167,12 @@ __constant__ unsigned char kLevelIdx[15][4] = {
 // the model does not describe, 4000 bins from 0.1 mHz, link levels a factor of 2 apart: rms error
 // of the likelihood against 80 bits 1.1e-10 -> 1.2e-11 (sums by bin, as the reference: 1.1e-11).
 __device__ __forceinline__ void noise_model_load(NoiseModel &M, const double *in, const double *sg, double fstep) {
-  if (threadIdx.x >= 32) return;
-  const int lane = threadIdx.x;
+  if (threadIdx.x >= 64) return;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x >= 32) {
+    if (sg) noise_foreground_load(M, sg, fstep);
+    return;
+  }
   double lev = 0.0;
   if (lane < 15) {
     double s = 0.0;
@@ -170,26 +195,6 @@ __device__ __forceinline__ void noise_model_load(NoiseModel &M, const double *in
     if (lane >= 6 && lane < 9) lev = (sa + sb) - a;
   }
   if (lane < 15) M.lev[lane] = lev * (lane < 3 ? 0.25 : lane < 9 ? 1.0 : lane < 12 ? 0.5 : 2.0);
-  if (sg) {
-    const double v = lane < 5 ? sg[lane] : 0.0, x = lane == 2 ? 0.0 : v;
-    const double e = exp(x);
-    const double f2 = __shfl_sync(0xffffffffu, e, 4);
-    if (lane == 0) M.Amp = e;
-    if (lane == 1) {
-      M.l1 = v;
-      M.f10 = e * 10;
-    }
-    if (lane == 2) M.alpha = v;
-    if (lane == 3) M.fk = e;
-    if (lane == 4) {
-      // a step of the sequence by more than e^1 could leave the exponent range
-      // within a thread's bins and not come back
-      const double st = 2.0 * fstep / f2;
-      M.i2 = 2.0 / f2;
-      M.estep = exp(st);
-      M.chain = st < 1.0;
-    }
-  }
 }
 
 // The six covariance entries of one bin or layer from the model's sums and the
