@@ -1,4 +1,4 @@
-"""The checker built from the reference's sources is left out where they are absent."""
+"""The shared object of the reference's sources is left out where they are absent."""
 import oracle as orc
 
 
